@@ -122,8 +122,11 @@ def draw(rng):
 
 @functools.lru_cache(maxsize=64)
 def _lattice(side, seed):
-    """A jittered lattice in the map layout: per node one connection list in ascending
-    road id, roads that end at the node listed twice, count = roads at the node."""
+    """A jittered lattice in the map layout.  A road end with three or more entries draws
+    one of the entries 1 .. count after its first (one with two always takes entry 1),
+    so a node's list is one entry to skip, then its roads, twice over where there are
+    two: every road of a node is drawn equally often, and a population stays spread out
+    however long it runs."""
     g = np.random.default_rng([side, seed])
     node = np.arange(side * side)
     a, b = node % side, node // side
@@ -134,11 +137,16 @@ def _lattice(side, seed):
     order = np.argsort(start, kind="stable")
     start, end = start[order], end[order]
     road = np.arange(start.size)
-    at = np.concatenate([start, end, end])
-    conn = np.concatenate([road, road, road])
-    conn = conn[np.argsort(at * road.size + conn, kind="stable")].astype(np.uint32)
-    begins = np.concatenate([[0], np.cumsum(np.bincount(at, minlength=side * side))])
-    count = np.bincount(np.concatenate([start, end]), minlength=side * side)
+    at, conn = np.concatenate([start, end]), np.concatenate([road, road])
+    two = np.bincount(at, minlength=side * side)[at] == 2
+    at, conn = np.append(at, at[two]), np.append(conn, conn[two])
+    order = np.argsort(at, kind="stable")  # by node
+    at, conn = at[order], conn[order]
+    count = np.bincount(at, minlength=side * side)
+    first = np.concatenate([[0], np.cumsum(count)])[:-1]
+    used = np.unique(at)
+    conn = np.insert(conn, first[used], conn[first[used]]).astype(np.uint32)  # the entry to skip
+    begins = first + np.cumsum(count > 0) - (count > 0)
     road_pos = np.concatenate([xy[start], xy[end]], 1)
     road_conn = np.stack([begins[start], count[start], begins[end], count[end]], 1).astype(np.uint32)
     width, height = xy[np.concatenate([start, end])].max(0)
