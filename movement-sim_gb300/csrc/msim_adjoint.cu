@@ -66,56 +66,6 @@ struct AdjArgs {
     uint32_t* err;
 };
 
-// One tick; returns whether the entity snapped to its road end.  force < 0:
-// natural decision (len <= step); 0 / 1: the recorded decision.
-template <int RNG>
-__device__ __forceinline__ bool adj_step(const DeviceMap& m, float dt, float speed, float2& p, uint32_t& h, uint4& r,
-                                         int force, uint32_t* err) {
-    const uint32_t road = h & kHeadRoad;
-    if (road >= m.num_roads) {
-        atomicOr(err, kErrOob);
-        return false;
-    }
-    const bool to_end = (h & kHeadToEnd) != 0;
-    const float4 rp = __ldg(&m.road_pos[road]);
-    const float tx = to_end ? rp.z : rp.x, ty = to_end ? rp.w : rp.y;
-    const float f = m.factor ? __ldg(&m.factor[road]) : 1.0f;
-    const float step = __fmul_rn(__fmul_rn(speed, f), dt);
-    const float dx = __fsub_rn(tx, p.x), dy = __fsub_rn(ty, p.y);
-    const float len = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-    const bool snap = force < 0 ? !(len > step) : force != 0;
-    if (!snap) {
-        if (len > 0.f) {
-            p.x = __fadd_rn(p.x, __fmul_rn(__fdiv_rn(dx, len), step));
-            p.y = __fadd_rn(p.y, __fmul_rn(__fdiv_rn(dy, len), step));
-        }
-        return false;
-    }
-    p.x = tx;
-    p.y = ty;
-    const uint4 rc = __ldg(&m.road_conn[road]);
-    const uint32_t cidx = to_end ? rc.z : rc.x, ccnt = to_end ? rc.w : rc.y;
-    if (ccnt <= 1) {
-        h = to_end ? road : (road | kHeadToEnd);
-        return true;
-    }
-    uint32_t off = 1;
-    if (ccnt != 2) off = ranged(rng_next<RNG>(r), 1u, ccnt);
-    uint32_t ci = cidx + off;
-    if (ci > m.num_conn) {
-        atomicOr(err, kErrOob);
-        ci = m.num_conn;
-    }
-    const uint32_t nr = __ldg(&m.conn[ci]);
-    if (nr >= m.num_roads) {
-        atomicOr(err, kErrOob);
-        return true;
-    }
-    const float4 np = __ldg(&m.road_pos[nr]);
-    h = (np.x == tx && np.y == ty) ? (nr | kHeadToEnd) : nr;
-    return true;
-}
-
 // Cell coordinates of a position: u = x * (gw / W) - 1/2 in binary32 (cell-centred),
 // then U = floor(u * 2^fbits) as an integer (exact: a binary32 u below 2^(30-fbits)
 // has no fractional bits beyond fbits once truncated there).  The cell is
@@ -171,6 +121,8 @@ __global__ __launch_bounds__(256) void k_adj_forward(AdjArgs a) {
     uint32_t h = a.head0[e];
     uint4 r = a.rng0[e];
     const float s = a.speed[e];
+    Leg l;
+    if (!leg_load(a.map, a.dt, s, h, l, a.err)) return;  // unreachable: headings come from the initializer
     int bi = INT32_MIN, bj = INT32_MIN;
     BlockSums acc{0u, 0ull, 0ull, 0ull};
     uint32_t bits = 0;
@@ -188,8 +140,8 @@ __global__ __launch_bounds__(256) void k_adj_forward(AdjArgs a) {
         const uint32_t w = (t - 1) >> 5, b = (t - 1) & 31u;
         int force = -1;
         if (a.mode == 2) force = (a.sched[(size_t)e * a.sched_words + w] >> b) & 1u;
-        const bool snapped = RNG == 1 ? adj_step<1>(a.map, a.dt, s, p, h, r, force, a.err)
-                                      : adj_step<0>(a.map, a.dt, s, p, h, r, force, a.err);
+        const bool snapped =
+            step_leg<true>(a.map, a.dt, s, p, h, l, a.err, force, [&]() { return rng_next<RNG>(r); });
         if (a.mode != 2) {  // the schedule of the last forward, replayed by the backward
             if (snapped) bits |= 1u << b;
             if (b == 31 || t == a.ticks) {

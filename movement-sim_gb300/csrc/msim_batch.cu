@@ -74,6 +74,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
         uint32_t h[E], h0[E];
         float sp[E];
         uint4 r[E];
+        Leg l[E];
         bool rl[E], rd[E], ok[E];
 #pragma unroll
         for (int k = 0; k < E; k++) {
@@ -84,13 +85,23 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
             h[k] = h0[k] = a.head[e];
             sp[k] = a.speed[e];
             r[k] = make_uint4(0u, 0u, 0u, 0u);
-            rl[k] = rd[k] = false;
+            rd[k] = false;
+            rl[k] = a.ticks >= kRngAheadTicks;
+            if (rl[k]) r[k] = a.rng[e];
+            ok[k] = ok[k] && leg_load(m, a.dt, sp[k], h[k], l[k], a.err);
         }
         for (uint32_t t = 0; t < a.ticks; t++) {
 #pragma unroll
             for (int k = 0; k < E; k++) {
-                const uint32_t e = it.begin + off + threadIdx.x + k * blockDim.x;
-                if (ok[k]) step_entity<RNG>(m, a.dt, sp[k], p[k], h[k], r[k], rl[k], rd[k], a.rng + e, a.err);
+                if (!ok[k]) continue;
+                step_leg<false>(m, a.dt, sp[k], p[k], h[k], l[k], a.err, -1, [&]() {
+                    if (!rl[k]) {
+                        r[k] = a.rng[it.begin + off + threadIdx.x + k * blockDim.x];
+                        rl[k] = true;
+                    }
+                    rd[k] = true;
+                    return rng_next<RNG>(r[k]);
+                });
             }
         }
 #pragma unroll

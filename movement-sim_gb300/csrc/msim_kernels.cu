@@ -165,12 +165,14 @@ __device__ __forceinline__ void digit_counts(uint32_t key, bool valid, uint32_t 
     }
 }
 
-// Move-only ticks (several per launch, the state in registers between them): one
-// entity per thread in 128-thread blocks, so a small entity count still spreads
-// over many SMs (10,000 entities: 0.264 us per tick against 0.278 with the
-// two-per-thread, 512-thread shape of k_step; equal at 200,000).
-template <int RNG>
-__global__ __launch_bounds__(kMoveThreads) void k_move(StepLaunch a) {
+// Move-only ticks: one entity per thread in 128-thread blocks, so a small entity count
+// still spreads over many SMs.  ONE: a single tick (the tick that reuses the index
+// places its positions too); else several ticks with the state and the road's leg in
+// registers between them, bound by the ticks' serial chain (small counts) or by issue:
+// with read-back, 10,000 entities for 1,000 ticks 316 -> 216 us and 1 M for 200 ticks
+// 867 -> 581 us against reloading the road and three intrinsics every tick.
+template <int RNG, bool ONE>
+__global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch a) {
     chain_enter();
     const uint32_t stride = gridDim.x * kMoveThreads;
     for (uint32_t s = blockIdx.x * kMoveThreads + threadIdx.x; s < a.n; s += stride) {
@@ -179,12 +181,12 @@ __global__ __launch_bounds__(kMoveThreads) void k_move(StepLaunch a) {
         const uint32_t h0 = h;
         const float sp = a.st.speed[s];
         uint4 r = make_uint4(0u, 0u, 0u, 0u);
-        bool rl = false, rd = false;
-        for (uint32_t t = 0; t < a.ticks; t++) step_entity<RNG>(a.map, a.dt, sp, p, h, r, rl, rd, a.st.rng + s, a.err);
+        bool rd = false;
+        step_entity<RNG, ONE ? 1 : 0>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
         a.st.pos[s] = p;
         if (h != h0) a.st.head[s] = h;
         if (rd) a.st.rng[s] = r;
-        if (a.rank_pos) {  // uniform: a tick that reuses the index
+        if (ONE && a.rank_pos) {  // uniform: a tick that reuses the index
             const uint32_t q = a.rank[s];
             if (q < a.rank_n) a.rank_pos[q] = p;
         }
@@ -242,9 +244,8 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
             if (!valid[u]) continue;
             if (a.ticks) {
                 uint4 r = make_uint4(0u, 0u, 0u, 0u);
-                bool rl = false, rd = false;
-                for (uint32_t t = 0; t < a.ticks; t++)
-                    step_entity<RNG>(a.map, a.dt, sp[u], p[u], h[u], r, rl, rd, a.st.rng + sl[u], a.err);
+                bool rd = false;
+                step_entity<RNG, 1>(a.map, a.dt, sp[u], 1u, p[u], h[u], r, rd, a.st.rng + sl[u], a.err);
                 a.st.pos[sl[u]] = p[u];
                 if (h[u] != h0[u]) {
                     a.st.head[sl[u]] = h[u];
@@ -800,9 +801,13 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const unsigned blocks = std::min<unsigned>(blocks_for(a.n, kMoveThreads), 16u * (unsigned)std::max(sms, 1));
-        return a.rng_kind == 1 ? launch_chained(k_move<1>, blocks, kMoveThreads, s, a)
-                               : launch_chained(k_move<0>, blocks, kMoveThreads, s, a);
+        if (a.ticks == 1)
+            return a.rng_kind == 1 ? launch_chained(k_move<1, true>, blocks, kMoveThreads, s, a)
+                                   : launch_chained(k_move<0, true>, blocks, kMoveThreads, s, a);
+        return a.rng_kind == 1 ? launch_chained(k_move<1, false>, blocks, kMoveThreads, s, a)
+                               : launch_chained(k_move<0, false>, blocks, kMoveThreads, s, a);
     }
+    if (a.ticks > 1) return cudaErrorInvalidValue;  // k_step moves one tick at most
     if (a.disp_max) {  // a host tick that queries the previous index (keys, one tick)
         if (!key || !a.index_pos || a.ticks != 1) return cudaErrorInvalidValue;
         return a.rng_kind == 1 ? launch_chained(k_step<1, true, true>, a.blocks, kStepThreads, s, a)
