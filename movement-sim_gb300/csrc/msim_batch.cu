@@ -3,10 +3,10 @@
 //
 // All instances' entity state is concatenated (structure of arrays) and so are
 // their road tables (road_pos, road_conn, connections + one pad entry each).  The
-// host cuts every instance into tiles of entities; each tile is a work item with
-// an entities-per-thread factor.  A persistent grid (a few blocks per SM) pulls
-// items through an atomic ticket and runs all requested ticks of a tile with the
-// state in registers.  The per-entity math is step_entity, the same function as
+// host cuts every instance into tiles of entities with an entities-per-thread factor
+// and, where that leaves too few to fill and balance the chip, the tiles into smaller
+// pieces.  The warps of a persistent grid (a few blocks per SM) pull pieces through an
+// atomic ticket and run all requested ticks with the state in registers.  The per-entity math is step_entity, the same function as
 // the single-instance path, so every instance's result is bit-identical to
 // running it alone.  The ticket reset and the launch are captured once per tick
 // count into a CUDA graph and replayed.
@@ -64,11 +64,12 @@ struct BatchArgs {
     uint32_t* err;
 };
 
-// E independent entities per thread, interleaved tick by tick so their
-// dependency chains overlap.
+// One warp's piece.  E independent entities per thread, interleaved tick by tick so
+// their dependency chains overlap.
 template <int RNG, int E>
-__device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m, const WorkItem& it) {
-    const uint32_t span = blockDim.x * E;
+__device__ __forceinline__ void run_piece(const BatchArgs& a, const DeviceMap& m, const WorkItem& it) {
+    const uint32_t lane = threadIdx.x & 31u;
+    constexpr uint32_t span = 32u * E;
     for (uint32_t off = 0; off < it.count; off += span) {
         float2 p[E];
         uint32_t h[E], h0[E];
@@ -78,7 +79,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
         bool rl[E], rd[E], ok[E];
 #pragma unroll
         for (int k = 0; k < E; k++) {
-            const uint32_t local = off + threadIdx.x + k * blockDim.x;
+            const uint32_t local = off + lane + k * 32u;
             ok[k] = local < it.count;
             const uint32_t e = it.begin + (ok[k] ? local : 0u);
             p[k] = a.pos[e];
@@ -96,7 +97,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
                 if (!ok[k]) continue;
                 step_leg<false>(m, a.dt, sp[k], p[k], h[k], l[k], a.err, -1, [&]() {
                     if (!rl[k]) {
-                        r[k] = a.rng[it.begin + off + threadIdx.x + k * blockDim.x];
+                        r[k] = a.rng[it.begin + off + lane + k * 32u];
                         rl[k] = true;
                     }
                     rd[k] = true;
@@ -107,7 +108,7 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
 #pragma unroll
         for (int k = 0; k < E; k++) {
             if (!ok[k]) continue;
-            const uint32_t e = it.begin + off + threadIdx.x + k * blockDim.x;
+            const uint32_t e = it.begin + off + lane + k * 32u;
             a.pos[e] = p[k];
             if (h[k] != h0[k]) a.head[e] = h[k];
             if (rd[k]) a.rng[e] = r[k];
@@ -119,14 +120,14 @@ __device__ __forceinline__ void run_tile(const BatchArgs& a, const DeviceMap& m,
 // kernel, so a schedule of one entity per thread does not pay the registers of the
 // four-entity path (72 registers and 43 % of the warps resident with all three paths
 // in one kernel).
+// Every warp takes its own pieces: no block barrier, and a block's slow warp (road ends)
+// holds up no other.
 template <int RNG, int EMAX>
-__global__ void k_batch_step(BatchArgs a) {
-    __shared__ uint32_t s_item;
+__global__ void __maxnreg__(EMAX == 1 ? 40 : EMAX == 2 ? 56 : 72) k_batch_step(BatchArgs a) {
     while (true) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(a.ticket, 1u);
-        __syncthreads();
-        const uint32_t i = s_item;
+        uint32_t i = 0;
+        if ((threadIdx.x & 31u) == 0) i = atomicAdd(a.ticket, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
         if (i >= a.num_items) return;
         const WorkItem it = a.items[i];
         const InstanceDesc d = a.inst[it.instance];
@@ -137,9 +138,9 @@ __global__ void k_batch_step(BatchArgs a) {
         m.factor = nullptr;
         m.num_roads = d.num_roads;
         m.num_conn = d.num_conn;
-        if (EMAX >= 4 && it.ept == 4) run_tile<RNG, 4>(a, m, it);
-        else if (EMAX >= 2 && it.ept == 2) run_tile<RNG, 2>(a, m, it);
-        else run_tile<RNG, 1>(a, m, it);
+        if (EMAX >= 4 && it.ept == 4) run_piece<RNG, 4>(a, m, it);
+        else if (EMAX >= 2 && it.ept == 2) run_piece<RNG, 2>(a, m, it);
+        else run_piece<RNG, 1>(a, m, it);
     }
 }
 
@@ -174,7 +175,9 @@ struct msim_batch {
     uint32_t* conn = nullptr;
     InstanceDesc* d_inst = nullptr;
     WorkItem* d_items = nullptr;
-    uint32_t num_items = 0;
+    uint32_t num_items = 0;   // tiles of the schedule
+    uint32_t num_pieces = 0;  // what the warps take: the tiles or parts of them
+    size_t items_capacity = 0;
     uint32_t* ticket = nullptr;
     uint32_t* err = nullptr;
     float2* pos = nullptr;
@@ -253,24 +256,6 @@ int check_schedule(const msim_batch_schedule& s) {
     return MSIM_OK;
 }
 
-int upload_items(msim_batch* b, const std::vector<WorkItem>& items) {
-    if (items.size() > b->num_items || !b->d_items) {
-        if (b->d_items) {
-            cudaFree(b->d_items);
-            b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void*)b->d_items));
-            b->d_items = nullptr;
-        }
-        int rc = balloc(b, &b->d_items, items.size());
-        if (rc != MSIM_OK) return rc;
-    }
-    b->num_items = (uint32_t)items.size();
-    if (!items.empty())
-        BCK(cudaMemcpy(b->d_items, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice),
-            "upload work items");
-    drop_graphs(b);
-    return MSIM_OK;
-}
-
 // The kernel instantiation for a schedule: RNG and its largest entities per thread.
 using BatchKernel = void (*)(BatchArgs);
 BatchKernel batch_kernel(uint32_t rng_kind, const msim_batch_schedule& s) {
@@ -287,6 +272,51 @@ int occupancy(msim_batch* b, uint32_t threads) {
     return std::max(per_sm, 1);
 }
 
+// The pieces of a work list: tiles cut further so that every resident warp finds about
+// kPiecesPerWarp of them, in whole rounds of a warp (32 x entities per thread).  A tile
+// of 4096 entities taken by one block left most of the chip idle on small ensembles
+// (20 instances, 832 K entities, 1,000 ticks: 203 tiles for 912 resident blocks) and
+// the last tiles unbalanced on large ones; many more pieces than that only add tickets.
+constexpr uint64_t kPiecesPerWarp = 8;
+std::vector<WorkItem> cut_pieces(msim_batch* b, const std::vector<WorkItem>& items) {
+    uint64_t total = 0;
+    for (const WorkItem& it : items) total += it.count;
+    const uint64_t warps = (uint64_t)b->sms * occupancy(b, b->sched.block_threads) * (b->sched.block_threads / 32u);
+    const uint64_t want = total / std::max<uint64_t>(warps * kPiecesPerWarp, 1u);
+    std::vector<WorkItem> pieces;
+    for (const WorkItem& it : items) {
+        const uint32_t span = 32u * it.ept;
+        const uint32_t size = (uint32_t)std::min<uint64_t>(it.count, (want + span) / span * span);
+        for (uint32_t off = 0; off < it.count; off += size)
+            pieces.push_back(WorkItem{it.instance, it.begin + off, std::min(size, it.count - off), it.ept});
+    }
+    return pieces;
+}
+
+int upload_items(msim_batch* b, const std::vector<WorkItem>& items) {
+    const std::vector<WorkItem> pieces = cut_pieces(b, items);
+    if (pieces.size() > b->items_capacity || !b->d_items) {
+        drop_graphs(b);
+        b->num_items = b->num_pieces = 0;
+        if (b->d_items) {
+            cudaFree(b->d_items);
+            b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void*)b->d_items));
+            b->d_items = nullptr;
+            b->items_capacity = 0;
+        }
+        int rc = balloc(b, &b->d_items, pieces.size());
+        if (rc != MSIM_OK) return rc;
+        b->items_capacity = pieces.size();
+    }
+    b->num_items = (uint32_t)items.size();
+    b->num_pieces = (uint32_t)pieces.size();
+    if (!pieces.empty())
+        BCK(cudaMemcpy(b->d_items, pieces.data(), sizeof(WorkItem) * pieces.size(), cudaMemcpyHostToDevice),
+            "upload work items");
+    drop_graphs(b);
+    return MSIM_OK;
+}
+
 BatchArgs args_of(msim_batch* b, uint32_t ticks) {
     BatchArgs a;
     a.road_pos = b->road_pos;
@@ -294,7 +324,7 @@ BatchArgs args_of(msim_batch* b, uint32_t ticks) {
     a.conn = b->conn;
     a.inst = b->d_inst;
     a.items = b->d_items;
-    a.num_items = b->num_items;
+    a.num_items = b->num_pieces;
     a.ticket = b->ticket;
     a.pos = b->pos;
     a.head = b->head;
