@@ -20,7 +20,7 @@
 //
 // Backward, per segment of K ticks from the last to the first
 // (k_adj_backward): recompute the segment from its checkpoint with the recorded
-// events, store positions and headings, then sweep backwards:
+// events, store its positions, then sweep backwards:
 //   a_t += (1/T) d splat(p_t)/dp . lambda,     lambda = dL/dD = 2/G (D - D*)
 //   snap tick:     a_{t-1} = 0 (p_t = road end does not depend on p, speed, factor)
 //   otherwise:     n = (target - p_{t-1})/L, l = s*f*dt, g = n . a_t
@@ -28,8 +28,8 @@
 //                  a_{t-1} = a_t - (l/L)(a_t - n g)
 // Speed gradients are owned by their entity (no reduction).  Road-factor
 // contributions are flushed as (road, value) records, one per road visit per
-// segment, then sorted by road with the stable onesweep radix sort and summed per
-// road in record order: a deterministic segmented reduction, no float atomics.
+// segment, then packed, sorted by road with the stable onesweep radix sort and summed
+// per road in a fixed order: a deterministic segmented reduction, no float atomics.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -46,7 +46,7 @@ namespace msim {
 namespace {
 
 constexpr uint32_t kRecPerSeg = 8;  // road-visit records per entity and segment
-constexpr uint32_t kSnapBit = 1u << 30;
+constexpr uint32_t kRecBlock = 1024;  // entities whose records one block packs
 
 struct AdjArgs {
     DeviceMap map;
@@ -62,9 +62,24 @@ struct AdjArgs {
     uint4* ck_rng;
     unsigned long long* dacc;
     uint32_t* sched;  // one bit per entity and tick
-    uint32_t mode;    // 0 / 1 natural (the schedule is stored), 2 replay the stored schedule
+    uint32_t lanes;   // entities per warp (adj_entity)
     uint32_t* err;
 };
+
+// Threads of a block of the forward and backward kernels, and blocks per SM.  Both are
+// bound by issue; the backward's history (800 B per entity at K = 100) of the resident
+// threads then also fits the L2 it is read back from.
+constexpr uint32_t kAdjThreads = 128;
+constexpr int kAdjForwardBlocks = 7;
+constexpr int kAdjBackwardBlocks = 7;
+
+// The entity of a thread: `lanes` entities to a warp (32, fewer for small counts: the
+// road ends and cell changes of one entity hold up the others of its warp).
+__device__ __forceinline__ uint32_t adj_entity(uint32_t n, uint32_t lanes) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint64_t e = (uint64_t)warp * lanes + lane;
+    return lane < lanes && e < n ? (uint32_t)e : 0xffffffffu;
+}
 
 // Cell coordinates of a position: u = x * (gw / W) - 1/2 in binary32 (cell-centred),
 // then U = floor(u * 2^fbits) as an integer (exact: a binary32 u below 2^(30-fbits)
@@ -80,9 +95,10 @@ __device__ __forceinline__ int fixed_coord(float u, uint32_t fbits) {
     u = fminf(fmaxf(u, -lim), lim);                                  // off-grid positions stay off-grid
     return __float2int_rd(__fmul_rn(u, __int_as_float((127 + (int)fbits) << 23)));
 }
-__device__ __forceinline__ Splat splat_of(float x, float y, float inv_cw, float inv_ch, uint32_t fbits) {
-    const int U = fixed_coord(__fsub_rn(__fmul_rn(x, inv_cw), 0.5f), fbits);
-    const int V = fixed_coord(__fsub_rn(__fmul_rn(y, inv_ch), 0.5f), fbits);
+__device__ __forceinline__ float cell_coord(float x, float inv_c) { return __fsub_rn(__fmul_rn(x, inv_c), 0.5f); }
+__device__ __forceinline__ Splat splat_of(float ux, float uy, uint32_t fbits) {
+    const int U = fixed_coord(ux, fbits);
+    const int V = fixed_coord(uy, fbits);
     const uint32_t mask = (1u << fbits) - 1u;
     Splat s;
     s.i0 = U >> fbits;  // arithmetic shift: floor
@@ -91,6 +107,23 @@ __device__ __forceinline__ Splat splat_of(float x, float y, float inv_cw, float 
     s.fy = (uint32_t)V & mask;
     return s;
 }
+// The same without conversions while a position stays in the cell (fi, fj) of an
+// earlier splat: u - fi towards zero is in [0, 1) exactly when floor(u) = fi (u - fi is
+// exact for u >= 0; for u in [-1, 0) its truncation keeps every bit above 2^-24), and
+// adding 2^(23 - fbits) towards zero leaves the fraction's first fbits bits as the low
+// bits of the sum.  An entity stays about a hundred ticks in a cell.
+struct CellFrame {
+    float fi, fj;
+    float one;  // 2^(23 - fbits)
+};
+__device__ __forceinline__ bool in_cell(const CellFrame& c, float ux, float uy, float& wx, float& wy) {
+    const float dx = __fadd_rz(ux, -c.fi), dy = __fadd_rz(uy, -c.fj);
+    wx = __fadd_rz(dx, c.one);
+    wy = __fadd_rz(dy, c.one);
+    return max(__float_as_uint(dx), __float_as_uint(dy)) < 0x3f800000u;
+}
+__device__ __forceinline__ float frame_one(uint32_t fbits) { return __int_as_float((150 - (int)fbits) << 23); }
+
 // Per-entity sums over the ticks spent in one 2 x 2 cell block: the tick count and
 // the sums of fx, fy and fx*fy give the four bilinear corner weights exactly.
 struct BlockSums {
@@ -113,22 +146,53 @@ __device__ __forceinline__ void flush_block(unsigned long long* dacc, uint32_t g
     }
 }
 
-template <int RNG>
-__global__ __launch_bounds__(256) void k_adj_forward(AdjArgs a) {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= a.n) return;
+// Sums of blocks an entity has left, one per thread, until a lane of the warp leaves a
+// second one: then every lane that has one flushes it.  An entity changes its cell once
+// in about 70 ticks, so some lane of a warp does in 37 % of its ticks; waiting for the second
+// change brings the flushes of about eight lanes together.
+struct LeftBlocks {
+    int i[kAdjThreads], j[kAdjThreads];
+    uint32_t n[kAdjThreads];  // 0: none
+    unsigned long long sx[kAdjThreads], sy[kAdjThreads], sxy[kAdjThreads];
+};
+__device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
+    const uint32_t t = threadIdx.x;
+    if (left.n[t]) {
+        flush_block(a.dacc, a.gw, a.gh, left.i[t], left.j[t], BlockSums{left.n[t], left.sx[t], left.sy[t], left.sxy[t]},
+                    a.fbits);
+        left.n[t] = 0u;
+    }
+}
+
+// REPLAY: the stored event schedule is forced; else events come from the step and the
+// schedule is stored.  Ticks run in stretches of at most 32 that end where a schedule
+// word or a checkpoint does, so a tick itself is the step, the cell test and three
+// sums (32-bit within a stretch).  Bound by issue (82 % active): 118 warp instructions
+// per tick against 190 with the road reloaded, two conversions and a flush at every
+// cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.92 ms.
+template <int RNG, bool REPLAY>
+__global__ __launch_bounds__(kAdjThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
+    __shared__ LeftBlocks left;
+    const uint32_t e = adj_entity(a.n, a.lanes);
+    left.n[threadIdx.x] = 0u;
+    const unsigned warp_mask = __ballot_sync(0xffffffffu, e != 0xffffffffu);
+    if (e == 0xffffffffu) return;
     float2 p = a.pos0[e];
     uint32_t h = a.head0[e];
     uint4 r = a.rng0[e];
     const float s = a.speed[e];
-    Leg l;
-    if (!leg_load(a.map, a.dt, s, h, l, a.err)) return;  // unreachable: headings come from the initializer
+    Leg l{};
+    if (!leg_load(a.map, a.dt, s, h, l, a.err)) {  // unreachable: headings come from the initializer
+        h = 0u;
+        leg_load(a.map, a.dt, s, h, l, a.err);
+    }
+    const uint32_t low = (1u << a.fbits) - 1u;
+    CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};  // NaN: in no cell yet
     int bi = INT32_MIN, bj = INT32_MIN;
     BlockSums acc{0u, 0ull, 0ull, 0ull};
-    uint32_t bits = 0;
-    uint32_t until_ck = 0;  // ticks until the next checkpoint
     size_t ck = e;
-    for (uint32_t t = 1; t <= a.ticks; t++) {
+    uint32_t until_ck = 0, bits = 0;
+    for (uint32_t t = 0; t < a.ticks;) {
         if (until_ck == 0) {
             a.ck_pos[ck] = p;
             a.ck_head[ck] = h;
@@ -136,32 +200,64 @@ __global__ __launch_bounds__(256) void k_adj_forward(AdjArgs a) {
             ck += a.n;
             until_ck = a.K;
         }
-        until_ck--;
-        const uint32_t w = (t - 1) >> 5, b = (t - 1) & 31u;
-        int force = -1;
-        if (a.mode == 2) force = (a.sched[(size_t)e * a.sched_words + w] >> b) & 1u;
-        const bool snapped =
-            step_leg<true>(a.map, a.dt, s, p, h, l, a.err, force, [&]() { return rng_next<RNG>(r); });
-        if (a.mode != 2) {  // the schedule of the last forward, replayed by the backward
-            if (snapped) bits |= 1u << b;
-            if (b == 31 || t == a.ticks) {
-                a.sched[(size_t)e * a.sched_words + w] = bits;
-                bits = 0;
+        const uint32_t first = t & 31u;
+        const uint32_t len = min(min(32u - first, until_ck), a.ticks - t);
+        uint32_t* word = a.sched + (size_t)e * a.sched_words + (t >> 5);
+        if (REPLAY) bits = *word >> first;
+        uint32_t sx = 0u, sy = 0u, began = 0u;  // sums and first tick of this stretch in the block
+        for (uint32_t k = 0; k < len; k++) {
+            const int force = REPLAY ? (int)(bits & 1u) : -1;
+            const bool snapped = step_leg<true>(a.map, a.dt, s, p, h, l, a.err, force,
+                                                [&]() { return rng_next<RNG>(r); });
+            if (REPLAY) bits >>= 1;
+            else if (snapped) bits |= 1u << (first + k);
+            const float ux = cell_coord(p.x, a.inv_cw), uy = cell_coord(p.y, a.inv_ch);
+            float wx, wy;
+            const bool stays = in_cell(c, ux, uy, wx, wy);
+            uint32_t fx = __float_as_uint(wx) & low, fy = __float_as_uint(wy) & low;
+            bool leaves = false;
+            Splat sp{};
+            if (!stays) {
+                sp = splat_of(ux, uy, a.fbits);
+                fx = sp.fx;
+                fy = sp.fy;
+                leaves = sp.i0 != bi || sp.j0 != bj;
             }
+            if (__any_sync(warp_mask, leaves && left.n[threadIdx.x] != 0u)) flush_left(left, a);
+            if (leaves) {
+                acc.n += k - began;
+                if (acc.n) {
+                    left.i[threadIdx.x] = bi;
+                    left.j[threadIdx.x] = bj;
+                    left.n[threadIdx.x] = acc.n;
+                    left.sx[threadIdx.x] = acc.sx + sx;
+                    left.sy[threadIdx.x] = acc.sy + sy;
+                    left.sxy[threadIdx.x] = acc.sxy;
+                }
+                bi = sp.i0;
+                bj = sp.j0;
+                c.fi = (float)bi;
+                c.fj = (float)bj;
+                acc = BlockSums{0u, 0ull, 0ull, 0ull};
+                sx = sy = 0u;
+                began = k;
+            }
+            sx += fx;
+            sy += fy;
+            acc.sxy += (unsigned long long)fx * fy;
         }
-        const Splat sp = splat_of(p.x, p.y, a.inv_cw, a.inv_ch, a.fbits);
-        if (sp.i0 != bi || sp.j0 != bj) {
-            if (bi != INT32_MIN) flush_block(a.dacc, a.gw, a.gh, bi, bj, acc, a.fbits);
-            bi = sp.i0;
-            bj = sp.j0;
-            acc = BlockSums{0u, 0ull, 0ull, 0ull};
+        acc.n += len - began;
+        acc.sx += sx;
+        acc.sy += sy;
+        t += len;
+        until_ck -= len;
+        if (!REPLAY && ((t & 31u) == 0u || t == a.ticks)) {
+            *word = bits;
+            bits = 0u;
         }
-        acc.n++;
-        acc.sx += sp.fx;
-        acc.sy += sp.fy;
-        acc.sxy += (unsigned long long)sp.fx * sp.fy;
     }
-    if (bi != INT32_MIN) flush_block(a.dacc, a.gw, a.gh, bi, bj, acc, a.fbits);
+    flush_left(left, a);
+    if (acc.n) flush_block(a.dacc, a.gw, a.gh, bi, bj, acc, a.fbits);
 }
 
 // density, lambda = 2/G (D - D*), per-block partial sums of (D - D*)^2
@@ -187,23 +283,34 @@ __global__ __launch_bounds__(256) void k_adj_loss(const unsigned long long* __re
     if (threadIdx.x == 0) partial[blockIdx.x] = s_sum[0];
 }
 
-__global__ void k_adj_loss_final(const double* partial, uint32_t blocks, uint32_t G, double* loss) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// The blocks' partial sums in a fixed order: strided by thread, then a tree (one thread
+// adding 1,024 partials one after another took 54 us).
+__global__ __launch_bounds__(256) void k_adj_loss_final(const double* partial, uint32_t blocks, uint32_t G,
+                                                        double* loss) {
+    __shared__ double s_sum[256];
     double s = 0.0;
-    for (uint32_t b = 0; b < blocks; b++) s += partial[b];
-    *loss = s / (double)G;
+    for (uint32_t b = threadIdx.x; b < blocks; b += 256u) s += partial[b];
+    s_sum[threadIdx.x] = s;
+    __syncthreads();
+    for (uint32_t o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) s_sum[threadIdx.x] += s_sum[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = s_sum[0] / (double)G;
 }
 
 struct AdjBack {
     AdjArgs f;
-    uint32_t seg;
+    uint32_t segments;
     const float* lambda;
-    float2* hist_pos;     // [K][n]
-    uint32_t* hist_head;  // [K][n], heading before the tick | snap bit
-    float2* carry;        // adjoint of the position at the segment's end
+    float2* hist_pos;     // [K + 1][n]: the segment's positions, its checkpoint first
+    uint32_t* hist_head;  // [K][n]: headings before the segment's road ends, in order
     double* gspeed;
-    uint32_t* rec_road;   // [segments][n][kRecPerSeg], unused = num_roads
-    double* rec_val;
+    float* gspeed_out;    // by entity id (may be NULL)
+    const uint32_t* perm;
+    uint2* rec;           // [n][segments * kRecPerSeg]: road, float bits of the gradient part
+    uint32_t* rec_count;  // [n]
+    uint32_t* rec_block;  // records per kRecBlock entities (accumulated)
     uint32_t num_roads;
 };
 
@@ -211,217 +318,277 @@ __device__ __forceinline__ float lam_at(const float* lambda, uint32_t gw, uint32
     return (i < 0 || j < 0 || i >= (int)gw || j >= (int)gh) ? 0.f : __ldg(&lambda[(size_t)j * gw + i]);
 }
 
-// The recorded step for the backward's recompute: the event decision comes from the
-// schedule, the road choice from the checkpointed RNG (both exact); the position
-// update uses the hardware reciprocal square root, since the adjoint needs the
-// positions only to about 1e-6 relative (snaps put them back on exact road ends).
+// Backward of one entity, segment by segment from the last to the first: recompute
+// the segment's positions from its checkpoint (the event decisions from the schedule,
+// the road choices from the checkpointed RNG, both exact; the position update with
+// the hardware reciprocal square root, since the adjoint needs the positions only to
+// about 1e-6 relative and snaps put them back on exact road ends), then sweep
+// backwards over them.  The road's leg, and the four cell values' differences, stay in
+// registers until a road end or a cell change; headings are kept only for road ends
+// (12 -> 8 B of history per tick), and all segments run in one launch, which a launch
+// per segment rounded up to two waves each.
 template <int RNG>
-__device__ __forceinline__ void adj_replay_step(const DeviceMap& m, float dt, float speed, float2& p, uint32_t& h,
-                                                uint4& r, bool snap, uint32_t* err) {
-    const uint32_t road = h & kHeadRoad;
-    if (road >= m.num_roads) {
-        atomicOr(err, kErrOob);
-        return;
-    }
-    const bool to_end = (h & kHeadToEnd) != 0;
-    const float4 rp = __ldg(&m.road_pos[road]);
-    const float tx = to_end ? rp.z : rp.x, ty = to_end ? rp.w : rp.y;
-    if (!snap) {
-        const float f = m.factor ? __ldg(&m.factor[road]) : 1.0f;
-        const float step = speed * f * dt;
-        const float dx = tx - p.x, dy = ty - p.y;
-        const float d2 = dx * dx + dy * dy;
-        if (d2 > 0.f) {
-            const float k = rsqrtf(d2) * step;
-            p.x += dx * k;
-            p.y += dy * k;
-        }
-        return;
-    }
-    p.x = tx;
-    p.y = ty;
-    const uint4 rc = __ldg(&m.road_conn[road]);
-    const uint32_t cidx = to_end ? rc.z : rc.x, ccnt = to_end ? rc.w : rc.y;
-    if (ccnt <= 1) {
-        h = to_end ? road : (road | kHeadToEnd);
-        return;
-    }
-    uint32_t off = 1;
-    if (ccnt != 2) off = ranged(rng_next<RNG>(r), 1u, ccnt);
-    uint32_t ci = cidx + off;
-    if (ci > m.num_conn) {
-        atomicOr(err, kErrOob);
-        ci = m.num_conn;
-    }
-    const uint32_t nr = __ldg(&m.conn[ci]);
-    if (nr >= m.num_roads) {
-        atomicOr(err, kErrOob);
-        return;
-    }
-    const float4 np = __ldg(&m.road_pos[nr]);
-    h = (np.x == tx && np.y == ty) ? (nr | kHeadToEnd) : nr;
-}
-
-// lambda at the four corners of p's cell block, and the fractions
-struct SplatLam {
-    float l00, l10, l01, l11, fx, fy;
-};
-__device__ __forceinline__ SplatLam splat_lam(const AdjBack& b, float2 p) {
-    const Splat sp = splat_of(p.x, p.y, b.f.inv_cw, b.f.inv_ch, b.f.fbits);
-    const float scale = __int_as_float((127 - (int)b.f.fbits) << 23);  // 2^-fbits
-    SplatLam o;
-    o.l00 = lam_at(b.lambda, b.f.gw, b.f.gh, sp.i0, sp.j0);
-    o.l10 = lam_at(b.lambda, b.f.gw, b.f.gh, sp.i0 + 1, sp.j0);
-    o.l01 = lam_at(b.lambda, b.f.gw, b.f.gh, sp.i0, sp.j0 + 1);
-    o.l11 = lam_at(b.lambda, b.f.gw, b.f.gh, sp.i0 + 1, sp.j0 + 1);
-    o.fx = (float)sp.fx * scale;  // exact: fewer than 24 bits
-    o.fy = (float)sp.fy * scale;
-    return o;
-}
-
-template <int RNG>
-__global__ __launch_bounds__(256) void k_adj_backward(AdjBack b) {
+__global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backward(AdjBack b) {
     const AdjArgs& a = b.f;
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= a.n) return;
-    const uint32_t t0 = b.seg * a.K + 1, t1 = min((b.seg + 1) * a.K, a.ticks);
-    const size_t ck = (size_t)b.seg * a.n + e;
-    const float2 pk = a.ck_pos[ck];
-    float2 p = pk;
-    uint32_t h = a.ck_head[ck];
-    uint4 r = a.ck_rng[ck];
+    const uint32_t e = adj_entity(a.n, a.lanes);
+    if (e == 0xffffffffu) return;
+    const size_t n = a.n;
     const float s = a.speed[e];
     const uint32_t* sched = a.sched + (size_t)e * a.sched_words;
-    uint32_t word = 0;
-    for (uint32_t t = t0; t <= t1; t++) {  // recompute the segment with the recorded events
-        const uint32_t bit = (t - 1) & 31u;
-        if (t == t0 || bit == 0) word = sched[(t - 1) >> 5];
-        const bool snap = (word >> bit) & 1u;
-        const uint32_t hb = h;
-        adj_replay_step<RNG>(a.map, a.dt, s, p, h, r, snap, a.err);
-        const size_t hi = (size_t)(t - t0) * a.n + e;
-        b.hist_pos[hi] = p;
-        b.hist_head[hi] = hb | (snap ? kSnapBit : 0u);
-    }
-    // reverse sweep; positions, headings and lambda are fetched one tick ahead
-    float2 adj = b.carry[e];
-    float gs = 0.f, cur_sum = 0.f;
-    uint32_t cur_road = b.num_roads, nrec = 0;
-    const size_t rec0 = ((size_t)b.seg * a.n + e) * kRecPerSeg;
+    uint2* rec = b.rec + (size_t)e * b.segments * kRecPerSeg;
+    float2* hist = b.hist_pos + e;
+    uint32_t* ends = b.hist_head + e;
     const float sx = a.inv_cw, sy = a.inv_ch, invT = 1.0f / (float)a.ticks;
-    const size_t n = a.n;
-    float2 pt = b.hist_pos[(size_t)(t1 - t0) * n + e];
-    uint32_t hw = b.hist_head[(size_t)(t1 - t0) * n + e];
-    float2 pp = t1 > t0 ? b.hist_pos[(size_t)(t1 - 1 - t0) * n + e] : pk;
-    SplatLam sl = splat_lam(b, pt);
-    for (uint32_t t = t1;; t--) {
-        uint32_t hw_n = 0;
-        float2 pp_n = pk;
-        if (t > t0) {
-            hw_n = b.hist_head[(size_t)(t - 1 - t0) * n + e];
-            if (t - 1 > t0) pp_n = b.hist_pos[(size_t)(t - 2 - t0) * n + e];
+    const float scale = __int_as_float((127 - (int)a.fbits) << 23);  // 2^-fbits
+    float2 adj = make_float2(0.f, 0.f);
+    double gspeed = 0.0;
+    uint32_t records = 0;
+    CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};
+    float dx0 = 0.f, dx1 = 0.f, dy0 = 0.f, dy1 = 0.f;  // lambda differences of the cell block
+    for (uint32_t seg = b.segments; seg-- > 0;) {
+        const uint32_t t0 = seg * a.K, len = min(a.K, a.ticks - t0);  // ticks t0 + 1 .. t0 + len
+        const size_t ck = (size_t)seg * n + e;
+        float2 p = a.ck_pos[ck];
+        uint32_t h = a.ck_head[ck];
+        uint4 r = a.ck_rng[ck];
+        Leg l{};
+        if (!leg_load(a.map, a.dt, s, h, l, a.err)) {  // unreachable: the forward's headings
+            h = 0u;
+            leg_load(a.map, a.dt, s, h, l, a.err);
         }
-        const SplatLam sl_n = splat_lam(b, pp);  // lambda for the next (earlier) tick
-        {  // + (1/T) d splat(p_t)/dp . lambda
-            const float gx = ((1.f - sl.fy) * (sl.l10 - sl.l00) + sl.fy * (sl.l11 - sl.l01)) * sx;
-            const float gy = ((1.f - sl.fx) * (sl.l01 - sl.l00) + sl.fx * (sl.l11 - sl.l10)) * sy;
-            adj.x += gx * invT;
-            adj.y += gy * invT;
-        }
-        if (hw & kSnapBit) {
-            adj = make_float2(0.f, 0.f);
-        } else {
-            const uint32_t h0 = hw & ~kSnapBit;
-            const uint32_t road = h0 & kHeadRoad;
-            const float4 rp = __ldg(&a.map.road_pos[road]);
-            const float tx = (h0 & kHeadToEnd) ? rp.z : rp.x, ty = (h0 & kHeadToEnd) ? rp.w : rp.y;
-            const float dx = tx - pp.x, dy = ty - pp.y;
-            const float d2 = dx * dx + dy * dy;
-            if (d2 > 0.f) {
-                const float invL = rsqrtf(d2);
-                const float f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
-                const float nx = dx * invL, ny = dy * invL;
-                const float g = nx * adj.x + ny * adj.y;
-                gs += g * f * a.dt;
-                if (road != cur_road) {
-                    if (cur_road != b.num_roads) {
-                        if (nrec < kRecPerSeg) {
-                            b.rec_road[rec0 + nrec] = cur_road;
-                            b.rec_val[rec0 + nrec] = (double)cur_sum;
-                            nrec++;
-                        } else {
-                            atomicOr(a.err, kErrOob);
-                        }
-                    }
-                    cur_road = road;
-                    cur_sum = 0.f;
+        hist[0] = p;
+        uint32_t num_ends = 0, word = 0;
+        for (uint32_t k = 0; k < len; k++) {  // recompute with the recorded events
+            const uint32_t bit = (t0 + k) & 31u;
+            if (k == 0 || bit == 0) word = sched[(t0 + k) >> 5];
+            if ((word >> bit) & 1u) {
+                p.x = l.tx;
+                p.y = l.ty;
+                ends[(size_t)num_ends++ * n] = h;
+                road_end(a.map, a.dt, s, h, l, a.err, [&]() { return rng_next<RNG>(r); });
+            } else {
+                const float dx = l.tx - p.x, dy = l.ty - p.y;
+                const float d2 = dx * dx + dy * dy;
+                if (d2 > 0.f) {
+                    const float q = rsqrtf(d2) * l.step;
+                    p.x += dx * q;
+                    p.y += dy * q;
                 }
-                cur_sum += g * s * a.dt;
-                const float k = s * f * a.dt * invL;
-                adj.x -= k * (adj.x - nx * g);
-                adj.y -= k * (adj.y - ny * g);
             }
+            hist[(size_t)(k + 1u) * n] = p;
         }
-        if (t == t0) break;
-        pt = pp;
-        pp = pp_n;
-        hw = hw_n;
-        sl = sl_n;
-    }
-    if (cur_road != b.num_roads) {
-        if (nrec < kRecPerSeg) {
-            b.rec_road[rec0 + nrec] = cur_road;
-            b.rec_val[rec0 + nrec] = (double)cur_sum;
-            nrec++;
-        } else {
-            atomicOr(a.err, kErrOob);
+        // reverse sweep: p is the position after the tick, pp before it; the history is
+        // fetched kAhead ticks early
+        constexpr int kAhead = 4;
+        float2 ahead[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) ahead[q] = hist[(size_t)(len > 1u + q ? len - 1u - q : 0u) * n];
+        float gs = 0.f, cur_sum = 0.f;
+        uint32_t cur_road = b.num_roads, nrec = 0;
+        uint32_t road = h & kHeadRoad;
+        float f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
+        auto record = [&]() {
+            if (cur_road == b.num_roads) return;
+            if (nrec < kRecPerSeg) {
+                rec[records++] = make_uint2(cur_road, __float_as_uint(cur_sum));
+                nrec++;
+            } else {
+                atomicOr(a.err, kErrOob);
+            }
+        };
+        for (uint32_t k = len; k-- > 0;) {  // tick t0 + k + 1
+            const uint32_t bit = (t0 + k) & 31u;
+            if (k == len - 1u || bit == 31u) word = sched[(t0 + k) >> 5];
+            const float2 pp = ahead[0];
+#pragma unroll
+            for (int q = 0; q + 1 < kAhead; q++) ahead[q] = ahead[q + 1];
+            ahead[kAhead - 1] = hist[(size_t)(k > (uint32_t)kAhead ? k - kAhead : 0u) * n];
+            {  // + (1/T) d splat(p_t)/dp . lambda
+                const float ux = cell_coord(p.x, sx), uy = cell_coord(p.y, sy);
+                float wx, wy;
+                float fx, fy;
+                if (in_cell(c, ux, uy, wx, wy)) {
+                    fx = wx - c.one;  // exact: fbits bits
+                    fy = wy - c.one;
+                } else {
+                    const Splat sp = splat_of(ux, uy, a.fbits);
+                    const float l00 = lam_at(b.lambda, a.gw, a.gh, sp.i0, sp.j0);
+                    const float l10 = lam_at(b.lambda, a.gw, a.gh, sp.i0 + 1, sp.j0);
+                    const float l01 = lam_at(b.lambda, a.gw, a.gh, sp.i0, sp.j0 + 1);
+                    const float l11 = lam_at(b.lambda, a.gw, a.gh, sp.i0 + 1, sp.j0 + 1);
+                    dx0 = l10 - l00;
+                    dx1 = l11 - l01;
+                    dy0 = l01 - l00;
+                    dy1 = l11 - l10;
+                    fx = (float)sp.fx * scale;  // exact: fewer than 24 bits
+                    fy = (float)sp.fy * scale;
+                    c.fi = (float)sp.i0;
+                    c.fj = (float)sp.j0;
+                }
+                const float gx = ((1.f - fy) * dx0 + fy * dx1) * sx;
+                const float gy = ((1.f - fx) * dy0 + fx * dy1) * sy;
+                adj.x += gx * invT;
+                adj.y += gy * invT;
+            }
+            if ((word >> bit) & 1u) {
+                adj = make_float2(0.f, 0.f);
+                h = ends[(size_t)--num_ends * n];  // the road before this tick
+                road = h & kHeadRoad;
+                l = leg_of(a.map, a.dt, s, road, __ldg(&a.map.road_pos[road]), (h & kHeadToEnd) != 0);
+                f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
+            } else {
+                const float dx = l.tx - pp.x, dy = l.ty - pp.y;
+                const float d2 = dx * dx + dy * dy;
+                if (d2 > 0.f) {
+                    const float invL = rsqrtf(d2);
+                    const float nx = dx * invL, ny = dy * invL;
+                    const float g = nx * adj.x + ny * adj.y;
+                    gs += g * f * a.dt;
+                    if (road != cur_road) {
+                        record();
+                        cur_road = road;
+                        cur_sum = 0.f;
+                    }
+                    cur_sum += g * s * a.dt;
+                    const float q = l.step * invL;
+                    adj.x -= q * (adj.x - nx * g);
+                    adj.y -= q * (adj.y - ny * g);
+                }
+            }
+            p = pp;
         }
+        record();
+        gspeed += (double)gs;
     }
-    for (uint32_t j = nrec; j < kRecPerSeg; j++) {
-        b.rec_road[rec0 + j] = b.num_roads;
-        b.rec_val[rec0 + j] = 0.0;
-    }
-    b.carry[e] = adj;
-    b.gspeed[e] += (double)gs;
+    b.gspeed[e] = gspeed;
+    if (b.gspeed_out) b.gspeed_out[b.perm[e]] = (float)gspeed;
+    b.rec_count[e] = records;
+    if (records) atomicAdd(&b.rec_block[e / kRecBlock], records);
 }
 
-// sum of every road's records in sorted (stable) order
-__global__ void k_adj_road_sum(const uint32_t* __restrict__ kstart, const uint32_t* __restrict__ sorted_rec,
-                               const double* __restrict__ rec_val, uint32_t num_roads, uint32_t total,
-                               double* gfactor, float* out) {
-    const uint32_t rd = blockIdx.x * blockDim.x + threadIdx.x;
-    if (rd >= num_roads) return;
-    const uint32_t lo = kstart[rd], hi = min(kstart[rd + 1], total);
+// Road gradients: the entities' records (about 30 of the 160 places of an entity are
+// used at K = 100) are packed in entity order, sorted by road with the stable radix
+// sort and summed per road.  One block: the exclusive scan of the records per
+// kRecBlock entities (rec_block is left zeroed for the next backward), the total, and
+// zeroed digit counts.
+__global__ __launch_bounds__(1024) void k_adj_rec_scan(uint32_t* rec_block, uint32_t* rec_base, uint32_t blocks,
+                                                       uint32_t* total, uint32_t* hist) {
+    __shared__ uint32_t s_warp[32];
+    __shared__ uint32_t s_run;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (tid < kMaxPasses * kRadix) hist[tid] = 0u;
+    if (tid == 0) s_run = 0u;
+    __syncthreads();
+    for (uint32_t b0 = 0; b0 < blocks; b0 += 1024u) {
+        const uint32_t i = b0 + tid;
+        const uint32_t v = i < blocks ? rec_block[i] : 0u;
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t before = s_run;
+        for (uint32_t w = 0; w < warp; w++) before += s_warp[w];
+        if (i < blocks) {
+            rec_base[i] = before + incl - v;
+            rec_block[i] = 0u;
+        }
+        __syncthreads();
+        if (tid == 1023u) s_run = before + incl;
+        __syncthreads();
+    }
+    if (tid == 0) *total = s_run;
+}
+
+// One block per kRecBlock entities: their records end to end, 256 at a time (the
+// entity of a record by binary search in the scanned counts), and the roads' digits.
+__global__ __launch_bounds__(256) void k_adj_rec_pack(const uint2* __restrict__ rec,
+                                                      const uint32_t* __restrict__ rec_count,
+                                                      const uint32_t* __restrict__ rec_base, uint32_t n, uint32_t places,
+                                                      uint32_t passes, uint32_t* __restrict__ key,
+                                                      uint32_t* __restrict__ val, uint32_t* hist) {
+    constexpr uint32_t kPer = kRecBlock / 256u;
+    __shared__ uint32_t s_first[kRecBlock + 1];  // records before each entity of the block
+    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_hist[kMaxPasses * kRadix];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    for (uint32_t i = tid; i < passes * kRadix; i += 256u) s_hist[i] = 0u;
+    const uint32_t e0 = blockIdx.x * kRecBlock;
+    uint32_t v[kPer], sum = 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) {
+        const uint32_t e = e0 + tid * kPer + k;
+        v[k] = e < n ? rec_count[e] : 0u;
+        sum += v[k];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t run = incl - sum;
+    for (uint32_t w = 0; w < warp; w++) run += s_warp[w];
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) {
+        s_first[tid * kPer + k] = run;
+        run += v[k];
+    }
+    if (tid == 255u) s_first[kRecBlock] = run;
+    __syncthreads();
+    const uint32_t count = s_first[kRecBlock], base = rec_base[blockIdx.x];
+    for (uint32_t i = tid; i < count; i += 256u) {
+        uint32_t o = 0;  // last entity that begins at or before record i
+#pragma unroll
+        for (uint32_t st = kRecBlock / 2u; st > 0; st >>= 1)
+            if (s_first[o + st] <= i) o += st;
+        const uint2 x = rec[(size_t)(e0 + o) * places + (i - s_first[o])];
+        key[base + i] = x.x;
+        val[base + i] = x.y;
+        for (uint32_t ps = 0; ps < passes; ps++) atomicAdd(&s_hist[ps * kRadix + ((x.x >> (8u * ps)) & 0xffu)], 1u);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < passes * kRadix; i += 256u)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+// One warp per road: its run of the sorted records by two binary searches (lanes 0 and
+// 1), summed in double strided by lane, then a tree: a fixed order.
+__global__ __launch_bounds__(256) void k_adj_road_sum(const uint32_t* __restrict__ key, const float* __restrict__ val,
+                                                      const uint32_t* __restrict__ total, uint32_t num_roads,
+                                                      double* gfactor, float* out, const uint32_t* err) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t rd = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (rd >= num_roads || (*err & kErrTimeout)) return;  // uniform per warp
+    uint32_t lo = 0, hi = *total;
+    const uint32_t want = rd + (lane & 1u);  // first record of road `want` or later
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (key[mid] < want) lo = mid + 1u;
+        else hi = mid;
+    }
+    const uint32_t from = __shfl_sync(FULL, lo, 0), to = __shfl_sync(FULL, lo, 1);
     double s = 0.0;
-    for (uint32_t q = lo; q < hi; q++) s += rec_val[sorted_rec[q]];
-    gfactor[rd] = s;
-    if (out) out[rd] = (float)s;
+    for (uint32_t q = from + lane; q < to; q += 32u) s += (double)val[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o);
+    if (lane == 0) {
+        gfactor[rd] = s;
+        if (out) out[rd] = (float)s;
+    }
 }
 
 // Entities are kept in spatial order inside the context (perm[i] = entity id of
-// internal index i); these move per-entity arrays across that boundary.
-__global__ void k_adj_speed_out(const double* gspeed, const uint32_t* perm, uint32_t n, float* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[perm[i]] = (float)gspeed[i];
-}
+// internal index i); this moves a per-entity array across that boundary.
 __global__ void k_adj_gather(const float* __restrict__ in, const uint32_t* __restrict__ perm, uint32_t n,
                              float* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = in[perm[i]];
-}
-
-// Digit histograms of the record keys for the radix sort (keys < 2^(8*passes)).
-__global__ void k_adj_hist(const uint32_t* __restrict__ keys, size_t count, uint32_t passes, uint32_t* hist) {
-    __shared__ uint32_t s_hist[kMaxPasses * kRadix];
-    for (uint32_t i = threadIdx.x; i < passes * kRadix; i += blockDim.x) s_hist[i] = 0;
-    __syncthreads();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t k = keys[i];
-        for (uint32_t ps = 0; ps < passes; ps++) atomicAdd(&s_hist[ps * kRadix + ((k >> (8 * ps)) & 0xffu)], 1u);
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < passes * kRadix; i += blockDim.x)
-        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
@@ -465,22 +632,27 @@ struct msim_adj {
     uint32_t* sched = nullptr;
     float2* hist_pos = nullptr;
     uint32_t* hist_head = nullptr;
-    float2* carry = nullptr;
     double* gspeed = nullptr;
     double* gfactor = nullptr;
-    uint32_t* rec_road = nullptr;
-    double* rec_val = nullptr;
+    uint2* rec = nullptr;             // road-visit records, a fixed place count per entity
+    uint32_t* rec_used = nullptr;     // records of each entity
+    uint32_t* rec_block = nullptr;    // records per kRecBlock entities (zero between backwards)
+    uint32_t* rec_base = nullptr;     // their exclusive scan
+    uint32_t* rec_total = nullptr;
     uint32_t* sk[2] = {nullptr, nullptr};
     uint32_t* sv[2] = {nullptr, nullptr};
     uint32_t* hist = nullptr;
     uint32_t* lookback = nullptr;
     uint32_t* tickets = nullptr;
-    uint32_t* kstart = nullptr;
+    uint32_t* sort_dirty = nullptr;   // look-back words each region's last pass published
+    bool sort_clean = false;          // regions, tickets and extents are as the chained passes expect
+    uint32_t lanes = 32;
     uint32_t* err = nullptr;
     uint32_t* perm = nullptr;        // device: entity id of each internal index
     std::vector<uint32_t> hperm;     // host copy
     size_t rec_count = 0;
-    uint32_t rec_tiles = 0;
+    size_t sort_region = 0;           // look-back words per pass
+    bool sort_large = false;          // 4096-record tiles (else 1024)
     bool have_forward = false;
     bool have_backward = false;
     bool have_sched = false;
@@ -521,7 +693,21 @@ uint32_t splat_fraction_bits(uint32_t gw, uint32_t gh) {
     return (uint32_t)std::max(16, std::min(22, fb));
 }
 
-AdjArgs fwd_args(msim_adj* a, uint32_t mode) {
+// Entities per warp: 32, halved (to kAdjMinLanes) while that leaves the schedulers
+// fewer than two warps each.  Small counts are bound by the latency of a tick, and the
+// road end or cell change of one lane adds to every lane of its warp.
+constexpr uint32_t kAdjMinLanes = 4;
+uint32_t adj_lanes(uint32_t n, int sms) {
+    uint32_t lanes = 32;
+    while (lanes > kAdjMinLanes && n / lanes < 8u * (uint32_t)std::max(sms, 1)) lanes /= 2;
+    return lanes;
+}
+unsigned adj_blocks(const msim_adj* a) {
+    const uint64_t warps = ((uint64_t)a->n + a->lanes - 1u) / a->lanes;
+    return (unsigned)((warps * 32u + kAdjThreads - 1u) / kAdjThreads);
+}
+
+AdjArgs fwd_args(msim_adj* a) {
     AdjArgs f{};
     f.map.road_pos = a->road_pos;
     f.map.road_conn = a->road_conn;
@@ -548,7 +734,7 @@ AdjArgs fwd_args(msim_adj* a, uint32_t mode) {
     f.ck_rng = a->ck_rng;
     f.dacc = a->dacc;
     f.sched = a->sched;
-    f.mode = mode;
+    f.lanes = a->lanes;
     f.err = a->err;
     return f;
 }
@@ -559,6 +745,7 @@ int check_status(msim_adj* a) {
     ACK(cudaMemcpy(&h, a->err, sizeof(h), cudaMemcpyDeviceToHost), "read device status");
     if (h) {
         ACK(cudaMemset(a->err, 0, sizeof(uint32_t)), "clear device status");
+        a->sort_clean = false;
         if (h & kErrTimeout) return fail(MSIM_ERR_TIMEOUT, "a bounded device wait gave up in the road-gradient sort");
         return fail(MSIM_ERR_OOB, "device-side index check failed in the adjoint (or more than 8 road visits per "
                                   "entity in one checkpoint segment)");
@@ -616,7 +803,14 @@ int msim_adj_create(const msim_map* map, const msim_adj_params* params, msim_adj
     if (a->passes > kMaxPasses) return bail(fail(MSIM_ERR_INVALID, "too many roads for the record sort"));
     a->rec_count = (size_t)a->S * a->n * kRecPerSeg;
     if (a->rec_count >= (1ull << 30)) return bail(fail(MSIM_ERR_INVALID, "ticks x entities too large for the record sort"));
-    a->rec_tiles = (uint32_t)((a->rec_count + kSortTile - 1) / kSortTile);
+    // about one record place in six is used: 1024-record tiles where 4096-record ones
+    // would leave most of the chip idle
+    a->sort_large = a->rec_count >= (1u << 22);
+    a->sort_region = a->sort_large ? (a->rec_count + kSortTile - 1) / kSortTile * kRadix
+                                   : sort_lookback_words((uint32_t)a->rec_count);
+    int sms = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device);
+    a->lanes = adj_lanes(a->n, sms);
     cudaError_t e = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
     cudaEventCreate(&a->t0);
@@ -630,14 +824,16 @@ int msim_adj_create(const msim_map* map, const msim_adj_params* params, msim_adj
         (rc = aalloc(a, &a->ck_head, a->S * n)) || (rc = aalloc(a, &a->ck_rng, a->S * n)) ||
         (rc = aalloc(a, &a->dacc, G)) || (rc = aalloc(a, &a->density, G)) || (rc = aalloc(a, &a->lambda, G)) ||
         (rc = aalloc(a, &a->partial, (G + 255) / 256)) || (rc = aalloc(a, &a->loss, 1)) ||
-        (rc = aalloc(a, &a->sched, n * a->sched_words)) || (rc = aalloc(a, &a->hist_pos, K * n)) ||
-        (rc = aalloc(a, &a->hist_head, K * n)) || (rc = aalloc(a, &a->carry, n)) || (rc = aalloc(a, &a->gspeed, n)) ||
-        (rc = aalloc(a, &a->gfactor, a->R)) || (rc = aalloc(a, &a->rec_road, a->rec_count)) ||
-        (rc = aalloc(a, &a->rec_val, a->rec_count)) || (rc = aalloc(a, &a->sk[0], a->rec_count)) ||
+        (rc = aalloc(a, &a->sched, n * a->sched_words)) || (rc = aalloc(a, &a->hist_pos, (K + 1) * n)) ||
+        (rc = aalloc(a, &a->hist_head, K * n)) || (rc = aalloc(a, &a->gspeed, n)) ||
+        (rc = aalloc(a, &a->gfactor, a->R)) || (rc = aalloc(a, &a->rec, a->rec_count)) ||
+        (rc = aalloc(a, &a->rec_used, n)) || (rc = aalloc(a, &a->rec_block, (n + kRecBlock - 1) / kRecBlock)) ||
+        (rc = aalloc(a, &a->rec_base, (n + kRecBlock - 1) / kRecBlock)) || (rc = aalloc(a, &a->rec_total, 1)) ||
+        (rc = aalloc(a, &a->sk[0], a->rec_count)) ||
         (rc = aalloc(a, &a->sk[1], a->rec_count)) || (rc = aalloc(a, &a->sv[0], a->rec_count)) ||
         (rc = aalloc(a, &a->sv[1], a->rec_count)) || (rc = aalloc(a, &a->hist, (size_t)kMaxPasses * kRadix)) ||
-        (rc = aalloc(a, &a->lookback, (size_t)kMaxPasses * a->rec_tiles * kRadix)) ||
-        (rc = aalloc(a, &a->tickets, (size_t)kMaxPasses)) || (rc = aalloc(a, &a->kstart, (size_t)a->R + 2)) ||
+        (rc = aalloc(a, &a->lookback, a->passes * a->sort_region)) ||
+        (rc = aalloc(a, &a->tickets, (size_t)kMaxPasses)) || (rc = aalloc(a, &a->sort_dirty, (size_t)kMaxPasses)) ||
         (rc = aalloc(a, &a->err, 1)) || (rc = aalloc(a, &a->perm, n)))
         return bail(rc);
     std::vector<uint32_t> conn(a->C + 1);
@@ -649,6 +845,7 @@ int msim_adj_create(const msim_map* map, const msim_adj_params* params, msim_adj
     if (e == cudaSuccess) e = cudaMemcpy(a->conn, conn.data(), sizeof(uint32_t) * (a->C + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(a->factor, ones.data(), sizeof(float) * a->R, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(a->err, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(a->rec_block, 0, sizeof(uint32_t) * ((n + kRecBlock - 1) / kRecBlock));
     if (e == cudaSuccess) e = cudaMemset(a->target, 0, sizeof(float) * G);
     if (e != cudaSuccess) return bail(cuda_fail(e, "adjoint set-up"));
     // initial entity state: the deterministic initializer of msim_init_entities
@@ -762,17 +959,22 @@ int msim_adj_forward(msim_adj* a, const float* d_speed, const float* d_factor, c
     if (d_target)
         ACK(cudaMemcpyAsync(a->target, d_target, sizeof(float) * G, cudaMemcpyDeviceToDevice, a->stream), "target");
     ACK(cudaMemsetAsync(a->dacc, 0, sizeof(unsigned long long) * G, a->stream), "memset density");
-    AdjArgs f = fwd_args(a, mode);
-    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const AdjArgs f = fwd_args(a);
+    const unsigned blocks = adj_blocks(a);
     cudaEventRecord(a->ph[0], a->stream);
-    if (a->p.rng_kind == 1) k_adj_forward<1><<<blocks, 256, 0, a->stream>>>(f);
-    else k_adj_forward<0><<<blocks, 256, 0, a->stream>>>(f);
+    if (a->p.rng_kind == 1) {
+        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<1, true><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+        else k_adj_forward<1, false><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+    } else {
+        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<0, true><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+        else k_adj_forward<0, false><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+    }
     ACK(cudaGetLastError(), "k_adj_forward");
     cudaEventRecord(a->ph[1], a->stream);
     const unsigned gb = (unsigned)((G + 255) / 256);
     k_adj_loss<<<gb, 256, 0, a->stream>>>(a->dacc, a->target, (uint32_t)G, a->p.ticks, a->density, a->lambda,
                                           a->partial);
-    k_adj_loss_final<<<1, 32, 0, a->stream>>>(a->partial, gb, (uint32_t)G, a->loss);
+    k_adj_loss_final<<<1, 256, 0, a->stream>>>(a->partial, gb, (uint32_t)G, a->loss);
     ACK(cudaGetLastError(), "k_adj_loss");
     cudaEventRecord(a->ph[2], a->stream);
     if (d_density)
@@ -791,54 +993,56 @@ int msim_adj_backward(msim_adj* a, float* d_grad_speed, float* d_grad_factor) {
     if (!a) return fail(MSIM_ERR_INVALID, "NULL argument");
     if (!a->have_forward) return fail(MSIM_ERR_INVALID, "backward needs a forward first");
     cudaSetDevice(a->device);
-    const size_t n = a->n;
-    ACK(cudaMemsetAsync(a->carry, 0, sizeof(float2) * n, a->stream), "memset carry");
-    ACK(cudaMemsetAsync(a->gspeed, 0, sizeof(double) * n, a->stream), "memset gspeed");
     AdjBack b{};
-    b.f = fwd_args(a, 2u);  // the backward replays the last forward's schedule
+    b.f = fwd_args(a);
+    b.segments = a->S;
     b.lambda = a->lambda;
     b.hist_pos = a->hist_pos;
     b.hist_head = a->hist_head;
-    b.carry = a->carry;
     b.gspeed = a->gspeed;
-    b.rec_road = a->rec_road;
-    b.rec_val = a->rec_val;
+    b.gspeed_out = d_grad_speed;
+    b.perm = a->perm;
+    b.rec = a->rec;
+    b.rec_count = a->rec_used;
+    b.rec_block = a->rec_block;
     b.num_roads = a->R;
-    const unsigned blocks = (unsigned)((n + 255) / 256);
     cudaEventRecord(a->ph[3], a->stream);
-    for (int seg = (int)a->S - 1; seg >= 0; seg--) {
-        b.seg = (uint32_t)seg;
-        if (a->p.rng_kind == 1) k_adj_backward<1><<<blocks, 256, 0, a->stream>>>(b);
-        else k_adj_backward<0><<<blocks, 256, 0, a->stream>>>(b);
-        ACK(cudaGetLastError(), "k_adj_backward");
-    }
+    if (a->p.rng_kind == 1) k_adj_backward<1><<<adj_blocks(a), kAdjThreads, 0, a->stream>>>(b);
+    else k_adj_backward<0><<<adj_blocks(a), kAdjThreads, 0, a->stream>>>(b);
+    ACK(cudaGetLastError(), "k_adj_backward");
     cudaEventRecord(a->ph[4], a->stream);
-    // road gradients: stable sort of the records by road, then per-road sums in order
-    const uint32_t total = (uint32_t)a->rec_count;
-    ACK(cudaMemsetAsync(a->hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, a->stream), "memset hist");
-    k_adj_hist<<<1024, 256, 0, a->stream>>>(a->rec_road, a->rec_count, a->passes, a->hist);
-    ACK(cudaGetLastError(), "k_adj_hist");
-    ACK(cudaMemsetAsync(a->lookback, 0, sizeof(uint32_t) * (size_t)a->passes * a->rec_tiles * kRadix, a->stream),
-        "memset lookback");
-    ACK(cudaMemsetAsync(a->tickets, 0, sizeof(uint32_t) * kMaxPasses, a->stream), "memset tickets");
+    // road gradients: the records packed, stably sorted by road, summed per road
+    const uint32_t rec_blocks = (a->n + kRecBlock - 1u) / kRecBlock;
+    k_adj_rec_scan<<<1, 1024, 0, a->stream>>>(a->rec_block, a->rec_base, rec_blocks, a->rec_total, a->hist);
+    k_adj_rec_pack<<<rec_blocks, 256, 0, a->stream>>>(a->rec, a->rec_used, a->rec_base, a->n, a->S * kRecPerSeg,
+                                                      a->passes, a->sk[0], a->sv[0], a->hist);
+    ACK(cudaGetLastError(), "k_adj_rec_pack");
+    // with two or more passes each clears the next one's look-back words and ticket
+    const bool chained = a->passes >= 2;
+    if (!a->sort_clean || !chained) {
+        ACK(cudaMemsetAsync(a->lookback, 0, sizeof(uint32_t) * a->passes * a->sort_region, a->stream), "memset lookback");
+        ACK(cudaMemsetAsync(a->tickets, 0, sizeof(uint32_t) * kMaxPasses, a->stream), "memset tickets");
+        ACK(cudaMemsetAsync(a->sort_dirty, 0, sizeof(uint32_t) * kMaxPasses, a->stream), "memset look-back extents");
+    }
+    a->sort_clean = false;  // until every pass has launched
     for (uint32_t ps = 0; ps < a->passes; ps++) {
-        const uint32_t* kin = ps == 0 ? a->rec_road : a->sk[(ps - 1) & 1];
-        const uint32_t* vin = ps == 0 ? nullptr : a->sv[(ps - 1) & 1];
-        ACK(launch_onesweep(a->stream, kin, vin, a->sk[ps & 1], a->sv[ps & 1], total, 8u * ps,
-                            a->hist + ps * kRadix, a->lookback + (size_t)ps * a->rec_tiles * kRadix,
-                            a->tickets + ps, a->err),
+        SweepChain ch;
+        const uint32_t nx = (ps + 1u) % a->passes;
+        ch.next_lookback = a->lookback + nx * a->sort_region;
+        ch.next_ticket = a->tickets + nx;
+        ch.next_dirty = a->sort_dirty + nx;
+        ch.my_dirty = a->sort_dirty + ps;
+        ACK(launch_onesweep(a->stream, a->sk[ps & 1], a->sv[ps & 1], a->sk[(ps + 1) & 1], a->sv[(ps + 1) & 1],
+                            (uint32_t)a->rec_count, 8u * ps, a->hist + ps * kRadix, a->lookback + ps * a->sort_region,
+                            a->tickets + ps, a->err, a->rec_total, chained ? &ch : nullptr, kDefaultSpinLimit,
+                            a->sort_large),
             "k_onesweep");
     }
-    const uint32_t* sorted_key = a->sk[(a->passes - 1) & 1];
-    const uint32_t* sorted_rec = a->sv[(a->passes - 1) & 1];
-    ACK(launch_kstart(a->stream, sorted_key, total, a->kstart, a->R + 1), "k_kstart");
-    k_adj_road_sum<<<(a->R + 255) / 256, 256, 0, a->stream>>>(a->kstart, sorted_rec, a->rec_val, a->R, total,
-                                                              a->gfactor, d_grad_factor);
+    a->sort_clean = true;
+    k_adj_road_sum<<<(a->R + 7u) / 8u, 256, 0, a->stream>>>(a->sk[a->passes & 1],
+                                                          reinterpret_cast<const float*>(a->sv[a->passes & 1]),
+                                                          a->rec_total, a->R, a->gfactor, d_grad_factor, a->err);
     ACK(cudaGetLastError(), "k_adj_road_sum");
-    if (d_grad_speed) {
-        k_adj_speed_out<<<blocks, 256, 0, a->stream>>>(a->gspeed, a->perm, a->n, d_grad_speed);
-        ACK(cudaGetLastError(), "k_adj_speed_out");
-    }
     cudaEventRecord(a->ph[5], a->stream);
     a->have_backward = true;
     return check_status(a);

@@ -826,13 +826,15 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
 cudaError_t launch_onesweep(cudaStream_t s, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                             uint32_t* vals_out, uint32_t n, uint32_t shift, const uint32_t* digit_count,
                             uint32_t* lookback, uint32_t* ticket, uint32_t* err, const uint32_t* n_dev,
-                            const SweepChain* chain, uint32_t spin_limit) {
+                            const SweepChain* chain, uint32_t spin_limit, bool many) {
     if (n == 0) return cudaSuccess;
     static bool carveout = false;  // prefer the largest shared-memory carveout: 4 blocks of 43 KB per SM
     if (!carveout) {
         cudaFuncSetAttribute(k_onesweep<false, kSortRows>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cudaFuncSetAttribute(k_onesweep<true, kSortRowsDev>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(k_onesweep<true, kSortRows>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cudaGetLastError();
         carveout = true;
@@ -842,8 +844,11 @@ cudaError_t launch_onesweep(cudaStream_t s, const uint32_t* keys_in, const uint3
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const unsigned grid =
-            std::min<unsigned>(blocks_for(n, kSortThreads * kSortRowsDev), 4u * (unsigned)(sms > 0 ? sms : 1));
+        const unsigned grid = std::min<unsigned>(blocks_for(n, many ? kSortTile : kSortThreads * kSortRowsDev),
+                                                 4u * (unsigned)(sms > 0 ? sms : 1));
+        if (many)
+            return launch_chained(k_onesweep<true, kSortRows>, grid, kSortThreads, s, keys_in, vals_in, keys_out,
+                                  vals_out, n, shift, digit_count, lookback, ticket, err, n_dev, ch, spin_limit);
         return launch_chained(k_onesweep<true, kSortRowsDev>, grid, kSortThreads, s, keys_in, vals_in, keys_out,
                               vals_out, n, shift, digit_count, lookback, ticket, err, n_dev, ch, spin_limit);
     }
