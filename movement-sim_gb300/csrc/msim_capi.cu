@@ -180,6 +180,7 @@ struct msim_ctx {
     uint32_t* err = nullptr;
     uint32_t* check = nullptr;  // first invalid heading found by msim_set_entities
     TileGrid grid{};
+    bool dense = false;  // many neighbours expected (see msim_create): the query's dense kernel
     uint32_t passes = 1;
     uint32_t resort = 16;
     uint32_t since_permute = 0;
@@ -373,6 +374,11 @@ EntityState& cur_state(msim_ctx* c) { return c->st[c->cur]; }
 // 0.0437, 2.0 0.558 / 0.0437, 3.0 0.568 / 0.0437.  At densities where a query meets
 // 17 or 70 neighbours it costs the same at 0 and 1.0 (1.41 and 22.4 ms at 1 M).
 constexpr float kWidenLimit = 1.0f;
+
+// Expected neighbours along the road above which the query's dense kernel is used.
+// Measured at 1 M entities, sparse / dense kernel: 0.68 33.1 / 37.6 us, 1.02 40.0 / 40.5,
+// 1.36 46.5 / 45.5, 2.0 55.1 / 52.5, 2.7 81.3 / 63.2, 3.4 170 / 104.
+constexpr double kDenseNeighbours = 1.2;
 
 // rank[slot] (written by every later merge once allocated): false when the allocation
 // fails.
@@ -838,7 +844,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
         CKL(p, launch_query(qs, c->params.cap, c->kstart, c->sorted_slot, pos ? pos : c->sorted_pos,
                         c->slots_identity ? nullptr : cur_state(c).slot_id, grid ? *grid : c->grid,
                         c->n, c->nbr_count, c->nbr_list, c->pairs, c->err,
-                        c->slots_identity ? count_by_id : nullptr),
+                        c->slots_identity ? count_by_id : nullptr, c->dense),
            "k_query");
     }
     if (qs != c->stream) {
@@ -979,6 +985,17 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     c->grid.reach = (float)reach;
     c->grid.radius = p.radius;
     c->grid.d2_limit = sqrt_limit(p.radius);
+    // Entities within the radius along an entity's own road, both ways, were all roads
+    // filled evenly: picks the query kernel (the results are the same).  The road length
+    // from at most 4,096 roads spread over the list.
+    double road_length = 0.0;
+    const uint64_t every = std::max<uint64_t>(1u, c->R / 4096u);
+    for (uint64_t r = 0; r < c->R; r += every) {
+        const float* q = map->road_pos + 4 * r;
+        const double dx = (double)q[2] - (double)q[0], dy = (double)q[3] - (double)q[1];
+        road_length += std::sqrt(dx * dx + dy * dy) * (double)every;
+    }
+    c->dense = 2.0 * radius * (double)c->n > kDenseNeighbours * road_length;
     // y bands inside a tile fill the key up to 24 bits (3 radix passes), at most 64
     // bands, and keep the key-start table within about four entries per entity
     uint32_t nbits = 0;

@@ -533,11 +533,8 @@ __global__ void k_ranges(const uint32_t* __restrict__ sk, uint32_t n, uint32_t* 
     }
 }
 
-// The query keeps the sorted positions of an entity's first kRegKeep neighbours in
-// shared memory; entities with more take list_overflow, which walks their tiles again
-// and holds up the whole warp.  At the 16 M workload 0.9 % of the entities have more
-// than 4 neighbours (a quarter of the warps would wait) and 0.001 % more than 8.
-constexpr int kRegKeep = 8;
+// Lists of up to this many ids are sorted in registers.
+constexpr int kSortInRegisters = 8;
 
 // Exact ascending list of the cap smallest ids of one entity, written by
 // insertion straight into its output slots; for the rare entities with more
@@ -912,25 +909,25 @@ cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n
 
 cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, const uint32_t* sorted_slot,
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
-                         uint32_t* list, unsigned long long* pair_bins, const uint32_t* err, uint32_t* count_by_id) {
+                         uint32_t* list, unsigned long long* pair_bins, const uint32_t* err, uint32_t* count_by_id,
+                         bool dense) {
     if (n == 0) return cudaSuccess;
-    static bool carveout = false;  // 16 blocks of ~9.5 KB per SM
+    using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
+                           uint32_t*, uint32_t*, unsigned long long*, const uint32_t*, uint32_t*);
+    static const Query kernels[2][2] = {{k_query<false, kQueryKeep, false>, k_query<false, kQueryKeepDense, true>},
+                                        {k_query<true, kQueryKeep, false>, k_query<true, kQueryKeepDense, true>}};
+    static bool carveout = false;  // 16 blocks of ~11.5 KB per SM (dense: 9 of ~23.5 KB)
     if (!carveout) {
-        cudaFuncSetAttribute(k_query<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(k_query<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+        for (int i = 0; i < 4; i++)
+            cudaFuncSetAttribute(kernels[i >> 1][i & 1], cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared);
         cudaGetLastError();
         carveout = true;
     }
-    if (cap > 0 && list)
-        k_query<true><<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(kstart, sorted_slot, sorted_pos, slot_id,
-                                                                            grid, n, cap, count, list, pair_bins, err,
-                                                                            count_by_id);
-    else
-        k_query<false><<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(kstart, sorted_slot, sorted_pos, slot_id,
-                                                                             grid, n, 0u, count, nullptr, pair_bins, err,
-                                                                             count_by_id);
+    const bool lists = cap > 0 && list;
+    kernels[lists][dense]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
+        kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins, err,
+        count_by_id);
     return cudaGetLastError();
 }
 

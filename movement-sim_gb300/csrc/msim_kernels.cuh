@@ -20,6 +20,8 @@ constexpr int kStepThreads = 512;  // measured at 16 M: 0.122 ms per tick agains
 constexpr int kStepPer = 1;        // entities per thread and iteration of k_step
 constexpr int kMoveThreads = 128;  // move-only multi-tick launches (k_move)
 constexpr uint32_t kMaxCap = 256;
+constexpr int kQueryKeep = 8;        // neighbours the query keeps per entity (more are collected again)
+constexpr int kQueryKeepDense = 32;  // the same in its kernel for dense populations
 constexpr uint32_t kPairBins = 256;  // pair counters (summed on read), spread to avoid one hot atomic
 
 // Entity state in slot order (structure of arrays)
@@ -116,7 +118,8 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          const uint32_t* err = nullptr,  // err: the status word (skip after a failed wait)
                          // count_by_id (may be NULL; only when slot = entity id): every count also
                          // written at its entity's id
-                         uint32_t* count_by_id = nullptr);
+                         uint32_t* count_by_id = nullptr,
+                         bool dense = false);  // dense: the kernel for many neighbours (the same results)
 // Incremental index update: split the previous sorted order P (keys PK; P[q] = q when
 // identity) by whether the new key NK[slot] changed (A: unchanged, B: changed; counts
 // -> counts[0..1]; B's digit counts -> hist), then, after B is sorted, merge A and B

@@ -259,31 +259,49 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 // run lengths; the run of each pair comes from a bit mask of the runs that start in
 // the current window of 32 pairs.  Every candidate is tested with the predicate of
 // random_move.comp:551-562; candidate positions come from the sorted copy, read in
-// runs.  A hit adds one to the owner's count and, for the first kRegKeep hits,
-// keeps the candidate's sorted position; ids are looked up only for those.  An
-// entity with more than kRegKeep neighbours redoes an exact pass into its output
-// slots.  The predicate is symmetric (fl(a - b) = -fl(b - a)), so the pair count is
-// half the sum of the counts, and a pair of entities of the same warp (most pairs:
-// consecutive sorted entities share their band runs) is tested once, by the lower
-// lane, which credits both.  Each warp writes its lists contiguously at
-// warp * 32 * cap and adds its count sum to one of kPairBins counters; the kernel has
-// no block-wide barrier.
+// runs.  A hit counts for the owner and, for the first KEEP hits, keeps the
+// candidate's sorted position; ids are looked up only for those.  An entity with more
+// than KEEP neighbours has them collected again by its whole warp.  The predicate is
+// symmetric (fl(a - b) = -fl(b - a)), so the pair count is half the sum of the counts,
+// and a pair of entities of the same warp (most pairs: consecutive sorted entities
+// share their band runs) is tested once, by the lower lane, which credits both.  Each
+// warp writes its lists contiguously at warp * 32 * cap and adds its count sum to one
+// of kPairBins counters; the kernel has no block-wide barrier.
+//
+// KEEP and DENSE (chosen by kDenseNeighbours): sparse populations keep 8 and count every hit with
+// a shared atomic; dense ones keep 32 and count an owner's hits by ballot - its pairs lie
+// side by side in a window, where up to 32 atomics on its counter took turns - with
+// atomics only for the credited lanes, and rank longer lists in shared memory.  1 M
+// entities with 4.5 neighbours 170 -> 104 us, 200,000 with 14.6 261 -> 118 us (keeping
+// 16 with more blocks resident 131 and 204, 24 111 and 150: entities beyond pay for
+// list_by_warp).
 constexpr uint32_t kRuns = 4;                  // runs per lane and round
 constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 
+template <int KEEP>
 struct QueryShared {
     float2 me[kQueryThreads];
     uint32_t cnt[kQueryThreads];
-    uint32_t keep[kRegKeep][kQueryThreads];    // sorted positions of the first kRegKeep hits
+    // sorted positions of the first hits; DENSE: the owner's own from the front, those
+    // credited by lower lanes from the back
+    uint32_t keep[KEEP][kQueryThreads];
     uint32_t rq[kQueryThreads / 32][kWarpRuns];   // run start position minus its flat start
     uint32_t rfs[kQueryThreads / 32][kWarpRuns];  // flat start of the run
     uint32_t rown[kQueryThreads / 32][kWarpRuns]; // owner lane
 };
 
-template <bool LIST>
+// Bits [from, to) of a word, both clamped to 0 .. 32.
+__device__ __forceinline__ uint32_t bit_range(int from, int to) {
+    from = max(from, 0);
+    to = min(to, 32);
+    return to > from ? (0xffffffffu >> (32 - (to - from))) << from : 0u;
+}
+
+// own: DENSE: the lane's hits as owner so far.
+template <bool LIST, int KEEP, bool DENSE>
 __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const uint32_t (&len_in)[kRuns],
-                                           uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared& sh,
-                                           const float2* __restrict__ sorted_pos, const TileGrid& g) {
+                                           uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP>& sh,
+                                           const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own) {
     constexpr uint32_t FULL = 0xffffffffu;
     // A pair of entities of this warp is tested once, by the lower lane, which credits
     // both (the predicate is symmetric, and an in-range pair lies in both entities'
@@ -342,28 +360,113 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
         const uint32_t run = ra + (uint32_t)__popc(le) - 1u;  // le == 0: the run begun before the window
         ra += (uint32_t)__popc(marks);
         const uint32_t i = base + lane;
-        if (i >= total) continue;
-        const uint32_t q = sh.rq[warp][run] + i;
-        const uint32_t owner = sh.rown[warp][run];
-        const uint32_t other = q - pwarp;  // the candidate's lane when it is in this warp
-        if (other <= owner) continue;      // the owner itself or a lower lane: tested from there
-        const uint32_t ot = warp * 32u + owner;
-        if (!in_range_fast(sorted_pos[q], sh.me[ot], g.radius, g.d2_limit)) continue;
-        const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
-        if (LIST && c < (uint32_t)kRegKeep) sh.keep[c][ot] = q;  // sorted position; the id comes later
-        if (other < 32u) {  // a higher lane of this warp: the pair counts for it too
-            const uint32_t om = warp * 32u + other;
-            const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
-            if (LIST && c2 < (uint32_t)kRegKeep) sh.keep[c2][om] = pwarp + owner;
+        if constexpr (!DENSE) {
+            if (i >= total) continue;
+            const uint32_t q = sh.rq[warp][run] + i;
+            const uint32_t owner = sh.rown[warp][run];
+            const uint32_t other = q - pwarp;  // the candidate's lane when it is in this warp
+            if (other <= owner) continue;      // the owner itself or a lower lane: tested from there
+            const uint32_t ot = warp * 32u + owner;
+            if (!in_range_fast(sorted_pos[q], sh.me[ot], g.radius, g.d2_limit)) continue;
+            const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
+            if (LIST && c < (uint32_t)KEEP) sh.keep[c][ot] = q;  // sorted position; the id comes later
+            if (other < 32u) {  // a higher lane of this warp: the pair counts for it too
+                const uint32_t om = warp * 32u + other;
+                const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
+                if (LIST && c2 < (uint32_t)KEEP) sh.keep[c2][om] = pwarp + owner;
+            }
+        } else {
+            uint32_t q = 0u, owner = lane, other = 0u;
+            bool hit = false;
+            if (i < total) {
+                q = sh.rq[warp][run] + i;
+                owner = sh.rown[warp][run];
+                other = q - pwarp;
+                hit = other > owner &&
+                      in_range_fast(sorted_pos[q], sh.me[warp * 32u + owner], g.radius, g.d2_limit);
+            }
+            const uint32_t hits = __ballot_sync(FULL, hit);
+            const uint32_t mine = bit_range((int)(fi - flat - base), (int)(fi - base));  // this lane's pairs
+            if (LIST) {
+                const uint32_t before = __shfl_sync(FULL, own, owner), pairs = __shfl_sync(FULL, mine, owner);
+                const uint32_t c = before + (uint32_t)__popc(hits & pairs & lanemask_lt());
+                if (hit && c < (uint32_t)KEEP) sh.keep[c][warp * 32u + owner] = q;
+            }
+            own += (uint32_t)__popc(hits & mine);
+            if (hit && other < 32u) {
+                const uint32_t om = warp * 32u + other;
+                const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
+                if (LIST && c2 < (uint32_t)KEEP) sh.keep[KEEP - 1 - c2][om] = pwarp + owner;
+            }
         }
     }
     __syncwarp();  // before the run list is rewritten
 }
 
+// The ascending list of lane o's entity (count > KEEP neighbours, at most the 32 * KEEP
+// that the warp's keep words hold) by the whole warp: its runs again, 32 candidates at a
+// time, every hit's id into the keep words, then each id to its rank among them.  One
+// lane walking its tiles and inserting into its output slots held up its warp: at a
+// million entities with 10 m radius three of four warps have such an entity.
+template <int KEEP>
+__device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_slot,
+                                          const float2* __restrict__ sorted_pos, const uint32_t* __restrict__ slot_id,
+                                          const uint32_t* __restrict__ kstart, const TileGrid& g, uint32_t n,
+                                          uint32_t p, float2 me, uint32_t count, uint32_t cap, uint32_t* words,
+                                          uint32_t* out) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    auto word = [&](uint32_t k) -> uint32_t& { return words[(k >> 5) * kQueryThreads + (k & 31u)]; };
+    const float ylo = __fsub_rn(me.y, g.reach), yhi = __fadd_rn(me.y, g.reach);
+    const uint32_t x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
+    const uint32_t x1 = tile_coord(__fadd_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
+    const uint32_t y0 = tile_coord(ylo, g.inv_cell, g.tiles_y), y1 = tile_coord(yhi, g.inv_cell, g.tiles_y);
+    const uint32_t nx = x1 - x0 + 1u, slots = nx * (y1 - y0 + 1u);
+    uint32_t m = 0;
+    for (uint32_t j0 = 0; j0 < slots; j0 += 32u) {  // a tile's run per lane
+        const uint32_t j = j0 + lane;
+        uint32_t lo = 0, len = 0;
+        if (j < slots) {
+            const uint32_t jy = j / nx, tx = x0 + (j - jy * nx), ty = y0 + jy;
+            const uint32_t t = morton2(tx, ty) << g.ybits;
+            lo = kstart[t | (g.ybits ? y_band(g, ylo, ty) : 0u)];
+            const uint32_t hi = min(kstart[(t | (g.ybits ? y_band(g, yhi, ty) : 0u)) + 1u], n);
+            len = hi > lo ? hi - lo : 0u;
+        }
+        uint32_t runs = __ballot_sync(FULL, len != 0u);
+        while (runs) {
+            const uint32_t o = (uint32_t)__ffs(runs) - 1u;
+            runs &= runs - 1u;
+            const uint32_t from = __shfl_sync(FULL, lo, o), to = from + __shfl_sync(FULL, len, o);
+            for (uint32_t q0 = from; q0 < to; q0 += 32u) {
+                const uint32_t q = q0 + lane;
+                uint32_t id = 0xffffffffu;
+                if (q < to && q != p && in_range_fast(sorted_pos[q], me, g.radius, g.d2_limit)) {
+                    const uint32_t s2 = sorted_slot[q];
+                    if (s2 < n) id = slot_id ? slot_id[s2] : s2;
+                }
+                const uint32_t hits = __ballot_sync(FULL, id != 0xffffffffu);
+                const uint32_t k = m + (uint32_t)__popc(hits & lanemask_lt());
+                if (id != 0xffffffffu && k < count) word(k) = id;
+                m += (uint32_t)__popc(hits);
+            }
+        }
+    }
+    m = min(m, count);
+    __syncwarp();
+    for (uint32_t i = lane; i < m; i += 32u) {
+        const uint32_t id = word(i);
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < m; j++) rank += word(j) < id ? 1u : 0u;
+        if (rank < cap) out[rank] = id;
+    }
+    __syncwarp();  // before the words are used again
+}
+
 // 16 blocks (64 warps) per SM: at 40 registers (12 blocks) the symmetric pair loop
 // gained nothing (0.435 against 0.437 ms at 16 M), at 32 it takes 0.395.
-template <bool LIST>
-__global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __restrict__ kstart,
+template <bool LIST, int KEEP, bool DENSE>
+__global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const uint32_t* __restrict__ kstart,
                                                          const uint32_t* __restrict__ sorted_slot,
                                                          const float2* __restrict__ sorted_pos,
                                                          const uint32_t* __restrict__ slot_id, TileGrid g,
@@ -372,7 +475,7 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
                                                          unsigned long long* __restrict__ pair_bins,
                                                          const uint32_t* err, uint32_t* __restrict__ count_by_id) {
     constexpr uint32_t FULL = 0xffffffffu;
-    __shared__ QueryShared sh;
+    __shared__ QueryShared<KEEP> sh;
     if (index_failed(err)) return;  // uniform per block
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31;
@@ -394,6 +497,7 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
     }
     sh.me[tid] = me;
     sh.cnt[tid] = 0u;
+    uint32_t own = 0u;
     const uint32_t nx = x1 >= x0 ? x1 - x0 + 1u : 0u, ny = y1 >= y0 ? y1 - y0 + 1u : 0u;
     if (__all_sync(FULL, nx <= 2u && ny <= 2u)) {
         // at most 2 x 2 tiles (always when the tile side is at least 2 x reach): the
@@ -422,7 +526,7 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
                 len[k] = hi > lo[k] ? hi - lo[k] : 0u;
             }
         }
-        query_runs<LIST>(lo, len, lane, warp, pwarp, sh, sorted_pos, g);
+        query_runs<LIST, KEEP, DENSE>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own);
     } else {
         // general boxes (tile side below 2 x reach): kRuns tiles per round
         const uint32_t nslots = nx * ny;
@@ -447,11 +551,11 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
                     len[k] = hi > lo[k] ? hi - lo[k] : 0u;
                 }
             }
-            query_runs<LIST>(lo, len, lane, warp, pwarp, sh, sorted_pos, g);
+            query_runs<LIST, KEEP, DENSE>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own);
         }
     }
     __syncwarp();
-    const uint32_t count = valid ? sh.cnt[tid] : 0u;
+    const uint32_t count = valid ? sh.cnt[tid] + own : 0u;
     if (valid) {
         count_out[p] = count;
         // slots that hold their own entity: the count also goes straight to its id's
@@ -469,23 +573,25 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
             if (lane >= (uint32_t)o) incl += y;
         }
         uint32_t* out = list + (size_t)(p >> 5) * 32u * cap + (incl - kept);
-        // the warp's largest kept list bounds the (warp-uniform) id fetch and insertion
-        const uint32_t wmax = __reduce_max_sync(FULL, count <= (uint32_t)kRegKeep ? count : 0u);
-        if (count <= (uint32_t)kRegKeep) {  // every neighbour is kept: ids, sort, write
-            uint32_t id[kRegKeep];
+        // the warp's largest list that was kept bounds the (warp-uniform) loops below
+        const uint32_t listed = count <= (uint32_t)KEEP ? count : 0u;
+        const uint32_t wmax = __reduce_max_sync(FULL, listed);
+        if (!DENSE || wmax <= kSortInRegisters) {
+            uint32_t id[kSortInRegisters];  // ascending; unused slots hold 0xffffffff
 #pragma unroll
-            for (int i = 0; i < kRegKeep; i++) {  // all fetches of a lane in flight together
+            for (int i = 0; i < kSortInRegisters; i++) {  // all fetches of a lane in flight together
                 id[i] = 0xffffffffu;
                 if ((uint32_t)i < wmax) {
-                    const uint32_t s2 = (uint32_t)i < count ? sorted_slot[sh.keep[i][tid]] : n;
+                    const uint32_t k = DENSE && (uint32_t)i >= own ? (uint32_t)i + (uint32_t)KEEP - listed : (uint32_t)i;
+                    const uint32_t s2 = (uint32_t)i < listed ? sorted_slot[sh.keep[k][tid]] : n;
                     id[i] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;  // NULL: slot = id
                 }
             }
-            uint32_t keep[kRegKeep];  // ascending; unused slots hold 0xffffffff
+            uint32_t keep[kSortInRegisters];
 #pragma unroll
-            for (int i = 0; i < kRegKeep; i++) keep[i] = 0xffffffffu;
+            for (int i = 0; i < kSortInRegisters; i++) keep[i] = 0xffffffffu;
 #pragma unroll
-            for (int i = 0; i < kRegKeep; i++) {
+            for (int i = 0; i < kSortInRegisters; i++) {
                 if ((uint32_t)i >= wmax) continue;  // uniform
                 // keep[0..i) is sorted and slot i is free: insert there and sink it, i
                 // compare-exchanges (w (w - 1) / 2 in all for a warp's largest list w)
@@ -498,12 +604,78 @@ __global__ __launch_bounds__(kQueryThreads, 16) void k_query(const uint32_t* __r
                 }
             }
 #pragma unroll
-            for (int i = 0; i < kRegKeep; i++) {
+            for (int i = 0; i < kSortInRegisters; i++) {
                 if ((uint32_t)i >= wmax) break;  // uniform
-                if ((uint32_t)i < kept) out[i] = keep[i];
+                if ((uint32_t)i < min(listed, cap)) out[i] = keep[i];
             }
         } else {
-            list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
+            // longer lists: every id to rows 0 .. of its lane's column (row i of the list lies
+            // at i, or at i + KEEP - listed for the credited ones: never below i), then two
+            // elements of a column per lane, the warp's pairs of elements end to end: each
+            // element to its rank in its column
+#pragma unroll 4
+            for (uint32_t i = 0; i < wmax; i++) {
+                if (i < listed) {
+                    const uint32_t s2 = sorted_slot[sh.keep[i < own ? i : i + (uint32_t)KEEP - listed][tid]];
+                    sh.keep[i][tid] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+                }
+            }
+            __syncwarp();
+            const uint32_t couples = (listed + 1u) / 2u;
+            uint32_t li = couples;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, li, o);
+                if (lane >= (uint32_t)o) li += y;
+            }
+            const uint32_t total = __shfl_sync(FULL, li, 31);
+            const uint32_t place = incl - kept;  // the lane's first place in the warp's output
+            uint32_t* warp_out = out - place;
+            for (uint32_t base = 0; base < total; base += 32u) {
+                const uint32_t i = base + lane;
+                uint32_t o = 0;  // first lane whose inclusive prefix exceeds i
+#pragma unroll
+                for (uint32_t st = 16; st > 0; st >>= 1) {
+                    const uint32_t v = __shfl_sync(FULL, li, o + st - 1u);
+                    if (v <= i) o += st;
+                }
+                o &= 31u;
+                const uint32_t m = __shfl_sync(FULL, listed, o), to = __shfl_sync(FULL, place, o);
+                const uint32_t first = __shfl_sync(FULL, li - couples, o);
+                if (i < total) {
+                    const uint32_t* col = &sh.keep[0][warp * 32u + o];
+                    const uint32_t j = 2u * (i - first);
+                    const uint32_t a = col[j * kQueryThreads];
+                    const uint32_t b = j + 1u < m ? col[(j + 1u) * kQueryThreads] : 0xffffffffu;
+                    uint32_t ra = 0, rb = 0;
+#pragma unroll 4
+                    for (uint32_t k = 0; k < m; k++) {
+                        const uint32_t x = col[k * kQueryThreads];
+                        ra += x < a ? 1u : 0u;
+                        rb += x < b ? 1u : 0u;
+                    }
+                    if (ra < cap) warp_out[to + ra] = a;
+                    if (j + 1u < m && rb < cap) warp_out[to + rb] = b;
+                }
+            }
+        }
+        if constexpr (!DENSE) {  // a few in a million
+            if (count > (uint32_t)KEEP) list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
+        } else {
+            uint32_t longer = __ballot_sync(FULL, count > (uint32_t)KEEP);
+            if (longer) __syncwarp();  // the kept lists are written out: their words are free
+            while (longer) {
+                const uint32_t o = (uint32_t)__ffs(longer) - 1u;
+                longer &= longer - 1u;
+                const uint32_t c = __shfl_sync(FULL, count, o);
+                if (c <= 32u * (uint32_t)KEEP) {
+                    list_by_warp<KEEP>(sorted_slot, sorted_pos, slot_id, kstart, g, n, pwarp + o,
+                                       sh.me[warp * 32u + o], c, cap, &sh.keep[0][warp * 32u],
+                                       list + (size_t)(p >> 5) * 32u * cap + __shfl_sync(FULL, incl - kept, o));
+                } else if (lane == o) {
+                    list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
+                }
+            }
         }
     }
 }
