@@ -148,6 +148,12 @@ struct msim_ctx {
     double maxc = 0.0;
     uint32_t* bounds_dev = nullptr;  // [max |speed|, max |coordinate|] as float bits
     float2* reuse_pos[2] = {nullptr, nullptr};
+    // pair lists of the current index (see msim_query.cuh): kept by the query of one of
+    // its ticks, they serve until pair_until move ticks after the index's keys (< 0: none)
+    uint32_t* pairs_kept = nullptr;
+    uint32_t* pair_sizes = nullptr;
+    uint32_t* pair_ids = nullptr;
+    int64_t pair_until = -1;
     // rank[slot] = sorted position of the slot in the current index, written by the
     // merge once allocated (rank_valid: it describes the current index); a reusing
     // tick's move then writes each position there itself (no gather pass)
@@ -372,7 +378,9 @@ EntityState& cur_state(msim_ctx* c) { return c->st[c->cur]; }
 // 6.4 m: 0.385-0.400 ms); per tick with reuse, measured at 16 M / 1 M: 0.25 of the
 // reach 0.616 / 0.0521 ms, 0.5 0.573 / 0.0473, 1.0 0.555 / 0.0447, 1.5 0.569 /
 // 0.0437, 2.0 0.558 / 0.0437, 3.0 0.568 / 0.0437.  At densities where a query meets
-// 17 or 70 neighbours it costs the same at 0 and 1.0 (1.41 and 22.4 ms at 1 M).
+// 17 or 70 neighbours it costs the same at 0 and 1.0 (1.41 and 22.4 ms at 1 M).  With
+// the pair lists of msim_query.cuh, 1.0 / 1.5 / 2.0 / 3.0: 16 M 0.371 / 0.396 / 0.386 /
+// 0.455 ms, 1 M 0.0346 / 0.0367 / 0.0341 / 0.0376.
 constexpr float kWidenLimit = 1.0f;
 
 // Expected neighbours along the road above which the query's dense kernel is used.
@@ -441,6 +449,48 @@ bool ensure_reuse(msim_ctx* c) {
         }
     }
     return true;
+}
+
+// Buffers of the pair lists: false when an allocation fails (the queries then look
+// their candidates up).
+bool ensure_pairs(msim_ctx* c) {
+    if (c->pairs_kept && c->pair_sizes && c->pair_ids) return true;
+    const size_t bytes[3] = {sizeof(uint32_t) * query_pair_places(c->n, c->dense),
+                             sizeof(uint32_t) * query_pair_sizes(c->n), sizeof(uint32_t) * c->n};
+    void* at[3] = {c->pairs_kept, c->pair_sizes, c->pair_ids};
+    bool all = true;
+    for (int k = 0; k < 3 && all; k++) {
+        if (at[k]) continue;
+        all = device_malloc(&at[k], bytes[k]);
+        if (!all) break;
+        c->allocs.push_back(at[k]);
+        c->device_bytes += bytes[k];
+    }
+    c->pairs_kept = static_cast<uint32_t*>(at[0]);
+    c->pair_sizes = static_cast<uint32_t*>(at[1]);
+    c->pair_ids = static_cast<uint32_t*>(at[2]);
+    return all;
+}
+
+// Ticks that pair lists kept `since` move ticks after the index's keys should serve (0:
+// look the candidates up).  More ticks keep more pairs (each one twice its displacement
+// further apart), fewer pay for the keeping query more often: with use cost growing by
+// 2 s / reach per tick and the keeping query worth kPairCost of it, the best count is
+// about the square root of kPairCost x reach / (2 s), as far as the index is reused.
+// Measured with costs 11 / 22 / 44 (sparse): 16 M 388 / 371 / 372 us per tick, 1 M 36.0 /
+// 36.0 / 35.2; 3 / 6 / 12 (dense): 1 M reference mode 105 / 108 / 124, 200,000 with 14.6
+// neighbours 110 / 118 / 122.
+int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
+    constexpr double kPairCost = 44.0, kPairCostDense = 3.0;
+    constexpr int64_t kFewest = 2;
+    if (!c->reuse || !c->bounds_valid || !(c->grid.reach > 0.f) || !(c->step_bound > 0.0) ||
+        c->n > kPairMaxEntities)
+        return 0;
+    const double per_reach = (double)c->grid.reach / c->step_bound;
+    const int64_t left = (int64_t)std::min(std::floor((double)kWidenLimit * per_reach), 1e9) - since;
+    const int64_t best = (int64_t)std::min(std::sqrt(0.5 * (c->dense ? kPairCostDense : kPairCost) * per_reach), 1e9);
+    const int64_t ticks = std::min(left, std::max(best, kFewest));
+    return ticks >= kFewest ? ticks : 0;
 }
 
 // Widened reach for queries that read an index built `ticks` move ticks ago: reach +
@@ -599,6 +649,7 @@ int permute_state(msim_ctx* c) {
 // runs a full sort, and the one after re-orders the state by it.
 void reset_index(msim_ctx* c) {
     c->reuse_ticks = -1;
+    c->pair_until = -1;
     c->rank_valid = false;
     c->state_free_event = false;
     c->have_nbr = false;
@@ -614,6 +665,7 @@ void reset_index(msim_ctx* c) {
 int build_index(msim_ctx* c) {
     c->have_nbr = false;
     c->reuse_ticks = -1;
+    c->pair_until = -1;
     c->bounds_valid = false;
     c->state_free_event = false;
     if (c->n == 0) return MSIM_OK;
@@ -711,14 +763,15 @@ int incremental_update(msim_ctx* c, bool positions, bool ranks) {
 
 int key_start_table(msim_ctx* c);
 int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id = nullptr, const float2* pos = nullptr,
-              const TileGrid* grid = nullptr);
+              const TileGrid* grid = nullptr, bool pairs = false, double keep_near = 0.0);
 
 // Bound on any entity's displacement in one move tick, per coordinate, for index
 // reuse.  A move advances at most step = |speed| * |road factor| * dt toward its target
 // and snaps to it when closer (the rest of the step is discarded), so it moves at most
-// step; each coordinate's rounding adds at most half an ulp of the largest coordinate,
-// which no later position exceeds (every move heads for a road end, so positions stay
-// within max(largest coordinate now, largest map coordinate)).  Computed from the
+// step, in either coordinate and in distance; each coordinate's rounding adds at most
+// half an ulp of the largest coordinate (four halves are allowed for), which no later
+// position exceeds (every move heads for a road end, so positions stay within
+// max(largest coordinate now, largest map coordinate)).  Computed from the
 // current state (one reduction and a read-back) while the index describes it
 // (reuse_ticks == 0), so the bound covers every tick since the build.
 int ensure_bounds(msim_ctx* c) {
@@ -736,6 +789,24 @@ int ensure_bounds(msim_ctx* c) {
     c->step_bound = std::isfinite(step) ? step : INFINITY;
     c->bounds_valid = true;
     return MSIM_OK;
+}
+
+// The query of a tick `ticks` move ticks after the index's keys (0: the tick that
+// updated it): from the pair lists while they serve, else looked up in the index with
+// boxes widened by how far any entity can have moved since, keeping pair lists for the
+// ticks after it when that pays (boxes and pairs then reach as far as both entities can
+// have moved until the last of them).
+int reusable_query(msim_ctx* c, int64_t ticks, const float2* pos) {
+    TileGrid g = c->grid;
+    if (ticks > 0) g.reach = widened_reach(c, (double)ticks);
+    else c->pair_until = -1;  // a new index
+    if (ticks <= c->pair_until) return run_query(c, true, nullptr, pos, &g, true);
+    const int64_t serve = pair_list_ticks(c, ticks);
+    if (!serve || !ensure_pairs(c)) return run_query(c, true, nullptr, pos, &g);
+    g.reach = widened_reach(c, (double)ticks + 2.0 * (double)serve);
+    const int rc = run_query(c, true, nullptr, pos, &g, true, widened_reach(c, 2.0 * (double)serve));
+    if (rc == MSIM_OK) c->pair_until = ticks + serve;
+    return rc;
 }
 
 int neighbour_tick(msim_ctx* c) {
@@ -770,7 +841,7 @@ int neighbour_tick(msim_ctx* c) {
             rc = key_start_table(c);
             if (rc != MSIM_OK) return rc;
         }
-        rc = run_query(c, true);
+        rc = reusable_query(c, 0, nullptr);
         if (rc == MSIM_OK) c->reuse_ticks = 0;
         return rc;
     }
@@ -796,9 +867,7 @@ int neighbour_tick(msim_ctx* c) {
         CKL(p, launch_gather_chunk(c->stream, c->sorted_slot, c->n, 0, c->n, cur_state(c).pos, c->reuse_pos[x]),
             "k_gather_chunk");
     }
-    TileGrid g = c->grid;
-    g.reach = widened_reach(c, ticks);
-    rc = run_query(c, true, nullptr, c->reuse_pos[x], &g);
+    rc = reusable_query(c, (int64_t)ticks, c->reuse_pos[x]);
     if (rc != MSIM_OK) return rc;
     if (!c->profiling) {  // the query ran on the query stream (see run_query)
         CK(cudaEventRecord(c->ev_reuse_read[x], c->qstream), "cudaEventRecord");
@@ -826,7 +895,9 @@ int key_start_table(msim_ctx* c) {
 // count_by_id (only with slots holding their own entity): the counts also by id.
 // pos / grid (may be NULL): the positions in sorted order and the grid (its reach)
 // instead of the index's own (the skin query of a host tick).
-int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* pos, const TileGrid* grid) {
+// pairs: the query keeps pair lists up to keep_near apart, or with keep_near 0 reads them.
+int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* pos, const TileGrid* grid, bool pairs,
+              double keep_near) {
     NvtxRange range("msim query");
     // The query reads only the index (key-start table, sorted slots and positions)
     // and slot ids: the next tick's move step may overwrite positions meanwhile.  With
@@ -841,10 +912,13 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
     {
         Prof p(c, K_QUERY);
         // slots that hold their own entity need no id lookup
-        CKL(p, launch_query(qs, c->params.cap, c->kstart, c->sorted_slot, pos ? pos : c->sorted_pos,
-                        c->slots_identity ? nullptr : cur_state(c).slot_id, grid ? *grid : c->grid,
+        const bool read_pairs = pairs && !(keep_near > 0.0);
+        CKL(p, launch_query(qs, c->params.cap, c->kstart, read_pairs ? c->pair_ids : c->sorted_slot,
+                        pos ? pos : c->sorted_pos,
+                        c->slots_identity || read_pairs ? nullptr : cur_state(c).slot_id, grid ? *grid : c->grid,
                         c->n, c->nbr_count, c->nbr_list, c->pairs, c->err,
-                        c->slots_identity ? count_by_id : nullptr, c->dense),
+                        c->slots_identity ? count_by_id : nullptr, c->dense, pairs ? c->pairs_kept : nullptr,
+                        c->pair_sizes, c->pair_ids, keep_near),
            "k_query");
     }
     if (qs != c->stream) {
@@ -1164,6 +1238,7 @@ int msim_set_road_factors(msim_ctx* c, const float* factors) {
     c->max_factor = fmax;
     c->bounds_valid = false;
     if (c->reuse_ticks > 0) c->reuse_ticks = -1;
+    c->pair_until = -1;  // kept for the old bound
     return MSIM_OK;
 }
 
@@ -1312,6 +1387,7 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     const bool state_free_event = c->state_free_event;
     bool skin = c->reuse && use_inc && c->reuse_ticks == 0 && c->grid.reach > 0.f && ensure_skin(c);
     c->reuse_ticks = -1;
+    c->pair_until = -1;  // this call builds another index
     c->bounds_valid = false;  // speeds and positions come from the host
     c->state_free_event = false;
     // In place (the same page-locked arrays for heading and RNG in and out): they

@@ -910,26 +910,38 @@ cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n
 cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, const uint32_t* sorted_slot,
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
                          uint32_t* list, unsigned long long* pair_bins, const uint32_t* err, uint32_t* count_by_id,
-                         bool dense) {
+                         bool dense, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near) {
     if (n == 0) return cudaSuccess;
     using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
-                           uint32_t*, uint32_t*, unsigned long long*, const uint32_t*, uint32_t*);
-    static const Query kernels[2][2] = {{k_query<false, kQueryKeep, false>, k_query<false, kQueryKeepDense, true>},
-                                        {k_query<true, kQueryKeep, false>, k_query<true, kQueryKeepDense, true>}};
+                           uint32_t*, uint32_t*, unsigned long long*, const uint32_t*, uint32_t*, PairStore);
+#define QUERY_KERNELS(LIST, KEEP, DENSE)                                                               \
+    {k_query<LIST, KEEP, DENSE, kPairsFound>, k_query<LIST, KEEP, DENSE, kPairsKept>, \
+     k_query<LIST, KEEP, DENSE, kPairsUsed>}
+    static const Query kernels[2][2][3] = {
+        {QUERY_KERNELS(false, kQueryKeep, false), QUERY_KERNELS(false, kQueryKeepDense, true)},
+        {QUERY_KERNELS(true, kQueryKeep, false), QUERY_KERNELS(true, kQueryKeepDense, true)}};
+#undef QUERY_KERNELS
     static bool carveout = false;  // 16 blocks of ~11.5 KB per SM (dense: 9 of ~23.5 KB)
     if (!carveout) {
-        for (int i = 0; i < 4; i++)
-            cudaFuncSetAttribute(kernels[i >> 1][i & 1], cudaFuncAttributePreferredSharedMemoryCarveout,
+        for (int i = 0; i < 12; i++)
+            cudaFuncSetAttribute(kernels[i / 6][i / 3 % 2][i % 3], cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
         cudaGetLastError();
         carveout = true;
     }
+    if (pairs && (!pair_sizes || !pair_ids || n > kPairMaxEntities)) return cudaErrorInvalidValue;
     const bool lists = cap > 0 && list;
-    kernels[lists][dense]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
+    const PairLists use = !pairs ? kPairsFound : keep_near > 0.0 ? kPairsKept : kPairsUsed;
+    // the squared distance's rounding and its operands' stay far below 2^-18 of it
+    const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18))};
+    kernels[lists][dense][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
         kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins, err,
-        count_by_id);
+        count_by_id, store);
     return cudaGetLastError();
 }
+
+size_t query_pair_sizes(uint32_t n) { return (size_t)blocks_for(n, kQueryThreads) * (kQueryThreads / 32); }
+size_t query_pair_places(uint32_t n, bool dense) { return query_pair_sizes(n) * pair_places(dense); }
 
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,
                                uint32_t* first_bad) {

@@ -119,7 +119,15 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // count_by_id (may be NULL; only when slot = entity id): every count also
                          // written at its entity's id
                          uint32_t* count_by_id = nullptr,
-                         bool dense = false);  // dense: the kernel for many neighbours (the same results)
+                         bool dense = false,  // dense: the kernel for many neighbours (the same results)
+                         // pair lists of a reused index (see msim_query.cuh): written with keep_near > 0
+                         // (pairs up to that distance), else read back (the ids then serve as
+                         // sorted_slot, slot_id NULL); NULL: not used
+                         uint32_t* pairs = nullptr, uint32_t* pair_sizes = nullptr, uint32_t* pair_ids = nullptr,
+                         double keep_near = 0.0);
+constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
+size_t query_pair_places(uint32_t n, bool dense);   // pairs of all lists
+size_t query_pair_sizes(uint32_t n);
 // Incremental index update: split the previous sorted order P (keys PK; P[q] = q when
 // identity) by whether the new key NK[slot] changed (A: unchanged, B: changed; counts
 // -> counts[0..1]; B's digit counts -> hist), then, after B is sorted, merge A and B

@@ -278,10 +278,41 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 constexpr uint32_t kRuns = 4;                  // runs per lane and round
 constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 
+// Pair lists, for the ticks that reuse an index.  The index does not change between
+// those ticks and entities move little, so a query can keep, per warp, the pairs it
+// tested that lie within radius + 2 x (the displacement of the next few ticks): every pair
+// in range in one of those ticks is among them, and their queries test the kept pairs
+// alone - no tiles, bands or key starts per entity, no search for the run of a pair, and
+// a quarter of the pairs.  One word per pair: owner lane | the candidate's sorted
+// position (pair_places words per warp; kNoPairs: more than that, look them up); and
+// the entity id of every sorted position, read beside the candidate's position so that
+// a hit keeps the id itself.
+// Bound by the latency of its three dependent loads (58 % issue active); 378 warp
+// instructions against 770.  1 M entities at 2 m 30.6 us looked up, 19.3 from pairs, 38
+// for the query that keeps them; the 16 M tick 532 -> 371 us, the 1 M tick 44.3 -> 34.6,
+// reference mode at 1 M 122 -> 105.  Keeping runs instead of pairs gave 31.1 us at 1 M,
+// ids beside the pairs 42 us for the keeping query.
+constexpr uint32_t kPairOwnerShift = 27;
+constexpr uint32_t kPairPosition = (1u << kPairOwnerShift) - 1u;
+constexpr uint32_t kNoPairs = 0xffffffffu;
+enum PairLists : int { kPairsFound, kPairsKept, kPairsUsed };  // looked up; looked up and kept; read back
+
+// Places per warp: about twice what the workloads keep (sparse 1 M and 16 M populations
+// 45 of 128; a crowd with 15 neighbours 500 of 1,024).
+__host__ __device__ constexpr uint32_t pair_places(bool dense) { return dense ? 1024u : 128u; }
+
+struct PairStore {
+    uint32_t* pairs;
+    uint32_t* sizes;
+    uint32_t* ids;
+    float near2;  // pairs up to this squared distance are kept
+};
+
 template <int KEEP>
 struct QueryShared {
     float2 me[kQueryThreads];
     uint32_t cnt[kQueryThreads];
+    uint32_t id[kQueryThreads];                // kept pairs: the entities' ids
     // sorted positions of the first hits; DENSE: the owner's own from the front, those
     // credited by lower lanes from the back
     uint32_t keep[KEEP][kQueryThreads];
@@ -297,11 +328,28 @@ __device__ __forceinline__ uint32_t bit_range(int from, int to) {
     return to > from ? (0xffffffffu >> (32 - (to - from))) << from : 0u;
 }
 
-// own: DENSE: the lane's hits as owner so far.
+// A hit of owner and candidate q by atomics on their counters; kept for the owner is
+// `theirs`, for a credited lane `mine` (sorted positions or ids).
 template <bool LIST, int KEEP, bool DENSE>
+__device__ __forceinline__ void count_hit(QueryShared<KEEP>& sh, uint32_t warp, uint32_t owner, uint32_t q,
+                                          uint32_t pwarp, uint32_t theirs, uint32_t mine) {
+    const uint32_t ot = warp * 32u + owner, other = q - pwarp;
+    const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
+    if (LIST && c < (uint32_t)KEEP) sh.keep[DENSE ? KEEP - 1 - c : c][ot] = theirs;
+    if (other < 32u) {  // a higher lane of this warp: the pair counts for it too
+        const uint32_t om = warp * 32u + other;
+        const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
+        if (LIST && c2 < (uint32_t)KEEP) sh.keep[DENSE ? KEEP - 1 - c2 : c2][om] = mine;
+    }
+}
+
+// own: DENSE: the lane's hits as owner so far.  KEPT: near pairs are appended to the
+// warp's places (near_count so far).
+template <bool LIST, int KEEP, bool DENSE, bool KEPT>
 __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const uint32_t (&len_in)[kRuns],
                                            uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP>& sh,
-                                           const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own) {
+                                           const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own,
+                                           PairStore store, uint32_t& near_count, uint32_t places) {
     constexpr uint32_t FULL = 0xffffffffu;
     // A pair of entities of this warp is tested once, by the lower lane, which credits
     // both (the predicate is symmetric, and an in-range pair lies in both entities'
@@ -360,30 +408,39 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
         const uint32_t run = ra + (uint32_t)__popc(le) - 1u;  // le == 0: the run begun before the window
         ra += (uint32_t)__popc(marks);
         const uint32_t i = base + lane;
-        if constexpr (!DENSE) {
+        if constexpr (!DENSE && !KEPT) {
             if (i >= total) continue;
             const uint32_t q = sh.rq[warp][run] + i;
             const uint32_t owner = sh.rown[warp][run];
-            const uint32_t other = q - pwarp;  // the candidate's lane when it is in this warp
-            if (other <= owner) continue;      // the owner itself or a lower lane: tested from there
-            const uint32_t ot = warp * 32u + owner;
-            if (!in_range_fast(sorted_pos[q], sh.me[ot], g.radius, g.d2_limit)) continue;
-            const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
-            if (LIST && c < (uint32_t)KEEP) sh.keep[c][ot] = q;  // sorted position; the id comes later
-            if (other < 32u) {  // a higher lane of this warp: the pair counts for it too
-                const uint32_t om = warp * 32u + other;
-                const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
-                if (LIST && c2 < (uint32_t)KEEP) sh.keep[c2][om] = pwarp + owner;
-            }
+            if (q - pwarp <= owner) continue;  // the owner itself or a lower lane: tested from there
+            if (!in_range_fast(sorted_pos[q], sh.me[warp * 32u + owner], g.radius, g.d2_limit)) continue;
+            count_hit<LIST, KEEP, DENSE>(sh, warp, owner, q, pwarp, q, pwarp + owner);
         } else {
             uint32_t q = 0u, owner = lane, other = 0u;
-            bool hit = false;
+            bool hit = false, near = false;
             if (i < total) {
                 q = sh.rq[warp][run] + i;
                 owner = sh.rown[warp][run];
                 other = q - pwarp;
-                hit = other > owner &&
-                      in_range_fast(sorted_pos[q], sh.me[warp * 32u + owner], g.radius, g.d2_limit);
+                if (other > owner) {
+                    const float2 o = sorted_pos[q], me = sh.me[warp * 32u + owner];
+                    hit = in_range_fast(o, me, g.radius, g.d2_limit);
+                    if (KEPT) {
+                        const float ex = __fsub_rn(o.x, me.x), ey = __fsub_rn(o.y, me.y);
+                        near = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)) <= store.near2;
+                    }
+                }
+            }
+            if constexpr (KEPT) {
+                const uint32_t m = __ballot_sync(FULL, near);
+                const uint32_t at = near_count + (uint32_t)__popc(m & lanemask_lt());
+                if (near && at < places)
+                    store.pairs[(size_t)(pwarp >> 5) * places + at] = q | (owner << kPairOwnerShift);
+                near_count += (uint32_t)__popc(m);
+            }
+            if constexpr (!DENSE) {
+                if (hit) count_hit<LIST, KEEP, DENSE>(sh, warp, owner, q, pwarp, q, pwarp + owner);
+                continue;
             }
             const uint32_t hits = __ballot_sync(FULL, hit);
             const uint32_t mine = bit_range((int)(fi - flat - base), (int)(fi - base));  // this lane's pairs
@@ -465,7 +522,7 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
 
 // 16 blocks (64 warps) per SM: at 40 registers (12 blocks) the symmetric pair loop
 // gained nothing (0.435 against 0.437 ms at 16 M), at 32 it takes 0.395.
-template <bool LIST, int KEEP, bool DENSE>
+template <bool LIST, int KEEP, bool DENSE, PairLists PAIRS>
 __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const uint32_t* __restrict__ kstart,
                                                          const uint32_t* __restrict__ sorted_slot,
                                                          const float2* __restrict__ sorted_pos,
@@ -473,7 +530,8 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                                                          uint32_t n, uint32_t cap, uint32_t* __restrict__ count_out,
                                                          uint32_t* __restrict__ list,
                                                          unsigned long long* __restrict__ pair_bins,
-                                                         const uint32_t* err, uint32_t* __restrict__ count_by_id) {
+                                                         const uint32_t* err, uint32_t* __restrict__ count_by_id,
+                                                         PairStore store) {
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ QueryShared<KEEP> sh;
     if (index_failed(err)) return;  // uniform per block
@@ -484,10 +542,52 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     const uint32_t pwarp = p - lane;
     const bool valid = p < n;
     float2 me = make_float2(0.f, 0.f);
+    constexpr uint32_t places = pair_places(DENSE);
+    const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * places : nullptr;
+    uint32_t size = kNoPairs;
+    uint32_t pair[2];
+    if (PAIRS == kPairsUsed) {  // the first pairs, their number, position and id in flight together
+        size = store.sizes[p >> 5];
+        pair[0] = pairs[lane];
+        pair[1] = pairs[lane + 32u];
+        if (valid) sh.id[tid] = store.ids[p];
+    }
+    if (valid) me = sorted_pos[p];
+    sh.me[tid] = me;
+    sh.cnt[tid] = 0u;
+    uint32_t own = 0u, near_count = 0u;
+    if (PAIRS == kPairsKept && valid) {
+        const uint32_t s2 = sorted_slot[p];
+        store.ids[p] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+    }
+    const bool have_ids = PAIRS == kPairsUsed && size != kNoPairs;  // uniform per warp
+    if (have_ids) {
+        __syncwarp();
+        for (uint32_t base = 0; base < size; base += 64u) {  // two pairs per lane in flight
+            float2 o[2];
+            uint32_t id[2];
+#pragma unroll
+            for (uint32_t k = 0; k < 2u; k++) {
+                if (base + 32u * k + lane >= size) continue;
+                const uint32_t q = pair[k] & kPairPosition;
+                o[k] = sorted_pos[q];
+                if (LIST) id[k] = store.ids[q];
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 2u; k++) {
+                const uint32_t i = base + 32u * k + lane;
+                if (i >= size) continue;
+                const uint32_t owner = pair[k] >> kPairOwnerShift;
+                if (in_range_fast(o[k], sh.me[warp * 32u + owner], g.radius, g.d2_limit))
+                    count_hit<LIST, KEEP, DENSE>(sh, warp, owner, pair[k] & kPairPosition, pwarp, id[k],
+                                                 sh.id[warp * 32u + owner]);
+                if (i + 64u < size) pair[k] = pairs[i + 64u];
+            }
+        }
+    } else {
     uint32_t x0 = 1, x1 = 0, y0 = 1, y1 = 0;  // empty box for invalid lanes
     float ylo = 0.f, yhi = 0.f;
     if (valid) {
-        me = sorted_pos[p];
         ylo = __fsub_rn(me.y, g.reach);
         yhi = __fadd_rn(me.y, g.reach);
         x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
@@ -495,9 +595,6 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
         y0 = tile_coord(ylo, g.inv_cell, g.tiles_y);
         y1 = tile_coord(yhi, g.inv_cell, g.tiles_y);
     }
-    sh.me[tid] = me;
-    sh.cnt[tid] = 0u;
-    uint32_t own = 0u;
     const uint32_t nx = x1 >= x0 ? x1 - x0 + 1u : 0u, ny = y1 >= y0 ? y1 - y0 + 1u : 0u;
     if (__all_sync(FULL, nx <= 2u && ny <= 2u)) {
         // at most 2 x 2 tiles (always when the tile side is at least 2 x reach): the
@@ -526,7 +623,8 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                 len[k] = hi > lo[k] ? hi - lo[k] : 0u;
             }
         }
-        query_runs<LIST, KEEP, DENSE>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own);
+        query_runs<LIST, KEEP, DENSE, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
+                                                           store, near_count, places);
     } else {
         // general boxes (tile side below 2 x reach): kRuns tiles per round
         const uint32_t nslots = nx * ny;
@@ -551,8 +649,11 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                     len[k] = hi > lo[k] ? hi - lo[k] : 0u;
                 }
             }
-            query_runs<LIST, KEEP, DENSE>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own);
+            query_runs<LIST, KEEP, DENSE, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
+                                                           store, near_count, places);
         }
+    }
+    if (PAIRS == kPairsKept && lane == 0) store.sizes[p >> 5] = near_count <= places ? near_count : kNoPairs;
     }
     __syncwarp();
     const uint32_t count = valid ? sh.cnt[tid] + own : 0u;
@@ -583,7 +684,12 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                 id[i] = 0xffffffffu;
                 if ((uint32_t)i < wmax) {
                     const uint32_t k = DENSE && (uint32_t)i >= own ? (uint32_t)i + (uint32_t)KEEP - listed : (uint32_t)i;
-                    const uint32_t s2 = (uint32_t)i < listed ? sorted_slot[sh.keep[k][tid]] : n;
+                    const uint32_t x = (uint32_t)i < listed ? sh.keep[k][tid] : 0xffffffffu;
+                    if (have_ids) {
+                        id[i] = x;
+                        continue;
+                    }
+                    const uint32_t s2 = (uint32_t)i < listed ? sorted_slot[x] : n;
                     id[i] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;  // NULL: slot = id
                 }
             }
@@ -616,8 +722,9 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
 #pragma unroll 4
             for (uint32_t i = 0; i < wmax; i++) {
                 if (i < listed) {
-                    const uint32_t s2 = sorted_slot[sh.keep[i < own ? i : i + (uint32_t)KEEP - listed][tid]];
-                    sh.keep[i][tid] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+                    const uint32_t x = sh.keep[i < own ? i : i + (uint32_t)KEEP - listed][tid];
+                    const uint32_t s2 = have_ids ? n : sorted_slot[x];
+                    sh.keep[i][tid] = have_ids ? x : s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
                 }
             }
             __syncwarp();
