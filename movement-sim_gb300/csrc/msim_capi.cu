@@ -1291,17 +1291,18 @@ int msim_get_state(msim_ctx* c, float* pos, uint32_t* heading, uint32_t* rng, fl
     if (rc != MSIM_OK) return rc;
     const size_t n = c->n;
     if (n == 0) return sync_and_check(c);
-    if ((rc = ensure_stage(c, n * (sizeof(float2) + sizeof(uint32_t) + sizeof(uint4) + sizeof(float)))) != MSIM_OK)
-        return rc;
-    char* b = static_cast<char*>(c->stage);
+    const size_t fields = sizeof(float2) + sizeof(uint32_t) + sizeof(uint4) + sizeof(float);
+    if ((rc = ensure_stage(c, n * (kStateRecordBytes + fields))) != MSIM_OK) return rc;
+    char* b = static_cast<char*>(c->stage) + n * kStateRecordBytes;  // the records, then the fields
     uint4* d_rng = reinterpret_cast<uint4*>(b);
     float2* d_pos = reinterpret_cast<float2*>(b + n * sizeof(uint4));
     uint32_t* d_head = reinterpret_cast<uint32_t*>(b + n * (sizeof(uint4) + sizeof(float2)));
     float* d_speed = reinterpret_cast<float*>(b + n * (sizeof(uint4) + sizeof(float2) + sizeof(uint32_t)));
     {
         Prof p(c, K_EXPORT);
+        c->launch_count++;  // two kernels
         CK(launch_export_state(c->stream, cur_state(c), c->n, pos ? d_pos : nullptr, heading ? d_head : nullptr,
-                               rng ? d_rng : nullptr, speed ? d_speed : nullptr),
+                               rng ? d_rng : nullptr, speed ? d_speed : nullptr, c->stage),
            "k_export_state");
     }
     if (pos) CK(cudaMemcpyAsync(pos, d_pos, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream), "download pos");
@@ -1321,8 +1322,8 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     if (n == 0) return MSIM_OK;
     const bool want_idx = idx && cap;
     if ((rc = ensure_stage(c, n * sizeof(uint32_t) * (1 + (want_idx ? cap : 0)))) != MSIM_OK) return rc;
-    uint32_t* d_count = static_cast<uint32_t*>(c->stage);
-    uint32_t* d_idx = want_idx ? d_count + n : nullptr;
+    uint32_t* d_idx = want_idx ? static_cast<uint32_t*>(c->stage) : nullptr;
+    uint32_t* d_count = static_cast<uint32_t*>(c->stage) + (want_idx ? n * cap : 0);
     {
         Prof p(c, K_EXPORT);
         CK(launch_export_neighbours(c->stream, c->query_slot, cur_state(c).slot_id, c->nbr_count, c->nbr_list,
@@ -1519,9 +1520,9 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     uint32_t* d_count = nullptr;
     if (nbr && (out_count || out_idx)) {
         if ((rc = ensure_stage(c, (size_t)n * sizeof(uint32_t) * (1 + (want_idx ? cap : 0)))) != MSIM_OK) return rc;
-        d_count = static_cast<uint32_t*>(c->stage);
+        d_count = static_cast<uint32_t*>(c->stage) + (want_idx ? (size_t)n * cap : 0);
     }
-    uint32_t* d_idx = want_idx ? d_count + n : nullptr;
+    uint32_t* d_idx = want_idx ? static_cast<uint32_t*>(c->stage) : nullptr;
     // the neighbour downloads go on `dl`: the context's stream, or (skin query) the
     // download stream, so the index update can follow the query on the context's stream
     cudaStream_t dl = c->stream;

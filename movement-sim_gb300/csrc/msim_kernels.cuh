@@ -168,8 +168,11 @@ cudaError_t launch_fill(cudaStream_t s, float* out, uint32_t n, float v);
 // With kErrTimeout in *err (may be NULL) the state is copied in its current order.
 cudaError_t launch_permute(cudaStream_t s, const uint32_t* sorted_slot, EntityState src,
                            EntityState dst, uint32_t n, const uint32_t* err = nullptr);
+// records: n x kStateRecordBytes of scratch, 32-byte aligned
+constexpr size_t kStateRecordBytes = 32;
 cudaError_t launch_export_state(cudaStream_t s, EntityState st, uint32_t n, float2* pos,
-                                uint32_t* head, uint4* rng, float* speed);
+                                uint32_t* head, uint4* rng, float* speed, void* records);
+// out_idx: 16-byte aligned
 cudaError_t launch_export_neighbours(cudaStream_t s, const uint32_t* sorted_slot, const uint32_t* slot_id,
                                      const uint32_t* count, const uint32_t* list, uint32_t n,
                                      uint32_t cap, uint32_t* out_count, uint32_t* out_idx);
