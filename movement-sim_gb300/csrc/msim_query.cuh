@@ -534,7 +534,9 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                                                          PairStore store) {
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ QueryShared<KEEP> sh;
-    if (index_failed(err)) return;  // uniform per block
+    // read first, tested once the other first loads are in flight (they stay in range
+    // whatever an index update left behind)
+    const uint32_t status = err ? ld_relaxed(err) : 0u;
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31;
     const uint32_t warp = tid >> 5;
@@ -545,14 +547,15 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     constexpr uint32_t places = pair_places(DENSE);
     const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * places : nullptr;
     uint32_t size = kNoPairs;
-    uint32_t pair[2];
+    uint32_t pair[2], my_id = 0u;
     if (PAIRS == kPairsUsed) {  // the first pairs, their number, position and id in flight together
         size = store.sizes[p >> 5];
         pair[0] = pairs[lane];
         pair[1] = pairs[lane + 32u];
-        if (valid) sh.id[tid] = store.ids[p];
+        my_id = valid ? store.ids[p] : 0u;
     }
     if (valid) me = sorted_pos[p];
+    if (status & kErrTimeout) return;  // an index update gave up (index_failed)
     sh.me[tid] = me;
     sh.cnt[tid] = 0u;
     uint32_t own = 0u, near_count = 0u;
@@ -562,6 +565,7 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     }
     const bool have_ids = PAIRS == kPairsUsed && size != kNoPairs;  // uniform per warp
     if (have_ids) {
+        sh.id[tid] = my_id;
         __syncwarp();
         for (uint32_t base = 0; base < size; base += 64u) {  // two pairs per lane in flight
             float2 o[2];
