@@ -284,7 +284,7 @@ int msim_quad_tree_build(const float* pos, uint32_t n, float width, float height
  * ok).  Work is queued on `stream` (a cudaStream_t, NULL = default stream) and not
  * waited for.  n <= MSIM_NOALLOC_MAX_ENTITIES, else MSIM_ERR_INVALID; tiles are
  * capped at 512 x 512 over world_w x world_h.  All intermediates live in one
- * ~7.5 MB static device array per device, held until the process exits; every
+ * ~6 MB static device array per device, held until the process exits; every
  * call shares it, so calls whose GPU work overlaps race (serialise them).  The
  * first call on a device looks the array up (cudaGetSymbolAddress) and sets a
  * kernel attribute: make that first call before any stream capture. */

@@ -503,36 +503,6 @@ __global__ __launch_bounds__(kSortThreads, 4) void k_onesweep(const uint32_t* __
   }
 }
 
-// [start, end) of every occupied tile; the tile of a key is key >> ybits.
-__global__ void k_ranges(const uint32_t* __restrict__ sk, uint32_t n, uint32_t* __restrict__ ranges,
-                         uint32_t num_keys, uint32_t ybits) {
-    // four consecutive sorted keys per thread (one 16-byte load when in range)
-    const uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
-    if (p0 >= n) return;
-    uint32_t k[6];  // k[0] = key before p0, k[1..4] = keys p0..p0+3, k[5] = key after
-    k[0] = p0 ? sk[p0 - 1] : 0xffffffffu;
-    if (p0 + 4 <= n) {
-        const uint4 v = *reinterpret_cast<const uint4*>(sk + p0);
-        k[1] = v.x;
-        k[2] = v.y;
-        k[3] = v.z;
-        k[4] = v.w;
-        k[5] = p0 + 4 < n ? sk[p0 + 4] : 0xffffffffu;
-    } else {
-#pragma unroll
-        for (int i = 1; i < 6; i++) k[i] = p0 + i - 1 < n ? sk[p0 + i - 1] : 0xffffffffu;
-    }
-#pragma unroll
-    for (int i = 0; i < 6; i++) k[i] >>= ybits;  // tile codes (the sentinels stay above every tile)
-#pragma unroll
-    for (int i = 1; i <= 4; i++) {
-        const uint32_t p = p0 + i - 1;
-        if (p >= n || k[i] >= num_keys) continue;  // tiles are Morton codes of clamped tile coordinates
-        if (k[i - 1] != k[i]) ranges[2ull * k[i]] = p;
-        if (k[i + 1] != k[i]) ranges[2ull * k[i] + 1] = p + 1;
-    }
-}
-
 // Lists of up to this many ids are sorted in registers.
 constexpr int kSortInRegisters = 8;
 
@@ -907,14 +877,6 @@ size_t sort_lookback_words(uint32_t n) {
     const size_t tiles = std::max<size_t>((n + kSortTile - 1) / kSortTile,
                                           (n + kSortThreads * kSortRowsDev - 1) / (kSortThreads * kSortRowsDev));
     return std::max<size_t>(tiles, 1) * kRadix;
-}
-
-cudaError_t launch_ranges(cudaStream_t s, const uint32_t* sorted_key, uint32_t n, uint2* ranges, uint32_t num_keys,
-                          uint32_t ybits) {
-    if (n == 0) return cudaSuccess;
-    k_ranges<<<blocks_for((n + 3) / 4, 256), 256, 0, s>>>(sorted_key, n, reinterpret_cast<uint32_t*>(ranges), num_keys,
-                                                          ybits);
-    return cudaGetLastError();
 }
 
 uint32_t kstart_chunks(uint64_t num_keys) { return kstart_chunk_cap(num_keys); }

@@ -100,8 +100,6 @@ cudaError_t launch_onesweep(cudaStream_t s, const uint32_t* keys_in, const uint3
                             uint32_t* err, const uint32_t* n_dev = nullptr,  // n_dev: count on the device (<= n)
                             const SweepChain* chain = nullptr, uint32_t spin_limit = kDefaultSpinLimit,
                             bool many = false);  // many: with n_dev, 4096-item tiles all the same
-cudaError_t launch_ranges(cudaStream_t s, const uint32_t* sorted_key, uint32_t n, uint2* ranges, uint32_t num_keys,
-                          uint32_t ybits = 0);
 // Key-start table of sorted keys (num_keys + 1 entries).  chunks / chunk_count
 // (kstart_chunks(num_keys) uint4 entries and one counter; may be NULL) enable the
 // per-position kernel, which also gathers pos into sorted order (sorted_pos, n entries)
