@@ -180,6 +180,7 @@ struct msim_batch {
     size_t items_capacity = 0;
     uint32_t* ticket = nullptr;
     uint32_t* err = nullptr;
+    uint32_t* status_host = nullptr;  // page-locked copy of *err
     float2* pos = nullptr;
     uint32_t* head = nullptr;
     uint4* rng = nullptr;
@@ -217,6 +218,7 @@ void free_batch(msim_batch* b) {
     drop_graphs(b);
     for (void* p : b->allocs) cudaFree(p);
     b->allocs.clear();
+    status_word_give(b->status_host);
     if (b->t0) cudaEventDestroy(b->t0);
     if (b->t1) cudaEventDestroy(b->t1);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -375,10 +377,10 @@ int run_ticks(msim_batch* b, uint32_t ticks, bool use_graph) {
 }
 
 int sync_batch(msim_batch* b) {
+    BCK(cudaMemcpyAsync(b->status_host, b->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream),
+        "read device status");
     BCK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
-    uint32_t h = 0;
-    BCK(cudaMemcpy(&h, b->err, sizeof(h), cudaMemcpyDeviceToHost), "read device status");
-    if (h) {
+    if (*static_cast<volatile uint32_t*>(b->status_host)) {
         BCK(cudaMemset(b->err, 0, sizeof(uint32_t)), "clear device status");
         return fail(MSIM_ERR_OOB, "a device-side index check failed in the batch");
     }
@@ -435,6 +437,8 @@ int msim_batch_create(const msim_map* maps, const uint32_t* num_entities, uint32
     b->n.assign(num_entities, num_entities + count);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
+    if (!(b->status_host = status_word_take()))
+        return bail(fail(MSIM_ERR_NOMEM, "page-locked allocation of the status word failed"));
     if (cudaEventCreate(&b->t0) != cudaSuccess || cudaEventCreate(&b->t1) != cudaSuccess)
         return bail(fail(MSIM_ERR_CUDA, "cudaEventCreate failed"));
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
@@ -528,14 +532,13 @@ int msim_batch_get_state(msim_batch* b, uint32_t instance, float* pos, uint32_t*
     if (!b) return fail(MSIM_ERR_INVALID, "batch is NULL");
     if (instance >= b->count) return fail(MSIM_ERR_INVALID, "instance out of range");
     cudaSetDevice(b->device);
-    int rc = sync_batch(b);
-    if (rc != MSIM_OK) return rc;
     const size_t e0 = b->ebase[instance], n = b->n[instance];
-    if (pos) BCK(cudaMemcpy(pos, b->pos + e0, sizeof(float2) * n, cudaMemcpyDeviceToHost), "download pos");
-    if (heading) BCK(cudaMemcpy(heading, b->head + e0, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost), "download heading");
-    if (rng) BCK(cudaMemcpy(rng, b->rng + e0, sizeof(uint4) * n, cudaMemcpyDeviceToHost), "download rng");
-    if (speed) BCK(cudaMemcpy(speed, b->speed + e0, sizeof(float) * n, cudaMemcpyDeviceToHost), "download speed");
-    return MSIM_OK;
+    cudaStream_t s = b->stream;  // one wait behind the copies and the status
+    if (pos) BCK(cudaMemcpyAsync(pos, b->pos + e0, sizeof(float2) * n, cudaMemcpyDeviceToHost, s), "download pos");
+    if (heading) BCK(cudaMemcpyAsync(heading, b->head + e0, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s), "download heading");
+    if (rng) BCK(cudaMemcpyAsync(rng, b->rng + e0, sizeof(uint4) * n, cudaMemcpyDeviceToHost, s), "download rng");
+    if (speed) BCK(cudaMemcpyAsync(speed, b->speed + e0, sizeof(float) * n, cudaMemcpyDeviceToHost, s), "download speed");
+    return sync_batch(b);
 }
 
 int msim_batch_set_schedule(msim_batch* b, const msim_batch_schedule* s) {

@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -42,6 +43,49 @@ bool device_malloc(void** p, size_t bytes) {
         return false;
     }
     return true;
+}
+
+namespace {
+constexpr uint32_t kStatusWords = 1024;
+std::mutex g_status_mutex;
+uint32_t* g_status_slab = nullptr;
+std::vector<uint32_t> g_status_free;  // indexes of the slab's free words
+}  // namespace
+
+uint32_t* status_word_take() {
+    std::lock_guard<std::mutex> lk(g_status_mutex);
+    if (!g_status_slab) {
+        void* raw = nullptr;
+        if (cudaHostAlloc(&raw, sizeof(uint32_t) * kStatusWords, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        g_status_slab = static_cast<uint32_t*>(raw);
+        for (uint32_t i = kStatusWords; i-- > 0;) g_status_free.push_back(i);
+    }
+    uint32_t* word = nullptr;
+    if (!g_status_free.empty()) {
+        word = g_status_slab + g_status_free.back();
+        g_status_free.pop_back();
+    } else {
+        void* raw = nullptr;
+        if (cudaHostAlloc(&raw, sizeof(uint32_t), cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        word = static_cast<uint32_t*>(raw);
+    }
+    *word = 0u;
+    return word;
+}
+
+void status_word_give(uint32_t* word) {
+    if (!word) return;
+    std::lock_guard<std::mutex> lk(g_status_mutex);
+    if (g_status_slab && word >= g_status_slab && word < g_status_slab + kStatusWords)
+        g_status_free.push_back((uint32_t)(word - g_status_slab));
+    else
+        cudaFreeHost(word);
 }
 
 enum KernelId : uint32_t {
@@ -184,6 +228,7 @@ struct msim_ctx {
     unsigned long long* pairs = nullptr;
     bool have_nbr = false;
     uint32_t* err = nullptr;
+    uint32_t* status_host = nullptr;  // page-locked copy of *err, written behind the work it describes
     uint32_t* check = nullptr;  // first invalid heading found by msim_set_entities
     TileGrid grid{};
     bool dense = false;  // many neighbours expected (see msim_create): the query's dense kernel
@@ -293,6 +338,8 @@ void free_all(msim_ctx* c) {
     }
     for (cudaEvent_t e : {c->ev_disp, c->ev_query, c->ev_state_free, c->ev_reuse_read[0], c->ev_reuse_read[1]})
         if (e) cudaEventDestroy(e);
+    status_word_give(c->status_host);
+    c->status_host = nullptr;
     if (c->disp_host) cudaFreeHost(c->disp_host);
     c->disp_host = nullptr;
     if (c->up) cudaStreamDestroy(c->up);
@@ -528,6 +575,19 @@ void* mapped_host(const void* p) {
         return nullptr;
     }
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
+// Where an export kernel writes an output: the caller's array itself when it is
+// page-locked, aligned for the kernel's stores and small (below kDirectEntities
+// entities the copies' own latency is most of a read-back), else its staging place;
+// nullptr when the output is not wanted.
+constexpr uint32_t kDirectEntities = 65536;
+template <typename T>
+T* direct_out(const msim_ctx* c, void* out, T* staged) {
+    if (!out) return nullptr;
+    if (c->n > kDirectEntities) return staged;
+    void* mapped = mapped_host(out);
+    return mapped && (reinterpret_cast<uintptr_t>(mapped) & (sizeof(T) - 1)) == 0 ? static_cast<T*>(mapped) : staged;
 }
 
 // The main stream waits for the queries still running on qstream that read index
@@ -942,10 +1002,15 @@ int check_ctx(msim_ctx* c) {
     return MSIM_OK;
 }
 
-int sync_and_check(msim_ctx* c) {
+// Waits for the stream and reports the status word.  status_queued: a kernel already
+// queued writes it to status_host; else a copy behind the queued work does, so that one
+// wait covers both (a blocking copy after the wait cost 8 us a call).
+int sync_and_check(msim_ctx* c, bool status_queued = false) {
+    if (!status_queued)
+        CK(cudaMemcpyAsync(c->status_host, c->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
+           "read device status");
     CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-    uint32_t h = 0;
-    CK(cudaMemcpy(&h, c->err, sizeof(h), cudaMemcpyDeviceToHost), "read device status");
+    const uint32_t h = *static_cast<volatile uint32_t*>(c->status_host);
     if (h) {
         CK(cudaMemsetAsync(c->err, 0, sizeof(uint32_t), c->stream), "clear device status");
         if (h & kErrTimeout) {
@@ -1017,6 +1082,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->qstream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
+    if (!(c->status_host = status_word_take()))
+        return bail(fail(MSIM_ERR_NOMEM, "page-locked allocation of the status word failed"));
     if (cudaEventCreate(&c->t0) != cudaSuccess || cudaEventCreate(&c->t1) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_index, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_read[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -1298,19 +1365,27 @@ int msim_get_state(msim_ctx* c, float* pos, uint32_t* heading, uint32_t* rng, fl
     float2* d_pos = reinterpret_cast<float2*>(b + n * sizeof(uint4));
     uint32_t* d_head = reinterpret_cast<uint32_t*>(b + n * (sizeof(uint4) + sizeof(float2)));
     float* d_speed = reinterpret_cast<float*>(b + n * (sizeof(uint4) + sizeof(float2) + sizeof(uint32_t)));
+    // page-locked outputs are written by the kernel itself, others staged and copied
+    float2* to_pos = direct_out<float2>(c, pos, d_pos);
+    uint32_t* to_head = direct_out<uint32_t>(c, heading, d_head);
+    uint4* to_rng = direct_out<uint4>(c, rng, d_rng);
+    float* to_speed = direct_out<float>(c, speed, d_speed);
     {
         Prof p(c, K_EXPORT);
         c->launch_count++;  // two kernels
-        CK(launch_export_state(c->stream, cur_state(c), c->n, pos ? d_pos : nullptr, heading ? d_head : nullptr,
-                               rng ? d_rng : nullptr, speed ? d_speed : nullptr, c->stage),
+        CK(launch_export_state(c->stream, cur_state(c), c->n, to_pos, to_head, to_rng, to_speed, c->stage, c->err,
+                               c->status_host),
            "k_export_state");
     }
-    if (pos) CK(cudaMemcpyAsync(pos, d_pos, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream), "download pos");
-    if (heading)
+    if (to_pos == d_pos && pos)
+        CK(cudaMemcpyAsync(pos, d_pos, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream), "download pos");
+    if (to_head == d_head && heading)
         CK(cudaMemcpyAsync(heading, d_head, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download heading");
-    if (rng) CK(cudaMemcpyAsync(rng, d_rng, sizeof(uint4) * n, cudaMemcpyDeviceToHost, c->stream), "download rng");
-    if (speed) CK(cudaMemcpyAsync(speed, d_speed, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream), "download speed");
-    return sync_and_check(c);
+    if (to_rng == d_rng && rng)
+        CK(cudaMemcpyAsync(rng, d_rng, sizeof(uint4) * n, cudaMemcpyDeviceToHost, c->stream), "download rng");
+    if (to_speed == d_speed && speed)
+        CK(cudaMemcpyAsync(speed, d_speed, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream), "download speed");
+    return sync_and_check(c, true);
 }
 
 int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
@@ -1324,17 +1399,21 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     if ((rc = ensure_stage(c, n * sizeof(uint32_t) * (1 + (want_idx ? cap : 0)))) != MSIM_OK) return rc;
     uint32_t* d_idx = want_idx ? static_cast<uint32_t*>(c->stage) : nullptr;
     uint32_t* d_count = static_cast<uint32_t*>(c->stage) + (want_idx ? n * cap : 0);
+    uint32_t* to_count = direct_out<uint32_t>(c, count, d_count);
+    uint32_t* to_idx = nullptr;
+    if (want_idx) to_idx = reinterpret_cast<uint32_t*>(direct_out<uint4>(c, idx, reinterpret_cast<uint4*>(d_idx)));
     {
         Prof p(c, K_EXPORT);
         CK(launch_export_neighbours(c->stream, c->query_slot, cur_state(c).slot_id, c->nbr_count, c->nbr_list,
-                                    c->n, c->params.cap, d_count, d_idx),
+                                    c->n, c->params.cap, to_count, to_idx, c->err, c->status_host),
            "k_export_nbr");
     }
-    CK(cudaMemcpyAsync(count, d_count, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download counts");
-    if (want_idx)
+    if (to_count == d_count)
+        CK(cudaMemcpyAsync(count, d_count, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download counts");
+    if (want_idx && to_idx == d_idx)
         CK(cudaMemcpyAsync(idx, d_idx, sizeof(uint32_t) * n * cap, cudaMemcpyDeviceToHost, c->stream),
            "download neighbours");
-    return sync_and_check(c);
+    return sync_and_check(c, true);
 }
 
 int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading, const uint32_t* in_rng,

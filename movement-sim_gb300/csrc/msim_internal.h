@@ -29,6 +29,12 @@ int fail(int code, const std::string& msg);
 // failure injected by msim_debug_fail_device_alloc.  True on success.
 bool device_malloc(void** p, size_t bytes);
 
+// A zeroed page-locked word for a context's status read-back (page-locking one word costs
+// up to a millisecond, so 1,024 of them share one allocation for the life of the process),
+// or nullptr; status_word_give takes it back.  Safe from any thread.
+uint32_t* status_word_take();
+void status_word_give(uint32_t* word);
+
 // Owned map (JSON loader, lattice generator).
 struct MapData {
     std::vector<float> road_pos;      // 4 per road

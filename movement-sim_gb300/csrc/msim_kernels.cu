@@ -584,8 +584,10 @@ __global__ __launch_bounds__(256) void k_export_records(EntityState st, uint32_t
                  : "memory");
 }
 __global__ __launch_bounds__(256) void k_export_fields(const StateRecord* __restrict__ in, uint32_t n, float2* pos,
-                                                       uint32_t* head, uint4* rng, float* speed) {
+                                                       uint32_t* head, uint4* rng, float* speed, const uint32_t* err,
+                                                       uint32_t* status_out) {
     const uint32_t id = blockIdx.x * 256u + threadIdx.x;
+    if (id == 0 && status_out) *status_out = *err;
     if (id >= n) return;
     uint32_t w[8];
     asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -605,9 +607,11 @@ __global__ __launch_bounds__(256) void k_export_fields(const StateRecord* __rest
 __global__ __launch_bounds__(kQueryThreads) void k_export_nbr(const uint32_t* sorted_slot, const uint32_t* slot_id,
                                                               const uint32_t* count, const uint32_t* list,
                                                               uint32_t n, uint32_t cap, uint32_t* out_count,
-                                                              uint32_t* out_idx) {
+                                                              uint32_t* out_idx, const uint32_t* err,
+                                                              uint32_t* status_out) {
     constexpr uint32_t FULL = 0xffffffffu;
     const uint32_t p = blockIdx.x * kQueryThreads + threadIdx.x;
+    if (p == 0 && status_out) *status_out = *err;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t c = p < n ? count[p] : 0u;
     uint32_t id = 0xffffffffu;
@@ -1052,20 +1056,21 @@ cudaError_t launch_permute(cudaStream_t s, const uint32_t* sorted_slot, EntitySt
 }
 
 cudaError_t launch_export_state(cudaStream_t s, EntityState st, uint32_t n, float2* pos, uint32_t* head, uint4* rng,
-                                float* speed, void* records) {
+                                float* speed, void* records, const uint32_t* err, uint32_t* status_out) {
     if (n == 0) return cudaSuccess;
     StateRecord* rec = static_cast<StateRecord*>(records);
     k_export_records<<<blocks_for(n, 256), 256, 0, s>>>(st, n, rec);
-    k_export_fields<<<blocks_for(n, 256), 256, 0, s>>>(rec, n, pos, head, rng, speed);
+    k_export_fields<<<blocks_for(n, 256), 256, 0, s>>>(rec, n, pos, head, rng, speed, err, status_out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_export_neighbours(cudaStream_t s, const uint32_t* sorted_slot, const uint32_t* slot_id,
                                      const uint32_t* count, const uint32_t* list, uint32_t n, uint32_t cap,
-                                     uint32_t* out_count, uint32_t* out_idx) {
+                                     uint32_t* out_count, uint32_t* out_idx, const uint32_t* err,
+                                     uint32_t* status_out) {
     if (n == 0) return cudaSuccess;
     k_export_nbr<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(sorted_slot, slot_id, count, list, n, cap,
-                                                                        out_count, out_idx);
+                                                                        out_count, out_idx, err, status_out);
     return cudaGetLastError();
 }
 

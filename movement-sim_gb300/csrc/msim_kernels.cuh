@@ -169,11 +169,14 @@ cudaError_t launch_permute(cudaStream_t s, const uint32_t* sorted_slot, EntitySt
 // records: n x kStateRecordBytes of scratch, 32-byte aligned
 constexpr size_t kStateRecordBytes = 32;
 cudaError_t launch_export_state(cudaStream_t s, EntityState st, uint32_t n, float2* pos,
-                                uint32_t* head, uint4* rng, float* speed, void* records);
+                                uint32_t* head, uint4* rng, float* speed, void* records,
+                                // *status_out = *err (both or neither NULL)
+                                const uint32_t* err = nullptr, uint32_t* status_out = nullptr);
 // out_idx: 16-byte aligned
 cudaError_t launch_export_neighbours(cudaStream_t s, const uint32_t* sorted_slot, const uint32_t* slot_id,
                                      const uint32_t* count, const uint32_t* list, uint32_t n,
-                                     uint32_t cap, uint32_t* out_count, uint32_t* out_idx);
+                                     uint32_t cap, uint32_t* out_count, uint32_t* out_idx,
+                                     const uint32_t* err = nullptr, uint32_t* status_out = nullptr);
 cudaError_t launch_export_aos(cudaStream_t s, const DeviceMap& m, EntityState st, uint32_t n, float dt,
                               const uint32_t* sorted_slot, const uint32_t* count, void* out);
 
