@@ -180,16 +180,15 @@ __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch
         uint32_t h = a.st.head[s];
         const uint32_t h0 = h;
         const float sp = a.st.speed[s];
+        // the place of the moved position, in flight with the state
+        const uint32_t q = ONE && a.rank_pos ? a.rank[s] : 0xffffffffu;
         uint4 r = make_uint4(0u, 0u, 0u, 0u);
         bool rd = false;
         step_entity<RNG, ONE ? 1 : 0>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
         a.st.pos[s] = p;
         if (h != h0) a.st.head[s] = h;
         if (rd) a.st.rng[s] = r;
-        if (ONE && a.rank_pos) {  // uniform: a tick that reuses the index
-            const uint32_t q = a.rank[s];
-            if (q < a.rank_n) a.rank_pos[q] = p;
-        }
+        if (ONE && a.rank_pos && q < a.rank_n) a.rank_pos[q] = p;  // a tick that reuses the index
     }
 }
 
