@@ -182,9 +182,9 @@ __global__ __launch_bounds__(kAdjThreads, kAdjForwardBlocks) void k_adj_forward(
     uint4 r = a.rng0[e];
     const float s = a.speed[e];
     Leg l{};
-    if (!leg_load(a.map, a.dt, s, h, l, a.err)) {  // unreachable: headings come from the initializer
+    if (!leg_load<true>(a.map, a.dt, s, h, l, a.err)) {  // unreachable: headings come from the initializer
         h = 0u;
-        leg_load(a.map, a.dt, s, h, l, a.err);
+        leg_load<true>(a.map, a.dt, s, h, l, a.err);
     }
     const uint32_t low = (1u << a.fbits) - 1u;
     CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};  // NaN: in no cell yet
@@ -207,7 +207,7 @@ __global__ __launch_bounds__(kAdjThreads, kAdjForwardBlocks) void k_adj_forward(
         uint32_t sx = 0u, sy = 0u, began = 0u;  // sums and first tick of this stretch in the block
         for (uint32_t k = 0; k < len; k++) {
             const int force = REPLAY ? (int)(bits & 1u) : -1;
-            const bool snapped = step_leg<true>(a.map, a.dt, s, p, h, l, a.err, force,
+            const bool snapped = step_leg<true, true>(a.map, a.dt, s, p, h, l, a.err, force,
                                                 [&]() { return rng_next<RNG>(r); });
             if (REPLAY) bits >>= 1;
             else if (snapped) bits |= 1u << (first + k);
@@ -352,9 +352,9 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
         uint32_t h = a.ck_head[ck];
         uint4 r = a.ck_rng[ck];
         Leg l{};
-        if (!leg_load(a.map, a.dt, s, h, l, a.err)) {  // unreachable: the forward's headings
+        if (!leg_load<true>(a.map, a.dt, s, h, l, a.err)) {  // unreachable: the forward's headings
             h = 0u;
-            leg_load(a.map, a.dt, s, h, l, a.err);
+            leg_load<true>(a.map, a.dt, s, h, l, a.err);
         }
         hist[0] = p;
         uint32_t num_ends = 0, word = 0;
@@ -365,7 +365,7 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
                 p.x = l.tx;
                 p.y = l.ty;
                 ends[(size_t)num_ends++ * n] = h;
-                road_end(a.map, a.dt, s, h, l, a.err, [&]() { return rng_next<RNG>(r); });
+                road_end<true>(a.map, a.dt, s, h, l, a.err, [&]() { return rng_next<RNG>(r); });
             } else {
                 const float dx = l.tx - p.x, dy = l.ty - p.y;
                 const float d2 = dx * dx + dy * dy;
@@ -434,7 +434,7 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
                 adj = make_float2(0.f, 0.f);
                 h = ends[(size_t)--num_ends * n];  // the road before this tick
                 road = h & kHeadRoad;
-                l = leg_of(a.map, a.dt, s, road, __ldg(&a.map.road_pos[road]), (h & kHeadToEnd) != 0);
+                l = leg_of<false>(a.map, a.dt, s, road, __ldg(&a.map.road_pos[road]), (h & kHeadToEnd) != 0);
                 f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
             } else {
                 const float dx = l.tx - pp.x, dy = l.ty - pp.y;
@@ -698,7 +698,7 @@ uint32_t splat_fraction_bits(uint32_t gw, uint32_t gh) {
 // Entities per warp: 32, halved (to kAdjMinLanes) while that leaves the schedulers
 // fewer than two warps each.  Small counts are bound by the latency of a tick, and the
 // road end or cell change of one lane adds to every lane of its warp.
-constexpr uint32_t kAdjMinLanes = 4;
+constexpr uint32_t kAdjMinLanes = 8;
 uint32_t adj_lanes(uint32_t n, int sms) {
     uint32_t lanes = 32;
     while (lanes > kAdjMinLanes && n / lanes < 8u * (uint32_t)std::max(sms, 1)) lanes /= 2;

@@ -66,7 +66,7 @@ struct BatchArgs {
 
 // One warp's piece.  E independent entities per thread, interleaved tick by tick so
 // their dependency chains overlap.
-template <int RNG, int E>
+template <int RNG, int E, bool AHEAD>
 __device__ __forceinline__ void run_piece(const BatchArgs& a, const DeviceMap& m, const WorkItem& it) {
     const uint32_t lane = threadIdx.x & 31u;
     constexpr uint32_t span = 32u * E;
@@ -87,15 +87,17 @@ __device__ __forceinline__ void run_piece(const BatchArgs& a, const DeviceMap& m
             sp[k] = a.speed[e];
             r[k] = make_uint4(0u, 0u, 0u, 0u);
             rd[k] = false;
-            rl[k] = a.ticks >= kRngAheadTicks;
+            rl[k] = AHEAD;
             if (rl[k]) r[k] = a.rng[e];
-            ok[k] = ok[k] && leg_load(m, a.dt, sp[k], h[k], l[k], a.err);
+            ok[k] = ok[k] && leg_load<AHEAD>(m, a.dt, sp[k], h[k], l[k], a.err);
         }
+        constexpr int kUnroll = E == 1 ? 4 : 1;  // more than one entity: registers
+#pragma unroll kUnroll
         for (uint32_t t = 0; t < a.ticks; t++) {
 #pragma unroll
             for (int k = 0; k < E; k++) {
                 if (!ok[k]) continue;
-                step_leg<false>(m, a.dt, sp[k], p[k], h[k], l[k], a.err, -1, [&]() {
+                step_leg<false, AHEAD>(m, a.dt, sp[k], p[k], h[k], l[k], a.err, -1, [&]() {
                     if (!rl[k]) {
                         r[k] = a.rng[it.begin + off + lane + k * 32u];
                         rl[k] = true;
@@ -122,7 +124,7 @@ __device__ __forceinline__ void run_piece(const BatchArgs& a, const DeviceMap& m
 // in one kernel).
 // Every warp takes its own pieces: no block barrier, and a block's slow warp (road ends)
 // holds up no other.
-template <int RNG, int EMAX>
+template <int RNG, int EMAX, bool AHEAD>
 __global__ void __maxnreg__(EMAX == 1 ? 40 : EMAX == 2 ? 56 : 72) k_batch_step(BatchArgs a) {
     while (true) {
         uint32_t i = 0;
@@ -138,9 +140,9 @@ __global__ void __maxnreg__(EMAX == 1 ? 40 : EMAX == 2 ? 56 : 72) k_batch_step(B
         m.factor = nullptr;
         m.num_roads = d.num_roads;
         m.num_conn = d.num_conn;
-        if (EMAX >= 4 && it.ept == 4) run_piece<RNG, 4>(a, m, it);
-        else if (EMAX >= 2 && it.ept == 2) run_piece<RNG, 2>(a, m, it);
-        else run_piece<RNG, 1>(a, m, it);
+        if (EMAX >= 4 && it.ept == 4) run_piece<RNG, 4, AHEAD>(a, m, it);
+        else if (EMAX >= 2 && it.ept == 2) run_piece<RNG, 2, AHEAD>(a, m, it);
+        else run_piece<RNG, 1, AHEAD>(a, m, it);
     }
 }
 
@@ -258,19 +260,23 @@ int check_schedule(const msim_batch_schedule& s) {
     return MSIM_OK;
 }
 
-// The kernel instantiation for a schedule: RNG and its largest entities per thread.
+// The kernel instantiation for a schedule and a run: RNG, and for long runs its largest
+// entities per thread; short runs take one entity per thread whatever the schedule says
+// (128 instances, 1 tick: 69 us against 83 for four per thread; 32 ticks 308 and 444).
 using BatchKernel = void (*)(BatchArgs);
-BatchKernel batch_kernel(uint32_t rng_kind, const msim_batch_schedule& s) {
+BatchKernel batch_kernel(uint32_t rng_kind, const msim_batch_schedule& s, uint32_t ticks) {
+    static const BatchKernel kernels[2][4] = {
+        {k_batch_step<0, 1, false>, k_batch_step<0, 1, true>, k_batch_step<0, 2, true>, k_batch_step<0, 4, true>},
+        {k_batch_step<1, 1, false>, k_batch_step<1, 1, true>, k_batch_step<1, 2, true>, k_batch_step<1, 4, true>}};
     uint32_t emax = 1;
     for (uint32_t c = 0; c < s.num_classes && c < MSIM_BATCH_MAX_CLASSES; c++)
         emax = std::max(emax, s.entities_per_thread[c]);
-    if (rng_kind == 1) return emax >= 4 ? k_batch_step<1, 4> : emax == 2 ? k_batch_step<1, 2> : k_batch_step<1, 1>;
-    return emax >= 4 ? k_batch_step<0, 4> : emax == 2 ? k_batch_step<0, 2> : k_batch_step<0, 1>;
+    return kernels[rng_kind == 1][ticks < kAheadTicks ? 0 : emax >= 4 ? 3 : emax];
 }
 
-int occupancy(msim_batch* b, uint32_t threads) {
+int occupancy(msim_batch* b, uint32_t threads, uint32_t ticks = kAheadTicks) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel(b->rng_kind, b->sched), (int)threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel(b->rng_kind, b->sched, ticks), (int)threads, 0);
     return std::max(per_sm, 1);
 }
 
@@ -342,9 +348,9 @@ cudaError_t enqueue(msim_batch* b, uint32_t ticks) {
     cudaError_t e = cudaMemsetAsync(b->ticket, 0, sizeof(uint32_t), b->stream);
     if (e != cudaSuccess) return e;
     const uint32_t threads = b->sched.block_threads;
-    const int grid = b->sms * occupancy(b, threads);
+    const int grid = b->sms * occupancy(b, threads, ticks);
     BatchArgs a = args_of(b, ticks);
-    batch_kernel(b->rng_kind, b->sched)<<<grid, threads, 0, b->stream>>>(a);
+    batch_kernel(b->rng_kind, b->sched, ticks)<<<grid, threads, 0, b->stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -171,11 +171,18 @@ __device__ __forceinline__ void digit_counts(uint32_t key, bool valid, uint32_t 
 // registers between them, bound by the ticks' serial chain (small counts) or by issue:
 // with read-back, 10,000 entities for 1,000 ticks 316 -> 216 us and 1 M for 200 ticks
 // 867 -> 581 us against reloading the road and three intrinsics every tick.
-template <int RNG, bool ONE>
+template <int RNG, bool ONE, bool AHEAD>
 __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch a) {
     chain_enter();
-    const uint32_t stride = gridDim.x * kMoveThreads;
-    for (uint32_t s = blockIdx.x * kMoveThreads + threadIdx.x; s < a.n; s += stride) {
+    const uint32_t thread = blockIdx.x * kMoveThreads + threadIdx.x;
+    uint32_t s = thread, stride = gridDim.x * kMoveThreads;
+    if (!ONE) {  // a.lanes entities to a warp
+        const uint32_t lane = thread & 31u;
+        if (lane >= a.lanes) return;
+        s = (thread >> 5) * a.lanes + lane;
+        stride = (stride >> 5) * a.lanes;
+    }
+    for (; s < a.n; s += stride) {
         float2 p = a.st.pos[s];
         uint32_t h = a.st.head[s];
         const uint32_t h0 = h;
@@ -184,7 +191,7 @@ __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch
         const uint32_t q = ONE && a.rank_pos ? a.rank[s] : 0xffffffffu;
         uint4 r = make_uint4(0u, 0u, 0u, 0u);
         bool rd = false;
-        step_entity<RNG, ONE ? 1 : 0>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
+        step_entity<RNG, ONE ? 1 : 0, AHEAD>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
         a.st.pos[s] = p;
         if (h != h0) a.st.head[s] = h;
         if (rd) a.st.rng[s] = r;
@@ -244,7 +251,7 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
             if (a.ticks) {
                 uint4 r = make_uint4(0u, 0u, 0u, 0u);
                 bool rd = false;
-                step_entity<RNG, 1>(a.map, a.dt, sp[u], 1u, p[u], h[u], r, rd, a.st.rng + sl[u], a.err);
+                step_entity<RNG, 1, false>(a.map, a.dt, sp[u], 1u, p[u], h[u], r, rd, a.st.rng + sl[u], a.err);
                 a.st.pos[sl[u]] = p[u];
                 if (h[u] != h0[u]) {
                     a.st.head[sl[u]] = h[u];
@@ -770,6 +777,17 @@ __global__ void k_iota(uint32_t* out, uint32_t n) {
 
 inline unsigned blocks_for(uint32_t n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
 
+// Entities per warp of a run of many ticks: 32, halved while that leaves the
+// schedulers fewer than kFewWarps warps each.  Small counts are bound by the latency of
+// a tick, and the road end of one lane adds to every lane of its warp (1,000 entities
+// 154 -> 133 ns per tick, 10,000 162 -> 151; four warps 184).
+uint32_t warp_lanes(uint32_t n, int sms) {
+    constexpr uint32_t kFewWarps = 2, kFewestLanes = 4;
+    uint32_t lanes = 32;
+    while (lanes > kFewestLanes && n / lanes < kFewWarps * 4u * (uint32_t)std::max(sms, 1)) lanes /= 2;
+    return lanes;
+}
+
 // Launch of a chain kernel (see chain_enter).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args) {
@@ -820,12 +838,20 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const unsigned blocks = std::min<unsigned>(blocks_for(a.n, kMoveThreads), 16u * (unsigned)std::max(sms, 1));
-        if (a.ticks == 1)
-            return a.rng_kind == 1 ? launch_chained(k_move<1, true>, blocks, kMoveThreads, s, a)
-                                   : launch_chained(k_move<0, true>, blocks, kMoveThreads, s, a);
-        return a.rng_kind == 1 ? launch_chained(k_move<1, false>, blocks, kMoveThreads, s, a)
-                               : launch_chained(k_move<0, false>, blocks, kMoveThreads, s, a);
+        const unsigned most = 16u * (unsigned)std::max(sms, 1);
+        if (a.ticks > 1) {
+            StepLaunch b = a;
+            b.lanes = warp_lanes(a.n, sms);
+            const unsigned blocks = std::min(most, blocks_for(blocks_for(a.n, b.lanes) * 32u, kMoveThreads));
+            if (a.ticks < kAheadTicks)
+                return a.rng_kind == 1 ? launch_chained(k_move<1, false, false>, blocks, kMoveThreads, s, b)
+                                       : launch_chained(k_move<0, false, false>, blocks, kMoveThreads, s, b);
+            return a.rng_kind == 1 ? launch_chained(k_move<1, false, true>, blocks, kMoveThreads, s, b)
+                                   : launch_chained(k_move<0, false, true>, blocks, kMoveThreads, s, b);
+        }
+        const unsigned blocks = std::min(most, blocks_for(a.n, kMoveThreads));
+        return a.rng_kind == 1 ? launch_chained(k_move<1, true, false>, blocks, kMoveThreads, s, a)
+                               : launch_chained(k_move<0, true, false>, blocks, kMoveThreads, s, a);
     }
     if (a.ticks > 1) return cudaErrorInvalidValue;  // k_step moves one tick at most
     if (a.disp_max) {  // a host tick that queries the previous index (keys, one tick)

@@ -74,6 +74,7 @@ struct StepLaunch {
     const uint32_t* rank = nullptr;
     float2* rank_pos = nullptr;
     uint32_t rank_n = 0;
+    uint32_t lanes = 32;  // several ticks: entities per warp (set by launch_step)
 };
 
 cudaError_t launch_init_entities(cudaStream_t s, const DeviceMap& m, EntityState st, uint32_t n,
