@@ -318,15 +318,41 @@ __device__ __forceinline__ float lam_at(const float* lambda, uint32_t gw, uint32
     return (i < 0 || j < 0 || i >= (int)gw || j >= (int)gh) ? 0.f : __ldg(&lambda[(size_t)j * gw + i]);
 }
 
+// 1 / sqrt(d2) by the hardware instruction (rsqrtf's bits for normal d2, without its
+// test for subnormal ones); 0 for d2 = 0, where the adjoint's terms then vanish.
+__device__ __forceinline__ float inv_length(float d2) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d2));
+    return d2 >= 1.17549435e-38f ? y : d2 > 0.f ? rsqrtf(d2) : 0.f;
+}
+
+// Gradient of the splat at a position, scaled by cells per metre and 1 / ticks, as two
+// linear functions of the cell fractions: x = x0 + fy * x1, y = y0 + fx * y1.
+struct SplatGrad {
+    float x0, x1, y0, y1;
+};
+__device__ __noinline__ SplatGrad splat_grad(const float* lambda, uint32_t gw, uint32_t gh, int i, int j, float sx,
+                                             float sy) {
+    const float l00 = lam_at(lambda, gw, gh, i, j), l10 = lam_at(lambda, gw, gh, i + 1, j);
+    const float l01 = lam_at(lambda, gw, gh, i, j + 1), l11 = lam_at(lambda, gw, gh, i + 1, j + 1);
+    SplatGrad g;
+    g.x0 = (l10 - l00) * sx;
+    g.x1 = ((l11 - l01) - (l10 - l00)) * sx;
+    g.y0 = (l01 - l00) * sy;
+    g.y1 = ((l11 - l10) - (l01 - l00)) * sy;
+    return g;
+}
+
 // Backward of one entity, segment by segment from the last to the first: recompute
 // the segment's positions from its checkpoint (the event decisions from the schedule,
 // the road choices from the checkpointed RNG, both exact; the position update with
 // the hardware reciprocal square root, since the adjoint needs the positions only to
 // about 1e-6 relative and snaps put them back on exact road ends), then sweep
-// backwards over them.  The road's leg, and the four cell values' differences, stay in
-// registers until a road end or a cell change; headings are kept only for road ends
-// (12 -> 8 B of history per tick), and all segments run in one launch, which a launch
-// per segment rounded up to two waves each.
+// backwards over them.  The road's leg and the cell's gradient stay in registers until a
+// road end or a cell change, the leg's gradient parts are summed before they are scaled,
+// headings are kept only for road ends (12 -> 8 B of history per tick), ticks run in
+// stretches of one schedule word, and all segments run in one launch, which a launch per
+// segment rounded up to two waves each.
 template <int RNG>
 __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backward(AdjBack b) {
     const AdjArgs& a = b.f;
@@ -336,17 +362,17 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
     const float s = a.speed[e];
     const uint32_t* sched = a.sched + (size_t)e * a.sched_words;
     uint2* rec = b.rec + (size_t)e * b.segments * kRecPerSeg;
-    float2* hist = b.hist_pos + e;
     uint32_t* ends = b.hist_head + e;
-    const float sx = a.inv_cw, sy = a.inv_ch, invT = 1.0f / (float)a.ticks;
+    const float invT = 1.0f / (float)a.ticks;
+    const float sx = a.inv_cw * invT, sy = a.inv_ch * invT;
     const float scale = __int_as_float((127 - (int)a.fbits) << 23);  // 2^-fbits
     float2 adj = make_float2(0.f, 0.f);
     double gspeed = 0.0;
     uint32_t records = 0;
     CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};
-    float dx0 = 0.f, dx1 = 0.f, dy0 = 0.f, dy1 = 0.f;  // lambda differences of the cell block
+    SplatGrad sg{};
     for (uint32_t seg = b.segments; seg-- > 0;) {
-        const uint32_t t0 = seg * a.K, len = min(a.K, a.ticks - t0);  // ticks t0 + 1 .. t0 + len
+        const uint32_t t0 = seg * a.K, t1 = t0 + min(a.K, a.ticks - t0);  // ticks t0 + 1 .. t1
         const size_t ck = (size_t)seg * n + e;
         float2 p = a.ck_pos[ck];
         uint32_t h = a.ck_head[ck];
@@ -356,37 +382,47 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
             h = 0u;
             leg_load<true>(a.map, a.dt, s, h, l, a.err);
         }
-        hist[0] = p;
-        uint32_t num_ends = 0, word = 0;
-        for (uint32_t k = 0; k < len; k++) {  // recompute with the recorded events
-            const uint32_t bit = (t0 + k) & 31u;
-            if (k == 0 || bit == 0) word = sched[(t0 + k) >> 5];
-            if ((word >> bit) & 1u) {
-                p.x = l.tx;
-                p.y = l.ty;
-                ends[(size_t)num_ends++ * n] = h;
-                road_end<true>(a.map, a.dt, s, h, l, a.err, [&]() { return rng_next<RNG>(r); });
-            } else {
-                const float dx = l.tx - p.x, dy = l.ty - p.y;
-                const float d2 = dx * dx + dy * dy;
-                if (d2 > 0.f) {
-                    const float q = rsqrtf(d2) * l.step;
+        float2* at = b.hist_pos + e;  // the segment's positions, its checkpoint first
+        *at = p;
+        uint32_t num_ends = 0;
+        for (uint32_t t = t0; t < t1;) {  // recompute with the recorded events
+            const uint32_t first = t & 31u, len = min(32u - first, t1 - t);
+            uint32_t bits = __brev(sched[t >> 5]) << first;  // the next tick's event in the sign bit
+            t += len;
+#pragma unroll 4
+            for (uint32_t k = 0; k < len; k++) {
+                if ((int)bits >= 0) {
+                    const float dx = l.tx - p.x, dy = l.ty - p.y;
+                    const float q = inv_length(dx * dx + dy * dy) * l.step;
                     p.x += dx * q;
                     p.y += dy * q;
+                } else {
+                    p.x = l.tx;
+                    p.y = l.ty;
+                    ends[(size_t)num_ends++ * n] = h;
+                    road_end<true>(a.map, a.dt, s, h, l, a.err, [&]() { return rng_next<RNG>(r); });
                 }
+                bits <<= 1;
+                at += n;
+                *at = p;
             }
-            hist[(size_t)(k + 1u) * n] = p;
         }
-        // reverse sweep: p is the position after the tick, pp before it; the history is
-        // fetched kAhead ticks early
-        constexpr int kAhead = 4;
+        // reverse sweep: p is the position after the tick, the history (fetched kAhead
+        // ticks early) holds the one before it
+        constexpr uint32_t kAhead = 4;
         float2 ahead[kAhead];
+        uint32_t left = t1 - t0;  // ticks to sweep; the position before the next one is hist[left - 1]
 #pragma unroll
-        for (int q = 0; q < kAhead; q++) ahead[q] = hist[(size_t)(len > 1u + q ? len - 1u - q : 0u) * n];
+        for (uint32_t q = 0; q < kAhead; q++) {
+            if (q < left) at -= n;
+            ahead[q] = *at;
+        }
         float gs = 0.f, cur_sum = 0.f;
         uint32_t cur_road = b.num_roads, nrec = 0;
         uint32_t road = h & kHeadRoad;
         float f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
+        float part = 0.f;  // sum of n . adj over the leg
+        bool any = false;
         auto record = [&]() {
             if (cur_road == b.num_roads) return;
             if (nrec < kRecPerSeg) {
@@ -396,67 +432,72 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
                 atomicOr(a.err, kErrOob);
             }
         };
-        for (uint32_t k = len; k-- > 0;) {  // tick t0 + k + 1
-            const uint32_t bit = (t0 + k) & 31u;
-            if (k == len - 1u || bit == 31u) word = sched[(t0 + k) >> 5];
-            const float2 pp = ahead[0];
+        auto end_leg = [&]() {
+            if (!any) return;
+            if (road != cur_road) {
+                record();
+                cur_road = road;
+                cur_sum = 0.f;
+            }
+            cur_sum += part * s * a.dt;
+            gs += part * f * a.dt;
+            part = 0.f;
+            any = false;
+        };
+        for (uint32_t t = t1; t > t0;) {
+            const uint32_t word_from = (t - 1u) & ~31u, from = max(word_from, t0), len = t - from;
+            uint32_t bits = sched[word_from >> 5] << (31u - ((t - 1u) & 31u));  // this tick's event in the sign bit
+            t = from;
+#pragma unroll 4
+            for (uint32_t k = 0; k < len; k++) {
+                const float2 pp = ahead[0];
 #pragma unroll
-            for (int q = 0; q + 1 < kAhead; q++) ahead[q] = ahead[q + 1];
-            ahead[kAhead - 1] = hist[(size_t)(k > (uint32_t)kAhead ? k - kAhead : 0u) * n];
-            {  // + (1/T) d splat(p_t)/dp . lambda
-                const float ux = cell_coord(p.x, sx), uy = cell_coord(p.y, sy);
-                float wx, wy;
-                float fx, fy;
-                if (in_cell(c, ux, uy, wx, wy)) {
-                    fx = wx - c.one;  // exact: fbits bits
-                    fy = wy - c.one;
-                } else {
-                    const Splat sp = splat_of(ux, uy, a.fbits);
-                    const float l00 = lam_at(b.lambda, a.gw, a.gh, sp.i0, sp.j0);
-                    const float l10 = lam_at(b.lambda, a.gw, a.gh, sp.i0 + 1, sp.j0);
-                    const float l01 = lam_at(b.lambda, a.gw, a.gh, sp.i0, sp.j0 + 1);
-                    const float l11 = lam_at(b.lambda, a.gw, a.gh, sp.i0 + 1, sp.j0 + 1);
-                    dx0 = l10 - l00;
-                    dx1 = l11 - l01;
-                    dy0 = l01 - l00;
-                    dy1 = l11 - l10;
-                    fx = (float)sp.fx * scale;  // exact: fewer than 24 bits
-                    fy = (float)sp.fy * scale;
-                    c.fi = (float)sp.i0;
-                    c.fj = (float)sp.j0;
-                }
-                const float gx = ((1.f - fy) * dx0 + fy * dx1) * sx;
-                const float gy = ((1.f - fx) * dy0 + fx * dy1) * sy;
-                adj.x += gx * invT;
-                adj.y += gy * invT;
-            }
-            if ((word >> bit) & 1u) {
-                adj = make_float2(0.f, 0.f);
-                h = ends[(size_t)--num_ends * n];  // the road before this tick
-                road = h & kHeadRoad;
-                l = leg_of<false>(a.map, a.dt, s, road, __ldg(&a.map.road_pos[road]), (h & kHeadToEnd) != 0);
-                f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
-            } else {
-                const float dx = l.tx - pp.x, dy = l.ty - pp.y;
-                const float d2 = dx * dx + dy * dy;
-                if (d2 > 0.f) {
-                    const float invL = rsqrtf(d2);
-                    const float nx = dx * invL, ny = dy * invL;
-                    const float g = nx * adj.x + ny * adj.y;
-                    gs += g * f * a.dt;
-                    if (road != cur_road) {
-                        record();
-                        cur_road = road;
-                        cur_sum = 0.f;
+                for (uint32_t q = 0; q + 1u < kAhead; q++) ahead[q] = ahead[q + 1u];
+                left--;
+                if (left >= kAhead) at -= n;  // else the checkpoint again, not used
+                ahead[kAhead - 1u] = *at;
+                {  // + (1/T) d splat(p_t)/dp . lambda
+                    const float ux = cell_coord(p.x, a.inv_cw), uy = cell_coord(p.y, a.inv_ch);
+                    float wx, wy;
+                    float fx, fy;
+                    if (in_cell(c, ux, uy, wx, wy)) {
+                        fx = wx - c.one;  // exact: fbits bits
+                        fy = wy - c.one;
+                    } else {
+                        const Splat sp = splat_of(ux, uy, a.fbits);
+                        sg = splat_grad(b.lambda, a.gw, a.gh, sp.i0, sp.j0, sx, sy);
+                        fx = (float)sp.fx * scale;  // exact: fewer than 24 bits
+                        fy = (float)sp.fy * scale;
+                        c.fi = (float)sp.i0;
+                        c.fj = (float)sp.j0;
                     }
-                    cur_sum += g * s * a.dt;
-                    const float q = l.step * invL;
-                    adj.x -= q * (adj.x - nx * g);
-                    adj.y -= q * (adj.y - ny * g);
+                    adj.x += __fmaf_rn(fy, sg.x1, sg.x0);
+                    adj.y += __fmaf_rn(fx, sg.y1, sg.y0);
                 }
+                if ((int)bits >= 0) {
+                    const float dx = l.tx - pp.x, dy = l.ty - pp.y;
+                    const float d2 = __fmaf_rn(dx, dx, dy * dy);
+                    const float inv = inv_length(d2);
+                    const float g = __fmaf_rn(dx, adj.x, dy * adj.y) * inv;  // n . adj
+                    part += g;
+                    any = any || d2 > 0.f;
+                    const float gi = g * inv, q = l.step * inv;
+                    const float cx = __fmaf_rn(-dx, gi, adj.x), cy = __fmaf_rn(-dy, gi, adj.y);  // adj - n g
+                    adj.x = __fmaf_rn(-q, cx, adj.x);
+                    adj.y = __fmaf_rn(-q, cy, adj.y);
+                } else {
+                    end_leg();
+                    adj = make_float2(0.f, 0.f);
+                    h = ends[(size_t)--num_ends * n];  // the road before this tick
+                    road = h & kHeadRoad;
+                    l = leg_of<false>(a.map, a.dt, s, road, __ldg(&a.map.road_pos[road]), (h & kHeadToEnd) != 0);
+                    f = a.map.factor ? __ldg(&a.map.factor[road]) : 1.0f;
+                }
+                bits <<= 1;
+                p = pp;
             }
-            p = pp;
         }
+        end_leg();
         record();
         gspeed += (double)gs;
     }
