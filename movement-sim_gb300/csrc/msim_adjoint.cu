@@ -67,10 +67,13 @@ struct AdjArgs {
 };
 
 // Threads of a block of the forward and backward kernels, and blocks per SM.  Both are
-// bound by issue; the backward's history (800 B per entity at K = 100) of the resident
-// threads then also fits the L2 it is read back from.
+// bound by issue.  Forward: one warp a block, so that a slow warp keeps no finished one's
+// place (262,144 entities 1.68 ms; 128 threads 1.80).  Backward: the history (800 B per
+// entity at K = 100) of the resident threads then mostly stays in the L2 it is read back
+// from (7 blocks of 128 threads 2.63 ms; 6 3.01, 8 at fewer registers 2.96, 24 of 32 2.94).
+constexpr uint32_t kAdjForwardThreads = 32;
+constexpr int kAdjForwardBlocks = 28;
 constexpr uint32_t kAdjThreads = 128;
-constexpr int kAdjForwardBlocks = 7;
 constexpr int kAdjBackwardBlocks = 7;
 
 // The entity of a thread: `lanes` entities to a warp (32, fewer for small counts: the
@@ -151,9 +154,9 @@ __device__ __forceinline__ void flush_block(unsigned long long* dacc, uint32_t g
 // in about 70 ticks, so some lane of a warp does in 37 % of its ticks; waiting for the second
 // change brings the flushes of about eight lanes together.
 struct LeftBlocks {
-    int i[kAdjThreads], j[kAdjThreads];
-    uint32_t n[kAdjThreads];  // 0: none
-    unsigned long long sx[kAdjThreads], sy[kAdjThreads], sxy[kAdjThreads];
+    int i[kAdjForwardThreads], j[kAdjForwardThreads];
+    uint32_t n[kAdjForwardThreads];  // 0: none
+    unsigned long long sx[kAdjForwardThreads], sy[kAdjForwardThreads], sxy[kAdjForwardThreads];
 };
 __device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
     const uint32_t t = threadIdx.x;
@@ -169,9 +172,9 @@ __device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
 // word or a checkpoint does, so a tick itself is the step, the cell test and three
 // sums (32-bit within a stretch).  Bound by issue (82 % active): 118 warp instructions
 // per tick against 190 with the road reloaded, two conversions and a flush at every
-// cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.92 ms.
+// cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.68 ms.
 template <int RNG, bool REPLAY>
-__global__ __launch_bounds__(kAdjThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
+__global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
     __shared__ LeftBlocks left;
     const uint32_t e = adj_entity(a.n, a.lanes);
     left.n[threadIdx.x] = 0u;
@@ -205,6 +208,7 @@ __global__ __launch_bounds__(kAdjThreads, kAdjForwardBlocks) void k_adj_forward(
         uint32_t* word = a.sched + (size_t)e * a.sched_words + (t >> 5);
         if (REPLAY) bits = *word >> first;
         uint32_t sx = 0u, sy = 0u, began = 0u;  // sums and first tick of this stretch in the block
+#pragma unroll 2
         for (uint32_t k = 0; k < len; k++) {
             const int force = REPLAY ? (int)(bits & 1u) : -1;
             const bool snapped = step_leg<true, true>(a.map, a.dt, s, p, h, l, a.err, force,
@@ -745,9 +749,9 @@ uint32_t adj_lanes(uint32_t n, int sms) {
     while (lanes > kAdjMinLanes && n / lanes < 8u * (uint32_t)std::max(sms, 1)) lanes /= 2;
     return lanes;
 }
-unsigned adj_blocks(const msim_adj* a) {
+unsigned adj_blocks(const msim_adj* a, uint32_t threads) {
     const uint64_t warps = ((uint64_t)a->n + a->lanes - 1u) / a->lanes;
-    return (unsigned)((warps * 32u + kAdjThreads - 1u) / kAdjThreads);
+    return (unsigned)((warps * 32u + threads - 1u) / threads);
 }
 
 AdjArgs fwd_args(msim_adj* a) {
@@ -1006,14 +1010,14 @@ int msim_adj_forward(msim_adj* a, const float* d_speed, const float* d_factor, c
         ACK(cudaMemcpyAsync(a->target, d_target, sizeof(float) * G, cudaMemcpyDeviceToDevice, a->stream), "target");
     ACK(cudaMemsetAsync(a->dacc, 0, sizeof(unsigned long long) * G, a->stream), "memset density");
     const AdjArgs f = fwd_args(a);
-    const unsigned blocks = adj_blocks(a);
+    const unsigned blocks = adj_blocks(a, kAdjForwardThreads);
     cudaEventRecord(a->ph[0], a->stream);
     if (a->p.rng_kind == 1) {
-        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<1, true><<<blocks, kAdjThreads, 0, a->stream>>>(f);
-        else k_adj_forward<1, false><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<1, true><<<blocks, kAdjForwardThreads, 0, a->stream>>>(f);
+        else k_adj_forward<1, false><<<blocks, kAdjForwardThreads, 0, a->stream>>>(f);
     } else {
-        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<0, true><<<blocks, kAdjThreads, 0, a->stream>>>(f);
-        else k_adj_forward<0, false><<<blocks, kAdjThreads, 0, a->stream>>>(f);
+        if (mode == MSIM_ADJ_REPLAY) k_adj_forward<0, true><<<blocks, kAdjForwardThreads, 0, a->stream>>>(f);
+        else k_adj_forward<0, false><<<blocks, kAdjForwardThreads, 0, a->stream>>>(f);
     }
     ACK(cudaGetLastError(), "k_adj_forward");
     cudaEventRecord(a->ph[1], a->stream);
@@ -1053,8 +1057,8 @@ int msim_adj_backward(msim_adj* a, float* d_grad_speed, float* d_grad_factor) {
     b.rec_block = a->rec_block;
     b.num_roads = a->R;
     cudaEventRecord(a->ph[3], a->stream);
-    if (a->p.rng_kind == 1) k_adj_backward<1><<<adj_blocks(a), kAdjThreads, 0, a->stream>>>(b);
-    else k_adj_backward<0><<<adj_blocks(a), kAdjThreads, 0, a->stream>>>(b);
+    if (a->p.rng_kind == 1) k_adj_backward<1><<<adj_blocks(a, kAdjThreads), kAdjThreads, 0, a->stream>>>(b);
+    else k_adj_backward<0><<<adj_blocks(a, kAdjThreads), kAdjThreads, 0, a->stream>>>(b);
     ACK(cudaGetLastError(), "k_adj_backward");
     cudaEventRecord(a->ph[4], a->stream);
     // road gradients: the records packed, stably sorted by road, summed per road
