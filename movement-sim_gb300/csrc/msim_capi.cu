@@ -225,7 +225,9 @@ struct msim_ctx {
     const uint32_t* query_slot = nullptr;
     uint32_t* nbr_count = nullptr;
     uint32_t* nbr_list = nullptr;
-    unsigned long long* pairs = nullptr;
+    unsigned long long* pairs = nullptr;  // the last query's counters
+    unsigned long long* pairs_b[2] = {nullptr, nullptr};  // used in turn
+    bool pairs_zeroed = false;  // the spare counters are zero (the last query zeroed them)
     bool have_nbr = false;
     uint32_t* err = nullptr;
     uint32_t* status_host = nullptr;  // page-locked copy of *err, written behind the work it describes
@@ -968,7 +970,10 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
         CK(cudaStreamWaitEvent(c->qstream, c->ev_index, 0), "cudaStreamWaitEvent");
         qs = c->qstream;
     }
-    CK(cudaMemsetAsync(c->pairs, 0, sizeof(unsigned long long) * kPairBins, qs), "memset pairs");
+    c->pairs = c->pairs_b[c->pairs == c->pairs_b[0] ? 1 : 0];
+    if (!c->pairs_zeroed)  // the first query, or after one that may not have run
+        CK(cudaMemsetAsync(c->pairs, 0, sizeof(unsigned long long) * kPairBins, qs), "memset pairs");
+    c->pairs_zeroed = false;
     {
         Prof p(c, K_QUERY);
         // slots that hold their own entity need no id lookup
@@ -976,7 +981,8 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
         CKL(p, launch_query(qs, c->params.cap, c->kstart, read_pairs ? c->pair_ids : c->sorted_slot,
                         pos ? pos : c->sorted_pos,
                         c->slots_identity || read_pairs ? nullptr : cur_state(c).slot_id, grid ? *grid : c->grid,
-                        c->n, c->nbr_count, c->nbr_list, c->pairs, c->err,
+                        c->n, c->nbr_count, c->nbr_list, c->pairs,
+                        c->pairs_b[c->pairs == c->pairs_b[0] ? 1 : 0], c->err,
                         c->slots_identity ? count_by_id : nullptr, c->dense, pairs ? c->pairs_kept : nullptr,
                         c->pair_sizes, c->pair_ids, keep_near),
            "k_query");
@@ -989,6 +995,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
         CK(cudaEventRecord(c->ev_tick[2], qs), "cudaEventRecord");
         c->tick_recorded = true;
     }
+    c->pairs_zeroed = true;
     c->query_slot = c->sorted_slot;
     c->have_nbr = true;
     c->since_permute++;
@@ -1018,6 +1025,7 @@ int sync_and_check(msim_ctx* c, bool status_queued = false) {
             // up, so the entity state is intact; the index is rebuilt from scratch (full
             // sort, every look-back region zeroed again) by the next neighbour tick.
             c->chain_broken = true;
+            c->pairs_zeroed = false;  // its query skipped its work
             reset_index(c);
             return fail(MSIM_ERR_TIMEOUT, "a bounded device wait (index look-back) gave up; the neighbour results "
                                           "since the last successful sync are invalid, the entity state is kept");
@@ -1173,7 +1181,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
         (rc = dalloc(c, &c->b_key[0], n)) || (rc = dalloc(c, &c->b_key[1], n)) || (rc = dalloc(c, &c->b_val[0], n)) ||
         (rc = dalloc(c, &c->b_val[1], n)) || (rc = dalloc(c, &c->ab_counts, 2)) ||
         (rc = dalloc(c, &c->merge_split, (size_t)merge_tiles(c->n) + 1)) || (rc = dalloc(c, &c->sorted_dev, 1)) ||
-        (rc = dalloc(c, &c->nbr_count, n)) || (rc = dalloc(c, &c->pairs, kPairBins)) || (rc = dalloc(c, &c->err, 1)) ||
+        (rc = dalloc(c, &c->nbr_count, n)) || (rc = dalloc(c, &c->pairs_b[0], kPairBins)) ||
+        (rc = dalloc(c, &c->pairs_b[1], kPairBins)) || (rc = dalloc(c, &c->err, 1)) ||
         (rc = dalloc(c, &c->check, 1)) || (rc = dalloc(c, &c->bounds_dev, 2)))
         return bail(rc);
     for (int b = 0; b < 2; b++) {
@@ -1185,6 +1194,7 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     c->mark_ticket = c->hist + (size_t)kMaxPasses * kRadix;
     c->mark_lookback = reinterpret_cast<unsigned long long*>(c->hist + (size_t)kMaxPasses * kRadix + 2u);
     use_index_buffers(c, 0);
+    c->pairs = c->pairs_b[0];
     if (p.cap > 0) {
         size_t blocks = (n + kQueryThreads - 1) / kQueryThreads;
         if ((rc = dalloc(c, &c->nbr_list, blocks * kQueryThreads * (size_t)p.cap))) return bail(rc);

@@ -950,11 +950,13 @@ cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n
 
 cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, const uint32_t* sorted_slot,
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
-                         uint32_t* list, unsigned long long* pair_bins, const uint32_t* err, uint32_t* count_by_id,
+                         uint32_t* list, unsigned long long* pair_bins, unsigned long long* next_bins, const uint32_t* err,
+                         uint32_t* count_by_id,
                          bool dense, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near) {
     if (n == 0) return cudaSuccess;
     using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
-                           uint32_t*, uint32_t*, unsigned long long*, const uint32_t*, uint32_t*, PairStore);
+                           uint32_t*, uint32_t*, unsigned long long*, unsigned long long*, const uint32_t*, uint32_t*,
+                           PairStore);
 #define QUERY_KERNELS(LIST, KEEP, DENSE)                                                               \
     {k_query<LIST, KEEP, DENSE, kPairsFound>, k_query<LIST, KEEP, DENSE, kPairsKept>, \
      k_query<LIST, KEEP, DENSE, kPairsUsed>}
@@ -976,8 +978,8 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
     // the squared distance's rounding and its operands' stay far below 2^-18 of it
     const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18))};
     kernels[lists][dense][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
-        kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins, err,
-        count_by_id, store);
+        kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins,
+        next_bins, err, count_by_id, store);
     return cudaGetLastError();
 }
 

@@ -113,7 +113,9 @@ cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n
                           float2* sorted_pos = nullptr, const uint32_t* err = nullptr);
 cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, const uint32_t* sorted_slot,
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
-                         uint32_t* list, unsigned long long* pair_bins,  // pair_bins: kPairBins counters
+                         uint32_t* list,
+                         // kPairBins counters, zero before this query, and those it zeroes for the next
+                         unsigned long long* pair_bins, unsigned long long* next_bins,
                          const uint32_t* err = nullptr,  // err: the status word (skip after a failed wait)
                          // count_by_id (may be NULL; only when slot = entity id): every count also
                          // written at its entity's id

@@ -530,6 +530,7 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                                                          uint32_t n, uint32_t cap, uint32_t* __restrict__ count_out,
                                                          uint32_t* __restrict__ list,
                                                          unsigned long long* __restrict__ pair_bins,
+                                                         unsigned long long* __restrict__ next_bins,
                                                          const uint32_t* err, uint32_t* __restrict__ count_by_id,
                                                          PairStore store) {
     constexpr uint32_t FULL = 0xffffffffu;
@@ -668,6 +669,8 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
         if (count_by_id) count_by_id[sorted_slot[p]] = count;
     }
     const uint32_t warp_sum = __reduce_add_sync(FULL, count);  // every pair is seen from both ends
+    // the next query's counters (a memset for them stood between two queries)
+    if (p < kPairBins) next_bins[p] = 0ull;
     if (lane == 0 && warp_sum) atomicAdd(&pair_bins[(p >> 5) & (kPairBins - 1u)], (unsigned long long)warp_sum);
     if (LIST) {
         const uint32_t kept = count < cap ? count : cap;
