@@ -63,13 +63,13 @@ def b_nbr(k_mean: float, updates_per_tick: float = 1.0) -> float:
 # per-kernel algorithmic bytes per entity and launch: the per-entity figures of a
 # neighbour tick (24 B move + 36 + 4 k B index and query) split over the kernels
 KERNEL_BYTES = {
-    "k_step": lambda k: B_STEP + 4,        # move + key write
+    "k_step": lambda k: B_STEP + 8,        # move + key and rank write
     "k_onesweep": lambda k: 16,            # (key, id) read + write
     "k_kstart": lambda k: 4 + 20,          # sorted key read, slot read + position gather + write
                                            # (+ 4 B per key slot, added below)
-    "k_mark": lambda k: 20,                # previous order 4 + old key 4 + new key 4, split write 8
-    "k_merge": lambda k: 32,               # split read 8, sorted key+slot write 8, position gather 8 + write 8
-                                           # (+ 4 B per key slot, added below)
+    "k_mark": lambda k: 0,                 # 12 B per key slot (count read and zeroed, start written; below)
+    "k_place": lambda k: 36,               # key, rank in its key and start 12, position 8, sorted slot 4,
+                                           # position 8 and place 4 written
     "k_query": lambda k: 12 + 4 * k,       # own pos 8 + count 4 + kept ids
     "k_gather": lambda k: 20,              # order read 4, position read 8 + write 8
     "k_move": lambda k: B_STEP + 12,       # reusing tick: move + rank read 4 + placed position write 8
@@ -91,7 +91,7 @@ NCU_BATCH_WARP_INSTR_PER_ENTITY_STEP = 1.971
 NCU_QUERY_WARP_INSTR_PER_ENTITY = 24.04
 
 NCU_DRAM_BYTES_PER_ENTITY = {
-    "scale": {"k_query": 26.87, "k_merge": 32.78, "k_mark": 16.91, "k_step": 27.98},
+    "scale": {"k_query": 26.87},
     "neighbours": {"k_query": 24.07, "k_onesweep": 6.91},
 }
 
@@ -277,8 +277,10 @@ def run_ours(args, cfg, world, rank, local):
             per_launch_bytes = KERNEL_BYTES[name](k_mean) * sorted_per_update
         else:
             per_launch_bytes = KERNEL_BYTES.get(name, lambda k: 0)(k_mean) * n
-            if name in ("k_kstart", "k_merge"):  # write one word per key of the key space
+            if name == "k_kstart":  # writes one word per key of the key space
                 per_launch_bytes += 4 * (2 ** info["key_bits"] + 1)
+            if name == "k_mark":
+                per_launch_bytes += 12 * 2 ** info["key_bits"]
         kernels[name] = {"launches": v["launches"], "avg_ms": avg, "share": v["ms"] / total_ms,
                          "algo_bytes_per_launch": per_launch_bytes,
                          "achieved_gbs": per_launch_bytes / (avg / 1e3) / 1e9 if avg > 0 else None}

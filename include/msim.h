@@ -127,8 +127,8 @@ typedef struct msim_params {
 } msim_params;
 
 /* msim_params.flags: how neighbour ticks rebuild the index (same results either way).
- * By default the previous order is updated (only entries whose key changed are
- * sorted and merged back; the first neighbour tick sorts fully), and between updates
+ * By default the index is updated by a counting sort over the keys (the first
+ * neighbour tick after entities were set sorts fully), and between updates
  * the index is reused: a neighbour tick queries the index built a few ticks earlier
  * with every box widened by a bound on how far any entity can have moved since
  * (ticks x max |speed| x max |road factor| x dt, plus rounding), and the index is
@@ -136,7 +136,7 @@ typedef struct msim_params {
  * the entities were set, moved by the host or re-ordered).  An entity within the
  * radius of another now lay within radius + bound of it, in each coordinate, when
  * the index was built, so the results are the same.
- * FULL_SORT: always a full radix sort (e.g. entities that move far between ticks);
+ * FULL_SORT: always a full radix sort;
  * INCREMENTAL: the update (the default; kept for callers that name it);
  * NO_REUSE: update the index on every neighbour tick (host ticks included). */
 #define MSIM_PARAM_FULL_SORT 1u
@@ -328,10 +328,8 @@ int msim_reset_kernel_stats(msim_ctx* ctx);
 int msim_get_kernel_stats(msim_ctx* ctx, uint32_t kernel, uint64_t* launches, double* total_ms);
 uint32_t msim_kernel_count(void);
 const char* msim_kernel_name(uint32_t kernel);
-/* Index updates (full sorts and incremental updates) since the stats were reset, and
- * the entries that went through their radix passes (n per full sort, the entries
- * whose key changed per incremental update): the sort's work per tick.
- * Synchronises the context's stream. */
+/* Index updates (full sorts and counting updates) since the stats were reset, and the
+ * entries they sorted (n per update).  Synchronises the context's stream. */
 int msim_get_sort_stats(msim_ctx* ctx, uint64_t* index_updates, uint64_t* sorted_entries);
 /* msim_tick_host calls since the stats were reset, those whose query read the
  * previous state's index with widened boxes, and the largest displacement measured by

@@ -334,7 +334,7 @@ class Simulation:
         return out
 
     def sort_stats(self) -> dict:
-        """Index updates since the stats were reset and the entries their radix passes sorted."""
+        """Index updates since the stats were reset and the entries they sorted."""
         u, e = ctypes.c_uint64(), ctypes.c_uint64()
         check(lib().msim_get_sort_stats(self._ctx, ctypes.byref(u), ctypes.byref(e)))
         return {"index_updates": u.value, "sorted_entries": e.value}

@@ -97,15 +97,15 @@ enum KernelId : uint32_t {
     K_QUERY,
     K_PERMUTE,
     K_EXPORT,
-    K_MARK,   // split of the previous order into unchanged / changed keys
-    K_MERGE,  // merge + key-start table + sorted positions
+    K_MARK,   // index update: key counts scanned into the key-start table
+    K_MERGE,  // index update: entities to their places
     K_GATHER, // host tick: an uploaded chunk's positions into the previous sorted order
     K_MOVE,   // a tick that reuses the index: move + each position at its sorted position
     K_COUNT
 };
 static const char* const kKernelNames[K_COUNT] = {"k_init",   "k_step",   "k_step_multi", "k_onesweep",
                                                   "k_kstart", "k_query",  "k_permute",    "k_export",
-                                                  "k_mark",   "k_merge",  "k_gather", "k_move"};
+                                                  "k_mark",   "k_place",  "k_gather", "k_move"};
 
 // msim_tick_host: at most this many chunks, each at least kHostChunkMin entities
 constexpr uint32_t kHostChunks = 4;  // at 16 M: 4.09 ms per host tick; 8 chunks 4.16-4.18, 16 4.31
@@ -157,24 +157,20 @@ struct msim_ctx {
     const uint32_t* sorted_key = nullptr;
     const uint32_t* sorted_slot = nullptr;
     bool have_sort = false;
-    // incremental index update: the previous order split into unchanged (a) and
-    // changed (b, sorted in place with ping-pong) keys, then merged
     bool order_identity = false;  // sorted_slot[q] == q (right after a re-ordering)
-    bool chunk_count_zeroed = false;  // the move step of this tick zeroed the merge's long-gap counter
     bool slots_identity = false;  // slot s holds entity s (state set from the host, not re-ordered since)
-    bool incremental = true;      // index updates from the previous order (else full sorts)
-    uint32_t* a_key = nullptr;
-    uint32_t* a_val = nullptr;
-    uint32_t* b_key[2] = {nullptr, nullptr};
-    uint32_t* b_val[2] = {nullptr, nullptr};
-    uint32_t* ab_counts = nullptr;
-    unsigned long long* mark_lookback = nullptr;
+    bool incremental = true;      // index updates by counting (else full radix sorts)
+    // index update by counting: entities per key (zero between updates; counts_pending: a
+    // step has counted into them and the scan that zeroes them has not been launched) and
+    // every slot's rank among its key
+    uint32_t* key_count = nullptr;
+    uint32_t* key_rank = nullptr;
+    bool counts_pending = false;
+    uint32_t* mark_lookback = nullptr;
     uint32_t* mark_ticket = nullptr;
-    size_t update_words = 0;  // hist, mark ticket and mark look-back lie together: one memset per update
-    uint32_t* merge_split = nullptr;
-    // entries that went through the radix passes since the stats were reset: full
-    // sorts counted on the host, incremental updates' changed entries on the device
-    unsigned long long* sorted_dev = nullptr;
+    size_t update_words = 0;  // ticket and look-back words of the scan lie together
+    uint32_t* update_scratch = nullptr;
+    // entries placed by index updates since the stats were reset
     uint64_t sorted_host = 0;
     uint64_t index_updates = 0;
     // Index reuse: neighbour ticks between index updates query the last index with
@@ -736,87 +732,71 @@ int build_index(msim_ctx* c) {
     return permute_state(c);
 }
 
-// One tick of the move plus the index, from the previous sorted order: split it by
-// whether each key changed, sort the changed entries, merge (writing the key-start
-// table and the sorted positions on the way).  The update's scratch (digit counts,
-// split ticket and look-back words) is cleared first, in one memset, before the
-// move, so that the move step and the split run back to back.
+// One tick of the move plus the index by a counting sort.  The move step clears the
+// scan's ticket and look-back words, so that the three kernels run back to back.
 int incremental_update(msim_ctx* c, bool positions = true, bool ranks = true);
 
 int clear_update_scratch(msim_ctx* c) {
-    CK(cudaMemsetAsync(c->hist, 0, sizeof(uint32_t) * c->update_words, c->stream), "memset update scratch");
+    CK(cudaMemsetAsync(c->update_scratch, 0, sizeof(uint32_t) * c->update_words, c->stream), "memset update scratch");
+    return MSIM_OK;
+}
+
+// Before a step that counts keys: the counters are zero (the last update's scan zeroed
+// them, unless it never ran or gave up).
+int begin_counts(msim_ctx* c) {
+    if (c->counts_pending)
+        CK(cudaMemsetAsync(c->key_count, 0, sizeof(uint32_t) * c->num_keys, c->stream), "memset key counts");
+    c->counts_pending = true;
     return MSIM_OK;
 }
 
 int incremental_index(msim_ctx* c) {
-    c->chunk_count_zeroed = false;
+    int rc = begin_counts(c);
+    if (rc != MSIM_OK) return rc;
     {
         Prof p(c, K_STEP);
         StepLaunch a = step_args(c, 1, true);
-        a.hist = nullptr;  // the changed keys' digits are counted by k_mark
-        // the move step clears the update's scratch and the long-gap counter of the index
-        // set the merge will write (no memsets between the chained launches)
-        a.zero_a = c->hist;
+        a.hist = nullptr;
+        a.key_count = c->key_count;
+        a.key_rank = c->key_rank;
+        a.zero_a = c->update_scratch;
         a.zero_a_words = (uint32_t)c->update_words;
-        a.zero_b = c->kstart_chunk_count_b[c->sorted_key == c->sk[0] ? 1 : 0];
         CKL(p, launch_step(c->stream, a), "k_step");
-        c->chunk_count_zeroed = true;
     }
     if (c->tick_timing) CK(cudaEventRecord(c->ev_tick[1], c->stream), "cudaEventRecord");
     return incremental_update(c);
 }
 
-// The update itself, for new keys (by slot) already in c->key.  positions = false:
-// the sorted positions are not written (a host tick whose next query reads the
-// positions it gathers itself).  ranks = false: no ranks either (a host tick's slots
-// are entity ids, in no spatial order: writing rank[slot] scatters at random, 0.12 ms
-// more per update at 16 M, and moves placing positions by them cost 0.11 ms more per
-// 4 M chunk than the gather passes).
+// The update itself, for keys, counts and ranks already taken by the step.  positions =
+// false: the sorted positions are not written (a host tick whose next query reads the
+// positions it gathers itself).  ranks = false: no ranks either (host ticks; see
+// msim_tick_host).
 int incremental_update(msim_ctx* c, bool positions, bool ranks) {
     NvtxRange range("msim index update");
     int rc = inject_sort_tile(c, c->mark_ticket);
     if (rc != MSIM_OK) return rc;
-    {
-        Prof p(c, K_MARK);
-        CKL(p, launch_mark(c->stream, c->sorted_slot, c->order_identity, c->sorted_key, c->key, c->n, c->passes,
-                       c->a_key, c->a_val, c->b_key[0], c->b_val[0], c->hist, c->mark_lookback, c->mark_ticket,
-                       c->ab_counts, c->err, c->sorted_dev, c->spin_limit),
-           "k_mark");
-        c->index_updates++;
-    }
-    rc = clear_unchained(c);
-    if (rc != MSIM_OK) return rc;
-    c->chain_broken = true;  // until every pass has launched
-    for (uint32_t ps = 0; ps < c->passes; ps++) {  // stable radix sort of the changed entries
-        const SweepChain ch = sweep_chain(c, ps);
-        Prof p(c, K_SORT_PASS);
-        CKL(p, launch_onesweep(c->stream, c->b_key[ps & 1], c->b_val[ps & 1], c->b_key[(ps + 1) & 1],
-                           c->b_val[(ps + 1) & 1], c->n, 8u * ps, c->hist + ps * kRadix,
-                           c->lookback + ps * c->sort_region, c->tickets + ps, c->err, c->ab_counts + 1,
-                           c->passes >= 2 ? &ch : nullptr, c->spin_limit),
-           "k_onesweep");
-    }
-    c->chain_broken = false;
-    // The merge writes the sorted slots and index buffer set the previous tick's query
+    // The update writes the sorted slots and index buffer set the previous tick's query
     // does not read (that query may still run); it waits for the query before that.
-    const int out = c->sorted_key == c->sk[0] ? 1 : 0;
-    rc = wait_reads(c, out);
-    if (rc != MSIM_OK) return rc;
+    const int out = 1 - c->ib;
+    if ((rc = wait_reads(c, out)) != MSIM_OK) return rc;
     use_index_buffers(c, out);
     {
-        Prof p(c, K_MERGE);
-        uint32_t launched = 0;
-        CKL(p, launch_merge(c->stream, c->a_key, c->a_val, c->b_key[c->passes & 1], c->b_val[c->passes & 1],
-                        c->ab_counts, c->merge_split, c->n, c->sk[out], c->sv[out],
-                        positions ? cur_state(c).pos : nullptr, positions ? c->sorted_pos : nullptr,
-                        c->kstart, (uint32_t)c->num_keys, c->kstart_chunks, c->kstart_chunk_count, c->err,
-                        &launched, c->chunk_count_zeroed, ranks ? c->rank : nullptr),
-           "k_merge");
-        c->rank_valid = ranks && c->rank != nullptr;
-        c->chunk_count_zeroed = false;
-        if (launched > 1) c->launch_count += launched - 1;
+        Prof p(c, K_MARK);
+        CKL(p, launch_mark(c->stream, c->key_count, (uint32_t)c->num_keys, c->n, c->kstart, c->mark_lookback,
+                           c->mark_ticket, c->err, c->spin_limit),
+           "k_mark");
+        c->index_updates++;
+        c->sorted_host += c->n;
     }
-    c->sorted_key = c->sk[out];
+    {
+        Prof p(c, K_MERGE);
+        CKL(p, launch_place(c->stream, c->key, c->key_rank, c->kstart, (uint32_t)c->num_keys, c->n,
+                            positions ? cur_state(c).pos : nullptr, c->sv[out], positions ? c->sorted_pos : nullptr,
+                            ranks ? c->rank : nullptr, c->err),
+           "k_place");
+        c->rank_valid = ranks && c->rank != nullptr;
+    }
+    c->counts_pending = false;
     c->sorted_slot = c->sv[out];
     c->order_identity = false;
     c->have_sort = true;
@@ -883,7 +863,7 @@ int neighbour_tick(msim_ctx* c) {
     // against 0.36-0.39), the update it skips (split, passes, merge) about 0.30 ms.
     const double ticks = c->reuse_ticks >= 0 ? (double)c->reuse_ticks + 1.0 : 0.0;
     bool reuse = false;
-    if (c->reuse && c->sorted_key && !c->order_identity && c->reuse_ticks >= 0 && c->grid.reach > 0.f &&
+    if (c->reuse && c->sorted_slot && !c->order_identity && c->reuse_ticks >= 0 && c->grid.reach > 0.f &&
         (c->bounds_valid || c->reuse_ticks == 0)) {
         if ((rc = ensure_bounds(c)) != MSIM_OK) return rc;
         reuse = ticks * c->step_bound <= (double)kWidenLimit * (double)c->grid.reach && ensure_reuse(c);
@@ -894,7 +874,7 @@ int neighbour_tick(msim_ctx* c) {
             if (rc != MSIM_OK) return rc;
         }
         if (c->reuse) ensure_reuse(c);  // so this update writes the ranks the next ticks use
-        if (c->sorted_key && c->incremental) {
+        if (c->sorted_slot && c->incremental) {
             rc = incremental_index(c);
             if (rc != MSIM_OK) return rc;
         } else {
@@ -1026,6 +1006,7 @@ int sync_and_check(msim_ctx* c, bool status_queued = false) {
             // sort, every look-back region zeroed again) by the next neighbour tick.
             c->chain_broken = true;
             c->pairs_zeroed = false;  // its query skipped its work
+            c->counts_pending = true;
             reset_index(c);
             return fail(MSIM_ERR_TIMEOUT, "a bounded device wait (index look-back) gave up; the neighbour results "
                                           "since the last successful sync are invalid, the entity state is kept");
@@ -1071,9 +1052,9 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
         return cuda_fail(e, "cudaGetDevice");
     }
     c->params = p;
-    // the incremental index update is the faster one at every size measured (62.5 K,
-    // 250 K, 1 M and 16 M entities at the lattice density: 0.051 against 0.060 ms per
-    // tick at 62.5 K, 0.092 against 0.114 at 1 M)
+    // the counting update is the faster one at every size measured (per update, move step
+    // included, against the earlier update from the previous order: 3,001 entities 57 ->
+    // 22 us, 1 M 117 -> 50, 16 M 531 -> 388; a full radix sort took longer at all of them)
     c->incremental = (p.flags & MSIM_PARAM_FULL_SORT) == 0;
     c->reuse = (p.flags & MSIM_PARAM_NO_REUSE) == 0;
     c->n = p.num_entities;
@@ -1172,15 +1153,14 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
             (rc = dalloc(c, &c->st[b].slot_id, n)) || (rc = dalloc(c, &c->sk[b], n)) || (rc = dalloc(c, &c->sv[b], n)))
             return bail(rc);
     }
-    // [digit counts | split ticket, pad | split look-back words (8-byte aligned)]
-    c->update_words = (size_t)kMaxPasses * kRadix + 2u + 2u * (size_t)mark_tiles(c->n);
-    if ((rc = dalloc(c, &c->key, n)) || (rc = dalloc(c, &c->hist, c->update_words)) ||
+    // [scan ticket, pad | scan look-back words]
+    c->update_words = 2u + (size_t)mark_tiles((uint32_t)c->num_keys);
+    if ((rc = dalloc(c, &c->key, n)) || (rc = dalloc(c, &c->hist, (size_t)kMaxPasses * kRadix)) ||
+        (rc = dalloc(c, &c->update_scratch, c->update_words)) ||
         (rc = dalloc(c, &c->lookback, (size_t)kMaxPasses * c->sort_region)) ||
         (rc = dalloc(c, &c->sort_dirty, (size_t)kMaxPasses)) ||
-        (rc = dalloc(c, &c->tickets, (size_t)kMaxPasses)) || (rc = dalloc(c, &c->a_key, n)) || (rc = dalloc(c, &c->a_val, n)) ||
-        (rc = dalloc(c, &c->b_key[0], n)) || (rc = dalloc(c, &c->b_key[1], n)) || (rc = dalloc(c, &c->b_val[0], n)) ||
-        (rc = dalloc(c, &c->b_val[1], n)) || (rc = dalloc(c, &c->ab_counts, 2)) ||
-        (rc = dalloc(c, &c->merge_split, (size_t)merge_tiles(c->n) + 1)) || (rc = dalloc(c, &c->sorted_dev, 1)) ||
+        (rc = dalloc(c, &c->tickets, (size_t)kMaxPasses)) || (rc = dalloc(c, &c->key_rank, n)) ||
+        (rc = dalloc(c, &c->key_count, c->num_keys)) ||
         (rc = dalloc(c, &c->nbr_count, n)) || (rc = dalloc(c, &c->pairs_b[0], kPairBins)) ||
         (rc = dalloc(c, &c->pairs_b[1], kPairBins)) || (rc = dalloc(c, &c->err, 1)) ||
         (rc = dalloc(c, &c->check, 1)) || (rc = dalloc(c, &c->bounds_dev, 2)))
@@ -1191,8 +1171,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
             (rc = dalloc(c, &c->kstart_chunk_count_b[b], 1)) || (rc = dalloc(c, &c->sorted_pos_b[b], n)))
             return bail(rc);
     }
-    c->mark_ticket = c->hist + (size_t)kMaxPasses * kRadix;
-    c->mark_lookback = reinterpret_cast<unsigned long long*>(c->hist + (size_t)kMaxPasses * kRadix + 2u);
+    c->mark_ticket = c->update_scratch;
+    c->mark_lookback = c->update_scratch + 2u;
     use_index_buffers(c, 0);
     c->pairs = c->pairs_b[0];
     if (p.cap > 0) {
@@ -1208,7 +1188,7 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     if (e == cudaSuccess) e = cudaMemcpy(c->road_conn, map->road_conn, sizeof(uint4) * c->R, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(c->conn, conn.data(), sizeof(uint32_t) * (c->C + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->err, 0, sizeof(uint32_t), c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->sorted_dev, 0, sizeof(unsigned long long), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->key_count, 0, sizeof(uint32_t) * c->num_keys, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->lookback, 0, sizeof(uint32_t) * kMaxPasses * c->sort_region, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->tickets, 0, sizeof(uint32_t) * kMaxPasses, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->sort_dirty, 0, sizeof(uint32_t) * kMaxPasses, c->stream);
@@ -1463,7 +1443,7 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     // its slots already held entity ids (the previous call was a host tick, or a set
     // followed by one tick): the new state goes to the same slots.
     const bool old_slots_identity = c->slots_identity;
-    const bool use_inc = nbr && c->incremental && c->sorted_key && c->slots_identity;
+    const bool use_inc = nbr && c->incremental && c->sorted_slot && c->slots_identity;
     // Skin query: when the current index was built from the keys of the state this
     // tick starts from (the previous call was a neighbour host tick and nothing moved
     // or set the state since), this tick's query reads that index with every box
@@ -1499,7 +1479,7 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     const bool in_place = dev_head != nullptr;
     CK(cudaMemsetAsync(c->check, 0xff, sizeof(uint32_t), c->stream), "memset check");
     if (nbr && !use_inc) CK(cudaMemsetAsync(c->hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, c->stream), "memset hist");
-    if (use_inc && (rc = clear_update_scratch(c)) != MSIM_OK) return rc;
+    if (use_inc && ((rc = clear_update_scratch(c)) != MSIM_OK || (rc = begin_counts(c)) != MSIM_OK)) return rc;
     if (skin) CK(cudaMemsetAsync(c->disp, 0, sizeof(uint32_t), c->stream), "memset displacement");
     // entity i in slot i (for later calls; this tick's query and export take the slot
     // as the id): written first, beside the first chunk's upload
@@ -1544,7 +1524,11 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
             a.st.slot_id = s.slot_id + lo;
             a.n = cnt;
             a.key = nbr ? c->key + lo : nullptr;
-            if (use_inc) a.hist = nullptr;  // the changed keys' digits are counted by k_mark
+            if (use_inc) {
+                a.hist = nullptr;
+                a.key_count = c->key_count;
+                a.key_rank = c->key_rank + lo;
+            }
             a.blocks = std::min<int>(c->step_blocks, (int)((cnt + kStepThreads - 1) / kStepThreads));
             a.host_head = dev_head;
             a.host_rng = dev_rng;
@@ -1891,7 +1875,6 @@ int msim_reset_kernel_stats(msim_ctx* c) {
     c->index_updates = 0;
     c->host_ticks = 0;
     c->skin_queries = 0;
-    CK(cudaMemsetAsync(c->sorted_dev, 0, sizeof(unsigned long long), c->stream), "memset sort stats");
     return rc;
 }
 
@@ -1906,11 +1889,9 @@ int msim_get_host_tick_stats(msim_ctx* c, uint64_t* host_ticks, uint64_t* skin_q
 int msim_get_sort_stats(msim_ctx* c, uint64_t* index_updates, uint64_t* sorted_entries) {
     int rc = check_ctx(c);
     if (rc != MSIM_OK) return rc;
-    unsigned long long dev = 0;
-    CK(cudaMemcpyAsync(&dev, c->sorted_dev, sizeof(dev), cudaMemcpyDeviceToHost, c->stream), "read sort stats");
     CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
     if (index_updates) *index_updates = c->index_updates;
-    if (sorted_entries) *sorted_entries = c->sorted_host + dev;
+    if (sorted_entries) *sorted_entries = c->sorted_host;
     return MSIM_OK;
 }
 

@@ -11,10 +11,10 @@
 //   k_kstart    key-start table: first sorted position of every key (tile + band)
 //   k_query     radius neighbour query (random_move.comp:541-719 semantics: the
 //               pair predicate of :551-562), count + the cap smallest ids
-// After the first neighbour tick the sort is replaced by an incremental update of the
-// previous order (msim_incsort.cuh): k_mark splits it by changed keys, k_onesweep
-// sorts the changed entries, k_merge_path + k_merge merge them back and write the
-// key-start table and the sorted positions.
+// After the first neighbour tick the sort is replaced by a counting sort
+// (msim_indexsort.cuh): the step takes every entity's rank among its key, k_mark scans
+// the keys' counts into the key-start table, k_place writes the sorted slots and
+// positions.
 // Every few ticks k_permute re-orders the entity state by the sorted order so
 // that the step and the query keep reading memory almost sequentially.
 #include <algorithm>
@@ -165,6 +165,24 @@ __device__ __forceinline__ void digit_counts(uint32_t key, bool valid, uint32_t 
     }
 }
 
+// Rank of an entity among those of its key (any order): one atomic per run of equal keys
+// among consecutive lanes, which keeps crowds on one key off its counter.
+__device__ __forceinline__ uint32_t key_rank(uint32_t key, bool valid, uint32_t lane, uint32_t* key_count) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const unsigned vm = __ballot_sync(FULL, valid);
+    const uint32_t prev = __shfl_up_sync(FULL, key, 1);
+    const bool head = valid && (lane == 0 || key != prev);
+    const unsigned heads = __ballot_sync(FULL, head);
+    uint32_t base = 0u;
+    if (head) {
+        const unsigned later = heads & ~((2u << lane) - 1u);  // heads after this lane
+        const uint32_t end = later ? (uint32_t)(__ffs(later) - 1) : (uint32_t)(32 - __clz(vm));
+        base = atomicAdd(key_count + key, end - lane);
+    }
+    const uint32_t first = 31u - (uint32_t)__clz((heads & (0xffffffffu >> (31u - lane))) | 1u);
+    return __shfl_sync(FULL, base, first) + lane - first;
+}
+
 // Move-only ticks: one entity per thread in 128-thread blocks, so a small entity count
 // still spreads over many SMs.  ONE: a single tick (the tick that reuses the index
 // places its positions too); else several ticks with the state and the road's leg in
@@ -219,7 +237,6 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * kStepThreads;
     for (uint32_t i = blockIdx.x * kStepThreads + threadIdx.x; i < a.zero_a_words; i += stride) a.zero_a[i] = 0u;
-    if (a.zero_b && blockIdx.x == 0 && threadIdx.x == 0) *a.zero_b = 0u;
     for (uint32_t base = blockIdx.x * kStepThreads; base < a.n; base += kStepPer * stride) {
         uint32_t sl[kStepPer];
         bool valid[kStepPer];
@@ -265,6 +282,13 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
             if (KEY) {
                 key[u] = tile_key(a.grid, p[u], s_morton);
                 a.key[sl[u]] = key[u];
+            }
+        }
+        if (KEY && a.key_count) {
+#pragma unroll
+            for (int u = 0; u < kStepPer; u++) {
+                const uint32_t r = key_rank(key[u], valid[u], lane, a.key_count);
+                if (valid[u]) a.key_rank[sl[u]] = r;
             }
         }
         if (KEY && a.hist) {
@@ -552,7 +576,7 @@ __device__ __noinline__ void list_overflow(const uint32_t* __restrict__ sorted_s
 }
 
 #include "msim_query.cuh"
-#include "msim_incsort.cuh"
+#include "msim_indexsort.cuh"
 
 __global__ void k_permute(const uint32_t* __restrict__ ss, EntityState src, EntityState dst, uint32_t n,
                           const uint32_t* err) {
@@ -1006,45 +1030,21 @@ cudaError_t launch_fill(cudaStream_t s, float* out, uint32_t n, float v) {
     return cudaGetLastError();
 }
 
-uint32_t mark_tiles(uint32_t n) { return (n + kMarkTile - 1u) / kMarkTile; }
-uint32_t merge_tiles(uint32_t n) { return (n + kMergeTile - 1u) / kMergeTile; }
+uint32_t mark_tiles(uint32_t num_keys) { return (num_keys + kScanTile - 1u) / kScanTile; }
 
-cudaError_t launch_mark(cudaStream_t s, const uint32_t* P, bool identity, const uint32_t* PK, const uint32_t* NK,
-                        uint32_t n, uint32_t passes, uint32_t* a_key, uint32_t* a_val, uint32_t* b_key,
-                        uint32_t* b_val, uint32_t* hist, unsigned long long* lookback, uint32_t* ticket,
-                        uint32_t* counts, uint32_t* err, unsigned long long* changed_total, uint32_t spin_limit) {
-    if (n == 0) return cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s);
-    const uint32_t tiles = mark_tiles(n);
-    return launch_chained(k_mark, tiles, kMarkThreads, s, P, identity ? 1u : 0u, PK, NK, n, passes, a_key, a_val, b_key,
-                          b_val, hist, lookback, ticket, tiles, counts, err, changed_total, spin_limit);
+cudaError_t launch_mark(cudaStream_t s, uint32_t* key_count, uint32_t num_keys, uint32_t n, uint32_t* kstart,
+                        uint32_t* lookback, uint32_t* ticket, uint32_t* err, uint32_t spin_limit) {
+    const uint32_t tiles = mark_tiles(num_keys);
+    return launch_chained(k_mark, tiles, kScanThreads, s, key_count, num_keys, n, kstart, lookback, ticket, tiles, err,
+                          spin_limit);
 }
 
-cudaError_t launch_merge(cudaStream_t s, const uint32_t* a_key, const uint32_t* a_val, const uint32_t* b_key,
-                         const uint32_t* b_val, const uint32_t* counts, uint32_t* split, uint32_t n,
-                         uint32_t* out_key, uint32_t* out_val, const float2* pos, float2* sorted_pos,
-                         uint32_t* kstart, uint32_t num_keys, uint4* chunks, uint32_t* chunk_count, uint32_t* err,
-                         uint32_t* kernels, bool chunk_count_zeroed, uint32_t* rank) {
-    if (kernels) *kernels = 0;
-    if (n == 0 || num_keys == 0) return cudaSuccess;
-    const uint32_t tiles = merge_tiles(n);
-    const uint32_t cap = kstart_chunk_cap(num_keys);
-    cudaError_t e = cudaSuccess;
-    if (!chunk_count_zeroed)  // first: the three kernels chain
-        e = cudaMemsetAsync(chunk_count, 0, sizeof(uint32_t), s);
-    if (e == cudaSuccess)  // a warp per tile boundary
-        e = launch_chained(k_merge_path, (tiles + 1u + 7u) / 8u, 256, s, a_key, b_key, counts, n, tiles + 1u, split,
-                           static_cast<const uint32_t*>(err));
-    if (e == cudaSuccess)
-        e = launch_chained(k_merge, tiles, kMergeThreads, s, a_key, a_val, b_key, b_val, counts, split, n, out_key,
-                           out_val, pos, sorted_pos, kstart, num_keys, chunks, chunk_count, cap, err, rank);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = launch_chained(k_kstart_fill, 4u * (sms > 0 ? sms : 1), 256, s, chunks, chunk_count, cap, kstart,
-                       static_cast<const uint32_t*>(err));
-    if (e == cudaSuccess && kernels) *kernels = 3;
-    return e;
+cudaError_t launch_place(cudaStream_t s, const uint32_t* key, const uint32_t* key_rank, const uint32_t* kstart,
+                         uint32_t num_keys, uint32_t n, const float2* pos, uint32_t* sorted_slot, float2* sorted_pos,
+                         uint32_t* rank, uint32_t* err) {
+    if (n == 0) return cudaSuccess;
+    return launch_chained(k_place, blocks_for(n, 256), 256, s, key, key_rank, kstart, num_keys, n, pos, sorted_slot,
+                          sorted_pos, rank, err);
 }
 
 cudaError_t launch_gather_chunk(cudaStream_t s, const uint32_t* P, uint32_t n, uint32_t lo, uint32_t cnt,

@@ -41,7 +41,9 @@ struct StepLaunch {
     uint32_t ticks;       // 0: only keys/histogram of the current positions
     uint32_t rng_kind;
     uint32_t* key;        // nullptr: no spatial key
-    uint32_t* hist;       // passes * 256 digit counts (accumulated)
+    uint32_t* hist;       // passes * 256 digit counts (accumulated); or, with NULL,
+    uint32_t* key_count = nullptr;  // entities per key (accumulated) and each one's rank
+    uint32_t* key_rank = nullptr;   // among its key, by slot
     TileGrid grid;
     uint32_t passes;
     uint32_t* err;
@@ -58,7 +60,6 @@ struct StepLaunch {
     // chained launches of the tick.
     uint32_t* zero_a = nullptr;
     uint32_t zero_a_words = 0;
-    uint32_t* zero_b = nullptr;  // one word
     // Largest displacement of the tick (nullptr: not measured): every moved entity's
     // max(|x - x0|, |y - y0|) against index_pos (by slot, the positions the current
     // index was built from) is atomically maxed into *disp_max as float bits (a
@@ -129,27 +130,16 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
 constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
 size_t query_pair_places(uint32_t n, bool dense);   // pairs of all lists
 size_t query_pair_sizes(uint32_t n);
-// Incremental index update: split the previous sorted order P (keys PK; P[q] = q when
-// identity) by whether the new key NK[slot] changed (A: unchanged, B: changed; counts
-// -> counts[0..1]; B's digit counts -> hist), then, after B is sorted, merge A and B
-// into out_key / out_val, writing the key-start table and the sorted positions.
-// changed_total (may be NULL) accumulates |B| (entries that go through the sort).
-// lookback (mark_tiles(n) words), ticket and hist must be zero when the split starts.
-uint32_t mark_tiles(uint32_t n);
-uint32_t merge_tiles(uint32_t n);
-cudaError_t launch_mark(cudaStream_t s, const uint32_t* P, bool identity, const uint32_t* PK, const uint32_t* NK,
-                        uint32_t n, uint32_t passes, uint32_t* a_key, uint32_t* a_val, uint32_t* b_key,
-                        uint32_t* b_val, uint32_t* hist, unsigned long long* lookback, uint32_t* ticket,
-                        uint32_t* counts, uint32_t* err, unsigned long long* changed_total = nullptr,
+// Index update by counting (msim_indexsort.cuh): the keys' counters become the key-start
+// table (and are zeroed), then every slot goes to its place; sorted_pos and rank may be
+// NULL.  lookback (mark_tiles(num_keys) words) and ticket must be zero when it starts.
+uint32_t mark_tiles(uint32_t num_keys);
+cudaError_t launch_mark(cudaStream_t s, uint32_t* key_count, uint32_t num_keys, uint32_t n, uint32_t* kstart,
+                        uint32_t* lookback, uint32_t* ticket, uint32_t* err,
                         uint32_t spin_limit = kDefaultSpinLimit);
-// chunk_count_zeroed: the long-gap counter was already zeroed in the tick (else a
-// memset does it first).  sorted_pos NULL: no positions are gathered (pos unused).
-cudaError_t launch_merge(cudaStream_t s, const uint32_t* a_key, const uint32_t* a_val, const uint32_t* b_key,
-                         const uint32_t* b_val, const uint32_t* counts, uint32_t* split, uint32_t n,
-                         uint32_t* out_key, uint32_t* out_val, const float2* pos, float2* sorted_pos,
-                         uint32_t* kstart, uint32_t num_keys, uint4* chunks, uint32_t* chunk_count, uint32_t* err,
-                         uint32_t* kernels, bool chunk_count_zeroed = false,
-                         uint32_t* rank = nullptr);  // rank (may be NULL): rank[out_val[p]] = p
+cudaError_t launch_place(cudaStream_t s, const uint32_t* key, const uint32_t* key_rank, const uint32_t* kstart,
+                         uint32_t num_keys, uint32_t n, const float2* pos, uint32_t* sorted_slot, float2* sorted_pos,
+                         uint32_t* rank, uint32_t* err);
 // out[q] = pos[P[q]] for the q whose slot P[q] lies in [lo, lo + cnt) (q < n; the
 // other entries are left as they are): the positions of one uploaded chunk of a host
 // tick copied to their places in the sorted order P.
