@@ -205,8 +205,9 @@ struct msim_ctx {
     // Host ticks: with the index built from the state they start from (reuse_ticks ==
     // 0, slot = id), the query reads it with boxes widened by the tick's measured
     // largest displacement (the skin query); skin_pos = the new positions in that
-    // index's sorted order; disp = that displacement (device word, float bits);
-    // disp_host = page-locked words: [0] its copy, [1] the device status as the query
+    // index's sorted order; disp = device words: [0] that displacement (float bits),
+    // [1] the largest ~entity whose heading is invalid (0: none); disp_host =
+    // page-locked words: [0], [1] their copies, [2] the device status as the query
     // left it.
     bool state_free_event = false;
     uint64_t host_ticks = 0, skin_queries = 0;  // since the stats were reset
@@ -214,7 +215,8 @@ struct msim_ctx {
     float2* skin_pos = nullptr;
     uint32_t* disp = nullptr;
     uint32_t* disp_host = nullptr;
-    cudaEvent_t ev_disp = nullptr, ev_query = nullptr, ev_state_free = nullptr;
+    bool disp_zeroed = false;  // disp is zero (the last host tick zeroed it)
+    cudaEvent_t ev_query = nullptr, ev_state_free = nullptr;
     // neighbours
     // query_slot: the sorted slots of the index the last query ran on (its counts and
     // lists are in that order; a host tick's background update moves sorted_slot on)
@@ -334,7 +336,7 @@ void free_all(msim_ctx* c) {
         if (c->ev_up[k]) cudaEventDestroy(c->ev_up[k]);
         if (c->ev_moved[k]) cudaEventDestroy(c->ev_moved[k]);
     }
-    for (cudaEvent_t e : {c->ev_disp, c->ev_query, c->ev_state_free, c->ev_reuse_read[0], c->ev_reuse_read[1]})
+    for (cudaEvent_t e : {c->ev_query, c->ev_state_free, c->ev_reuse_read[0], c->ev_reuse_read[1]})
         if (e) cudaEventDestroy(e);
     status_word_give(c->status_host);
     c->status_host = nullptr;
@@ -459,14 +461,14 @@ bool ensure_skin(msim_ctx* c) {
     }
     if (!c->disp) {
         void* raw = nullptr;
-        if (!device_malloc(&raw, sizeof(uint32_t))) return false;
+        if (!device_malloc(&raw, 2 * sizeof(uint32_t))) return false;
         c->allocs.push_back(raw);
-        c->device_bytes += sizeof(uint32_t);
+        c->device_bytes += 2 * sizeof(uint32_t);
         c->disp = static_cast<uint32_t*>(raw);
     }
     if (!c->disp_host) {
         void* h = nullptr;
-        if (cudaMallocHost(&h, 2 * sizeof(uint32_t)) != cudaSuccess) {
+        if (cudaMallocHost(&h, 3 * sizeof(uint32_t)) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
@@ -573,6 +575,16 @@ void* mapped_host(const void* p) {
         return nullptr;
     }
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
+// The same for count elements that all lie in one page-locked range, aligned for the
+// kernels' loads and stores.
+template <typename T>
+T* mapped_range(const void* p, size_t count) {
+    char* first = static_cast<char*>(mapped_host(p));
+    if (!first || (reinterpret_cast<uintptr_t>(first) & (sizeof(T) - 1))) return nullptr;
+    const size_t last = count * sizeof(T) - 1;
+    return mapped_host(static_cast<const char*>(p) + last) == first + last ? reinterpret_cast<T*>(first) : nullptr;
 }
 
 // Where an export kernel writes an output: the caller's array itself when it is
@@ -736,11 +748,6 @@ int build_index(msim_ctx* c) {
 // scan's ticket and look-back words, so that the three kernels run back to back.
 int incremental_update(msim_ctx* c, bool positions = true, bool ranks = true);
 
-int clear_update_scratch(msim_ctx* c) {
-    CK(cudaMemsetAsync(c->update_scratch, 0, sizeof(uint32_t) * c->update_words, c->stream), "memset update scratch");
-    return MSIM_OK;
-}
-
 // Before a step that counts keys: the counters are zero (the last update's scan zeroed
 // them, unless it never ran or gave up).
 int begin_counts(msim_ctx* c) {
@@ -805,7 +812,7 @@ int incremental_update(msim_ctx* c, bool positions, bool ranks) {
 
 int key_start_table(msim_ctx* c);
 int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id = nullptr, const float2* pos = nullptr,
-              const TileGrid* grid = nullptr, bool pairs = false, double keep_near = 0.0);
+              const TileGrid* grid = nullptr, bool pairs = false, double keep_near = 0.0, const uint32_t* disp = nullptr);
 
 // Bound on any entity's displacement in one move tick, per coordinate, for index
 // reuse.  A move advances at most step = |speed| * |road factor| * dt toward its target
@@ -939,7 +946,7 @@ int key_start_table(msim_ctx* c) {
 // instead of the index's own (the skin query of a host tick).
 // pairs: the query keeps pair lists up to keep_near apart, or with keep_near 0 reads them.
 int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* pos, const TileGrid* grid, bool pairs,
-              double keep_near) {
+              double keep_near, const uint32_t* disp) {
     NvtxRange range("msim query");
     // The query reads only the index (key-start table, sorted slots and positions)
     // and slot ids: the next tick's move step may overwrite positions meanwhile.  With
@@ -964,7 +971,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
                         c->n, c->nbr_count, c->nbr_list, c->pairs,
                         c->pairs_b[c->pairs == c->pairs_b[0] ? 1 : 0], c->err,
                         c->slots_identity ? count_by_id : nullptr, c->dense, pairs ? c->pairs_kept : nullptr,
-                        c->pair_sizes, c->pair_ids, keep_near),
+                        c->pair_sizes, c->pair_ids, keep_near, disp, kWidenLimit * c->grid.reach),
            "k_query");
     }
     if (qs != c->stream) {
@@ -1257,7 +1264,7 @@ int msim_set_entities(msim_ctx* c, const float* pos, const uint32_t* heading, co
     if (speed) {
         CK(cudaMemcpyAsync(s.speed, speed, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream), "upload speed");
     } else {
-        CK(launch_fill(c->stream, s.speed, c->n, 1.4f), "k_fill");  // SPEED, random_move.comp:750
+        CK(launch_fill(c->stream, s.speed, c->n, kDefaultSpeed), "k_fill");
     }
     uint32_t first_bad = 0;
     CK(cudaMemcpyAsync(&first_bad, c->check, sizeof(first_bad), cudaMemcpyDeviceToHost, c->stream), "read check");
@@ -1425,7 +1432,6 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
         CK(cudaStreamCreateWithFlags(&c->up, cudaStreamNonBlocking), "cudaStreamCreate");
         CK(cudaStreamCreateWithFlags(&c->down, cudaStreamNonBlocking), "cudaStreamCreate");
         CK(cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming), "cudaEventCreate");
-        CK(cudaEventCreateWithFlags(&c->ev_disp, cudaEventDisableTiming), "cudaEventCreate");
         CK(cudaEventCreateWithFlags(&c->ev_query, cudaEventDisableTiming), "cudaEventCreate");
         CK(cudaEventCreateWithFlags(&c->ev_state_free, cudaEventDisableTiming), "cudaEventCreate");
         for (uint32_t k = 0; k < kHostChunks; k++) {
@@ -1449,11 +1455,12 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     // or set the state since), this tick's query reads that index with every box
     // widened by the tick's largest displacement d (an entity within the radius of
     // another now lay within radius + d of it when the index was built, in each
-    // coordinate).  The move measures d; the new positions are gathered into the
-    // index's order chunk by chunk behind the uploads; the index update for the new
-    // state then runs after the query, beside the downloads and the next call's
-    // uploads.  A d above kWidenLimit of the reach (host edits between ticks, large
-    // steps) takes the usual order: index update, then query.
+    // coordinate).  The move measures d, and the query reads it on the device: the host
+    // waits once, at the end.  The new positions go into the index's order chunk by
+    // chunk behind the uploads (or with the move itself, see below); the index update
+    // for the new state runs after the query, beside the downloads and the next call's
+    // uploads.  With a d above kWidenLimit of the reach (host edits between ticks, large
+    // steps) the query does nothing and runs again on the updated index.
     const bool state_free_event = c->state_free_event;
     bool skin = c->reuse && use_inc && c->reuse_ticks == 0 && c->grid.reach > 0.f && ensure_skin(c);
     c->reuse_ticks = -1;
@@ -1477,14 +1484,31 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
         }
     }
     const bool in_place = dev_head != nullptr;
-    CK(cudaMemsetAsync(c->check, 0xff, sizeof(uint32_t), c->stream), "memset check");
+    // Direct: with every array page-locked and in place the move kernel reads the state from the host
+    // itself and writes the moved positions back, and the positions also go to their
+    // places in the index by the ranks of the last update.
+    HostState host_in;
+    float2* host_pos = nullptr;
+    bool direct = skin && in_place;
+    if (direct) {
+        host_in.pos = mapped_range<float2>(in_pos, n);
+        host_in.head = mapped_range<uint32_t>(in_heading, n);
+        host_in.rng = mapped_range<uint4>(in_rng, n);
+        host_in.speed = in_speed ? mapped_range<float>(in_speed, n) : nullptr;
+        host_pos = out_pos ? mapped_range<float2>(out_pos, n) : nullptr;
+        direct = host_in.pos && host_in.head && host_in.rng && (host_in.speed || !in_speed) && (host_pos || !out_pos);
+    }
+    if (!skin) CK(cudaMemsetAsync(c->check, 0xff, sizeof(uint32_t), c->stream), "memset check");
     if (nbr && !use_inc) CK(cudaMemsetAsync(c->hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, c->stream), "memset hist");
-    if (use_inc && ((rc = clear_update_scratch(c)) != MSIM_OK || (rc = begin_counts(c)) != MSIM_OK)) return rc;
-    if (skin) CK(cudaMemsetAsync(c->disp, 0, sizeof(uint32_t), c->stream), "memset displacement");
+    if (use_inc && (rc = begin_counts(c)) != MSIM_OK) return rc;
+    if (skin && !c->disp_zeroed)
+        CK(cudaMemsetAsync(c->disp, 0, 2 * sizeof(uint32_t), c->stream), "memset displacement");
+    if (skin) c->disp_zeroed = false;
     // entity i in slot i (for later calls; this tick's query and export take the slot
     // as the id): written first, beside the first chunk's upload
-    CK(launch_iota(c->stream, s.slot_id, n), "k_iota");
-    if (state_free_event) {
+    if (!direct) CK(launch_iota(c->stream, s.slot_id, n), "k_iota");
+    if (direct) {  // no upload stream
+    } else if (state_free_event) {
         // the last read of the spare buffer was recorded before the previous call's
         // index update, which so runs beside these uploads
         CK(cudaStreamWaitEvent(c->up, c->ev_state_free, 0), "cudaStreamWaitEvent");
@@ -1497,8 +1521,31 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     // download of the moved state (down); chunk k's download overlaps chunk k+1's upload
     const uint32_t chunk = std::max<uint32_t>(kHostChunkMin, (n + kHostChunks - 1) / kHostChunks);
     uint32_t k = 0;
-    uint32_t last_lo = 0, last_cnt = 0;
-    for (uint32_t lo = 0; lo < n; lo += chunk, k++) {
+    if (direct) {
+        Prof p(c, K_STEP);
+        StepLaunch a = step_args(c, 1, true);
+        a.st = s;
+        a.key = c->key;
+        a.hist = nullptr;
+        a.key_count = c->key_count;
+        a.key_rank = c->key_rank;
+        a.zero_a = c->update_scratch;
+        a.zero_a_words = (uint32_t)c->update_words;
+        a.host_in = host_in;
+        a.host_pos = host_pos;
+        a.host_head = dev_head;
+        a.host_rng = dev_rng;
+        a.index_pos = c->st[old].pos;
+        a.disp_max = c->disp;
+        a.first_bad = c->disp + 1;
+        if (c->rank_valid) {
+            a.rank = c->rank;
+            a.rank_pos = c->skin_pos;
+            a.rank_n = n;
+        }
+        CKL(p, launch_step(c->stream, a), "k_step");
+    }
+    for (uint32_t lo = 0; lo < n && !direct; lo += chunk, k++) {
         const uint32_t cnt = std::min(chunk, n - lo);
         CK(cudaMemcpyAsync(s.head + lo, in_heading + lo, sizeof(uint32_t) * cnt, cudaMemcpyHostToDevice, c->up),
            "upload heading");
@@ -1528,6 +1575,10 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
                 a.hist = nullptr;
                 a.key_count = c->key_count;
                 a.key_rank = c->key_rank + lo;
+                if (lo == 0) {
+                    a.zero_a = c->update_scratch;
+                    a.zero_a_words = (uint32_t)c->update_words;
+                }
             }
             a.blocks = std::min<int>(c->step_blocks, (int)((cnt + kStepThreads - 1) / kStepThreads));
             a.host_head = dev_head;
@@ -1536,7 +1587,7 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
             if (skin) {  // displacement against the positions the current index was built from
                 a.index_pos = c->st[old].pos + lo;
                 a.disp_max = c->disp;
-                a.first_bad = c->check;
+                a.first_bad = c->disp + 1;
             }
             CK(launch_step(c->stream, a), "k_step");
         }
@@ -1556,37 +1607,16 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
                                    cudaMemcpyDeviceToHost, c->down),
                    "download rng");
         }
-        last_lo = lo;
-        last_cnt = cnt;
-        if (skin && lo + cnt < n) {  // the last chunk's gather runs while the host reads d
+        if (skin) {
             Prof p(c, K_GATHER);
             CK(launch_gather_chunk(c->stream, c->sorted_slot, n, lo, cnt, s.pos, c->skin_pos), "k_gather_chunk");
         }
     }
     c->cur = b;
     c->slots_identity = true;
-    TileGrid skin_grid = c->grid;
-    if (skin) {
-        CK(cudaMemcpyAsync(c->disp_host, c->disp, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
-           "read displacement");
-        CK(cudaEventRecord(c->ev_disp, c->stream), "cudaEventRecord");
-        {
-            Prof p(c, K_GATHER);
-            CK(launch_gather_chunk(c->stream, c->sorted_slot, n, last_lo, last_cnt, s.pos, c->skin_pos),
-               "k_gather_chunk");
-        }
-        CK(cudaEventSynchronize(c->ev_disp), "cudaEventSynchronize");
-        float d = 0.f;
-        std::memcpy(&d, c->disp_host, sizeof(d));
-        c->last_disp = d;
-        skin = d <= kWidenLimit * c->grid.reach;  // false for +inf (a non-finite position)
-        if (skin) {
-            // widened reach, rounded up: the displacement was measured with one rounding
-            const double r = (double)c->grid.reach + (double)d * (1.0 + 0x1p-20);
-            float rf = (float)r;
-            if ((double)rf < r) rf = std::nextafter(rf, INFINITY);
-            skin_grid.reach = rf;
-        }
+    if (direct && !c->rank_valid) {
+        Prof p(c, K_GATHER);
+        CK(launch_gather_chunk(c->stream, c->sorted_slot, n, 0, n, s.pos, c->skin_pos), "k_gather_chunk");
     }
     const bool want_idx = nbr && out_idx && c->params.cap;
     const size_t cap = c->params.cap;
@@ -1601,18 +1631,18 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     cudaStream_t dl = c->stream;
     if (nbr && skin) {
         // slots hold entity ids: the query writes the counts by id itself
-        if ((rc = run_query(c, false, d_count, c->skin_pos, &skin_grid)) != MSIM_OK) return rc;
+        if ((rc = run_query(c, false, d_count, c->skin_pos, nullptr, false, 0.0, c->disp)) != MSIM_OK) return rc;
         if (want_idx) {
             Prof p(c, K_EXPORT);
             CK(launch_export_neighbours(c->stream, c->query_slot, nullptr, c->nbr_count, c->nbr_list, n,
                                         c->params.cap, d_count, d_idx),
                "k_export_nbr");
         }
-        // the status as the query left it, before the index update below can raise one
-        CK(cudaMemcpyAsync(c->disp_host + 1, c->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
-           "read device status");
         CK(cudaEventRecord(c->ev_query, c->stream), "cudaEventRecord");
         CK(cudaStreamWaitEvent(c->down, c->ev_query, 0), "cudaStreamWaitEvent");
+        // the status as the query left it, before the index update below can raise one
+        CK(launch_host_words(c->stream, c->disp, c->err, c->disp_host), "k_host_words");
+        c->disp_zeroed = true;
         // nothing after this point reads the spare state buffer: the next call's uploads
         // may start while the index update below runs
         CK(cudaEventRecord(c->ev_state_free, c->stream), "cudaEventRecord");
@@ -1642,14 +1672,24 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
            "download neighbours");
     // the index of the new state for the next call (no sorted positions: its query
     // gathers its own); with the skin query this runs after the query, off the host's path
-    if (nbr && skin && (rc = incremental_update(c, false, false)) != MSIM_OK) return rc;
+    if (skin && (rc = incremental_update(c, false, direct && ensure_rank(c))) != MSIM_OK) return rc;
     c->tick++;
     uint32_t first_bad = 0;
     // read after the query: the heading checks of every chunk ran before it
-    CK(cudaMemcpyAsync(&first_bad, c->check, sizeof(first_bad), cudaMemcpyDeviceToHost, dl), "read check");
+    if (!skin) CK(cudaMemcpyAsync(&first_bad, c->check, sizeof(first_bad), cudaMemcpyDeviceToHost, dl), "read check");
     CK(cudaStreamSynchronize(c->down), "cudaStreamSynchronize");
-    if (!skin) CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-    const uint32_t status = skin ? c->disp_host[1] : 0u;
+    uint32_t status = 0u;
+    float d = 0.f;
+    if (skin) {
+        CK(cudaEventSynchronize(c->ev_state_free), "cudaEventSynchronize");
+        const uint32_t words[3] = {c->disp_host[0], c->disp_host[1], c->disp_host[2]};
+        std::memcpy(&d, &words[0], sizeof(d));
+        c->last_disp = d;
+        first_bad = ~words[1];
+        status = words[2];
+    } else {
+        CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+    }
     if (first_bad != 0xffffffffu) {  // as msim_set_entities: the previous state stays
         CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
         c->cur = old;
@@ -1666,6 +1706,34 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
         // a status raised before the query (e.g. by the previous call's index update):
         // reported now, after everything on the context's stream
         if (status) return sync_and_check(c);
+        if (!(d <= kWidenLimit * c->grid.reach)) {
+            // too far for the previous index (also a non-finite position): the query did
+            // nothing and runs on the new one
+            c->pairs_zeroed = false;
+            {
+                Prof p(c, K_GATHER);
+                CK(launch_gather_chunk(c->stream, c->sorted_slot, n, 0, n, s.pos, c->skin_pos), "k_gather_chunk");
+            }
+            if ((rc = run_query(c, false, d_count, c->skin_pos)) != MSIM_OK) return rc;
+            if (want_idx) {
+                Prof p(c, K_EXPORT);
+                CK(launch_export_neighbours(c->stream, c->query_slot, nullptr, c->nbr_count, c->nbr_list, n,
+                                            c->params.cap, d_count, d_idx),
+                   "k_export_nbr");
+            }
+            if (out_count)
+                CK(cudaMemcpyAsync(out_count, d_count, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream),
+                   "download counts");
+            if (want_idx)
+                CK(cudaMemcpyAsync(out_idx, d_idx, sizeof(uint32_t) * n * cap, cudaMemcpyDeviceToHost, c->stream),
+                   "download neighbours");
+            rc = sync_and_check(c);
+            if (rc == MSIM_OK) {
+                c->reuse_ticks = 0;
+                c->host_ticks++;
+            }
+            return rc;
+        }
         c->reuse_ticks = 0;
         c->state_free_event = true;
         c->host_ticks++;

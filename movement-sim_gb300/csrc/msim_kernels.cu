@@ -221,7 +221,17 @@ __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch
 // in flight before any is stepped.  One per thread at four 512-thread blocks per SM
 // (32 registers): 0.122 ms at 16 M against 0.125 for two per thread at three blocks.
 // DISP: the tick's largest displacement is measured too (StepLaunch::disp_max).
-template <int RNG, bool KEY, bool DISP>
+//
+// HOST: the state comes from the caller's page-locked arrays and the results go back to
+// them from the same kernel: the link is busy both ways from the first block to the
+// last, where copies in four chunks of four arrays left 1.5 to 2 us idle between any two
+// of them and put the last chunk's move and gather behind the last copy.  Bound by the
+// link: 1 M entities, 32 MB up and 8 MB down in 165 us (194 GB/s up of the 211 a copy
+// alone reaches).  The writes to the index by rank, to the state arrays and the key
+// counts hide behind it.  A whole host tick with counts, chunked copies / this kernel:
+// 20,000 entities 91 / 54 us, 300,000 193 / 122, 1 M 348 / 255, 4 M 1011 / 857, 16 M
+// 3646 / 3361, so no size keeps the copies when the arrays allow it.
+template <int RNG, bool KEY, bool DISP, bool HOST>
 __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
     __shared__ uint32_t s_hist[kMaxPasses * kRadix];
     __shared__ uint32_t s_morton[KEY ? 2048 : 1];
@@ -243,6 +253,7 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
         float2 p[kStepPer];
         uint32_t h[kStepPer], h0[kStepPer];
         float sp[kStepPer];
+        uint4 host_rng[kStepPer];
 #pragma unroll
         for (int u = 0; u < kStepPer; u++) {
             sl[u] = base + u * stride + threadIdx.x;
@@ -250,15 +261,22 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
             p[u] = make_float2(0.f, 0.f);
             h[u] = h0[u] = 0u;
             sp[u] = 0.f;
-            if (valid[u]) {
+            if (HOST && valid[u]) {  // four loads in flight, each byte once over the link
+                h[u] = h0[u] = __ldcs(a.host_in.head + sl[u]);
+                p[u] = __ldcs(a.host_in.pos + sl[u]);
+                host_rng[u] = __ldcs(a.host_in.rng + sl[u]);
+                sp[u] = a.host_in.speed ? __ldcs(a.host_in.speed + sl[u]) : kDefaultSpeed;
+                a.st.slot_id[sl[u]] = a.id_base + sl[u];
+                a.st.speed[sl[u]] = sp[u];
+            } else if (valid[u]) {
                 p[u] = a.st.pos[sl[u]];
                 if (a.ticks) {
                     h[u] = h0[u] = a.st.head[sl[u]];
                     sp[u] = a.st.speed[sl[u]];
-                    if (DISP && a.first_bad && (h[u] & kHeadRoad) >= a.map.num_roads)
-                        atomicMin(a.first_bad, a.id_base + sl[u]);
                 }
             }
+            if (DISP && a.first_bad && valid[u] && (h[u] & kHeadRoad) >= a.map.num_roads)
+                atomicMax(a.first_bad, ~(a.id_base + sl[u]));
         }
         uint32_t key[kStepPer];
 #pragma unroll
@@ -268,16 +286,20 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
             if (a.ticks) {
                 uint4 r = make_uint4(0u, 0u, 0u, 0u);
                 bool rd = false;
-                step_entity<RNG, 1, false>(a.map, a.dt, sp[u], 1u, p[u], h[u], r, rd, a.st.rng + sl[u], a.err);
+                step_entity<RNG, 1, false>(a.map, a.dt, sp[u], 1u, p[u], h[u], r, rd,
+                                           HOST ? &host_rng[u] : a.st.rng + sl[u], a.err);
                 a.st.pos[sl[u]] = p[u];
-                if (h[u] != h0[u]) {
-                    a.st.head[sl[u]] = h[u];
-                    if (a.host_head) a.host_head[a.id_base + sl[u]] = h[u];  // the caller's copy, by id
+                if (HOST) {
+                    if (a.host_pos) __stcs(a.host_pos + sl[u], p[u]);
+                    if (a.rank_pos) {
+                        const uint32_t k = a.rank[sl[u]];
+                        if (k < a.rank_n) a.rank_pos[k] = p[u];
+                    }
                 }
-                if (rd) {
-                    a.st.rng[sl[u]] = r;
-                    if (a.host_rng) a.host_rng[a.id_base + sl[u]] = r;
-                }
+                if (HOST || h[u] != h0[u]) a.st.head[sl[u]] = h[u];
+                if (h[u] != h0[u] && a.host_head) a.host_head[a.id_base + sl[u]] = h[u];  // the caller's copy, by id
+                if (HOST || rd) a.st.rng[sl[u]] = HOST && !rd ? host_rng[u] : r;
+                if (rd && a.host_rng) a.host_rng[a.id_base + sl[u]] = r;
             }
             if (KEY) {
                 key[u] = tile_key(a.grid, p[u], s_morton);
@@ -765,6 +787,15 @@ __global__ __launch_bounds__(256) void k_gather_chunk(const uint32_t* __restrict
     }
 }
 
+// The words a host tick reads back (displacement, invalid heading, status), written to
+// page-locked memory by the device (three copies would queue behind the downloads), and
+// the first two zeroed for the next tick.
+__global__ void k_host_words(uint32_t* disp, const uint32_t* err, uint32_t* out) {
+    if (threadIdx.x >= 3u) return;
+    out[threadIdx.x] = threadIdx.x < 2u ? disp[threadIdx.x] : *err;
+    if (threadIdx.x < 2u) disp[threadIdx.x] = 0u;
+}
+
 __device__ __forceinline__ uint32_t abs_bits(float v) {  // |v| as ordered bits; NaN / inf: +inf
     const float a = fabsf(v);
     return a <= 3.0e38f ? __float_as_uint(a) : 0x7f800000u;
@@ -836,7 +867,7 @@ cudaError_t configure_kernels(uint32_t) { return cudaSuccess; }
 int step_blocks_for(int device, uint32_t n) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step<0, true, false>, kStepThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step<0, true, false, false>, kStepThreads, 0);
     if (sms <= 0) sms = 1;
     if (per_sm <= 0) per_sm = 1;
     long long want = (long long)sms * per_sm;
@@ -857,7 +888,8 @@ cudaError_t launch_init_entities(cudaStream_t s, const DeviceMap& m, EntityState
 cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
     if (a.n == 0) return cudaSuccess;
     const bool key = a.key != nullptr;
-    if (a.rank_pos && (key || a.ticks != 1 || !a.rank)) return cudaErrorInvalidValue;
+    if (a.rank_pos && ((key && !a.host_in.pos) || a.ticks != 1 || !a.rank)) return cudaErrorInvalidValue;
+    if (a.host_in.pos && !a.disp_max) return cudaErrorInvalidValue;
     if (!key && a.ticks > 0 && !a.host_head && !a.host_rng) {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
@@ -880,15 +912,20 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
     if (a.ticks > 1) return cudaErrorInvalidValue;  // k_step moves one tick at most
     if (a.disp_max) {  // a host tick that queries the previous index (keys, one tick)
         if (!key || !a.index_pos || a.ticks != 1) return cudaErrorInvalidValue;
-        return a.rng_kind == 1 ? launch_chained(k_step<1, true, true>, a.blocks, kStepThreads, s, a)
-                               : launch_chained(k_step<0, true, true>, a.blocks, kStepThreads, s, a);
+        if (a.host_in.pos) {
+            const unsigned blocks = blocks_for(a.n, kStepThreads);
+            return a.rng_kind == 1 ? launch_chained(k_step<1, true, true, true>, blocks, kStepThreads, s, a)
+                                   : launch_chained(k_step<0, true, true, true>, blocks, kStepThreads, s, a);
+        }
+        return a.rng_kind == 1 ? launch_chained(k_step<1, true, true, false>, a.blocks, kStepThreads, s, a)
+                               : launch_chained(k_step<0, true, true, false>, a.blocks, kStepThreads, s, a);
     }
     if (a.rng_kind == 1) {
-        return key ? launch_chained(k_step<1, true, false>, a.blocks, kStepThreads, s, a)
-                   : launch_chained(k_step<1, false, false>, a.blocks, kStepThreads, s, a);
+        return key ? launch_chained(k_step<1, true, false, false>, a.blocks, kStepThreads, s, a)
+                   : launch_chained(k_step<1, false, false, false>, a.blocks, kStepThreads, s, a);
     } else {
-        return key ? launch_chained(k_step<0, true, false>, a.blocks, kStepThreads, s, a)
-                   : launch_chained(k_step<0, false, false>, a.blocks, kStepThreads, s, a);
+        return key ? launch_chained(k_step<0, true, false, false>, a.blocks, kStepThreads, s, a)
+                   : launch_chained(k_step<0, false, false, false>, a.blocks, kStepThreads, s, a);
     }
     return cudaGetLastError();
 }
@@ -976,31 +1013,34 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
                          uint32_t* list, unsigned long long* pair_bins, unsigned long long* next_bins, const uint32_t* err,
                          uint32_t* count_by_id,
-                         bool dense, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near) {
+                         bool dense, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near,
+                         const uint32_t* disp, float widen_limit) {
     if (n == 0) return cudaSuccess;
     using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
                            uint32_t*, uint32_t*, unsigned long long*, unsigned long long*, const uint32_t*, uint32_t*,
                            PairStore);
 #define QUERY_KERNELS(LIST, KEEP, DENSE)                                                               \
     {k_query<LIST, KEEP, DENSE, kPairsFound>, k_query<LIST, KEEP, DENSE, kPairsKept>, \
-     k_query<LIST, KEEP, DENSE, kPairsUsed>}
-    static const Query kernels[2][2][3] = {
+     k_query<LIST, KEEP, DENSE, kPairsUsed>, k_query<LIST, KEEP, DENSE, kPairsWidened>}
+    static const Query kernels[2][2][4] = {
         {QUERY_KERNELS(false, kQueryKeep, false), QUERY_KERNELS(false, kQueryKeepDense, true)},
         {QUERY_KERNELS(true, kQueryKeep, false), QUERY_KERNELS(true, kQueryKeepDense, true)}};
 #undef QUERY_KERNELS
     static bool carveout = false;  // 16 blocks of ~11.5 KB per SM (dense: 9 of ~23.5 KB)
     if (!carveout) {
-        for (int i = 0; i < 12; i++)
-            cudaFuncSetAttribute(kernels[i / 6][i / 3 % 2][i % 3], cudaFuncAttributePreferredSharedMemoryCarveout,
+        for (int i = 0; i < 16; i++)
+            cudaFuncSetAttribute(kernels[i / 8][i / 4 % 2][i % 4], cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
         cudaGetLastError();
         carveout = true;
     }
     if (pairs && (!pair_sizes || !pair_ids || n > kPairMaxEntities)) return cudaErrorInvalidValue;
     const bool lists = cap > 0 && list;
-    const PairLists use = !pairs ? kPairsFound : keep_near > 0.0 ? kPairsKept : kPairsUsed;
+    if (pairs && disp) return cudaErrorInvalidValue;
+    const PairLists use = disp ? kPairsWidened : !pairs ? kPairsFound : keep_near > 0.0 ? kPairsKept : kPairsUsed;
     // the squared distance's rounding and its operands' stay far below 2^-18 of it
-    const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18))};
+    const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18)),
+                          disp, widen_limit};
     kernels[lists][dense][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
         kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins,
         next_bins, err, count_by_id, store);
@@ -1057,6 +1097,11 @@ cudaError_t launch_gather_chunk(cudaStream_t s, const uint32_t* P, uint32_t n, u
     const unsigned want = 8u * (unsigned)std::max(sms, 1);
     const unsigned blocks = std::min<unsigned>(want, blocks_for(n, 256u * kGatherPer));
     k_gather_chunk<<<blocks, 256, 0, s>>>(P, n, lo, cnt, pos, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out) {
+    k_host_words<<<1, 32, 0, s>>>(disp, err, out);
     return cudaGetLastError();
 }
 

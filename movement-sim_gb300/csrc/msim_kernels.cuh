@@ -18,6 +18,7 @@ constexpr int kMaxPasses = 3;                               // keys up to 24 bit
 constexpr int kQueryThreads = 128;
 constexpr int kStepThreads = 512;  // measured at 16 M: 0.122 ms per tick against 0.136 with 256
 constexpr int kStepPer = 1;        // entities per thread and iteration of k_step
+constexpr float kDefaultSpeed = 1.4f;  // SPEED, random_move.comp:750
 constexpr int kMoveThreads = 128;  // move-only multi-tick launches (k_move)
 constexpr uint32_t kMaxCap = 256;
 constexpr int kQueryKeep = 8;        // neighbours the query keeps per entity (more are collected again)
@@ -31,6 +32,14 @@ struct EntityState {
     uint4* rng;
     float* speed;
     uint32_t* slot_id;  // entity id held by each slot
+};
+
+// The caller's entity state in page-locked host memory, as the device addresses it.
+struct HostState {
+    const float2* pos = nullptr;  // nullptr: the state is on the device
+    const uint32_t* head = nullptr;
+    const uint4* rng = nullptr;
+    const float* speed = nullptr;
 };
 
 struct StepLaunch {
@@ -67,11 +76,16 @@ struct StepLaunch {
     const float2* index_pos = nullptr;
     uint32_t* disp_max = nullptr;
     // With disp_max: the first entity (id_base + slot) whose heading names a road out of
-    // range is atomically min-ed into *first_bad (NULL: not checked here).
+    // range, as the maximum of ~entity (0: none; NULL: not checked here).
     uint32_t* first_bad = nullptr;
-    // One move tick (move-only kernel): each moved position is also written to
-    // rank_pos[rank[slot]] (its place in a sorted order of rank_n entries; larger ranks
-    // are skipped).
+    // With disp_max: the state is read from the caller's page-locked arrays through their
+    // device mapping (by slot = entity id; speed NULL: all kDefaultSpeed) and every array
+    // of st is written, slot_id too; host_pos receives the moved positions.
+    HostState host_in;
+    float2* host_pos = nullptr;
+    // One move tick (move-only kernel, or with host_in): each moved position is also
+    // written to rank_pos[rank[slot]] (its place in a sorted order of rank_n entries;
+    // larger ranks are skipped).
     const uint32_t* rank = nullptr;
     float2* rank_pos = nullptr;
     uint32_t rank_n = 0;
@@ -126,7 +140,10 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // (pairs up to that distance), else read back (the ids then serve as
                          // sorted_slot, slot_id NULL); NULL: not used
                          uint32_t* pairs = nullptr, uint32_t* pair_sizes = nullptr, uint32_t* pair_ids = nullptr,
-                         double keep_near = 0.0);
+                         double keep_near = 0.0,
+                         // boxes widened by the displacement d = *disp (float bits); the query does
+                         // nothing when d exceeds widen_limit or is not finite
+                         const uint32_t* disp = nullptr, float widen_limit = 0.f);
 constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
 size_t query_pair_places(uint32_t n, bool dense);   // pairs of all lists
 size_t query_pair_sizes(uint32_t n);
@@ -148,6 +165,8 @@ cudaError_t launch_gather_chunk(cudaStream_t s, const uint32_t* P, uint32_t n, u
 // out[0] = largest |speed|, out[1] = largest |x| or |y| of the n entities, as float
 // bits (atomically maxed: out must hold zeros; NaN or infinite values count as +inf).
 cudaError_t launch_bounds(cudaStream_t s, const float* speed, const float2* pos, uint32_t n, uint32_t* out);
+// out[0..2] = disp[0], disp[1], *err (out: page-locked host memory); disp[0] = disp[1] = 0
+cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out);
 cudaError_t launch_iota(cudaStream_t s, uint32_t* out, uint32_t n);
 // *first_bad = first i with (head[i] & road mask) >= num_roads, or 0xffffffff
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,

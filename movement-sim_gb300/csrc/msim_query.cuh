@@ -295,7 +295,8 @@ constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 constexpr uint32_t kPairOwnerShift = 27;
 constexpr uint32_t kPairPosition = (1u << kPairOwnerShift) - 1u;
 constexpr uint32_t kNoPairs = 0xffffffffu;
-enum PairLists : int { kPairsFound, kPairsKept, kPairsUsed };  // looked up; looked up and kept; read back
+// looked up; looked up and kept; read back; looked up in boxes widened by *PairStore::disp
+enum PairLists : int { kPairsFound, kPairsKept, kPairsUsed, kPairsWidened };
 
 // Places per warp: about twice what the workloads keep (sparse 1 M and 16 M populations
 // 45 of 128; a crowd with 15 neighbours 500 of 1,024).
@@ -306,6 +307,8 @@ struct PairStore {
     uint32_t* sizes;
     uint32_t* ids;
     float near2;  // pairs up to this squared distance are kept
+    const uint32_t* disp;  // kPairsWidened: the tick's largest displacement d (float bits)
+    float widen_limit;     // and the d up to which the query runs
 };
 
 template <int KEEP>
@@ -557,6 +560,13 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     }
     if (valid) me = sorted_pos[p];
     if (status & kErrTimeout) return;  // an index update gave up (index_failed)
+    if (PAIRS == kPairsWidened) {
+        // an entity within the radius now lay within reach + d when the index was built;
+        // a d past the limit (or not finite) leaves the query to the host
+        const float d = __uint_as_float(*store.disp);
+        if (!(d <= store.widen_limit)) return;
+        g.reach = __fadd_ru(g.reach, __fmul_ru(d, 1.0f + 0x1p-20f));  // d was measured with one rounding
+    }
     sh.me[tid] = me;
     sh.cnt[tid] = 0u;
     uint32_t own = 0u, near_count = 0u;
