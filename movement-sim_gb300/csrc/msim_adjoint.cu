@@ -68,7 +68,8 @@ struct AdjArgs {
 
 // Threads of a block of the forward and backward kernels, and blocks per SM.  Both are
 // bound by issue.  Forward: one warp a block, so that a slow warp keeps no finished one's
-// place (262,144 entities 1.68 ms; 128 threads 1.80).  Backward: the history (800 B per
+// place (262,144 entities 1.68 ms; 128 threads 1.80; before the paired instructions, as
+// the figures that follow).  Backward: the history (800 B per
 // entity at K = 100) of the resident threads then mostly stays in the L2 it is read back
 // from (7 blocks of 128 threads 2.63 ms; 6 3.01, 8 at fewer registers 2.96, 24 of 32 2.94).
 constexpr uint32_t kAdjForwardThreads = 32;
@@ -98,7 +99,6 @@ __device__ __forceinline__ int fixed_coord(float u, uint32_t fbits) {
     u = fminf(fmaxf(u, -lim), lim);                                  // off-grid positions stay off-grid
     return __float2int_rd(__fmul_rn(u, __int_as_float((127 + (int)fbits) << 23)));
 }
-__device__ __forceinline__ float cell_coord(float x, float inv_c) { return __fsub_rn(__fmul_rn(x, inv_c), 0.5f); }
 __device__ __forceinline__ Splat splat_of(float ux, float uy, uint32_t fbits) {
     const int U = fixed_coord(ux, fbits);
     const int V = fixed_coord(uy, fbits);
@@ -116,14 +116,20 @@ __device__ __forceinline__ Splat splat_of(float ux, float uy, uint32_t fbits) {
 // adding 2^(23 - fbits) towards zero leaves the fraction's first fbits bits as the low
 // bits of the sum.  An entity stays about a hundred ticks in a cell.
 struct CellFrame {
-    float fi, fj;
-    float one;  // 2^(23 - fbits)
+    float2 back;  // (-fi, -fj); NaN: no cell
+    float one;    // 2^(23 - fbits)
 };
-__device__ __forceinline__ bool in_cell(const CellFrame& c, float ux, float uy, float& wx, float& wy) {
-    const float dx = __fadd_rz(ux, -c.fi), dy = __fadd_rz(uy, -c.fj);
-    wx = __fadd_rz(dx, c.one);
-    wy = __fadd_rz(dy, c.one);
-    return max(__float_as_uint(dx), __float_as_uint(dy)) < 0x3f800000u;
+__device__ __forceinline__ float2 add2_rz(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rz.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 cell_coords(float2 p, float2 inv_c) { return plus(both(-0.5f), mul2(p, inv_c)); }
+__device__ __forceinline__ bool in_cell(const CellFrame& c, float2 u, float2& w) {
+    const float2 d = add2_rz(u, c.back);
+    w = add2_rz(d, both(c.one));
+    return max(__float_as_uint(d.x), __float_as_uint(d.y)) < 0x3f800000u;
 }
 __device__ __forceinline__ float frame_one(uint32_t fbits) { return __int_as_float((150 - (int)fbits) << 23); }
 
@@ -170,9 +176,10 @@ __device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
 // REPLAY: the stored event schedule is forced; else events come from the step and the
 // schedule is stored.  Ticks run in stretches of at most 32 that end where a schedule
 // word or a checkpoint does, so a tick itself is the step, the cell test and three
-// sums (32-bit within a stretch).  Bound by issue (82 % active): 118 warp instructions
+// sums (32-bit within a stretch).  Bound by issue (83 % active): 105 warp instructions
 // per tick against 190 with the road reloaded, two conversions and a flush at every
-// cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.68 ms.
+// cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.68 ms, with the coordinates in
+// paired instructions 1.59.
 template <int RNG, bool REPLAY>
 __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
     __shared__ LeftBlocks left;
@@ -190,7 +197,7 @@ __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_f
         leg_load<true>(a.map, a.dt, s, h, l, a.err);
     }
     const uint32_t low = (1u << a.fbits) - 1u;
-    CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};  // NaN: in no cell yet
+    CellFrame c{both(__int_as_float(0x7fc00000)), frame_one(a.fbits)};  // in no cell yet
     int bi = INT32_MIN, bj = INT32_MIN;
     BlockSums acc{0u, 0ull, 0ull, 0ull};
     size_t ck = e;
@@ -215,14 +222,14 @@ __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_f
                                                 [&]() { return rng_next<RNG>(r); });
             if (REPLAY) bits >>= 1;
             else if (snapped) bits |= 1u << (first + k);
-            const float ux = cell_coord(p.x, a.inv_cw), uy = cell_coord(p.y, a.inv_ch);
-            float wx, wy;
-            const bool stays = in_cell(c, ux, uy, wx, wy);
-            uint32_t fx = __float_as_uint(wx) & low, fy = __float_as_uint(wy) & low;
+            const float2 u = cell_coords(p, make_float2(a.inv_cw, a.inv_ch));
+            float2 w;
+            const bool stays = in_cell(c, u, w);
+            uint32_t fx = __float_as_uint(w.x) & low, fy = __float_as_uint(w.y) & low;
             bool leaves = false;
             Splat sp{};
             if (!stays) {
-                sp = splat_of(ux, uy, a.fbits);
+                sp = splat_of(u.x, u.y, a.fbits);
                 fx = sp.fx;
                 fy = sp.fy;
                 leaves = sp.i0 != bi || sp.j0 != bj;
@@ -240,8 +247,7 @@ __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_f
                 }
                 bi = sp.i0;
                 bj = sp.j0;
-                c.fi = (float)bi;
-                c.fj = (float)bj;
+                c.back = make_float2(-(float)bi, -(float)bj);
                 acc = BlockSums{0u, 0ull, 0ull, 0ull};
                 sx = sy = 0u;
                 began = k;
@@ -356,7 +362,8 @@ __device__ __noinline__ SplatGrad splat_grad(const float* lambda, uint32_t gw, u
 // road end or a cell change, the leg's gradient parts are summed before they are scaled,
 // headings are kept only for road ends (12 -> 8 B of history per tick), ticks run in
 // stretches of one schedule word, and all segments run in one launch, which a launch per
-// segment rounded up to two waves each.
+// segment rounded up to two waves each.  262,144 entities x 2,000 ticks 5.06 -> 2.63 ms,
+// with the coordinates in paired instructions 2.52.
 template <int RNG>
 __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backward(AdjBack b) {
     const AdjArgs& a = b.f;
@@ -373,7 +380,7 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
     float2 adj = make_float2(0.f, 0.f);
     double gspeed = 0.0;
     uint32_t records = 0;
-    CellFrame c{__int_as_float(0x7fc00000), 0.f, frame_one(a.fbits)};
+    CellFrame c{both(__int_as_float(0x7fc00000)), frame_one(a.fbits)};
     SplatGrad sg{};
     for (uint32_t seg = b.segments; seg-- > 0;) {
         const uint32_t t0 = seg * a.K, t1 = t0 + min(a.K, a.ticks - t0);  // ticks t0 + 1 .. t1
@@ -396,10 +403,8 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
 #pragma unroll 4
             for (uint32_t k = 0; k < len; k++) {
                 if ((int)bits >= 0) {
-                    const float dx = l.tx - p.x, dy = l.ty - p.y;
-                    const float q = inv_length(dx * dx + dy * dy) * l.step;
-                    p.x += dx * q;
-                    p.y += dy * q;
+                    const float2 d = sub2(make_float2(l.tx, l.ty), p), dd = mul2(d, d);
+                    p = plus(p, mul2(d, both(inv_length(dd.x + dd.y) * l.step)));
                 } else {
                     p.x = l.tx;
                     p.y = l.ty;
@@ -461,34 +466,27 @@ __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backwar
                 if (left >= kAhead) at -= n;  // else the checkpoint again, not used
                 ahead[kAhead - 1u] = *at;
                 {  // + (1/T) d splat(p_t)/dp . lambda
-                    const float ux = cell_coord(p.x, a.inv_cw), uy = cell_coord(p.y, a.inv_ch);
-                    float wx, wy;
-                    float fx, fy;
-                    if (in_cell(c, ux, uy, wx, wy)) {
-                        fx = wx - c.one;  // exact: fbits bits
-                        fy = wy - c.one;
+                    const float2 u = cell_coords(p, make_float2(a.inv_cw, a.inv_ch));
+                    float2 w, fr;  // fr: the cell fractions
+                    if (in_cell(c, u, w)) {
+                        fr = add2(w, both(-c.one));  // exact: fbits bits
                     } else {
-                        const Splat sp = splat_of(ux, uy, a.fbits);
+                        const Splat sp = splat_of(u.x, u.y, a.fbits);
                         sg = splat_grad(b.lambda, a.gw, a.gh, sp.i0, sp.j0, sx, sy);
-                        fx = (float)sp.fx * scale;  // exact: fewer than 24 bits
-                        fy = (float)sp.fy * scale;
-                        c.fi = (float)sp.i0;
-                        c.fj = (float)sp.j0;
+                        fr = make_float2((float)sp.fx * scale, (float)sp.fy * scale);  // exact: fewer than 24 bits
+                        c.back = make_float2(-(float)sp.i0, -(float)sp.j0);
                     }
-                    adj.x += __fmaf_rn(fy, sg.x1, sg.x0);
-                    adj.y += __fmaf_rn(fx, sg.y1, sg.y0);
+                    adj = add2(adj, make_float2(__fmaf_rn(fr.y, sg.x1, sg.x0), __fmaf_rn(fr.x, sg.y1, sg.y0)));
                 }
                 if ((int)bits >= 0) {
-                    const float dx = l.tx - pp.x, dy = l.ty - pp.y;
-                    const float d2 = __fmaf_rn(dx, dx, dy * dy);
+                    const float2 d = sub2(make_float2(l.tx, l.ty), pp);
+                    const float d2 = __fmaf_rn(d.x, d.x, d.y * d.y);
                     const float inv = inv_length(d2);
-                    const float g = __fmaf_rn(dx, adj.x, dy * adj.y) * inv;  // n . adj
+                    const float g = __fmaf_rn(d.x, adj.x, d.y * adj.y) * inv;  // n . adj
                     part += g;
                     any = any || d2 > 0.f;
-                    const float gi = g * inv, q = l.step * inv;
-                    const float cx = __fmaf_rn(-dx, gi, adj.x), cy = __fmaf_rn(-dy, gi, adj.y);  // adj - n g
-                    adj.x = __fmaf_rn(-q, cx, adj.x);
-                    adj.y = __fmaf_rn(-q, cy, adj.y);
+                    const float2 across = fma2(d, both(g * -inv), adj);  // adj - n g
+                    adj = fma2(across, both(l.step * -inv), adj);
                 } else {
                     end_leg();
                     adj = make_float2(0.f, 0.f);

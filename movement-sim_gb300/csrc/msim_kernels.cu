@@ -187,20 +187,22 @@ __device__ __forceinline__ uint32_t key_rank(uint32_t key, bool valid, uint32_t 
 // still spreads over many SMs.  ONE: a single tick (the tick that reuses the index
 // places its positions too); else several ticks with the state and the road's leg in
 // registers between them, bound by the ticks' serial chain (small counts) or by issue:
-// with read-back, 10,000 entities for 1,000 ticks 316 -> 216 us and 1 M for 200 ticks
-// 867 -> 581 us against reloading the road and three intrinsics every tick.
+// with read-back, 10,000 entities for 1,000 ticks 316 -> 123 us and 1 M for 200 ticks
+// 865 -> 470 us against reloading the road and three intrinsics every tick.  A run's
+// blocks take one entity per thread and no more (the scheduler fills places as they come
+// free; a grid of 16 blocks per SM with 12 resident left its last blocks to run alone: 1 M
+// x 200 ticks 312 us, so 287, with the coordinates in paired instructions 268).
 template <int RNG, bool ONE, bool AHEAD>
-__global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch a) {
+__global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 10) void k_move(StepLaunch a) {
     chain_enter();
     const uint32_t thread = blockIdx.x * kMoveThreads + threadIdx.x;
-    uint32_t s = thread, stride = gridDim.x * kMoveThreads;
+    uint32_t s = thread;
     if (!ONE) {  // a.lanes entities to a warp
         const uint32_t lane = thread & 31u;
         if (lane >= a.lanes) return;
         s = (thread >> 5) * a.lanes + lane;
-        stride = (stride >> 5) * a.lanes;
     }
-    for (; s < a.n; s += stride) {
+    for (; s < a.n; s += gridDim.x * kMoveThreads) {
         float2 p = a.st.pos[s];
         uint32_t h = a.st.head[s];
         const uint32_t h0 = h;
@@ -214,6 +216,7 @@ __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 12) void k_move(StepLaunch
         if (h != h0) a.st.head[s] = h;
         if (rd) a.st.rng[s] = r;
         if (ONE && a.rank_pos && q < a.rank_n) a.rank_pos[q] = p;  // a tick that reuses the index
+        if (!ONE) break;
     }
 }
 
@@ -898,7 +901,7 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
         if (a.ticks > 1) {
             StepLaunch b = a;
             b.lanes = warp_lanes(a.n, sms);
-            const unsigned blocks = std::min(most, blocks_for(blocks_for(a.n, b.lanes) * 32u, kMoveThreads));
+            const unsigned blocks = blocks_for(blocks_for(a.n, b.lanes) * 32u, kMoveThreads);
             if (a.ticks < kAheadTicks)
                 return a.rng_kind == 1 ? launch_chained(k_move<1, false, false>, blocks, kMoveThreads, s, b)
                                        : launch_chained(k_move<0, false, false>, blocks, kMoveThreads, s, b);

@@ -19,7 +19,7 @@ constexpr int kQueryThreads = 128;
 constexpr int kStepThreads = 512;  // measured at 16 M: 0.122 ms per tick against 0.136 with 256
 constexpr int kStepPer = 1;        // entities per thread and iteration of k_step
 constexpr float kDefaultSpeed = 1.4f;  // SPEED, random_move.comp:750
-constexpr int kMoveThreads = 128;  // move-only multi-tick launches (k_move)
+constexpr int kMoveThreads = 128;  // move-only launches (k_move)
 constexpr uint32_t kMaxCap = 256;
 constexpr int kQueryKeep = 8;        // neighbours the query keeps per entity (more are collected again)
 constexpr int kQueryKeepDense = 32;  // the same in its kernel for dense populations
