@@ -231,7 +231,7 @@ struct msim_ctx {
     uint32_t* status_host = nullptr;  // page-locked copy of *err, written behind the work it describes
     uint32_t* check = nullptr;  // first invalid heading found by msim_set_entities
     TileGrid grid{};
-    bool dense = false;  // many neighbours expected (see msim_create): the query's dense kernel
+    uint32_t density = 0;  // how many neighbours are expected (see msim_create): the query's kernel
     uint32_t passes = 1;
     uint32_t resort = 16;
     uint32_t since_permute = 0;
@@ -434,6 +434,11 @@ constexpr float kWidenLimit = 1.0f;
 // Measured at 1 M entities, sparse / dense kernel: 0.68 33.1 / 37.6 us, 1.02 40.0 / 40.5,
 // 1.36 46.5 / 45.5, 2.0 55.1 / 52.5, 2.7 81.3 / 63.2, 3.4 170 / 104.
 constexpr double kDenseNeighbours = 1.2;
+// And above which its kernel for crowds is: 48 neighbours kept per entity in 7 blocks per SM
+// instead of 32 in 9.  32 / 48, us per tick at 200,000 entities: 5.4 expected (7.2
+// neighbours) 28.4 / 29.6, 7.6 (10.4) 41.0 / 35.6, 10.8 (15.5) 78.5 / 49.9, 15.2 (22.9) 119.6 /
+// 84.8; at 1 M 3.4 (4.8) 60.6 / 71.1, 8.6 (12.3) 155 / 162, 13.8 (21.4) 335 / 301.
+constexpr double kCrowdNeighbours = 6.5;
 
 // rank[slot] (written by every later merge once allocated): false when the allocation
 // fails.
@@ -502,7 +507,7 @@ bool ensure_reuse(msim_ctx* c) {
 // their candidates up).
 bool ensure_pairs(msim_ctx* c) {
     if (c->pairs_kept && c->pair_sizes && c->pair_ids) return true;
-    const size_t bytes[3] = {sizeof(uint32_t) * query_pair_places(c->n, c->dense),
+    const size_t bytes[3] = {sizeof(uint32_t) * query_pair_places(c->n, c->density),
                              sizeof(uint32_t) * query_pair_sizes(c->n), sizeof(uint32_t) * c->n};
     void* at[3] = {c->pairs_kept, c->pair_sizes, c->pair_ids};
     bool all = true;
@@ -535,7 +540,7 @@ int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
         return 0;
     const double per_reach = (double)c->grid.reach / c->step_bound;
     const int64_t left = (int64_t)std::min(std::floor((double)kWidenLimit * per_reach), 1e9) - since;
-    const int64_t best = (int64_t)std::min(std::sqrt(0.5 * (c->dense ? kPairCostDense : kPairCost) * per_reach), 1e9);
+    const int64_t best = (int64_t)std::min(std::sqrt(0.5 * (c->density ? kPairCostDense : kPairCost) * per_reach), 1e9);
     const int64_t ticks = std::min(left, std::max(best, kFewest));
     return ticks >= kFewest ? ticks : 0;
 }
@@ -970,7 +975,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
                         c->slots_identity || read_pairs ? nullptr : cur_state(c).slot_id, grid ? *grid : c->grid,
                         c->n, c->nbr_count, c->nbr_list, c->pairs,
                         c->pairs_b[c->pairs == c->pairs_b[0] ? 1 : 0], c->err,
-                        c->slots_identity ? count_by_id : nullptr, c->dense, pairs ? c->pairs_kept : nullptr,
+                        c->slots_identity ? count_by_id : nullptr, c->density, pairs ? c->pairs_kept : nullptr,
                         c->pair_sizes, c->pair_ids, keep_near, disp, kWidenLimit * c->grid.reach),
            "k_query");
     }
@@ -1132,7 +1137,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
         const double dx = (double)q[2] - (double)q[0], dy = (double)q[3] - (double)q[1];
         road_length += std::sqrt(dx * dx + dy * dy) * (double)every;
     }
-    c->dense = 2.0 * radius * (double)c->n > kDenseNeighbours * road_length;
+    const double along = 2.0 * radius * (double)c->n;
+    c->density = along > kCrowdNeighbours * road_length ? 2u : along > kDenseNeighbours * road_length ? 1u : 0u;
     // y bands inside a tile fill the key up to 24 bits (3 radix passes), at most 64
     // bands, and keep the key-start table within about four entries per entity
     uint32_t nbits = 0;

@@ -1016,42 +1016,45 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
                          uint32_t* list, unsigned long long* pair_bins, unsigned long long* next_bins, const uint32_t* err,
                          uint32_t* count_by_id,
-                         bool dense, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near,
+                         uint32_t density, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near,
                          const uint32_t* disp, float widen_limit) {
     if (n == 0) return cudaSuccess;
     using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
                            uint32_t*, uint32_t*, unsigned long long*, unsigned long long*, const uint32_t*, uint32_t*,
                            PairStore);
-#define QUERY_KERNELS(LIST, KEEP, DENSE)                                                               \
-    {k_query<LIST, KEEP, DENSE, kPairsFound>, k_query<LIST, KEEP, DENSE, kPairsKept>, \
-     k_query<LIST, KEEP, DENSE, kPairsUsed>, k_query<LIST, KEEP, DENSE, kPairsWidened>}
-    static const Query kernels[2][2][4] = {
-        {QUERY_KERNELS(false, kQueryKeep, false), QUERY_KERNELS(false, kQueryKeepDense, true)},
-        {QUERY_KERNELS(true, kQueryKeep, false), QUERY_KERNELS(true, kQueryKeepDense, true)}};
+#define QUERY_KERNELS(LIST, KEEP)                                                                \
+    {k_query<LIST, KEEP, kPairsFound>, k_query<LIST, KEEP, kPairsKept>, k_query<LIST, KEEP, kPairsUsed>, \
+     k_query<LIST, KEEP, kPairsWidened>}
+    static const Query kernels[2][3][4] = {
+        {QUERY_KERNELS(false, kQueryKeep), QUERY_KERNELS(false, kQueryKeepDense), QUERY_KERNELS(false, kQueryKeepCrowd)},
+        {QUERY_KERNELS(true, kQueryKeep), QUERY_KERNELS(true, kQueryKeepDense), QUERY_KERNELS(true, kQueryKeepCrowd)}};
 #undef QUERY_KERNELS
-    static bool carveout = false;  // 16 blocks of ~11.5 KB per SM (dense: 9 of ~23.5 KB)
+    static bool carveout = false;  // 16 blocks of 12 KB per SM, 9 of 24, 7 of 32
     if (!carveout) {
-        for (int i = 0; i < 16; i++)
-            cudaFuncSetAttribute(kernels[i / 8][i / 4 % 2][i % 4], cudaFuncAttributePreferredSharedMemoryCarveout,
+        for (int i = 0; i < 24; i++)
+            cudaFuncSetAttribute(kernels[i / 12][i / 4 % 3][i % 4], cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
         cudaGetLastError();
         carveout = true;
     }
     if (pairs && (!pair_sizes || !pair_ids || n > kPairMaxEntities)) return cudaErrorInvalidValue;
     const bool lists = cap > 0 && list;
-    if (pairs && disp) return cudaErrorInvalidValue;
+    if ((pairs && disp) || density > 2u) return cudaErrorInvalidValue;
     const PairLists use = disp ? kPairsWidened : !pairs ? kPairsFound : keep_near > 0.0 ? kPairsKept : kPairsUsed;
     // the squared distance's rounding and its operands' stay far below 2^-18 of it
     const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18)),
                           disp, widen_limit};
-    kernels[lists][dense][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
+    kernels[lists][density][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
         kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins,
         next_bins, err, count_by_id, store);
     return cudaGetLastError();
 }
 
 size_t query_pair_sizes(uint32_t n) { return (size_t)blocks_for(n, kQueryThreads) * (kQueryThreads / 32); }
-size_t query_pair_places(uint32_t n, bool dense) { return query_pair_sizes(n) * pair_places(dense); }
+size_t query_pair_places(uint32_t n, uint32_t density) {
+    constexpr int keep[3] = {kQueryKeep, kQueryKeepDense, kQueryKeepCrowd};
+    return query_pair_sizes(n) * pair_places(keep[std::min(density, 2u)]);
+}
 
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,
                                uint32_t* first_bad) {

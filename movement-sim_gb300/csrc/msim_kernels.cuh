@@ -23,6 +23,10 @@ constexpr int kMoveThreads = 128;  // move-only launches (k_move)
 constexpr uint32_t kMaxCap = 256;
 constexpr int kQueryKeep = 8;        // neighbours the query keeps per entity (more are collected again)
 constexpr int kQueryKeepDense = 32;  // the same in its kernel for dense populations
+constexpr int kQueryKeepCrowd = 48;  // and for crowded ones
+constexpr int query_blocks(int keep) {  // resident blocks per SM
+    return keep == kQueryKeep ? 16 : keep == kQueryKeepDense ? 9 : 7;
+}
 constexpr uint32_t kPairBins = 256;  // pair counters (summed on read), spread to avoid one hot atomic
 
 // Entity state in slot order (structure of arrays)
@@ -135,7 +139,7 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // count_by_id (may be NULL; only when slot = entity id): every count also
                          // written at its entity's id
                          uint32_t* count_by_id = nullptr,
-                         bool dense = false,  // dense: the kernel for many neighbours (the same results)
+                         uint32_t density = 0,  // 0, 1, 2: the kernel for few, some, many neighbours (the same results)
                          // pair lists of a reused index (see msim_query.cuh): written with keep_near > 0
                          // (pairs up to that distance), else read back (the ids then serve as
                          // sorted_slot, slot_id NULL); NULL: not used
@@ -145,7 +149,7 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // nothing when d exceeds widen_limit or is not finite
                          const uint32_t* disp = nullptr, float widen_limit = 0.f);
 constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
-size_t query_pair_places(uint32_t n, bool dense);   // pairs of all lists
+size_t query_pair_places(uint32_t n, uint32_t density);  // pairs of all lists
 size_t query_pair_sizes(uint32_t n);
 // Index update by counting (msim_indexsort.cuh): the keys' counters become the key-start
 // table (and are zeroed), then every slot goes to its place; sorted_pos and rank may be

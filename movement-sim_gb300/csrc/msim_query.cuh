@@ -268,13 +268,16 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 // warp writes its lists contiguously at warp * 32 * cap and adds its count sum to one
 // of kPairBins counters; the kernel has no block-wide barrier.
 //
-// KEEP and DENSE (chosen by kDenseNeighbours): sparse populations keep 8 and count every hit with
-// a shared atomic; dense ones keep 32 and count an owner's hits by ballot - its pairs lie
-// side by side in a window, where up to 32 atomics on its counter took turns - with
-// atomics only for the credited lanes, and rank longer lists in shared memory.  1 M
-// entities with 4.5 neighbours 170 -> 104 us, 200,000 with 14.6 261 -> 118 us (keeping
-// 16 with more blocks resident 131 and 204, 24 111 and 150: entities beyond pay for
-// list_by_warp).
+// KEEP (chosen by kDenseNeighbours and kCrowdNeighbours): sparse populations keep 8 and
+// count every hit with a shared atomic; dense ones keep 32, crowds 48, and a looked-up
+// window counts an owner's hits by ballot - its pairs lie side by side, where up to 32
+// atomics on its counter took turns - with atomics only for the credited lanes.  (Read
+// back from pair lists the hits thin out: one atomic per owner's run of pairs there was 15 %
+// slower than one per hit.)  Longer lists are ranked in shared memory.  1 M entities with
+// 4.5 neighbours 170 -> 86 us per tick, 200,000 with 14.6 261 -> 50.  A few warps with many
+// lists beyond KEEP decide how long a crowd's query takes (a list looked up again cost about
+// 4 us, and half the time half of the SMs stood idle), so those come from the kept pairs,
+// and crowds keep more at fewer blocks resident.
 constexpr uint32_t kRuns = 4;                  // runs per lane and round
 constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 
@@ -298,9 +301,12 @@ constexpr uint32_t kNoPairs = 0xffffffffu;
 // looked up; looked up and kept; read back; looked up in boxes widened by *PairStore::disp
 enum PairLists : int { kPairsFound, kPairsKept, kPairsUsed, kPairsWidened };
 
-// Places per warp: about twice what the workloads keep (sparse 1 M and 16 M populations
-// 45 of 128; a crowd with 15 neighbours 500 of 1,024).
-__host__ __device__ constexpr uint32_t pair_places(bool dense) { return dense ? 1024u : 128u; }
+// Places per warp: at least twice what the workloads keep (sparse 1 M and 16 M populations
+// 45 of 128; 4.5 neighbours 170 of 1,024; 15 neighbours 530 of 3,072; with 35 neighbours
+// 1,536 places overflow: 176 us per tick against 138).
+__host__ __device__ constexpr uint32_t pair_places(int keep) {
+    return keep == kQueryKeep ? 128u : keep == kQueryKeepDense ? 1024u : 3072u;
+}
 
 struct PairStore {
     uint32_t* pairs;
@@ -318,7 +324,13 @@ struct QueryShared {
     uint32_t id[kQueryThreads];                // kept pairs: the entities' ids
     // sorted positions of the first hits; DENSE: the owner's own from the front, those
     // credited by lower lanes from the back
-    uint32_t keep[KEEP][kQueryThreads];
+    uint32_t keep[KEEP * kQueryThreads];
+    // place c of a warp's lane; the dense kernel keeps a warp's places together, so that
+    // they can also hold its longer lists end to end
+    __device__ __forceinline__ uint32_t& place(uint32_t warp, uint32_t c, uint32_t lane) {
+        return KEEP != kQueryKeep ? keep[(warp * (uint32_t)KEEP + c) * 32u + lane]
+                                  : keep[c * (uint32_t)kQueryThreads + warp * 32u + lane];
+    }
     uint32_t rq[kQueryThreads / 32][kWarpRuns];   // run start position minus its flat start
     uint32_t rfs[kQueryThreads / 32][kWarpRuns];  // flat start of the run
     uint32_t rown[kQueryThreads / 32][kWarpRuns]; // owner lane
@@ -333,27 +345,29 @@ __device__ __forceinline__ uint32_t bit_range(int from, int to) {
 
 // A hit of owner and candidate q by atomics on their counters; kept for the owner is
 // `theirs`, for a credited lane `mine` (sorted positions or ids).
-template <bool LIST, int KEEP, bool DENSE>
+template <bool LIST, int KEEP>
 __device__ __forceinline__ void count_hit(QueryShared<KEEP>& sh, uint32_t warp, uint32_t owner, uint32_t q,
                                           uint32_t pwarp, uint32_t theirs, uint32_t mine) {
+    constexpr bool DENSE = KEEP != kQueryKeep;
     const uint32_t ot = warp * 32u + owner, other = q - pwarp;
     const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
-    if (LIST && c < (uint32_t)KEEP) sh.keep[DENSE ? KEEP - 1 - c : c][ot] = theirs;
+    if (LIST && c < (uint32_t)KEEP) sh.place(warp, DENSE ? KEEP - 1 - c : c, owner) = theirs;
     if (other < 32u) {  // a higher lane of this warp: the pair counts for it too
         const uint32_t om = warp * 32u + other;
         const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
-        if (LIST && c2 < (uint32_t)KEEP) sh.keep[DENSE ? KEEP - 1 - c2 : c2][om] = mine;
+        if (LIST && c2 < (uint32_t)KEEP) sh.place(warp, DENSE ? KEEP - 1 - c2 : c2, other) = mine;
     }
 }
 
 // own: DENSE: the lane's hits as owner so far.  KEPT: near pairs are appended to the
 // warp's places (near_count so far).
-template <bool LIST, int KEEP, bool DENSE, bool KEPT>
+template <bool LIST, int KEEP, bool KEPT>
 __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const uint32_t (&len_in)[kRuns],
                                            uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP>& sh,
                                            const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own,
-                                           PairStore store, uint32_t& near_count, uint32_t places) {
-    constexpr uint32_t FULL = 0xffffffffu;
+                                           PairStore store, uint32_t& near_count) {
+    constexpr uint32_t FULL = 0xffffffffu, places = pair_places(KEEP);
+    constexpr bool DENSE = KEEP != kQueryKeep;
     // A pair of entities of this warp is tested once, by the lower lane, which credits
     // both (the predicate is symmetric, and an in-range pair lies in both entities'
     // runs).  So a lane skips the warp's positions up to its own: a run that starts at
@@ -417,7 +431,7 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
             const uint32_t owner = sh.rown[warp][run];
             if (q - pwarp <= owner) continue;  // the owner itself or a lower lane: tested from there
             if (!in_range_fast(sorted_pos[q], sh.me[warp * 32u + owner], g.radius, g.d2_limit)) continue;
-            count_hit<LIST, KEEP, DENSE>(sh, warp, owner, q, pwarp, q, pwarp + owner);
+            count_hit<LIST, KEEP>(sh, warp, owner, q, pwarp, q, pwarp + owner);
         } else {
             uint32_t q = 0u, owner = lane, other = 0u;
             bool hit = false, near = false;
@@ -442,7 +456,7 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
                 near_count += (uint32_t)__popc(m);
             }
             if constexpr (!DENSE) {
-                if (hit) count_hit<LIST, KEEP, DENSE>(sh, warp, owner, q, pwarp, q, pwarp + owner);
+                if (hit) count_hit<LIST, KEEP>(sh, warp, owner, q, pwarp, q, pwarp + owner);
                 continue;
             }
             const uint32_t hits = __ballot_sync(FULL, hit);
@@ -450,23 +464,114 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
             if (LIST) {
                 const uint32_t before = __shfl_sync(FULL, own, owner), pairs = __shfl_sync(FULL, mine, owner);
                 const uint32_t c = before + (uint32_t)__popc(hits & pairs & lanemask_lt());
-                if (hit && c < (uint32_t)KEEP) sh.keep[c][warp * 32u + owner] = q;
+                if (hit && c < (uint32_t)KEEP) sh.place(warp, c, owner) = q;
             }
             own += (uint32_t)__popc(hits & mine);
             if (hit && other < 32u) {
                 const uint32_t om = warp * 32u + other;
                 const uint32_t c2 = atomicAdd(&sh.cnt[om], 1u);
-                if (LIST && c2 < (uint32_t)KEEP) sh.keep[KEEP - 1 - c2][om] = pwarp + owner;
+                if (LIST && c2 < (uint32_t)KEEP) sh.place(warp, KEEP - 1 - c2, other) = pwarp + owner;
             }
         }
     }
     __syncwarp();  // before the run list is rewritten
 }
 
+// Inclusive prefix sums over the warp, and the first lane whose sum exceeds i (31 when
+// none does).
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, uint32_t lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    return v;
+}
+__device__ __forceinline__ uint32_t first_above(uint32_t ends, uint32_t i) {
+    uint32_t o = 0;
+#pragma unroll
+    for (uint32_t st = 16; st > 0; st >>= 1)
+        if (__shfl_sync(0xffffffffu, ends, o + st - 1u) <= i) o += st;
+    return min(o, 31u);
+}
+
+// The ascending lists of the lanes with count > 0 (more than KEEP neighbours; 0 for the
+// others, whose lists are written) of a warp whose pairs are kept, by this tick's query or
+// an earlier one: those pairs again, every id into its entity's part of the keep words (the
+// lists end to end, as many lanes at a time as fit), then each id to its rank among its
+// list.  place: the lane's list in out.  False: a list alone is too long for the words.
+template <int KEEP>
+__device__ __noinline__ bool lists_from_pairs(const uint32_t* pairs, uint32_t size,
+                                              const uint32_t* __restrict__ sorted_slot,
+                                              const uint32_t* __restrict__ slot_id,
+                                              const float2* __restrict__ sorted_pos, float radius, float d2_limit,
+                                              uint32_t n, uint32_t pwarp, uint32_t count, uint32_t place,
+                                              uint32_t cap, QueryShared<KEEP>& sh, uint32_t* out) {
+    constexpr uint32_t FULL = 0xffffffffu, kWords = 32u * (uint32_t)KEEP;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (__any_sync(FULL, count > kWords)) return false;
+    uint32_t* const words = &sh.place(warp, 0u, 0u);
+    auto id_of = [&](uint32_t q) {
+        const uint32_t s2 = sorted_slot[q];
+        return s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+    };
+    sh.id[warp * 32u + lane] = pwarp + lane < n ? id_of(pwarp + lane) : 0xffffffffu;
+    const uint32_t ends = warp_inclusive(count, lane);
+    for (uint32_t from = 0; from < 32u;) {  // lanes from .. to - 1
+        const uint32_t before = __shfl_sync(FULL, ends - count, from);
+        const uint32_t to = (uint32_t)__popc(__ballot_sync(FULL, lane < from || ends - before <= kWords));
+        const uint32_t total = __shfl_sync(FULL, ends, to - 1u) - before;
+        sh.cnt[warp * 32u + lane] = ends - count - before;  // next free word
+        __syncwarp();
+        const uint32_t wanted = __ballot_sync(FULL, count != 0u && lane - from < to - from);
+        constexpr uint32_t kAtOnce = 4;  // per lane: each pair's loads wait for it
+        for (uint32_t base = lane; base < size; base += 32u * kAtOnce) {
+            uint32_t pair[kAtOnce], id[kAtOnce], who[kAtOnce];  // who: bit 0 the owner, bit 1 the other lane
+            float2 pos[kAtOnce];
+#pragma unroll
+            for (uint32_t k = 0; k < kAtOnce; k++) pair[k] = base + 32u * k < size ? pairs[base + 32u * k] : kNoPairs;
+#pragma unroll
+            for (uint32_t k = 0; k < kAtOnce; k++) {
+                const uint32_t q = pair[k] & kPairPosition, other = q - pwarp;
+                who[k] = 0u;
+                if (base + 32u * k < size)
+                    who[k] = ((wanted >> (pair[k] >> kPairOwnerShift)) & 1u) |
+                             (other < 32u ? ((wanted >> other) & 1u) << 1 : 0u);
+                if (who[k]) {
+                    id[k] = id_of(q);
+                    pos[k] = sorted_pos[q];
+                }
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kAtOnce; k++) {
+                const uint32_t owner = pair[k] >> kPairOwnerShift, other = (pair[k] & kPairPosition) - pwarp;
+                if (!who[k] || !in_range_fast(pos[k], sh.me[warp * 32u + owner], radius, d2_limit)) continue;
+                if (who[k] & 1u) words[atomicAdd(&sh.cnt[warp * 32u + owner], 1u)] = id[k];
+                if (who[k] & 2u) words[atomicAdd(&sh.cnt[warp * 32u + other], 1u)] = sh.id[warp * 32u + owner];
+            }
+        }
+        __syncwarp();
+        for (uint32_t base = 0; base < total; base += 32u) {
+            const uint32_t i = base + lane, o = first_above(ends, i + before);
+            const uint32_t m = __shfl_sync(FULL, count, o), first = __shfl_sync(FULL, ends, o) - m - before;
+            const uint32_t at = __shfl_sync(FULL, place, o);
+            if (i >= total) continue;
+            const uint32_t id = words[i];
+            uint32_t rank = 0;
+#pragma unroll 8
+            for (uint32_t k = 0; k < m; k++) rank += words[first + k] < id ? 1u : 0u;
+            if (rank < cap) out[at + rank] = id;
+        }
+        __syncwarp();  // before the words are used again
+        from = to;
+    }
+    return true;
+}
+
 // The ascending list of lane o's entity (count > KEEP neighbours, at most the 32 * KEEP
 // that the warp's keep words hold) by the whole warp: its runs again, 32 candidates at a
-// time, every hit's id into the keep words, then each id to its rank among them.  One
-// lane walking its tiles and inserting into its output slots held up its warp: at a
+// time, every hit's id into the keep words, then each id to its rank among them; for
+// warps without kept pairs.  One lane walking its tiles and inserting into its output slots held up its warp: at a
 // million entities with 10 m radius three of four warps have such an entity.
 template <int KEEP>
 __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_slot,
@@ -476,7 +581,6 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
                                           uint32_t* out) {
     constexpr uint32_t FULL = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
-    auto word = [&](uint32_t k) -> uint32_t& { return words[(k >> 5) * kQueryThreads + (k & 31u)]; };
     const float ylo = __fsub_rn(me.y, g.reach), yhi = __fadd_rn(me.y, g.reach);
     const uint32_t x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
     const uint32_t x1 = tile_coord(__fadd_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
@@ -493,21 +597,27 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
             const uint32_t hi = min(kstart[(t | (g.ybits ? y_band(g, yhi, ty) : 0u)) + 1u], n);
             len = hi > lo ? hi - lo : 0u;
         }
-        uint32_t runs = __ballot_sync(FULL, len != 0u);
-        while (runs) {
-            const uint32_t o = (uint32_t)__ffs(runs) - 1u;
-            runs &= runs - 1u;
-            const uint32_t from = __shfl_sync(FULL, lo, o), to = from + __shfl_sync(FULL, len, o);
-            for (uint32_t q0 = from; q0 < to; q0 += 32u) {
-                const uint32_t q = q0 + lane;
-                uint32_t id = 0xffffffffu;
-                if (q < to && q != p && in_range_fast(sorted_pos[q], me, g.radius, g.d2_limit)) {
-                    const uint32_t s2 = sorted_slot[q];
-                    if (s2 < n) id = slot_id ? slot_id[s2] : s2;
-                }
-                const uint32_t hits = __ballot_sync(FULL, id != 0xffffffffu);
-                const uint32_t k = m + (uint32_t)__popc(hits & lanemask_lt());
-                if (id != 0xffffffffu && k < count) word(k) = id;
+        const uint32_t ends = warp_inclusive(len, lane), total = __shfl_sync(FULL, ends, 31);
+        for (uint32_t base = 0; base < total; base += 64u) {  // the runs end to end, two candidates per lane
+            uint32_t q[2], id[2];
+            bool hit[2];
+#pragma unroll
+            for (uint32_t k = 0; k < 2u; k++) {
+                const uint32_t i = base + 32u * k + lane, o = first_above(ends, i);
+                q[k] = __shfl_sync(FULL, lo, o) + (i - (__shfl_sync(FULL, ends, o) - __shfl_sync(FULL, len, o)));
+                hit[k] = i < total && q[k] != p;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 2u; k++) {
+                hit[k] = hit[k] && in_range_fast(sorted_pos[q[k]], me, g.radius, g.d2_limit);
+                const uint32_t s2 = hit[k] ? sorted_slot[q[k]] : n;
+                id[k] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 2u; k++) {
+                const uint32_t hits = __ballot_sync(FULL, id[k] != 0xffffffffu);
+                const uint32_t w = m + (uint32_t)__popc(hits & lanemask_lt());
+                if (id[k] != 0xffffffffu && w < count) words[w] = id[k];
                 m += (uint32_t)__popc(hits);
             }
         }
@@ -515,9 +625,9 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
     m = min(m, count);
     __syncwarp();
     for (uint32_t i = lane; i < m; i += 32u) {
-        const uint32_t id = word(i);
+        const uint32_t id = words[i];
         uint32_t rank = 0;
-        for (uint32_t j = 0; j < m; j++) rank += word(j) < id ? 1u : 0u;
+        for (uint32_t j = 0; j < m; j++) rank += words[j] < id ? 1u : 0u;
         if (rank < cap) out[rank] = id;
     }
     __syncwarp();  // before the words are used again
@@ -525,8 +635,8 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
 
 // 16 blocks (64 warps) per SM: at 40 registers (12 blocks) the symmetric pair loop
 // gained nothing (0.435 against 0.437 ms at 16 M), at 32 it takes 0.395.
-template <bool LIST, int KEEP, bool DENSE, PairLists PAIRS>
-__global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const uint32_t* __restrict__ kstart,
+template <bool LIST, int KEEP, PairLists PAIRS>
+__global__ __launch_bounds__(kQueryThreads, query_blocks(KEEP)) void k_query(const uint32_t* __restrict__ kstart,
                                                          const uint32_t* __restrict__ sorted_slot,
                                                          const float2* __restrict__ sorted_pos,
                                                          const uint32_t* __restrict__ slot_id, TileGrid g,
@@ -548,14 +658,18 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     const uint32_t pwarp = p - lane;
     const bool valid = p < n;
     float2 me = make_float2(0.f, 0.f);
-    constexpr uint32_t places = pair_places(DENSE);
+    constexpr bool DENSE = KEEP != kQueryKeep;
+    constexpr uint32_t places = pair_places(KEEP);
+    // pairs in flight per lane (dense 2 / 4 / 6: 1 M entities with 4.5 neighbours 90.9 / 87.5 /
+    // 85.9 us per tick)
+    constexpr uint32_t kPairsAtOnce = DENSE ? 6 : 2;
     const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * places : nullptr;
     uint32_t size = kNoPairs;
-    uint32_t pair[2], my_id = 0u;
+    uint32_t pair[kPairsAtOnce], my_id = 0u;
     if (PAIRS == kPairsUsed) {  // the first pairs, their number, position and id in flight together
         size = store.sizes[p >> 5];
-        pair[0] = pairs[lane];
-        pair[1] = pairs[lane + 32u];
+#pragma unroll
+        for (uint32_t k = 0; k < kPairsAtOnce; k++) pair[k] = pairs[lane + 32u * k];
         my_id = valid ? store.ids[p] : 0u;
     }
     if (valid) me = sorted_pos[p];
@@ -578,25 +692,25 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
     if (have_ids) {
         sh.id[tid] = my_id;
         __syncwarp();
-        for (uint32_t base = 0; base < size; base += 64u) {  // two pairs per lane in flight
-            float2 o[2];
-            uint32_t id[2];
+        for (uint32_t base = 0; base < size; base += 32u * kPairsAtOnce) {
+            float2 o[kPairsAtOnce];
+            uint32_t id[kPairsAtOnce];
 #pragma unroll
-            for (uint32_t k = 0; k < 2u; k++) {
+            for (uint32_t k = 0; k < kPairsAtOnce; k++) {
                 if (base + 32u * k + lane >= size) continue;
                 const uint32_t q = pair[k] & kPairPosition;
                 o[k] = sorted_pos[q];
                 if (LIST) id[k] = store.ids[q];
             }
 #pragma unroll
-            for (uint32_t k = 0; k < 2u; k++) {
+            for (uint32_t k = 0; k < kPairsAtOnce; k++) {
                 const uint32_t i = base + 32u * k + lane;
                 if (i >= size) continue;
                 const uint32_t owner = pair[k] >> kPairOwnerShift;
                 if (in_range_fast(o[k], sh.me[warp * 32u + owner], g.radius, g.d2_limit))
-                    count_hit<LIST, KEEP, DENSE>(sh, warp, owner, pair[k] & kPairPosition, pwarp, id[k],
+                    count_hit<LIST, KEEP>(sh, warp, owner, pair[k] & kPairPosition, pwarp, id[k],
                                                  sh.id[warp * 32u + owner]);
-                if (i + 64u < size) pair[k] = pairs[i + 64u];
+                if (i + 32u * kPairsAtOnce < size) pair[k] = pairs[i + 32u * kPairsAtOnce];
             }
         }
     } else {
@@ -638,8 +752,8 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                 len[k] = hi > lo[k] ? hi - lo[k] : 0u;
             }
         }
-        query_runs<LIST, KEEP, DENSE, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
-                                                           store, near_count, places);
+        query_runs<LIST, KEEP, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
+                                                           store, near_count);
     } else {
         // general boxes (tile side below 2 x reach): kRuns tiles per round
         const uint32_t nslots = nx * ny;
@@ -664,8 +778,8 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                     len[k] = hi > lo[k] ? hi - lo[k] : 0u;
                 }
             }
-            query_runs<LIST, KEEP, DENSE, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
-                                                           store, near_count, places);
+            query_runs<LIST, KEEP, PAIRS == kPairsKept>(lo, len, lane, warp, pwarp, sh, sorted_pos, g, own,
+                                                           store, near_count);
         }
     }
     if (PAIRS == kPairsKept && lane == 0) store.sizes[p >> 5] = near_count <= places ? near_count : kNoPairs;
@@ -701,7 +815,7 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                 id[i] = 0xffffffffu;
                 if ((uint32_t)i < wmax) {
                     const uint32_t k = DENSE && (uint32_t)i >= own ? (uint32_t)i + (uint32_t)KEEP - listed : (uint32_t)i;
-                    const uint32_t x = (uint32_t)i < listed ? sh.keep[k][tid] : 0xffffffffu;
+                    const uint32_t x = (uint32_t)i < listed ? sh.place(warp, k, lane) : 0xffffffffu;
                     if (have_ids) {
                         id[i] = x;
                         continue;
@@ -739,9 +853,9 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
 #pragma unroll 4
             for (uint32_t i = 0; i < wmax; i++) {
                 if (i < listed) {
-                    const uint32_t x = sh.keep[i < own ? i : i + (uint32_t)KEEP - listed][tid];
+                    const uint32_t x = sh.place(warp, i < own ? i : i + (uint32_t)KEEP - listed, lane);
                     const uint32_t s2 = have_ids ? n : sorted_slot[x];
-                    sh.keep[i][tid] = have_ids ? x : s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+                    sh.place(warp, i, lane) = have_ids ? x : s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
                 }
             }
             __syncwarp();
@@ -767,14 +881,14 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
                 const uint32_t m = __shfl_sync(FULL, listed, o), to = __shfl_sync(FULL, place, o);
                 const uint32_t first = __shfl_sync(FULL, li - couples, o);
                 if (i < total) {
-                    const uint32_t* col = &sh.keep[0][warp * 32u + o];
+                    const uint32_t* col = &sh.place(warp, 0u, o);
                     const uint32_t j = 2u * (i - first);
-                    const uint32_t a = col[j * kQueryThreads];
-                    const uint32_t b = j + 1u < m ? col[(j + 1u) * kQueryThreads] : 0xffffffffu;
+                    const uint32_t a = col[j * 32u];
+                    const uint32_t b = j + 1u < m ? col[(j + 1u) * 32u] : 0xffffffffu;
                     uint32_t ra = 0, rb = 0;
 #pragma unroll 4
                     for (uint32_t k = 0; k < m; k++) {
-                        const uint32_t x = col[k * kQueryThreads];
+                        const uint32_t x = col[k * 32u];
                         ra += x < a ? 1u : 0u;
                         rb += x < b ? 1u : 0u;
                     }
@@ -788,13 +902,22 @@ __global__ __launch_bounds__(kQueryThreads, DENSE ? 9 : 16) void k_query(const u
         } else {
             uint32_t longer = __ballot_sync(FULL, count > (uint32_t)KEEP);
             if (longer) __syncwarp();  // the kept lists are written out: their words are free
+            if (longer && (PAIRS == kPairsUsed || PAIRS == kPairsKept)) {
+                const uint32_t known = PAIRS == kPairsUsed ? size : near_count <= places ? near_count : kNoPairs;
+                if (known != kNoPairs &&
+                    lists_from_pairs<KEEP>(store.pairs + (size_t)(p >> 5) * places, known, sorted_slot, slot_id,
+                                           sorted_pos, g.radius, g.d2_limit, n, pwarp,
+                                           count > (uint32_t)KEEP ? count : 0u, incl - kept, cap, sh,
+                                           list + (size_t)(p >> 5) * 32u * cap))
+                    return;
+            }
             while (longer) {
                 const uint32_t o = (uint32_t)__ffs(longer) - 1u;
                 longer &= longer - 1u;
                 const uint32_t c = __shfl_sync(FULL, count, o);
                 if (c <= 32u * (uint32_t)KEEP) {
                     list_by_warp<KEEP>(sorted_slot, sorted_pos, slot_id, kstart, g, n, pwarp + o,
-                                       sh.me[warp * 32u + o], c, cap, &sh.keep[0][warp * 32u],
+                                       sh.me[warp * 32u + o], c, cap, &sh.place(warp, 0u, 0u),
                                        list + (size_t)(p >> 5) * 32u * cap + __shfl_sync(FULL, incl - kept, o));
                 } else if (lane == o) {
                     list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
