@@ -231,7 +231,8 @@ struct msim_ctx {
     uint32_t* status_host = nullptr;  // page-locked copy of *err, written behind the work it describes
     uint32_t* check = nullptr;  // first invalid heading found by msim_set_entities
     TileGrid grid{};
-    uint32_t density = 0;  // how many neighbours are expected (see msim_create): the query's kernel
+    double expected = 0.0;  // neighbours expected along the road (see msim_create), and the
+    uint32_t density = 0;   // query's kernel for that many
     uint32_t passes = 1;
     uint32_t resort = 16;
     uint32_t since_permute = 0;
@@ -542,6 +543,12 @@ int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
     const int64_t left = (int64_t)std::min(std::floor((double)kWidenLimit * per_reach), 1e9) - since;
     const int64_t best = (int64_t)std::min(std::sqrt(0.5 * (c->density ? kPairCostDense : kPairCost) * per_reach), 1e9);
     const int64_t ticks = std::min(left, std::max(best, kFewest));
+    // a warp keeps about 24 pairs per expected neighbour within the reach (16 pairs per
+    // neighbour, 1.5 neighbours per one along the road), more the further they are kept;
+    // past its places it looks them up all the same (1 M with 192 neighbours, counts alone:
+    // 920 us per tick against 897)
+    if (24.0 * c->expected * (1.0 + 2.0 * (double)ticks / per_reach) > (double)pair_places(query_keep(c->density)))
+        return 0;
     return ticks >= kFewest ? ticks : 0;
 }
 
@@ -592,17 +599,21 @@ T* mapped_range(const void* p, size_t count) {
     return mapped_host(static_cast<const char*>(p) + last) == first + last ? reinterpret_cast<T*>(first) : nullptr;
 }
 
-// Where an export kernel writes an output: the caller's array itself when it is
-// page-locked, aligned for the kernel's stores and small (below kDirectEntities
-// entities the copies' own latency is most of a read-back), else its staging place;
-// nullptr when the output is not wanted.
-constexpr uint32_t kDirectEntities = 65536;
+// Where an export kernel writes an output of count elements: the caller's array itself
+// when it is page-locked and aligned for the kernel's stores, else its staging place;
+// nullptr when the output is not wanted.  The state's fields are written in entity
+// order, a line at a time, which keeps the link as busy as a copy and saves the staging
+// (1 M entities 20 us of 470); counts and id lists are written in the order of the query,
+// by id, which crosses the link in pieces, so above kDirectEntities entities counts and
+// lists of fewer than kDirectRow ids are staged (1 M counts 964 us for 25 ticks, 1,250
+// written in place; lists of 64 ids 643 us for five ticks at 200,000, 624 in place, of 16
+// 430 and 433; for few entities the copies' own latency is most of a read-back).
+constexpr uint32_t kDirectEntities = 65536, kDirectRow = 64;
 template <typename T>
-T* direct_out(const msim_ctx* c, void* out, T* staged) {
+T* direct_out(void* out, size_t count, T* staged) {
     if (!out) return nullptr;
-    if (c->n > kDirectEntities) return staged;
-    void* mapped = mapped_host(out);
-    return mapped && (reinterpret_cast<uintptr_t>(mapped) & (sizeof(T) - 1)) == 0 ? static_cast<T*>(mapped) : staged;
+    T* mapped = mapped_range<T>(out, count);
+    return mapped ? mapped : staged;
 }
 
 // The main stream waits for the queries still running on qstream that read index
@@ -1137,8 +1148,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
         const double dx = (double)q[2] - (double)q[0], dy = (double)q[3] - (double)q[1];
         road_length += std::sqrt(dx * dx + dy * dy) * (double)every;
     }
-    const double along = 2.0 * radius * (double)c->n;
-    c->density = along > kCrowdNeighbours * road_length ? 2u : along > kDenseNeighbours * road_length ? 1u : 0u;
+    c->expected = road_length > 0.0 ? 2.0 * radius * (double)c->n / road_length : INFINITY;
+    c->density = c->expected > kCrowdNeighbours ? 2u : c->expected > kDenseNeighbours ? 1u : 0u;
     // y bands inside a tile fill the key up to 24 bits (3 radix passes), at most 64
     // bands, and keep the key-start table within about four entries per entity
     uint32_t nbits = 0;
@@ -1369,10 +1380,10 @@ int msim_get_state(msim_ctx* c, float* pos, uint32_t* heading, uint32_t* rng, fl
     uint32_t* d_head = reinterpret_cast<uint32_t*>(b + n * (sizeof(uint4) + sizeof(float2)));
     float* d_speed = reinterpret_cast<float*>(b + n * (sizeof(uint4) + sizeof(float2) + sizeof(uint32_t)));
     // page-locked outputs are written by the kernel itself, others staged and copied
-    float2* to_pos = direct_out<float2>(c, pos, d_pos);
-    uint32_t* to_head = direct_out<uint32_t>(c, heading, d_head);
-    uint4* to_rng = direct_out<uint4>(c, rng, d_rng);
-    float* to_speed = direct_out<float>(c, speed, d_speed);
+    float2* to_pos = direct_out<float2>(pos, n, d_pos);
+    uint32_t* to_head = direct_out<uint32_t>(heading, n, d_head);
+    uint4* to_rng = direct_out<uint4>(rng, n, d_rng);
+    float* to_speed = direct_out<float>(speed, n, d_speed);
     {
         Prof p(c, K_EXPORT);
         c->launch_count++;  // two kernels
@@ -1402,9 +1413,16 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     if ((rc = ensure_stage(c, n * sizeof(uint32_t) * (1 + (want_idx ? cap : 0)))) != MSIM_OK) return rc;
     uint32_t* d_idx = want_idx ? static_cast<uint32_t*>(c->stage) : nullptr;
     uint32_t* d_count = static_cast<uint32_t*>(c->stage) + (want_idx ? n * cap : 0);
-    uint32_t* to_count = direct_out<uint32_t>(c, count, d_count);
+    const bool direct = n <= kDirectEntities;
+    uint32_t* to_count = direct ? direct_out<uint32_t>(count, n, d_count) : d_count;
     uint32_t* to_idx = nullptr;
-    if (want_idx) to_idx = reinterpret_cast<uint32_t*>(direct_out<uint4>(c, idx, reinterpret_cast<uint4*>(d_idx)));
+    if (want_idx) {
+        // whole rows, 16 bytes at a time where they allow it
+        const size_t rows = std::max<size_t>(n * cap / 4, 1);
+        to_idx = direct || cap >= kDirectRow
+                     ? reinterpret_cast<uint32_t*>(direct_out<uint4>(idx, rows, reinterpret_cast<uint4*>(d_idx)))
+                     : d_idx;
+    }
     {
         Prof p(c, K_EXPORT);
         CK(launch_export_neighbours(c->stream, c->query_slot, cur_state(c).slot_id, c->nbr_count, c->nbr_list,

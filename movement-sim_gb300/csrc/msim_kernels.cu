@@ -1052,8 +1052,7 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
 
 size_t query_pair_sizes(uint32_t n) { return (size_t)blocks_for(n, kQueryThreads) * (kQueryThreads / 32); }
 size_t query_pair_places(uint32_t n, uint32_t density) {
-    constexpr int keep[3] = {kQueryKeep, kQueryKeepDense, kQueryKeepCrowd};
-    return query_pair_sizes(n) * pair_places(keep[std::min(density, 2u)]);
+    return query_pair_sizes(n) * pair_places(query_keep(density));
 }
 
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,

@@ -24,8 +24,8 @@ constexpr uint32_t kMaxCap = 256;
 constexpr int kQueryKeep = 8;        // neighbours the query keeps per entity (more are collected again)
 constexpr int kQueryKeepDense = 32;  // the same in its kernel for dense populations
 constexpr int kQueryKeepCrowd = 48;  // and for crowded ones
-constexpr int query_blocks(int keep) {  // resident blocks per SM
-    return keep == kQueryKeep ? 16 : keep == kQueryKeepDense ? 9 : 7;
+constexpr int query_keep(uint32_t density) {  // 0, 1, 2: few, some, many neighbours expected
+    return density == 0 ? kQueryKeep : density == 1 ? kQueryKeepDense : kQueryKeepCrowd;
 }
 constexpr uint32_t kPairBins = 256;  // pair counters (summed on read), spread to avoid one hot atomic
 
@@ -149,6 +149,12 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // nothing when d exceeds widen_limit or is not finite
                          const uint32_t* disp = nullptr, float widen_limit = 0.f);
 constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
+// Places per warp: at least twice what the workloads keep (sparse 1 M and 16 M populations
+// 45 of 128; 4.5 neighbours 170 of 1,024; 15 neighbours 530 of 3,072; with 35 neighbours
+// 1,536 places overflow: 176 us per tick against 138).
+__host__ __device__ constexpr uint32_t pair_places(int keep) {
+    return keep == kQueryKeep ? 128u : keep == kQueryKeepDense ? 1024u : 3072u;
+}
 size_t query_pair_places(uint32_t n, uint32_t density);  // pairs of all lists
 size_t query_pair_sizes(uint32_t n);
 // Index update by counting (msim_indexsort.cuh): the keys' counters become the key-start

@@ -273,7 +273,7 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 // window counts an owner's hits by ballot - its pairs lie side by side, where up to 32
 // atomics on its counter took turns - with atomics only for the credited lanes.  (Read
 // back from pair lists the hits thin out: one atomic per owner's run of pairs there was 15 %
-// slower than one per hit.)  Longer lists are ranked in shared memory.  1 M entities with
+// slower than one per hit; counts alone take an atomic per hit everywhere.)  Longer lists are ranked in shared memory.  1 M entities with
 // 4.5 neighbours 170 -> 86 us per tick, 200,000 with 14.6 261 -> 50.  A few warps with many
 // lists beyond KEEP decide how long a crowd's query takes (a list looked up again cost about
 // 4 us, and half the time half of the SMs stood idle), so those come from the kept pairs,
@@ -301,13 +301,6 @@ constexpr uint32_t kNoPairs = 0xffffffffu;
 // looked up; looked up and kept; read back; looked up in boxes widened by *PairStore::disp
 enum PairLists : int { kPairsFound, kPairsKept, kPairsUsed, kPairsWidened };
 
-// Places per warp: at least twice what the workloads keep (sparse 1 M and 16 M populations
-// 45 of 128; 4.5 neighbours 170 of 1,024; 15 neighbours 530 of 3,072; with 35 neighbours
-// 1,536 places overflow: 176 us per tick against 138).
-__host__ __device__ constexpr uint32_t pair_places(int keep) {
-    return keep == kQueryKeep ? 128u : keep == kQueryKeepDense ? 1024u : 3072u;
-}
-
 struct PairStore {
     uint32_t* pairs;
     uint32_t* sizes;
@@ -317,14 +310,14 @@ struct PairStore {
     float widen_limit;     // and the d up to which the query runs
 };
 
-template <int KEEP>
+template <int KEEP, bool LIST>
 struct QueryShared {
     float2 me[kQueryThreads];
     uint32_t cnt[kQueryThreads];
     uint32_t id[kQueryThreads];                // kept pairs: the entities' ids
     // sorted positions of the first hits; DENSE: the owner's own from the front, those
     // credited by lower lanes from the back
-    uint32_t keep[KEEP * kQueryThreads];
+    uint32_t keep[LIST ? KEEP * kQueryThreads : 1];
     // place c of a warp's lane; the dense kernel keeps a warp's places together, so that
     // they can also hold its longer lists end to end
     __device__ __forceinline__ uint32_t& place(uint32_t warp, uint32_t c, uint32_t lane) {
@@ -346,9 +339,9 @@ __device__ __forceinline__ uint32_t bit_range(int from, int to) {
 // A hit of owner and candidate q by atomics on their counters; kept for the owner is
 // `theirs`, for a credited lane `mine` (sorted positions or ids).
 template <bool LIST, int KEEP>
-__device__ __forceinline__ void count_hit(QueryShared<KEEP>& sh, uint32_t warp, uint32_t owner, uint32_t q,
+__device__ __forceinline__ void count_hit(QueryShared<KEEP, LIST>& sh, uint32_t warp, uint32_t owner, uint32_t q,
                                           uint32_t pwarp, uint32_t theirs, uint32_t mine) {
-    constexpr bool DENSE = KEEP != kQueryKeep;
+    constexpr bool DENSE = LIST && KEEP != kQueryKeep;
     const uint32_t ot = warp * 32u + owner, other = q - pwarp;
     const uint32_t c = atomicAdd(&sh.cnt[ot], 1u);
     if (LIST && c < (uint32_t)KEEP) sh.place(warp, DENSE ? KEEP - 1 - c : c, owner) = theirs;
@@ -363,11 +356,11 @@ __device__ __forceinline__ void count_hit(QueryShared<KEEP>& sh, uint32_t warp, 
 // warp's places (near_count so far).
 template <bool LIST, int KEEP, bool KEPT>
 __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const uint32_t (&len_in)[kRuns],
-                                           uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP>& sh,
+                                           uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP, LIST>& sh,
                                            const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own,
                                            PairStore store, uint32_t& near_count) {
     constexpr uint32_t FULL = 0xffffffffu, places = pair_places(KEEP);
-    constexpr bool DENSE = KEEP != kQueryKeep;
+    constexpr bool DENSE = LIST && KEEP != kQueryKeep;
     // A pair of entities of this warp is tested once, by the lower lane, which credits
     // both (the predicate is symmetric, and an in-range pair lies in both entities'
     // runs).  So a lane skips the warp's positions up to its own: a run that starts at
@@ -506,7 +499,7 @@ __device__ __noinline__ bool lists_from_pairs(const uint32_t* pairs, uint32_t si
                                               const uint32_t* __restrict__ slot_id,
                                               const float2* __restrict__ sorted_pos, float radius, float d2_limit,
                                               uint32_t n, uint32_t pwarp, uint32_t count, uint32_t place,
-                                              uint32_t cap, QueryShared<KEEP>& sh, uint32_t* out) {
+                                              uint32_t cap, QueryShared<KEEP, true>& sh, uint32_t* out) {
     constexpr uint32_t FULL = 0xffffffffu, kWords = 32u * (uint32_t)KEEP;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (__any_sync(FULL, count > kWords)) return false;
@@ -633,10 +626,17 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
     __syncwarp();  // before the words are used again
 }
 
-// 16 blocks (64 warps) per SM: at 40 registers (12 blocks) the symmetric pair loop
-// gained nothing (0.435 against 0.437 ms at 16 M), at 32 it takes 0.395.
+// Resident blocks per SM.  Sparse and counts alone: 16 (64 warps), at 40 registers (12
+// blocks) the symmetric pair loop gained nothing (0.435 against 0.437 ms at 16 M), at 32 it
+// takes 0.395; reading back dense pair lists takes six in flight per lane and 12.  Lists of
+// dense populations: as many as their places in shared memory allow.
+constexpr int query_blocks(bool list, int keep, PairLists pairs) {
+    if (keep == kQueryKeep) return 16;
+    if (!list) return pairs == kPairsUsed ? 12 : 16;
+    return keep == kQueryKeepDense ? 9 : 7;
+}
 template <bool LIST, int KEEP, PairLists PAIRS>
-__global__ __launch_bounds__(kQueryThreads, query_blocks(KEEP)) void k_query(const uint32_t* __restrict__ kstart,
+__global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) void k_query(const uint32_t* __restrict__ kstart,
                                                          const uint32_t* __restrict__ sorted_slot,
                                                          const float2* __restrict__ sorted_pos,
                                                          const uint32_t* __restrict__ slot_id, TileGrid g,
@@ -647,7 +647,7 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(KEEP)) void k_query(con
                                                          const uint32_t* err, uint32_t* __restrict__ count_by_id,
                                                          PairStore store) {
     constexpr uint32_t FULL = 0xffffffffu;
-    __shared__ QueryShared<KEEP> sh;
+    __shared__ QueryShared<KEEP, LIST> sh;
     // read first, tested once the other first loads are in flight (they stay in range
     // whatever an index update left behind)
     const uint32_t status = err ? ld_relaxed(err) : 0u;
@@ -658,11 +658,11 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(KEEP)) void k_query(con
     const uint32_t pwarp = p - lane;
     const bool valid = p < n;
     float2 me = make_float2(0.f, 0.f);
-    constexpr bool DENSE = KEEP != kQueryKeep;
+    constexpr bool DENSE = LIST && KEEP != kQueryKeep;
     constexpr uint32_t places = pair_places(KEEP);
     // pairs in flight per lane (dense 2 / 4 / 6: 1 M entities with 4.5 neighbours 90.9 / 87.5 /
     // 85.9 us per tick)
-    constexpr uint32_t kPairsAtOnce = DENSE ? 6 : 2;
+    constexpr uint32_t kPairsAtOnce = KEEP != kQueryKeep ? 6 : 2;
     const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * places : nullptr;
     uint32_t size = kNoPairs;
     uint32_t pair[kPairsAtOnce], my_id = 0u;
@@ -796,7 +796,7 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(KEEP)) void k_query(con
     // the next query's counters (a memset for them stood between two queries)
     if (p < kPairBins) next_bins[p] = 0ull;
     if (lane == 0 && warp_sum) atomicAdd(&pair_bins[(p >> 5) & (kPairBins - 1u)], (unsigned long long)warp_sum);
-    if (LIST) {
+    if constexpr (LIST) {
         const uint32_t kept = count < cap ? count : cap;
         uint32_t incl = kept;
 #pragma unroll
