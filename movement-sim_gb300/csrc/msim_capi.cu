@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <string>
@@ -441,37 +442,43 @@ constexpr double kDenseNeighbours = 1.2;
 // 84.8; at 1 M 3.4 (4.8) 60.6 / 71.1, 8.6 (12.3) 155 / 162, 13.8 (21.4) 335 / 301.
 constexpr double kCrowdNeighbours = 6.5;
 
-// rank[slot] (written by every later merge once allocated): false when the allocation
-// fails.
-bool ensure_rank(msim_ctx* c) {
-    if (c->rank) return true;
+// One device block for those of the arrays that are not allocated yet (an allocation
+// costs about 10 us whatever its size, in the first pass of every context); false, and none
+// of them, when it fails.
+struct Part {
+    void** at;
+    size_t bytes;
+};
+bool allocate_parts(msim_ctx* c, std::initializer_list<Part> parts) {
+    constexpr size_t kAlign = 256;
+    size_t total = 0;
+    for (const Part& p : parts)
+        if (!*p.at) total += (std::max<size_t>(p.bytes, 1) + kAlign - 1) / kAlign * kAlign;
+    if (!total) return true;
     void* raw = nullptr;
-    if (!device_malloc(&raw, sizeof(uint32_t) * std::max<size_t>(c->n, 1))) return false;
+    if (!device_malloc(&raw, total)) return false;
     c->allocs.push_back(raw);
-    c->device_bytes += sizeof(uint32_t) * std::max<size_t>(c->n, 1);
-    c->rank = static_cast<uint32_t*>(raw);
-    c->rank_valid = false;
+    c->device_bytes += total;
+    char* next = static_cast<char*>(raw);
+    for (const Part& p : parts) {
+        if (*p.at) continue;
+        *p.at = next;
+        next += (std::max<size_t>(p.bytes, 1) + kAlign - 1) / kAlign * kAlign;
+    }
     return true;
 }
+template <typename T>
+Part part(T*& at, size_t count) {
+    return {reinterpret_cast<void**>(&at), count * sizeof(T)};
+}
+
+// Ranks of host ticks (rank[slot], written by every later update once allocated).
+bool ensure_rank(msim_ctx* c) { return allocate_parts(c, {part(c->rank, c->n)}); }
 
 // Buffers of the skin query (allocated by the first host tick that can use it): false
 // when an allocation fails, and the tick then takes the usual order.
 bool ensure_skin(msim_ctx* c) {
-    if (c->skin_pos && c->disp && c->disp_host) return true;
-    if (!c->skin_pos) {
-        void* raw = nullptr;
-        if (!device_malloc(&raw, sizeof(float2) * std::max<size_t>(c->n, 1))) return false;
-        c->allocs.push_back(raw);
-        c->device_bytes += sizeof(float2) * std::max<size_t>(c->n, 1);
-        c->skin_pos = static_cast<float2*>(raw);
-    }
-    if (!c->disp) {
-        void* raw = nullptr;
-        if (!device_malloc(&raw, 2 * sizeof(uint32_t))) return false;
-        c->allocs.push_back(raw);
-        c->device_bytes += 2 * sizeof(uint32_t);
-        c->disp = static_cast<uint32_t*>(raw);
-    }
+    if (!allocate_parts(c, {part(c->skin_pos, c->n), part(c->disp, 2)})) return false;
     if (!c->disp_host) {
         void* h = nullptr;
         if (cudaMallocHost(&h, 3 * sizeof(uint32_t)) != cudaSuccess) {
@@ -483,46 +490,25 @@ bool ensure_skin(msim_ctx* c) {
     return true;
 }
 
-// Buffers of index reuse on the device path (allocated by the first reusing tick):
-// false when an allocation fails, and the ticks then update the index every time.
+// Buffers and events of index reuse: ranks and two sets of sorted positions.
 bool ensure_reuse(msim_ctx* c) {
-    if (!ensure_rank(c)) return false;
-    for (int b = 0; b < 2; b++) {
-        if (!c->reuse_pos[b]) {
-            void* raw = nullptr;
-            if (!device_malloc(&raw, sizeof(float2) * std::max<size_t>(c->n, 1))) return false;
-            c->allocs.push_back(raw);
-            c->device_bytes += sizeof(float2) * std::max<size_t>(c->n, 1);
-            c->reuse_pos[b] = static_cast<float2*>(raw);
-        }
-        if (!c->ev_reuse_read[b] && cudaEventCreateWithFlags(&c->ev_reuse_read[b], cudaEventDisableTiming) != cudaSuccess) {
+    if (!allocate_parts(c, {part(c->rank, c->n), part(c->reuse_pos[0], c->n), part(c->reuse_pos[1], c->n)}))
+        return false;
+    for (cudaEvent_t& e : c->ev_reuse_read) {
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
-            c->ev_reuse_read[b] = nullptr;
+            e = nullptr;
             return false;
         }
     }
     return true;
 }
 
-// Buffers of the pair lists: false when an allocation fails (the queries then look
+// Buffers of the pair lists: false when their allocation fails (the queries then look
 // their candidates up).
 bool ensure_pairs(msim_ctx* c) {
-    if (c->pairs_kept && c->pair_sizes && c->pair_ids) return true;
-    const size_t bytes[3] = {sizeof(uint32_t) * query_pair_places(c->n, c->density),
-                             sizeof(uint32_t) * query_pair_sizes(c->n), sizeof(uint32_t) * c->n};
-    void* at[3] = {c->pairs_kept, c->pair_sizes, c->pair_ids};
-    bool all = true;
-    for (int k = 0; k < 3 && all; k++) {
-        if (at[k]) continue;
-        all = device_malloc(&at[k], bytes[k]);
-        if (!all) break;
-        c->allocs.push_back(at[k]);
-        c->device_bytes += bytes[k];
-    }
-    c->pairs_kept = static_cast<uint32_t*>(at[0]);
-    c->pair_sizes = static_cast<uint32_t*>(at[1]);
-    c->pair_ids = static_cast<uint32_t*>(at[2]);
-    return all;
+    return allocate_parts(c, {part(c->pairs_kept, query_pair_places(c->n, c->density)),
+                              part(c->pair_sizes, query_pair_sizes(c->n)), part(c->pair_ids, c->n)});
 }
 
 // Ticks that pair lists kept `since` move ticks after the index's keys should serve (0:
@@ -600,8 +586,8 @@ T* mapped_range(const void* p, size_t count) {
 }
 
 // Where an export kernel writes an output of count elements: the caller's array itself
-// when it is page-locked and aligned for the kernel's stores, else its staging place;
-// nullptr when the output is not wanted.  The state's fields are written in entity
+// when it is page-locked and aligned for the kernel's stores; else, or when it is not
+// wanted, nullptr.  The state's fields are written in entity
 // order, a line at a time, which keeps the link as busy as a copy and saves the staging
 // (1 M entities 20 us of 470); counts and id lists are written in the order of the query,
 // by id, which crosses the link in pieces, so above kDirectEntities entities counts and
@@ -610,10 +596,8 @@ T* mapped_range(const void* p, size_t count) {
 // 430 and 433; for few entities the copies' own latency is most of a read-back).
 constexpr uint32_t kDirectEntities = 65536, kDirectRow = 64;
 template <typename T>
-T* direct_out(void* out, size_t count, T* staged) {
-    if (!out) return nullptr;
-    T* mapped = mapped_range<T>(out, count);
-    return mapped ? mapped : staged;
+T* direct_out(void* out, size_t count) {
+    return out ? mapped_range<T>(out, count) : nullptr;
 }
 
 // The main stream waits for the queries still running on qstream that read index
@@ -1372,33 +1356,41 @@ int msim_get_state(msim_ctx* c, float* pos, uint32_t* heading, uint32_t* rng, fl
     if (rc != MSIM_OK) return rc;
     const size_t n = c->n;
     if (n == 0) return sync_and_check(c);
-    const size_t fields = sizeof(float2) + sizeof(uint32_t) + sizeof(uint4) + sizeof(float);
-    if ((rc = ensure_stage(c, n * (kStateRecordBytes + fields))) != MSIM_OK) return rc;
-    char* b = static_cast<char*>(c->stage) + n * kStateRecordBytes;  // the records, then the fields
-    uint4* d_rng = reinterpret_cast<uint4*>(b);
-    float2* d_pos = reinterpret_cast<float2*>(b + n * sizeof(uint4));
-    uint32_t* d_head = reinterpret_cast<uint32_t*>(b + n * (sizeof(uint4) + sizeof(float2)));
-    float* d_speed = reinterpret_cast<float*>(b + n * (sizeof(uint4) + sizeof(float2) + sizeof(uint32_t)));
-    // page-locked outputs are written by the kernel itself, others staged and copied
-    float2* to_pos = direct_out<float2>(pos, n, d_pos);
-    uint32_t* to_head = direct_out<uint32_t>(heading, n, d_head);
-    uint4* to_rng = direct_out<uint4>(rng, n, d_rng);
-    float* to_speed = direct_out<float>(speed, n, d_speed);
+    // Page-locked outputs are written by the kernel itself, others staged and copied; the
+    // staging holds the records and what is copied (above 2 MB an allocation costs 80 us).
+    struct Field {
+        void* out;
+        size_t bytes;
+        void* to;  // where the kernel writes
+        const char* what;
+    } field[4] = {{rng, sizeof(uint4) * n, direct_out<uint4>(rng, n), "download rng"},
+                  {pos, sizeof(float2) * n, direct_out<float2>(pos, n), "download pos"},
+                  {heading, sizeof(uint32_t) * n, direct_out<uint32_t>(heading, n), "download heading"},
+                  {speed, sizeof(float) * n, direct_out<float>(speed, n), "download speed"}};
+    size_t staged = n * kStateRecordBytes;
+    for (const Field& f : field)
+        if (f.out && !f.to) staged += f.bytes;
+    if ((rc = ensure_stage(c, staged)) != MSIM_OK) return rc;
+    char* next = static_cast<char*>(c->stage) + n * kStateRecordBytes;
+    bool copied[4] = {};
+    for (int k = 0; k < 4; k++) {
+        if (!field[k].out || field[k].to) continue;
+        field[k].to = next;
+        next += field[k].bytes;
+        copied[k] = true;
+    }
     {
         Prof p(c, K_EXPORT);
         c->launch_count++;  // two kernels
-        CK(launch_export_state(c->stream, cur_state(c), c->n, to_pos, to_head, to_rng, to_speed, c->stage, c->err,
-                               c->status_host),
+        CK(launch_export_state(c->stream, cur_state(c), c->n, static_cast<float2*>(field[1].to),
+                               static_cast<uint32_t*>(field[2].to), static_cast<uint4*>(field[0].to),
+                               static_cast<float*>(field[3].to), c->stage, c->err, c->status_host),
            "k_export_state");
     }
-    if (to_pos == d_pos && pos)
-        CK(cudaMemcpyAsync(pos, d_pos, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream), "download pos");
-    if (to_head == d_head && heading)
-        CK(cudaMemcpyAsync(heading, d_head, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download heading");
-    if (to_rng == d_rng && rng)
-        CK(cudaMemcpyAsync(rng, d_rng, sizeof(uint4) * n, cudaMemcpyDeviceToHost, c->stream), "download rng");
-    if (to_speed == d_speed && speed)
-        CK(cudaMemcpyAsync(speed, d_speed, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream), "download speed");
+    for (int k = 0; k < 4; k++)
+        if (copied[k])
+            CK(cudaMemcpyAsync(field[k].out, field[k].to, field[k].bytes, cudaMemcpyDeviceToHost, c->stream),
+               field[k].what);
     return sync_and_check(c, true);
 }
 
@@ -1410,29 +1402,27 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     const size_t n = c->n, cap = c->params.cap;
     if (n == 0) return MSIM_OK;
     const bool want_idx = idx && cap;
-    if ((rc = ensure_stage(c, n * sizeof(uint32_t) * (1 + (want_idx ? cap : 0)))) != MSIM_OK) return rc;
-    uint32_t* d_idx = want_idx ? static_cast<uint32_t*>(c->stage) : nullptr;
-    uint32_t* d_count = static_cast<uint32_t*>(c->stage) + (want_idx ? n * cap : 0);
+    // lists by whole rows, 16 bytes at a time where they allow it
     const bool direct = n <= kDirectEntities;
-    uint32_t* to_count = direct ? direct_out<uint32_t>(count, n, d_count) : d_count;
+    uint32_t* to_count = direct ? direct_out<uint32_t>(count, n) : nullptr;
     uint32_t* to_idx = nullptr;
-    if (want_idx) {
-        // whole rows, 16 bytes at a time where they allow it
-        const size_t rows = std::max<size_t>(n * cap / 4, 1);
-        to_idx = direct || cap >= kDirectRow
-                     ? reinterpret_cast<uint32_t*>(direct_out<uint4>(idx, rows, reinterpret_cast<uint4*>(d_idx)))
-                     : d_idx;
-    }
+    if (want_idx && (direct || cap >= kDirectRow))
+        to_idx = reinterpret_cast<uint32_t*>(direct_out<uint4>(idx, std::max<size_t>(n * cap / 4, 1)));
+    const bool copy_count = !to_count, copy_idx = want_idx && !to_idx;
+    if ((rc = ensure_stage(c, n * sizeof(uint32_t) * ((copy_idx ? cap : 0) + (copy_count ? 1 : 0)))) != MSIM_OK) return rc;
+    uint32_t* const stage = static_cast<uint32_t*>(c->stage);
+    if (copy_idx) to_idx = stage;
+    if (copy_count) to_count = stage + (copy_idx ? n * cap : 0);
     {
         Prof p(c, K_EXPORT);
         CK(launch_export_neighbours(c->stream, c->query_slot, cur_state(c).slot_id, c->nbr_count, c->nbr_list,
                                     c->n, c->params.cap, to_count, to_idx, c->err, c->status_host),
            "k_export_nbr");
     }
-    if (to_count == d_count)
-        CK(cudaMemcpyAsync(count, d_count, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download counts");
-    if (want_idx && to_idx == d_idx)
-        CK(cudaMemcpyAsync(idx, d_idx, sizeof(uint32_t) * n * cap, cudaMemcpyDeviceToHost, c->stream),
+    if (copy_count)
+        CK(cudaMemcpyAsync(count, to_count, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c->stream), "download counts");
+    if (copy_idx)
+        CK(cudaMemcpyAsync(idx, to_idx, sizeof(uint32_t) * n * cap, cudaMemcpyDeviceToHost, c->stream),
            "download neighbours");
     return sync_and_check(c, true);
 }
