@@ -73,7 +73,7 @@ struct AdjArgs {
 // entity at K = 100) of the resident threads then mostly stays in the L2 it is read back
 // from (7 blocks of 128 threads 2.63 ms; 6 3.01, 8 at fewer registers 2.96, 24 of 32 2.94).
 constexpr uint32_t kAdjForwardThreads = 32;
-constexpr int kAdjForwardBlocks = 28;
+constexpr int kAdjForwardBlocks = 32;
 constexpr uint32_t kAdjThreads = 128;
 constexpr int kAdjBackwardBlocks = 7;
 
@@ -179,7 +179,7 @@ __device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
 // sums (32-bit within a stretch).  Bound by issue (83 % active): 105 warp instructions
 // per tick against 190 with the road reloaded, two conversions and a flush at every
 // cell change; 262,144 entities x 2,000 ticks 3.13 -> 1.68 ms, with the coordinates in
-// paired instructions 1.59.
+// paired instructions 1.59, at 32 blocks per SM 1.57.
 template <int RNG, bool REPLAY>
 __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
     __shared__ LeftBlocks left;
