@@ -43,11 +43,11 @@ SPEED = (1.0, 1.6)
 B_STEP = 24  # algorithmic bytes per entity-step of the move (pos r/w 16, heading 4, speed 4)
 ADJ_GRID = (512, 512)
 ADJ_K = 100
-# algorithmic bytes per entity-tick of the calibration step: forward B_step + splat
-# position read 8; backward recompute B_step + splat position read 8 + reverse
-# (position and adjoint read + write) 16
-ADJ_FWD_BYTES = B_STEP + 8
-ADJ_BWD_BYTES = B_STEP + 8 + 16
+# bytes per entity-tick that the calibration step cannot do without: a checkpoint (28 B)
+# every ADJ_K ticks and one schedule bit per tick, written by the forward and read by the
+# backward, which also writes and reads back the positions of a segment (8 + 8 B)
+ADJ_FWD_BYTES = 28 / ADJ_K + 1 / 8
+ADJ_BWD_BYTES = ADJ_FWD_BYTES + 16
 
 
 def b_nbr(k_mean: float, updates_per_tick: float = 1.0) -> float:
@@ -77,22 +77,22 @@ KERNEL_BYTES = {
     "k_step_multi": lambda k: B_STEP,      # per tick
 }
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per entity and launch of
-# one ncu capture of the same workload at full size (third neighbour tick; 1-pass
-# metrics; profiles/scale_16M_dram_traffic.md); scaled by the entities of the run
 # warp instructions per entity-step of k_batch_step: smsp__inst_executed.sum of one
-# ncu capture (405.8 M for 64 instances, 2,058,939 entities, 100 ticks, tuned
-# schedule; profiles/batched_64_instances_k_batch_step_issue.md) over entities x ticks
-NCU_BATCH_WARP_INSTR_PER_ENTITY_STEP = 1.971
-# warp instructions per entity of k_query on a reused index (widened boxes):
-# smsp__inst_executed.sum of one ncu capture (96.2 M for 4,000,000 entities on the
-# 512 x 512 lattice, the 16 M and 1 M workloads' density;
-# profiles/mid_4M_k_query_widened_ncu.md)
-NCU_QUERY_WARP_INSTR_PER_ENTITY = 24.04
-
+# ncu capture (300.5 M for 64 instances, 2,058,939 entities, 100 ticks, default
+# schedule; profiles/kernels_issue_and_dram.md) over entities x ticks
+NCU_BATCH_WARP_INSTR_PER_ENTITY_STEP = 1.459
+# warp instructions per entity of k_query, mean over the queries of an index's reuse
+# (two that keep pair lists, 31.8, and 28 that read them, 12.0): smsp__inst_executed.sum
+# of an ncu capture of 4,000,000 entities on the 512 x 512 lattice, the 16 M and 1 M
+# workloads' density (profiles/kernels_issue_and_dram.md)
+NCU_QUERY_WARP_INSTR_PER_ENTITY = 13.33
+# warp instructions per entity-tick of the calibration kernels: smsp__inst_executed.sum of
+# one ncu capture (262,144 entities x 200 ticks, K = 100: 154.2 M and 205.8 M)
+NCU_ADJ_WARP_INSTR_PER_ENTITY_TICK = {"k_adj_forward": 2.941, "k_adj_backward": 3.925}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per entity and launch of the
+# same capture (a working set above L2), scaled by the entities of the run
 NCU_DRAM_BYTES_PER_ENTITY = {
-    "scale": {"k_query": 26.87},
-    "neighbours": {"k_query": 24.07, "k_onesweep": 6.91},
+    "scale": {"k_query": 24.2, "k_move": 26.3, "k_step": 34.3, "k_place": 30.0, "k_mark": 9.8},
 }
 
 
@@ -155,6 +155,7 @@ class ClockSampler:
     def __init__(self, gpu_index: int):
         self.gpu = gpu_index
         self.proc = None
+        self.result = None
         self.path = Path(tempfile.gettempdir()) / f"msim_clocks_{os.getpid()}_{gpu_index}.csv"
 
     def __enter__(self):
@@ -179,6 +180,12 @@ class ClockSampler:
             self.f.close()
 
     def summary(self):
+        """The samples' summary (read once, when first asked for)."""
+        if self.result is None:
+            self.result = self._read()
+        return self.result
+
+    def _read(self):
         if not self.proc or not self.path.exists():
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["unsampled"]}
         rows = []
@@ -265,8 +272,7 @@ def run_ours(args, cfg, world, rank, local):
     sim.set_profiling(False)
     total_ms = sum(v["ms"] for v in stats.values()) or 1.0
     peak, peak_kind = peaks()
-    # entries per radix pass: n for a full sort, the entries whose key changed for an
-    # incremental update (every pass of an update sorts the same entries)
+    # entries per radix pass (full sorts) or counting update: n
     sorted_per_update = sort["sorted_entries"] / sort["index_updates"] if sort["index_updates"] else float(n)
     kernels = {}
     for name, v in stats.items():
@@ -582,10 +588,9 @@ def run_adjoint(args, world, rank, local):
     fwd_ms = ph["forward"] + ph["loss"]
     bwd_ms = ph["backward_sweeps"] + ph["road_reduction"]
     peak, peak_kind = peaks()
-    S = (T + ADJ_K - 1) // ADJ_K
     kern = {"k_adj_forward": {"launches": 1, "avg_ms": ph["forward"], "algo_bytes_per_launch": ADJ_FWD_BYTES * n * T},
-            "k_adj_backward": {"launches": S, "avg_ms": ph["backward_sweeps"] / S,
-                               "algo_bytes_per_launch": ADJ_BWD_BYTES * n * ADJ_K}}
+            "k_adj_backward": {"launches": 1, "avg_ms": ph["backward_sweeps"],
+                               "algo_bytes_per_launch": ADJ_BWD_BYTES * n * T}}
     tot = sum(v["avg_ms"] * v["launches"] for v in kern.values())
     for v in kern.values():
         v["share"] = v["avg_ms"] * v["launches"] / tot
@@ -594,7 +599,17 @@ def run_adjoint(args, world, rank, local):
     roofline = {"bound": "hbm", "kernel": dom_name, "achieved": round(dom["achieved_gbs"], 1), "peak": peak,
                 "unit": "GB/s", "frac": round(dom["achieved_gbs"] / peak, 4), "traffic": None,
                 "peak_source": peak_kind,
-                "note": f"algorithmic bytes per entity-tick: forward {ADJ_FWD_BYTES}, backward {ADJ_BWD_BYTES}"}
+                "note": "not the bound: the state stays in registers between checkpoints (bytes per entity-tick: "
+                        f"forward {ADJ_FWD_BYTES:.2f}, backward {ADJ_BWD_BYTES:.2f}); see issue"}
+    # both kernels are bound by instruction issue: warp instructions per entity-tick (ncu)
+    # against one per cycle on each of the 4 schedulers of the 152 SMs
+    sm_mhz = clocks.summary().get("sm_mhz") or 2070.0
+    issue_peak = 152 * 4 * sm_mhz * 1e6
+    inst_s = NCU_ADJ_WARP_INSTR_PER_ENTITY_TICK[dom_name] * n * T / (dom["avg_ms"] / 1e3)
+    roofline["issue"] = {"bound": "issue", "achieved": round(inst_s, 1), "peak": issue_peak,
+                         "unit": "warp-instructions/s", "frac": round(inst_s / issue_peak, 4),
+                         "warp_instructions_per_entity_tick": NCU_ADJ_WARP_INSTR_PER_ENTITY_TICK[dom_name],
+                         "sm_mhz": sm_mhz}
     # end to end through the public API with host buffers: speeds and factors from
     # pinned host memory, forward + backward, gradients and loss back to the host
     e2e = None
@@ -627,7 +642,8 @@ def run_adjoint(args, world, rank, local):
             "kernels": kern, "phases_ms": ph, "forward_ms": fwd_ms, "backward_ms": bwd_ms,
             "backward_over_forward": bwd_ms / fwd_ms, "step_over_forward": (fwd_ms + bwd_ms) / fwd_ms,
             "loss": loss0, "roads": rm.num_roads, "e2e": e2e, "cpu": cpu,
-            "launches": args.steps * (3 + S + 3 + 3 + 2)}
+            # gather, forward, loss x 2; backward, record scan, pack, two radix passes, road sums
+            "launches": args.steps * 10}
 
 
 def cpu_adjoint(orc, rm, n, ticks, threads):
