@@ -20,10 +20,11 @@ extern "C" {
 #endif
 
 #define MSIM_FAULT_NONE 0u
-/* The next index update's first look-back chain (the split of an incremental update,
+/* The next index update's first look-back chain (the key scan of a counting update,
  * or the first radix pass of a full sort) starts handing out tiles at tile 1: tile 1
  * waits for tile 0, which never publishes, until its bounded wait (msim_set_wait_limit)
- * runs out.  Needs a chain of at least two tiles (4,096 entities for either). */
+ * runs out.  Needs a chain of at least two tiles (more than 4,096 keys, which about
+ * 1,000 entities have, or entities). */
 #define MSIM_FAULT_SORT_TILE 1u
 /* The (arg+1)-th kernel launch of the following msim_step calls reports
  * cudaErrorLaunchFailure instead of being issued; msim_step returns MSIM_ERR_CUDA. */

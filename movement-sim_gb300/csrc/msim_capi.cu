@@ -143,8 +143,8 @@ struct msim_ctx {
     bool chain_broken = false;      // a pass failed to launch: the regions' state is unknown
     size_t sort_region = 0;
     // The index the query reads (current buffer set).  Two sets, paired with the two
-    // sorted-slot buffers: a tick's merge writes the set the previous tick's query does
-    // not read, so that query overlaps the next tick up to its merge.
+    // sorted-slot buffers: a tick's update writes the set the previous tick's query does
+    // not read, so that query overlaps the next tick up to its update.
     uint32_t* kstart = nullptr;  // first sorted position of every key, 2^key_bits + 1 entries
     uint4* kstart_chunks = nullptr;  // long key gaps, filled by a second kernel
     float2* sorted_pos = nullptr;    // positions in sorted order (the query's candidates)
@@ -196,7 +196,7 @@ struct msim_ctx {
     uint32_t* pair_ids = nullptr;
     int64_t pair_until = -1;
     // rank[slot] = sorted position of the slot in the current index, written by the
-    // merge once allocated (rank_valid: it describes the current index); a reusing
+    // update once allocated (rank_valid: it describes the current index); a reusing
     // tick's move then writes each position there itself (no gather pass)
     uint32_t* rank = nullptr;
     bool rank_valid = false;
@@ -866,8 +866,9 @@ int neighbour_tick(msim_ctx* c) {
     // the reach, the tick moves the entities (each position also written at its sorted
     // position in the index, by the ranks of the last update, or gathered there after
     // a full sort) and queries the index built reuse_ticks + 1 ticks before; the
-    // widening costs about 10 % of the query over a reuse window at 16 M (0.40 ms
-    // against 0.36-0.39), the update it skips (split, passes, merge) about 0.30 ms.
+    // widening costs about 10 % of a looked-up query over a reuse window at 16 M, the
+    // update it skips (key scan and placement) 0.23 ms, and the pair lists serve only
+    // ticks that reuse an index.
     const double ticks = c->reuse_ticks >= 0 ? (double)c->reuse_ticks + 1.0 : 0.0;
     bool reuse = false;
     if (c->reuse && c->sorted_slot && !c->order_identity && c->reuse_ticks >= 0 && c->grid.reach > 0.f &&
@@ -1459,9 +1460,9 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     const int old = c->cur;
     const int b = 1 - old;
     EntityState& s = c->st[b];
-    // The previous index stays a valid starting order for an incremental update when
-    // its slots already held entity ids (the previous call was a host tick, or a set
-    // followed by one tick): the new state goes to the same slots.
+    // The index can be updated by counting when its slots already held entity ids (the
+    // previous call was a host tick, or a set followed by one tick): the new state goes to
+    // the same slots.
     const bool old_slots_identity = c->slots_identity;
     const bool use_inc = nbr && c->incremental && c->sorted_slot && c->slots_identity;
     // Skin query: when the current index was built from the keys of the state this

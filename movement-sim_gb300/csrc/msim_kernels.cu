@@ -33,8 +33,8 @@ constexpr uint32_t kValueMask = 0x3fffffffu;
 // limit (msim_set_wait_limit) defaults to kDefaultSpinLimit, about a second
 constexpr int kLookBack = 4;               // predecessor tiles read per look-back round of a radix pass
 
-// Kernels of the per-tick chain (move, split, radix passes, merge, key-start fill,
-// re-ordering) are launched with programmatic stream serialisation: a chain kernel
+// Kernels of the per-tick chain (move, radix passes or key scan and placement, key-start
+// fill, re-ordering) are launched with programmatic stream serialisation: a chain kernel
 // lets the next one launch once all its own blocks run, and waits for its
 // predecessor to finish, with its writes visible, before it touches global memory.
 // Only the launch and block dispatch overlap the predecessor's tail.  A dependent is
@@ -351,10 +351,9 @@ __global__ __launch_bounds__(kStepThreads, 4) void k_step(StepLaunch a) {
 // rank their ROWS x 256 items with warp-level multi-split (__match_any_sync) into
 // per-warp digit counters, publish per-digit counts and resolve their global
 // offsets by looking back over earlier tiles.  Every wait is bounded.  Tiles hold
-// 4096 items, or 1024 when the count is known only on the device: those passes sort
-// the few changed entries of an incremental update (about 230 K of 16 M), where a
-// pass lasts about as long as one tile takes, so smaller tiles finish sooner
-// (measured at 16 M: 15.7 us per pass against 22.9 with 4096).
+// 4096 items, or 1024 when the count is known only on the device and small (the records
+// of a small calibration), where a pass lasts about as long as one tile takes, so smaller
+// tiles finish sooner (measured over 230 K items: 15.7 us per pass against 22.9 with 4096).
 //
 // chain (pointers NULL: the caller clears the look-back words and the ticket):
 // before its tiles, the pass zeroes the next pass's look-back words that their last
