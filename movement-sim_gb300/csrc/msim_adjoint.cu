@@ -39,6 +39,7 @@
 
 #include <cuda_runtime.h>
 
+#include "msim_chain.cuh"
 #include "msim_internal.h"
 #include "msim_kernels.cuh"
 
@@ -183,6 +184,7 @@ __device__ __forceinline__ void flush_left(LeftBlocks& left, const AdjArgs& a) {
 template <int RNG, bool REPLAY>
 __global__ __launch_bounds__(kAdjForwardThreads, kAdjForwardBlocks) void k_adj_forward(AdjArgs a) {
     __shared__ LeftBlocks left;
+    chain_enter();
     const uint32_t e = adj_entity(a.n, a.lanes);
     left.n[threadIdx.x] = 0u;
     const unsigned warp_mask = __ballot_sync(0xffffffffu, e != 0xffffffffu);
@@ -275,6 +277,7 @@ __global__ __launch_bounds__(256) void k_adj_loss(const unsigned long long* __re
                                                   const float* __restrict__ target, uint32_t G, uint32_t ticks,
                                                   float* density, float* lambda, double* partial) {
     __shared__ double s_sum[256];
+    chain_enter();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     double d2 = 0.0;
     if (g < G) {
@@ -298,6 +301,7 @@ __global__ __launch_bounds__(256) void k_adj_loss(const unsigned long long* __re
 __global__ __launch_bounds__(256) void k_adj_loss_final(const double* partial, uint32_t blocks, uint32_t G,
                                                         double* loss) {
     __shared__ double s_sum[256];
+    chain_enter();
     double s = 0.0;
     for (uint32_t b = threadIdx.x; b < blocks; b += 256u) s += partial[b];
     s_sum[threadIdx.x] = s;
@@ -366,6 +370,7 @@ __device__ __noinline__ SplatGrad splat_grad(const float* lambda, uint32_t gw, u
 // with the coordinates in paired instructions 2.52.
 template <int RNG>
 __global__ __launch_bounds__(kAdjThreads, kAdjBackwardBlocks) void k_adj_backward(AdjBack b) {
+    chain_enter();
     const AdjArgs& a = b.f;
     const uint32_t e = adj_entity(a.n, a.lanes);
     if (e == 0xffffffffu) return;
@@ -518,6 +523,7 @@ __global__ __launch_bounds__(1024) void k_adj_rec_scan(uint32_t* rec_block, uint
                                                        uint32_t* total, uint32_t* hist) {
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_run;
+    chain_enter();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     if (tid < kMaxPasses * kRadix) hist[tid] = 0u;
     if (tid == 0) s_run = 0u;
@@ -557,6 +563,7 @@ __global__ __launch_bounds__(256) void k_adj_rec_pack(const uint2* __restrict__ 
     __shared__ uint32_t s_first[kRecBlock + 1];  // records before each entity of the block
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_hist[kMaxPasses * kRadix];
+    chain_enter();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     for (uint32_t i = tid; i < passes * kRadix; i += 256u) s_hist[i] = 0u;
     const uint32_t e0 = blockIdx.x * kRecBlock;
@@ -605,6 +612,7 @@ __global__ __launch_bounds__(256) void k_adj_rec_pack(const uint2* __restrict__ 
 __global__ __launch_bounds__(256) void k_adj_road_sum(const uint32_t* __restrict__ key, const float* __restrict__ val,
                                                       const uint32_t* __restrict__ total, uint32_t num_roads,
                                                       double* gfactor, float* out, const uint32_t* err) {
+    chain_enter();
     constexpr uint32_t FULL = 0xffffffffu;
     const uint32_t rd = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (rd >= num_roads || (*err & kErrTimeout)) return;  // uniform per warp
@@ -1020,10 +1028,10 @@ int msim_adj_forward(msim_adj* a, const float* d_speed, const float* d_factor, c
     ACK(cudaGetLastError(), "k_adj_forward");
     cudaEventRecord(a->ph[1], a->stream);
     const unsigned gb = (unsigned)((G + 255) / 256);
-    k_adj_loss<<<gb, 256, 0, a->stream>>>(a->dacc, a->target, (uint32_t)G, a->p.ticks, a->density, a->lambda,
-                                          a->partial);
-    k_adj_loss_final<<<1, 256, 0, a->stream>>>(a->partial, gb, (uint32_t)G, a->loss);
-    ACK(cudaGetLastError(), "k_adj_loss");
+    ACK(launch_chained(k_adj_loss, gb, 256, a->stream, a->dacc, a->target, (uint32_t)G, a->p.ticks, a->density,
+                       a->lambda, a->partial),
+        "k_adj_loss");
+    ACK(launch_chained(k_adj_loss_final, 1, 256, a->stream, a->partial, gb, (uint32_t)G, a->loss), "k_adj_loss_final");
     cudaEventRecord(a->ph[2], a->stream);
     if (d_density)
         ACK(cudaMemcpyAsync(d_density, a->density, sizeof(float) * G, cudaMemcpyDeviceToDevice, a->stream), "density");
@@ -1061,10 +1069,11 @@ int msim_adj_backward(msim_adj* a, float* d_grad_speed, float* d_grad_factor) {
     cudaEventRecord(a->ph[4], a->stream);
     // road gradients: the records packed, stably sorted by road, summed per road
     const uint32_t rec_blocks = (a->n + kRecBlock - 1u) / kRecBlock;
-    k_adj_rec_scan<<<1, 1024, 0, a->stream>>>(a->rec_block, a->rec_base, rec_blocks, a->rec_total, a->hist);
-    k_adj_rec_pack<<<rec_blocks, 256, 0, a->stream>>>(a->rec, a->rec_used, a->rec_base, a->n, a->S * kRecPerSeg,
-                                                      a->passes, a->sk[0], a->sv[0], a->hist);
-    ACK(cudaGetLastError(), "k_adj_rec_pack");
+    ACK(launch_chained(k_adj_rec_scan, 1, 1024, a->stream, a->rec_block, a->rec_base, rec_blocks, a->rec_total, a->hist),
+        "k_adj_rec_scan");
+    ACK(launch_chained(k_adj_rec_pack, rec_blocks, 256, a->stream, a->rec, a->rec_used, a->rec_base, a->n,
+                       a->S * kRecPerSeg, a->passes, a->sk[0], a->sv[0], a->hist),
+        "k_adj_rec_pack");
     // with two or more passes each clears the next one's look-back words and ticket
     const bool chained = a->passes >= 2;
     if (!a->sort_clean || !chained) {
@@ -1087,10 +1096,10 @@ int msim_adj_backward(msim_adj* a, float* d_grad_speed, float* d_grad_factor) {
             "k_onesweep");
     }
     a->sort_clean = true;
-    k_adj_road_sum<<<(a->R + 7u) / 8u, 256, 0, a->stream>>>(a->sk[a->passes & 1],
-                                                          reinterpret_cast<const float*>(a->sv[a->passes & 1]),
-                                                          a->rec_total, a->R, a->gfactor, d_grad_factor, a->err);
-    ACK(cudaGetLastError(), "k_adj_road_sum");
+    ACK(launch_chained(k_adj_road_sum, (a->R + 7u) / 8u, 256, a->stream, a->sk[a->passes & 1],
+                       reinterpret_cast<const float*>(a->sv[a->passes & 1]), a->rec_total, a->R, a->gfactor, d_grad_factor,
+                       a->err),
+        "k_adj_road_sum");
     cudaEventRecord(a->ph[5], a->stream);
     a->have_backward = true;
     return check_status(a);

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "msim_chain.cuh"
 #include "msim_kernels.cuh"
 
 namespace msim {
@@ -32,18 +33,6 @@ constexpr uint32_t kValueMask = 0x3fffffffu;
 // polls of a look-back word before a wait gives up with kErrTimeout: the per-context
 // limit (msim_set_wait_limit) defaults to kDefaultSpinLimit, about a second
 constexpr int kLookBack = 4;               // predecessor tiles read per look-back round of a radix pass
-
-// Kernels of the per-tick chain (move, radix passes or key scan and placement, key-start
-// fill, re-ordering) are launched with programmatic stream serialisation: a chain kernel
-// lets the next one launch once all its own blocks run, and waits for its
-// predecessor to finish, with its writes visible, before it touches global memory.
-// Only the launch and block dispatch overlap the predecessor's tail.  A dependent is
-// launched only when every block of its predecessor is resident, so waiting blocks
-// never keep a predecessor's block from being scheduled.
-__device__ __forceinline__ void chain_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -624,6 +613,7 @@ struct __align__(32) StateRecord {
     uint32_t w[8];  // rng, pos, heading, speed
 };
 __global__ __launch_bounds__(256) void k_export_records(EntityState st, uint32_t n, StateRecord* __restrict__ out) {
+    chain_enter();
     const uint32_t s = blockIdx.x * 256u + threadIdx.x;
     if (s >= n) return;
     const uint32_t id = st.slot_id[s];
@@ -640,6 +630,7 @@ __global__ __launch_bounds__(256) void k_export_records(EntityState st, uint32_t
 __global__ __launch_bounds__(256) void k_export_fields(const StateRecord* __restrict__ in, uint32_t n, float2* pos,
                                                        uint32_t* head, uint4* rng, float* speed, const uint32_t* err,
                                                        uint32_t* status_out) {
+    chain_enter();
     const uint32_t id = blockIdx.x * 256u + threadIdx.x;
     if (id == 0 && status_out) *status_out = *err;
     if (id >= n) return;
@@ -843,22 +834,6 @@ uint32_t warp_lanes(uint32_t n, int sms) {
     uint32_t lanes = 32;
     while (lanes > kFewestLanes && n / lanes < kFewWarps * 4u * (uint32_t)std::max(sms, 1)) lanes /= 2;
     return lanes;
-}
-
-// Launch of a chain kernel (see chain_enter).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 }  // namespace
@@ -1135,9 +1110,9 @@ cudaError_t launch_export_state(cudaStream_t s, EntityState st, uint32_t n, floa
                                 float* speed, void* records, const uint32_t* err, uint32_t* status_out) {
     if (n == 0) return cudaSuccess;
     StateRecord* rec = static_cast<StateRecord*>(records);
-    k_export_records<<<blocks_for(n, 256), 256, 0, s>>>(st, n, rec);
-    k_export_fields<<<blocks_for(n, 256), 256, 0, s>>>(rec, n, pos, head, rng, speed, err, status_out);
-    return cudaGetLastError();
+    cudaError_t e = launch_chained(k_export_records, blocks_for(n, 256), 256, s, st, n, rec);
+    if (e != cudaSuccess) return e;
+    return launch_chained(k_export_fields, blocks_for(n, 256), 256, s, rec, n, pos, head, rng, speed, err, status_out);
 }
 
 cudaError_t launch_export_neighbours(cudaStream_t s, const uint32_t* sorted_slot, const uint32_t* slot_id,

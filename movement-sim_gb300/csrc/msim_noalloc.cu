@@ -31,6 +31,7 @@
 
 #include <cuda_runtime.h>
 
+#include "msim_chain.cuh"
 #include "msim_internal.h"
 #include "msim_kernels.cuh"
 
@@ -57,11 +58,6 @@ struct CellGrid {
     float inv_cell, radius, d2_limit;
     uint32_t nx, ny, pitch;  // cell (x, y) is y * pitch + x
 };
-
-__device__ __forceinline__ void chain_enter() {  // see msim_kernels.cu
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 __device__ __forceinline__ uint32_t cell_of(const CellGrid& g, float2 p) {
     return tile_coord(p.y, g.inv_cell, g.ny) * g.pitch + tile_coord(p.x, g.inv_cell, g.nx);
@@ -214,23 +210,6 @@ __global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t*
     }
 }
 
-// Launch that may start under its predecessor's tail (see chain_enter).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                           Args... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 // Per-device set-up: the scratch array's device address (the host-side symbol is
 // only a stand-in, never a usable device pointer) and the query's shared-memory limit.
 struct DeviceSlot {
@@ -317,12 +296,12 @@ extern "C" int msim_query_neighbours_noalloc(const float* d_pos, uint32_t n, flo
     const bool quads = (cap & 3u) == 0u && (reinterpret_cast<uintptr_t>(d_idx) & 15u) == 0u;
 
     bool ok = cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * (kOffCount - kOffCursor + cells), s) == cudaSuccess;
-    ok = ok && launch_chained(k_noalloc_rank, blocks, 256, 0, s, pos, n, g, count, w + kOffRank, d_status) == cudaSuccess;
-    ok = ok && launch_chained(k_noalloc_scan, (cells + kScanCells - 1u) / kScanCells, 256, 0, s, count, cells,
+    ok = ok && launch_chained(k_noalloc_rank, blocks, 256, s, pos, n, g, count, w + kOffRank, d_status) == cudaSuccess;
+    ok = ok && launch_chained(k_noalloc_scan, (cells + kScanCells - 1u) / kScanCells, 256, s, count, cells,
                               w + kOffStart, cursor) == cudaSuccess;
-    ok = ok && launch_chained(k_noalloc_scatter, blocks, 256, 0, s, pos, n, g, w + kOffStart, w + kOffRank, cell_pos,
+    ok = ok && launch_chained(k_noalloc_scatter, blocks, 256, s, pos, n, g, w + kOffStart, w + kOffRank, cell_pos,
                               w + kOffId) == cudaSuccess;
-    ok = ok && launch_chained(quads ? k_noalloc_query<true> : k_noalloc_query<false>,
+    ok = ok && launch_chained_shared(quads ? k_noalloc_query<true> : k_noalloc_query<false>,
                               (n + kQueryThreads - 1) / kQueryThreads, kQueryThreads,
                               (size_t)cap * kQueryThreads * sizeof(uint32_t), s, w + kOffId, cell_pos, w + kOffStart,
                               count, g, n, cap, d_count, d_idx) == cudaSuccess;
