@@ -176,8 +176,8 @@ __device__ __forceinline__ uint32_t key_rank(uint32_t key, bool valid, uint32_t 
 // still spreads over many SMs.  ONE: a single tick (the tick that reuses the index
 // places its positions too); else several ticks with the state and the road's leg in
 // registers between them, bound by the ticks' serial chain (small counts) or by issue:
-// with read-back, 10,000 entities for 1,000 ticks 316 -> 123 us and 1 M for 200 ticks
-// 865 -> 470 us against reloading the road and three intrinsics every tick.  A run's
+// with read-back, 10,000 entities for 1,000 ticks 316 -> 118 us and 1 M for 200 ticks
+// 865 -> 448 us against reloading the road and three intrinsics every tick.  A run's
 // blocks take one entity per thread and no more (the scheduler fills places as they come
 // free; a grid of 16 blocks per SM with 12 resident left its last blocks to run alone: 1 M
 // x 200 ticks 312 us, so 287, with the coordinates in paired instructions 268).
