@@ -1203,8 +1203,11 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     if (e == cudaSuccess) e = cudaMemsetAsync(c->sort_dirty, 0, sizeof(uint32_t) * kMaxPasses, c->stream);
     // the index buffers start zeroed (every slot and key in range), so even an index
     // update that was cut short leaves nothing out of range behind
+    // the pair counters too: a query zeroes the next one's counters that have a thread, and
+    // those past the threads of a small context are never added to
     for (int b = 0; b < 2 && e == cudaSuccess; b++) {
-        e = cudaMemsetAsync(c->sk[b], 0, sizeof(uint32_t) * std::max<size_t>(n, 1), c->stream);
+        e = cudaMemsetAsync(c->pairs_b[b], 0, sizeof(unsigned long long) * kPairBins, c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->sk[b], 0, sizeof(uint32_t) * std::max<size_t>(n, 1), c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(c->sv[b], 0, sizeof(uint32_t) * std::max<size_t>(n, 1), c->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(c->kstart_b[b], 0, sizeof(uint32_t) * (c->num_keys + 1), c->stream);
     }
