@@ -983,7 +983,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
         CK(cudaEventRecord(c->ev_tick[2], qs), "cudaEventRecord");
         c->tick_recorded = true;
     }
-    c->pairs_zeroed = true;
+    c->pairs_zeroed = !disp;  // a widened query may do nothing: the host that reads d knows
     c->query_slot = c->sorted_slot;
     c->have_nbr = true;
     c->since_permute++;
@@ -1705,6 +1705,7 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
         c->last_disp = d;
         first_bad = ~words[1];
         status = words[2];
+        c->pairs_zeroed = d <= kWidenLimit * c->grid.reach && !(status & kErrTimeout);  // the query ran
     } else {
         CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
     }
@@ -1727,7 +1728,6 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
         if (!(d <= kWidenLimit * c->grid.reach)) {
             // too far for the previous index (also a non-finite position): the query did
             // nothing and runs on the new one
-            c->pairs_zeroed = false;
             {
                 Prof p(c, K_GATHER);
                 CK(launch_gather_chunk(c->stream, c->sorted_slot, n, 0, n, s.pos, c->skin_pos), "k_gather_chunk");
