@@ -730,6 +730,15 @@ void reset_index(msim_ctx* c) {
     c->since_permute = c->resort;
 }
 
+// The same after a device wait gave up: look-back regions, key counters and pair counters
+// hold whatever the kernels that skipped their work left.
+void restart_index(msim_ctx* c) {
+    c->chain_broken = true;
+    c->counts_pending = true;
+    c->pairs_zeroed = false;
+    reset_index(c);
+}
+
 // tick-0 index: the reference's first dispatch only inserts every entity into its
 // tree (random_move.comp:863-867); here: sort by tile and re-order the state.
 int build_index(msim_ctx* c) {
@@ -1012,10 +1021,7 @@ int sync_and_check(msim_ctx* c, bool status_queued = false) {
             // The kernels that read the index skipped their work after the wait gave
             // up, so the entity state is intact; the index is rebuilt from scratch (full
             // sort, every look-back region zeroed again) by the next neighbour tick.
-            c->chain_broken = true;
-            c->pairs_zeroed = false;  // its query skipped its work
-            c->counts_pending = true;
-            reset_index(c);
+            restart_index(c);
             return fail(MSIM_ERR_TIMEOUT, "a bounded device wait (index look-back) gave up; the neighbour results "
                                           "since the last successful sync are invalid, the entity state is kept");
         }
@@ -1712,7 +1718,9 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     if (first_bad != 0xffffffffu) {  // as msim_set_entities: the previous state stays
         CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
         c->cur = old;
-        reset_index(c);
+        // the status is cleared with this tick's own bits, so a wait that gave up in the update
+        // the call before left running is recovered from here, as in sync_and_check
+        restart_index(c);
         c->slots_identity = old_slots_identity;
         c->tick--;
         CK(cudaMemsetAsync(c->err, 0, sizeof(uint32_t), c->stream), "clear device status");

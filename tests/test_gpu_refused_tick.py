@@ -49,3 +49,42 @@ def test_refused_host_tick_leaves_no_counts(msim, pinned, moved):
             assert a.collision_pairs() == b.collision_pairs(), f"at tick {t + 1}"
         for buf in bufs.values():
             buf.free()
+
+
+def test_time_out_before_a_refused_host_tick(msim, orc):
+    """Refused while the index update that the call before left running had given up: the
+    key counters are zeroed before they count again, so the ticks after it match the oracle
+    (whole numbers and the same binary32 operations)."""
+    rm = msim.RoadMap.lattice(32, 3)
+    n, cap = 150_000, 8
+    pos, head, rng, speed = orc.init_entities(rm.road_pos, n, 1, 11, 1, 1.0, 1.6)
+    with msim.Simulation(rm, n, rng="pcg32", dt=0.1, radius=2.0, cap=cap) as sim:
+        state = {"pos": pos.copy(), "heading": head.copy(), "rng": rng.copy(), "speed": speed}
+
+        def host_tick(what):
+            nonlocal state
+            got = sim.tick_host(state, neighbours=True, with_idx=True)
+            orc.step(rm.road_pos, rm.road_conn, rm.connections, pos, head, rng, speed, 1, 0.1, 1, threads=8)
+            assert np.array_equal(got["pos"].view(np.uint32), pos.view(np.uint32)), what
+            count, idx, pairs = orc.neighbours(pos, 2.0, cap, threads=8)
+            assert np.array_equal(got["count"], count) and np.array_equal(got["idx"], idx), what
+            assert sim.collision_pairs() == pairs, what
+            state = {"pos": got["pos"].copy(), "heading": got["heading"].copy(), "rng": got["rng"].copy(),
+                     "speed": speed}
+
+        for t in range(2):
+            host_tick(f"tick {t + 1}")
+        sim.set_wait_limit(2048)
+        sim.inject_fault(msim._capi.FAULT_SORT_TILE)  # the update after this tick's query gives up
+        state = sim.tick_host(state, neighbours=True) | {"speed": speed}
+        orc.step(rm.road_pos, rm.road_conn, rm.connections, pos, head, rng, speed, 1, 0.1, 1, threads=8)
+        bad = {k: v.copy() for k, v in state.items()}
+        bad["heading"][3] = rm.num_roads
+        with pytest.raises(msim.MsimError) as e:
+            sim.tick_host(bad, neighbours=True)
+        assert e.value.code == 2
+        sim.set_wait_limit(0)
+        state = {k: state[k] for k in ("pos", "heading", "rng", "speed")}
+        for t in range(5):
+            host_tick(f"tick {t + 1} after the refusal")
+        sim.sync()
