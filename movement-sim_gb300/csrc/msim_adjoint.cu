@@ -699,7 +699,7 @@ struct msim_adj {
     bool sort_clean = false;          // regions, tickets and extents are as the chained passes expect
     uint32_t lanes = 32;
     uint32_t* err = nullptr;
-    uint32_t* status_host = nullptr; // page-locked copy of *err
+    StatusWord status_host;          // page-locked copy of *err
     uint32_t* perm = nullptr;        // device: entity id of each internal index
     std::vector<uint32_t> hperm;     // host copy
     size_t rec_count = 0;
@@ -728,7 +728,6 @@ int aalloc(msim_adj* a, T** ptr, size_t count) {
 void free_adj(msim_adj* a) {
     for (void* p : a->allocs) cudaFree(p);
     a->allocs.clear();
-    status_word_give(a->status_host);
     if (a->t0) cudaEventDestroy(a->t0);
     if (a->t1) cudaEventDestroy(a->t1);
     for (cudaEvent_t& ev : a->ph)
@@ -867,7 +866,7 @@ int msim_adj_create(const msim_map* map, const msim_adj_params* params, msim_adj
     a->lanes = adj_lanes(a->n, sms);
     cudaError_t e = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
-    if (!(a->status_host = status_word_take()))
+    if (!a->status_host.take())
         return bail(fail(MSIM_ERR_NOMEM, "page-locked allocation of the status word failed"));
     cudaEventCreate(&a->t0);
     cudaEventCreate(&a->t1);

@@ -182,7 +182,7 @@ struct msim_batch {
     size_t items_capacity = 0;
     uint32_t* ticket = nullptr;
     uint32_t* err = nullptr;
-    uint32_t* status_host = nullptr;  // page-locked copy of *err
+    StatusWord status_host;  // page-locked copy of *err
     float2* pos = nullptr;
     uint32_t* head = nullptr;
     uint4* rng = nullptr;
@@ -220,7 +220,6 @@ void free_batch(msim_batch* b) {
     drop_graphs(b);
     for (void* p : b->allocs) cudaFree(p);
     b->allocs.clear();
-    status_word_give(b->status_host);
     if (b->t0) cudaEventDestroy(b->t0);
     if (b->t1) cudaEventDestroy(b->t1);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -443,7 +442,7 @@ int msim_batch_create(const msim_map* maps, const uint32_t* num_entities, uint32
     b->n.assign(num_entities, num_entities + count);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
-    if (!(b->status_host = status_word_take()))
+    if (!b->status_host.take())
         return bail(fail(MSIM_ERR_NOMEM, "page-locked allocation of the status word failed"));
     if (cudaEventCreate(&b->t0) != cudaSuccess || cudaEventCreate(&b->t1) != cudaSuccess)
         return bail(fail(MSIM_ERR_CUDA, "cudaEventCreate failed"));

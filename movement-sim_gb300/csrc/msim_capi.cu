@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "msim_debug.h"
@@ -46,47 +47,61 @@ bool device_malloc(void** p, size_t bytes) {
     return true;
 }
 
-namespace {
-constexpr uint32_t kStatusWords = 1024;
-std::mutex g_status_mutex;
-uint32_t* g_status_slab = nullptr;
-std::vector<uint32_t> g_status_free;  // indexes of the slab's free words
-}  // namespace
+bool cuda_context_id(unsigned long long* id) {
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetId get_id = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<GetId>(p);
+    }();
+    return get_id && get_id(nullptr, id) == CUDA_SUCCESS;
+}
 
-uint32_t* status_word_take() {
+constexpr uint32_t kStatusWords = 1024;
+static std::mutex g_status_mutex;
+struct StatusSlab {
+    unsigned long long context = 0;
+    uint32_t* words = nullptr;
+    std::vector<uint32_t*> free;
+};
+
+bool StatusWord::take() try {
+    static auto* slabs = new std::vector<std::shared_ptr<StatusSlab>>;  // outlives every context
+    unsigned long long context = 0;
+    if (!cuda_context_id(&context)) return false;
     std::lock_guard<std::mutex> lk(g_status_mutex);
-    if (!g_status_slab) {
+    for (const auto& slab : *slabs)
+        if (slab->context == context && !slab->free.empty()) slab_ = slab;
+    if (!slab_) {
+        auto slab = std::make_shared<StatusSlab>();
         void* raw = nullptr;
         if (cudaHostAlloc(&raw, sizeof(uint32_t) * kStatusWords, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
-            return nullptr;
+            return false;
         }
-        g_status_slab = static_cast<uint32_t*>(raw);
-        for (uint32_t i = kStatusWords; i-- > 0;) g_status_free.push_back(i);
+        slab->context = context;
+        slab->words = static_cast<uint32_t*>(raw);
+        for (uint32_t i = kStatusWords; i-- > 0;) slab->free.push_back(slab->words + i);
+        slabs->push_back(slab);
+        slab_ = slab;
     }
-    uint32_t* word = nullptr;
-    if (!g_status_free.empty()) {
-        word = g_status_slab + g_status_free.back();
-        g_status_free.pop_back();
-    } else {
-        void* raw = nullptr;
-        if (cudaHostAlloc(&raw, sizeof(uint32_t), cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        word = static_cast<uint32_t*>(raw);
-    }
-    *word = 0u;
-    return word;
+    word_ = slab_->free.back();
+    slab_->free.pop_back();
+    *word_ = 0u;
+    return true;
+} catch (const std::bad_alloc&) {
+    return false;
 }
 
-void status_word_give(uint32_t* word) {
-    if (!word) return;
+StatusWord::~StatusWord() {
+    if (!slab_) return;
     std::lock_guard<std::mutex> lk(g_status_mutex);
-    if (g_status_slab && word >= g_status_slab && word < g_status_slab + kStatusWords)
-        g_status_free.push_back((uint32_t)(word - g_status_slab));
-    else
-        cudaFreeHost(word);
+    slab_->free.push_back(word_);
 }
 
 enum KernelId : uint32_t {
@@ -229,7 +244,7 @@ struct msim_ctx {
     bool pairs_zeroed = false;  // the spare counters are zero (the last query zeroed them)
     bool have_nbr = false;
     uint32_t* err = nullptr;
-    uint32_t* status_host = nullptr;  // page-locked copy of *err, written behind the work it describes
+    StatusWord status_host;  // page-locked copy of *err, written behind the work it describes
     uint32_t* check = nullptr;  // first invalid heading found by msim_set_entities
     TileGrid grid{};
     double expected = 0.0;  // neighbours expected along the road (see msim_create), and the
@@ -340,8 +355,6 @@ void free_all(msim_ctx* c) {
     }
     for (cudaEvent_t e : {c->ev_query, c->ev_state_free, c->ev_reuse_read[0], c->ev_reuse_read[1]})
         if (e) cudaEventDestroy(e);
-    status_word_give(c->status_host);
-    c->status_host = nullptr;
     if (c->disp_host) cudaFreeHost(c->disp_host);
     c->disp_host = nullptr;
     if (c->up) cudaStreamDestroy(c->up);
@@ -1085,7 +1098,7 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->qstream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
-    if (!(c->status_host = status_word_take()))
+    if (!c->status_host.take())
         return bail(fail(MSIM_ERR_NOMEM, "page-locked allocation of the status word failed"));
     if (cudaEventCreate(&c->t0) != cudaSuccess || cudaEventCreate(&c->t1) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_index, cudaEventDisableTiming) != cudaSuccess ||

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -29,11 +30,28 @@ int fail(int code, const std::string& msg);
 // failure injected by msim_debug_fail_device_alloc.  True on success.
 bool device_malloc(void** p, size_t bytes);
 
-// A zeroed page-locked word for a context's status read-back (page-locking one word costs
-// up to a millisecond, so 1,024 of them share one allocation for the life of the process),
-// or nullptr; status_word_give takes it back.  Safe from any thread.
-uint32_t* status_word_take();
-void status_word_give(uint32_t* word);
+// Number of the calling thread's CUDA context, never used again in the process: another one
+// after cudaDeviceReset.  False when the thread has no context.
+bool cuda_context_id(unsigned long long* id);
+
+// A zeroed page-locked word for a context's status read-back.  Page-locking one word costs
+// up to a millisecond, so 1,024 of them share an allocation, which is kept for the next
+// contexts.  It belongs to the CUDA context it was made in and ends with it: words taken
+// after a cudaDeviceReset come from a new one.  Safe from any thread.
+struct StatusSlab;
+class StatusWord {
+public:
+    StatusWord() = default;
+    StatusWord(const StatusWord&) = delete;
+    StatusWord& operator=(const StatusWord&) = delete;
+    ~StatusWord();
+    bool take();  // once; false when the allocation fails
+    operator uint32_t*() const { return word_; }
+
+private:
+    std::shared_ptr<StatusSlab> slab_;
+    uint32_t* word_ = nullptr;
+};
 
 // Owned map (JSON loader, lattice generator).
 struct MapData {
