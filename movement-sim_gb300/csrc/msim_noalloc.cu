@@ -212,8 +212,9 @@ __global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t*
 
 // Per-device set-up: the scratch array's device address (the host-side symbol is
 // only a stand-in, never a usable device pointer) and the query's shared-memory limit.
+// Both end with the device's CUDA context, so another one sets them up again.
 struct DeviceSlot {
-    bool ready = false;
+    unsigned long long context = 0;  // the CUDA context it was set up in (0: none)
     uint32_t* scratch = nullptr;
 };
 std::mutex g_setup_mutex;
@@ -223,7 +224,10 @@ int setup_device(int dev, DeviceSlot** out) {
     if (dev < 0 || dev >= 64) return fail(MSIM_ERR_INVALID, "device ordinal out of range for the no-allocation path");
     std::lock_guard<std::mutex> lk(g_setup_mutex);
     DeviceSlot& slot = g_slots[dev];
-    if (!slot.ready) {
+    unsigned long long context = 0;
+    if (!cuda_context_id(&context) && (cudaSetDevice(dev) != cudaSuccess || !cuda_context_id(&context)))
+        return fail(MSIM_ERR_CUDA, "no CUDA context for the no-allocation query");
+    if (slot.context != context) {
         void* ptr = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
         if (e != cudaSuccess || !ptr)
@@ -237,7 +241,7 @@ int setup_device(int dev, DeviceSlot** out) {
         if (e != cudaSuccess)
             return fail(MSIM_ERR_CUDA, std::string("cudaFuncSetAttribute failed: ") + cudaGetErrorString(e));
         slot.scratch = static_cast<uint32_t*>(ptr);
-        slot.ready = true;
+        slot.context = context;
     }
     *out = &slot;
     return MSIM_OK;
