@@ -782,11 +782,12 @@ __global__ __launch_bounds__(256) void k_gather_chunk(const uint32_t* __restrict
 
 // The words a host tick reads back (displacement, invalid heading, status), written to
 // page-locked memory by the device (three copies would queue behind the downloads), and
-// the first two zeroed for the next tick.
-__global__ void k_host_words(uint32_t* disp, const uint32_t* err, uint32_t* out) {
+// the first two zeroed for the next tick once its query has read them.
+__global__ void k_host_words(uint32_t* disp, const uint32_t* err, uint32_t* out, bool zero) {
+    chain_enter();
     if (threadIdx.x >= 3u) return;
     out[threadIdx.x] = threadIdx.x < 2u ? disp[threadIdx.x] : *err;
-    if (threadIdx.x < 2u) disp[threadIdx.x] = 0u;
+    if (zero && threadIdx.x < 2u) disp[threadIdx.x] = 0u;
 }
 
 __device__ __forceinline__ uint32_t abs_bits(float v) {  // |v| as ordered bits; NaN / inf: +inf
@@ -1079,9 +1080,8 @@ cudaError_t launch_gather_chunk(cudaStream_t s, const uint32_t* P, uint32_t n, u
     return cudaGetLastError();
 }
 
-cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out) {
-    k_host_words<<<1, 32, 0, s>>>(disp, err, out);
-    return cudaGetLastError();
+cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out, bool zero) {
+    return launch_chained(k_host_words, 1, 32, s, disp, err, out, zero);
 }
 
 cudaError_t launch_bounds(cudaStream_t s, const float* speed, const float2* pos, uint32_t n, uint32_t* out) {

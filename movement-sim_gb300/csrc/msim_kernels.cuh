@@ -175,8 +175,8 @@ cudaError_t launch_gather_chunk(cudaStream_t s, const uint32_t* P, uint32_t n, u
 // out[0] = largest |speed|, out[1] = largest |x| or |y| of the n entities, as float
 // bits (atomically maxed: out must hold zeros; NaN or infinite values count as +inf).
 cudaError_t launch_bounds(cudaStream_t s, const float* speed, const float2* pos, uint32_t n, uint32_t* out);
-// out[0..2] = disp[0], disp[1], *err (out: page-locked host memory); disp[0] = disp[1] = 0
-cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out);
+// out[0..2] = disp[0], disp[1], *err (out: page-locked host memory); zero: disp[0] = disp[1] = 0
+cudaError_t launch_host_words(cudaStream_t s, uint32_t* disp, const uint32_t* err, uint32_t* out, bool zero);
 cudaError_t launch_iota(cudaStream_t s, uint32_t* out, uint32_t n);
 // *first_bad = first i with (head[i] & road mask) >= num_roads, or 0xffffffff
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,
