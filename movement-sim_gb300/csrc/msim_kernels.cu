@@ -19,6 +19,7 @@
 // that the step and the query keep reading memory almost sequentially.
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "msim_chain.cuh"
 #include "msim_kernels.cuh"
@@ -548,45 +549,6 @@ __global__ __launch_bounds__(kSortThreads, 4) void k_onesweep(const uint32_t* __
 
 // Lists of up to this many ids are sorted in registers.
 constexpr int kSortInRegisters = 8;
-
-// Exact ascending list of the cap smallest ids of one entity, written by
-// insertion straight into its output slots; for the rare entities with more
-// than kRegKeep neighbours.
-__device__ __noinline__ void list_overflow(const uint32_t* __restrict__ sorted_slot,
-                                           const float2* __restrict__ sorted_pos,
-                                           const uint32_t* __restrict__ slot_id, const uint32_t* __restrict__ kstart,
-                                           const TileGrid& g, uint32_t n, uint32_t p, uint32_t cap,
-                                           uint32_t* out) {
-    // the entity and its query box's tiles, read and recomputed here so the caller
-    // keeps nothing live for them
-    const float2 me = sorted_pos[p];
-    const uint32_t x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
-    const uint32_t x1 = tile_coord(__fadd_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
-    const uint32_t y0 = tile_coord(__fsub_rn(me.y, g.reach), g.inv_cell, g.tiles_y);
-    const uint32_t y1 = tile_coord(__fadd_rn(me.y, g.reach), g.inv_cell, g.tiles_y);
-    uint32_t m = 0;
-    for (uint32_t ty = y0; ty <= y1; ty++) {
-        for (uint32_t tx = x0; tx <= x1; tx++) {
-            const uint32_t t = morton2(tx, ty);
-            const uint32_t q0 = kstart[t << g.ybits];
-            const uint32_t q1 = kstart[(t + 1u) << g.ybits];
-            const uint32_t qend = q1 < n ? q1 : n;
-            for (uint32_t q = q0; q < qend; q++) {
-                if (q == p || !in_range(sorted_pos[q], me, g.radius)) continue;
-                const uint32_t s2 = sorted_slot[q];
-                if (s2 >= n) continue;
-                const uint32_t oid = slot_id ? slot_id[s2] : s2;
-                if (m == cap && oid >= out[cap - 1]) continue;
-                uint32_t j = m < cap ? m++ : cap - 1;
-                while (j > 0 && out[j - 1] > oid) {
-                    out[j] = out[j - 1];
-                    j--;
-                }
-                out[j] = oid;
-            }
-        }
-    }
-}
 
 #include "msim_query.cuh"
 #include "msim_indexsort.cuh"

@@ -260,9 +260,9 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 // the current window of 32 pairs.  Every candidate is tested with the predicate of
 // random_move.comp:551-562; candidate positions come from the sorted copy, read in
 // runs.  A hit counts for the owner and, for the first KEEP hits, keeps the
-// candidate's sorted position; ids are looked up only for those.  An entity with more
-// than KEEP neighbours has them collected again by its whole warp.  The predicate is
-// symmetric (fl(a - b) = -fl(b - a)), so the pair count is half the sum of the counts,
+// candidate's sorted position; ids are looked up only for those.  The lists of entities
+// with more than KEEP neighbours are made afterwards (lists_from_pairs, longer_lists).  The
+// predicate is symmetric (fl(a - b) = -fl(b - a)), so the pair count is half the sum of the counts,
 // and a pair of entities of the same warp (most pairs: consecutive sorted entities
 // share their band runs) is tested once, by the lower lane, which credits both.  Each
 // warp writes its lists contiguously at warp * 32 * cap and adds its count sum to one
@@ -273,11 +273,12 @@ __global__ __launch_bounds__(256) void k_kstart_search(const uint32_t* __restric
 // window counts an owner's hits by ballot - its pairs lie side by side, where up to 32
 // atomics on its counter took turns - with atomics only for the credited lanes.  (Read
 // back from pair lists the hits thin out: one atomic per owner's run of pairs there was 15 %
-// slower than one per hit; counts alone take an atomic per hit everywhere.)  Longer lists are ranked in shared memory.  1 M entities with
-// 4.5 neighbours 170 -> 86 us per tick, 200,000 with 14.6 261 -> 50.  A few warps with many
-// lists beyond KEEP decide how long a crowd's query takes (a list looked up again cost about
-// 4 us, and half the time half of the SMs stood idle), so those come from the kept pairs,
-// and crowds keep more at fewer blocks resident.
+// slower than one per hit; counts alone take an atomic per hit everywhere.)  Lists of more
+// than eight are ranked in shared memory.  1 M entities with 4.5 neighbours 170 -> 83 us per
+// tick, 200,000 with 14.6 261 -> 50.  A few warps with many lists beyond KEEP decide how
+// long a crowd's query takes (a list looked up again cost about 4 us, and half the time half
+// of the SMs stood idle), so those come from the kept pairs where there are any, and crowds
+// keep more at fewer blocks resident.
 constexpr uint32_t kRuns = 4;                  // runs per lane and round
 constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 
@@ -315,18 +316,23 @@ struct QueryShared {
     float2 me[kQueryThreads];
     uint32_t cnt[kQueryThreads];
     uint32_t id[kQueryThreads];                // kept pairs: the entities' ids
-    // sorted positions of the first hits; DENSE: the owner's own from the front, those
-    // credited by lower lanes from the back
-    uint32_t keep[LIST ? KEEP * kQueryThreads : 1];
-    // place c of a warp's lane; the dense kernel keeps a warp's places together, so that
-    // they can also hold its longer lists end to end
+    // A warp's words: rows of one word per lane for the sorted positions of the first hits
+    // (DENSE: the owner's own from the front, those credited by lower lanes from the back),
+    // then the run list.  Together they hold the warp's longer lists once the others are
+    // written out.
+    static constexpr uint32_t kKept = LIST ? KEEP : 0, kRows = kKept + 3u * kRuns;
+    uint32_t words[kQueryThreads / 32][kRows * 32u];
     __device__ __forceinline__ uint32_t& place(uint32_t warp, uint32_t c, uint32_t lane) {
-        return KEEP != kQueryKeep ? keep[(warp * (uint32_t)KEEP + c) * 32u + lane]
-                                  : keep[c * (uint32_t)kQueryThreads + warp * 32u + lane];
+        return words[warp][c * 32u + lane];
     }
-    uint32_t rq[kQueryThreads / 32][kWarpRuns];   // run start position minus its flat start
-    uint32_t rfs[kQueryThreads / 32][kWarpRuns];  // flat start of the run
-    uint32_t rown[kQueryThreads / 32][kWarpRuns]; // owner lane
+    // of run j: its start position minus its flat start, its flat start, its owner lane
+    __device__ __forceinline__ uint32_t& rq(uint32_t warp, uint32_t j) { return words[warp][kKept * 32u + j]; }
+    __device__ __forceinline__ uint32_t& rfs(uint32_t warp, uint32_t j) {
+        return words[warp][kKept * 32u + kWarpRuns + j];
+    }
+    __device__ __forceinline__ uint32_t& rown(uint32_t warp, uint32_t j) {
+        return words[warp][kKept * 32u + 2u * kWarpRuns + j];
+    }
 };
 
 // Bits [from, to) of a word, both clamped to 0 .. 32.
@@ -401,9 +407,9 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
 #pragma unroll
     for (uint32_t k = 0; k < kRuns; k++) {
         if (len[k]) {
-            sh.rq[warp][j] = lo[k] - fs;
-            sh.rfs[warp][j] = fs;
-            sh.rown[warp][j] = lane;
+            sh.rq(warp, j) = lo[k] - fs;
+            sh.rfs(warp, j) = fs;
+            sh.rown(warp, j) = lane;
             j++;
             fs += len[k];
         }
@@ -412,7 +418,7 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
     uint32_t ra = 0;  // first run that starts at or after the current window
     for (uint32_t base = 0; base < total; base += 32u) {
         const uint32_t rr = ra + lane;
-        const uint32_t off = (rr < runs ? sh.rfs[warp][rr] : 0xffffffffu) - base;
+        const uint32_t off = (rr < runs ? sh.rfs(warp, rr) : 0xffffffffu) - base;
         const uint32_t marks = __reduce_or_sync(FULL, off < 32u ? (1u << off) : 0u);
         const uint32_t le = marks & (0xffffffffu >> (31u - lane));
         const uint32_t run = ra + (uint32_t)__popc(le) - 1u;  // le == 0: the run begun before the window
@@ -420,8 +426,8 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
         const uint32_t i = base + lane;
         if constexpr (!DENSE && !KEPT) {
             if (i >= total) continue;
-            const uint32_t q = sh.rq[warp][run] + i;
-            const uint32_t owner = sh.rown[warp][run];
+            const uint32_t q = sh.rq(warp, run) + i;
+            const uint32_t owner = sh.rown(warp, run);
             if (q - pwarp <= owner) continue;  // the owner itself or a lower lane: tested from there
             if (!in_range_fast(sorted_pos[q], sh.me[warp * 32u + owner], g.radius, g.d2_limit)) continue;
             count_hit<LIST, KEEP>(sh, warp, owner, q, pwarp, q, pwarp + owner);
@@ -429,8 +435,8 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
             uint32_t q = 0u, owner = lane, other = 0u;
             bool hit = false, near = false;
             if (i < total) {
-                q = sh.rq[warp][run] + i;
-                owner = sh.rown[warp][run];
+                q = sh.rq(warp, run) + i;
+                owner = sh.rown(warp, run);
                 other = q - pwarp;
                 if (other > owner) {
                     const float2 o = sorted_pos[q], me = sh.me[warp * 32u + owner];
@@ -500,7 +506,7 @@ __device__ __noinline__ bool lists_from_pairs(const uint32_t* pairs, uint32_t si
                                               const float2* __restrict__ sorted_pos, float radius, float d2_limit,
                                               uint32_t n, uint32_t pwarp, uint32_t count, uint32_t place,
                                               uint32_t cap, QueryShared<KEEP, true>& sh, uint32_t* out) {
-    constexpr uint32_t FULL = 0xffffffffu, kWords = 32u * (uint32_t)KEEP;
+    constexpr uint32_t FULL = 0xffffffffu, kWords = 32u * QueryShared<KEEP, true>::kRows;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (__any_sync(FULL, count > kWords)) return false;
     uint32_t* const words = &sh.place(warp, 0u, 0u);
@@ -561,25 +567,31 @@ __device__ __noinline__ bool lists_from_pairs(const uint32_t* pairs, uint32_t si
     return true;
 }
 
-// The ascending list of lane o's entity (count > KEEP neighbours, at most the 32 * KEEP
-// that the warp's keep words hold) by the whole warp: its runs again, 32 candidates at a
-// time, every hit's id into the keep words, then each id to its rank among them; for
-// warps without kept pairs.  One lane walking its tiles and inserting into its output slots held up its warp: at a
-// million entities with 10 m radius three of four warps have such an entity.
-template <int KEEP>
+// The ascending list of lane o's entity (more than KEEP neighbours) by the whole warp: its
+// runs again, 64 candidates at a time, every hit's id into the warp's words, then each id to
+// its rank among them.  Ranks cost the square of the ids held (200,000 entities with 727
+// neighbours, 64 ids: 17.8 ms with all of them, 6.5 so), so with `full` held the cap
+// smallest stay and larger ids are skipped from then on: any number of neighbours fits.
+template <uint32_t ROWS>
 __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_slot,
                                           const float2* __restrict__ sorted_pos, const uint32_t* __restrict__ slot_id,
-                                          const uint32_t* __restrict__ kstart, const TileGrid& g, uint32_t n,
-                                          uint32_t p, float2 me, uint32_t count, uint32_t cap, uint32_t* words,
-                                          uint32_t* out) {
-    constexpr uint32_t FULL = 0xffffffffu;
+                                          const uint32_t* __restrict__ kstart, const TileGrid& g, float reach,
+                                          uint32_t n, uint32_t p, float2 me, uint32_t cap, uint32_t* words, uint32_t* out) {
+    constexpr uint32_t FULL = 0xffffffffu, kNone = 0xffffffffu;
+    static_assert(2u * kMaxCap + 64u <= ROWS * 32u, "a full buffer and the hits of a round");
     const uint32_t lane = threadIdx.x & 31u;
-    const float ylo = __fsub_rn(me.y, g.reach), yhi = __fadd_rn(me.y, g.reach);
-    const uint32_t x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
-    const uint32_t x1 = tile_coord(__fadd_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
+    const float ylo = __fsub_rn(me.y, reach), yhi = __fadd_rn(me.y, reach);
+    const uint32_t x0 = tile_coord(__fsub_rn(me.x, reach), g.inv_cell, g.tiles_x);
+    const uint32_t x1 = tile_coord(__fadd_rn(me.x, reach), g.inv_cell, g.tiles_x);
     const uint32_t y0 = tile_coord(ylo, g.inv_cell, g.tiles_y), y1 = tile_coord(yhi, g.inv_cell, g.tiles_y);
     const uint32_t nx = x1 - x0 + 1u, slots = nx * (y1 - y0 + 1u);
-    uint32_t m = 0;
+    const uint32_t full = max(2u * cap, 384u);
+    uint32_t m = 0, below = kNone;  // ids held; only smaller ones are still wanted
+    auto rank_of = [&](uint32_t id) {
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < m; j++) rank += words[j] < id ? 1u : 0u;
+        return rank;
+    };
     for (uint32_t j0 = 0; j0 < slots; j0 += 32u) {  // a tile's run per lane
         const uint32_t j = j0 + lane;
         uint32_t lo = 0, len = 0;
@@ -604,26 +616,187 @@ __device__ __noinline__ void list_by_warp(const uint32_t* __restrict__ sorted_sl
             for (uint32_t k = 0; k < 2u; k++) {
                 hit[k] = hit[k] && in_range_fast(sorted_pos[q[k]], me, g.radius, g.d2_limit);
                 const uint32_t s2 = hit[k] ? sorted_slot[q[k]] : n;
-                id[k] = s2 < n ? (slot_id ? slot_id[s2] : s2) : 0xffffffffu;
+                id[k] = s2 < n ? (slot_id ? slot_id[s2] : s2) : kNone;
             }
 #pragma unroll
             for (uint32_t k = 0; k < 2u; k++) {
-                const uint32_t hits = __ballot_sync(FULL, id[k] != 0xffffffffu);
-                const uint32_t w = m + (uint32_t)__popc(hits & lanemask_lt());
-                if (id[k] != 0xffffffffu && w < count) words[w] = id[k];
+                const uint32_t hits = __ballot_sync(FULL, id[k] < below);
+                if (id[k] < below) words[m + (uint32_t)__popc(hits & lanemask_lt())] = id[k];
                 m += (uint32_t)__popc(hits);
             }
+            if (m < full) continue;
+            __syncwarp();
+            uint32_t last = 0u;  // the cap-th smallest, of the lane that holds it
+            for (uint32_t i = lane; i < m; i += 32u)
+                if (rank_of(words[i]) == cap - 1u) last = words[i];
+            below = __reduce_max_sync(FULL, last);
+            uint32_t kept = 0;
+            for (uint32_t i0 = 0; i0 < m; i0 += 32u) {  // towards the front, behind the reads
+                const uint32_t x = i0 + lane < m ? words[i0 + lane] : kNone;
+                const uint32_t stay = __ballot_sync(FULL, x <= below && x != kNone);
+                if ((stay >> lane) & 1u) words[kept + (uint32_t)__popc(stay & lanemask_lt())] = x;
+                kept += (uint32_t)__popc(stay);
+                __syncwarp();
+            }
+            m = kept;
         }
     }
-    m = min(m, count);
     __syncwarp();
     for (uint32_t i = lane; i < m; i += 32u) {
-        const uint32_t id = words[i];
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < m; j++) rank += words[j] < id ? 1u : 0u;
-        if (rank < cap) out[rank] = id;
+        const uint32_t rank = rank_of(words[i]);
+        if (rank < cap) out[rank] = words[i];
     }
     __syncwarp();  // before the words are used again
+}
+
+// How a lane holds the smallest ids it has met: in a column of the warp's words in no order,
+// the largest replaced and every id ranked in the end; in a column, ascending, by insertion;
+// or by insertion in its place of the output.
+enum HeldIds : int { kUnordered, kOrdered, kInPlace };
+
+// The ascending lists of the lanes with count > 0 (more than KEEP neighbours), each by its
+// own lane, `width` lanes at a time.  Candidates are tested 32 at a time into a mask and the
+// hits taken afterwards, so that the lanes take theirs together.
+template <HeldIds HELD>
+__device__ __forceinline__ void lists_by_lane(const uint32_t* __restrict__ sorted_slot,
+                                              const float2* __restrict__ sorted_pos,
+                                              const uint32_t* __restrict__ slot_id,
+                                              const uint32_t* __restrict__ kstart, const TileGrid& g, float reach,
+                                              uint32_t n, uint32_t p, uint32_t count, uint32_t cap, uint32_t width,
+                                              uint32_t* words, uint32_t* out) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t kept = min(count, cap), step = HELD == kInPlace ? 1u : width;
+    uint32_t todo = __ballot_sync(FULL, count != 0u);
+    while (todo) {
+        const uint32_t column = (uint32_t)__popc(todo & lanemask_lt());
+        const bool mine = ((todo >> (threadIdx.x & 31u)) & 1u) && column < width;
+        todo &= ~__ballot_sync(FULL, mine);
+        if (mine) {
+            uint32_t* const list = HELD == kInPlace ? out : words + column;
+            uint32_t m = 0, top = 0u, at = 0u;  // ids held; kUnordered: the largest and its place once all are
+            const float2 me = sorted_pos[p];
+            const float ylo = __fsub_rn(me.y, reach), yhi = __fadd_rn(me.y, reach);
+            const uint32_t x0 = tile_coord(__fsub_rn(me.x, reach), g.inv_cell, g.tiles_x);
+            const uint32_t x1 = tile_coord(__fadd_rn(me.x, reach), g.inv_cell, g.tiles_x);
+            const uint32_t y0 = tile_coord(ylo, g.inv_cell, g.tiles_y), y1 = tile_coord(yhi, g.inv_cell, g.tiles_y);
+            for (uint32_t ty = y0; ty <= y1; ty++) {
+                for (uint32_t tx = x0; tx <= x1; tx++) {
+                    const uint32_t t = morton2(tx, ty) << g.ybits;
+                    const uint32_t q1 = min(kstart[(t | (g.ybits ? y_band(g, yhi, ty) : 0u)) + 1u], n);
+                    for (uint32_t q0 = kstart[t | (g.ybits ? y_band(g, ylo, ty) : 0u)]; q0 < q1; q0 += 32u) {
+                        uint32_t hits = 0u;
+                        for (uint32_t k = 0; k < 32u && q0 + k < q1; k += 4u) {
+#pragma unroll
+                            for (uint32_t u = 0; u < 4u; u++) {
+                                const uint32_t q = min(q0 + k + u, q1 - 1u);  // past the end: the last one's again
+                                const bool hit = q != p && in_range_fast(sorted_pos[q], me, g.radius, g.d2_limit);
+                                hits |= hit ? 1u << (q - q0) : 0u;
+                            }
+                        }
+                        while (hits) {
+                            const uint32_t s2 = sorted_slot[q0 + (uint32_t)__ffs(hits) - 1u];
+                            hits &= hits - 1u;
+                            if (s2 >= n) continue;
+                            const uint32_t id = slot_id ? slot_id[s2] : s2;
+                            if constexpr (HELD == kUnordered) {
+                                if (m < kept) at = m++;
+                                else if (id >= top) continue;
+                                list[at * step] = id;
+                                if (m < kept) continue;
+                                top = 0u;
+#pragma unroll 4
+                                for (uint32_t j = 0; j < kept; j++) {
+                                    const uint32_t x = list[j * step];
+                                    if (x >= top) {
+                                        top = x;
+                                        at = j;
+                                    }
+                                }
+                            } else {
+                                uint32_t j = m;
+                                if (m < kept) m++;
+                                else if (id < list[(kept - 1u) * step]) j = kept - 1u;
+                                else continue;
+                                while (j > 0 && list[(j - 1u) * step] > id) {
+                                    list[j * step] = list[(j - 1u) * step];
+                                    j--;
+                                }
+                                list[j * step] = id;
+                            }
+                        }
+                    }
+                }
+            }
+            if constexpr (HELD == kOrdered) {
+                for (uint32_t j = 0; j < m; j++) out[j] = list[j * step];
+            } else if constexpr (HELD == kUnordered) {
+                for (uint32_t i = 0; i < m; i += 2u) {
+                    const uint32_t a = list[i * step], b = i + 1u < m ? list[(i + 1u) * step] : 0xffffffffu;
+                    uint32_t ra = 0, rb = 0;
+#pragma unroll 4
+                    for (uint32_t j = 0; j < m; j++) {
+                        const uint32_t x = list[j * step];
+                        ra += x < a ? 1u : 0u;
+                        rb += x < b ? 1u : 0u;
+                    }
+                    out[ra] = a;
+                    if (i + 1u < m) out[rb] = b;
+                }
+            }
+        }
+        __syncwarp();  // before the next lanes use the words
+    }
+}
+
+// The ascending lists of the lanes with count > KEEP (0 for the others, whose lists are
+// written), looked up again.  The only call of the kernel's tail, so that nothing stays live
+// across it.
+// Sparse populations have such lists where entities stand at one point; their ids then come
+// in a few ascending stretches, which suits insertion (1 M entities at the road starts, about
+// 30 neighbours, us per tick, by insertion / ranked in the end: 16 ids 178 / 199, 64 ids 234 /
+// 300).  In one turn of the warp's lanes, or two while the walk that is done twice is short;
+// lists of up to 96 ids in the output, where a third turn cost more than the slower
+// memory (3,000 entities on one spot, 64 ids: 2.2 ms, in four turns 4.7, list by list 3.7);
+// longer ones list by list (the same with 256 ids 6.8 ms, in the output 12).
+// In dense populations ids come in no order: ranked in the end 8 / 32 ids of 82 neighbours
+// 216 / 296 us at 50,000, by insertion 229 / 407, list by list 418 / 416.  A list alone costs
+// the warp what about 16 lanes' lists cost at once, more with longer lists, and two turns are
+// slower than list by list (64 ids of 570 neighbours, 1 M: 27 / 22 ms).
+template <int KEEP>
+__device__ __noinline__ void longer_lists(const uint32_t* __restrict__ sorted_slot,
+                                          const float2* __restrict__ sorted_pos,
+                                          const uint32_t* __restrict__ slot_id, const uint32_t* __restrict__ kstart,
+                                          const TileGrid& g, float reach, uint32_t n, uint32_t p, uint32_t count,
+                                          uint32_t cap, uint32_t* words, uint32_t* out) {
+    constexpr uint32_t FULL = 0xffffffffu, kRows = QueryShared<KEEP, true>::kRows;
+    uint32_t longer = __ballot_sync(FULL, count != 0u);
+    const uint32_t lanes = (uint32_t)__popc(longer), most = __reduce_max_sync(FULL, min(count, cap));
+    if constexpr (KEEP == kQueryKeep) {
+        uint32_t width = 32u;
+        while (most * width > kRows * 32u) width >>= 1;
+        const bool short_walk = __reduce_max_sync(FULL, count) <= 16u * most;
+        if (lanes <= (short_walk ? 2u * width : width)) {
+            lists_by_lane<kOrdered>(sorted_slot, sorted_pos, slot_id, kstart, g, reach, n, p, count, cap, width, words,
+                                    out);
+            return;
+        }
+        if (most <= 96u) {
+            lists_by_lane<kInPlace>(sorted_slot, sorted_pos, slot_id, kstart, g, reach, n, p, count, cap, 32u, words,
+                                    out);
+            return;
+        }
+    } else if (most <= kRows && lanes >= 16u + most / 4u) {
+        lists_by_lane<kUnordered>(sorted_slot, sorted_pos, slot_id, kstart, g, reach, n, p, count, cap, 32u, words, out);
+        return;
+    }
+    const float2 me = sorted_pos[min(p, n - 1u)];
+    for (; longer; longer &= longer - 1u) {
+        const int o = __ffs(longer) - 1;
+        list_by_warp<kRows>(sorted_slot, sorted_pos, slot_id, kstart, g, reach, n, p - (threadIdx.x & 31u) + (uint32_t)o,
+                            make_float2(__shfl_sync(FULL, me.x, o), __shfl_sync(FULL, me.y, o)), cap, words,
+                            reinterpret_cast<uint32_t*>(
+                                __shfl_sync(FULL, reinterpret_cast<unsigned long long>(out), o)));
+    }
 }
 
 // Resident blocks per SM.  Sparse and counts alone: 16 (64 warps), at 40 registers (12
@@ -639,7 +812,8 @@ template <bool LIST, int KEEP, PairLists PAIRS>
 __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) void k_query(const uint32_t* __restrict__ kstart,
                                                          const uint32_t* __restrict__ sorted_slot,
                                                          const float2* __restrict__ sorted_pos,
-                                                         const uint32_t* __restrict__ slot_id, TileGrid g,
+                                                         const uint32_t* __restrict__ slot_id,
+                                                         const __grid_constant__ TileGrid g,
                                                          uint32_t n, uint32_t cap, uint32_t* __restrict__ count_out,
                                                          uint32_t* __restrict__ list,
                                                          unsigned long long* __restrict__ pair_bins,
@@ -651,6 +825,7 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
     // read first, tested once the other first loads are in flight (they stay in range
     // whatever an index update left behind)
     const uint32_t status = err ? ld_relaxed(err) : 0u;
+    float reach = g.reach;
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31;
     const uint32_t warp = tid >> 5;
@@ -679,7 +854,7 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
         // a d past the limit (or not finite) leaves the query to the host
         const float d = __uint_as_float(*store.disp);
         if (!(d <= store.widen_limit)) return;
-        g.reach = __fadd_ru(g.reach, __fmul_ru(d, 1.0f + 0x1p-20f));  // d was measured with one rounding
+        reach = __fadd_ru(reach, __fmul_ru(d, 1.0f + 0x1p-20f));  // d was measured with one rounding
     }
     sh.me[tid] = me;
     sh.cnt[tid] = 0u;
@@ -717,10 +892,10 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
     uint32_t x0 = 1, x1 = 0, y0 = 1, y1 = 0;  // empty box for invalid lanes
     float ylo = 0.f, yhi = 0.f;
     if (valid) {
-        ylo = __fsub_rn(me.y, g.reach);
-        yhi = __fadd_rn(me.y, g.reach);
-        x0 = tile_coord(__fsub_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
-        x1 = tile_coord(__fadd_rn(me.x, g.reach), g.inv_cell, g.tiles_x);
+        ylo = __fsub_rn(me.y, reach);
+        yhi = __fadd_rn(me.y, reach);
+        x0 = tile_coord(__fsub_rn(me.x, reach), g.inv_cell, g.tiles_x);
+        x1 = tile_coord(__fadd_rn(me.x, reach), g.inv_cell, g.tiles_x);
         y0 = tile_coord(ylo, g.inv_cell, g.tiles_y);
         y1 = tile_coord(yhi, g.inv_cell, g.tiles_y);
     }
@@ -897,32 +1072,19 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
                 }
             }
         }
-        if constexpr (!DENSE) {  // a few in a million
-            if (count > (uint32_t)KEEP) list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
-        } else {
-            uint32_t longer = __ballot_sync(FULL, count > (uint32_t)KEEP);
-            if (longer) __syncwarp();  // the kept lists are written out: their words are free
-            if (longer && (PAIRS == kPairsUsed || PAIRS == kPairsKept)) {
-                const uint32_t known = PAIRS == kPairsUsed ? size : near_count <= places ? near_count : kNoPairs;
-                if (known != kNoPairs &&
-                    lists_from_pairs<KEEP>(store.pairs + (size_t)(p >> 5) * places, known, sorted_slot, slot_id,
-                                           sorted_pos, g.radius, g.d2_limit, n, pwarp,
-                                           count > (uint32_t)KEEP ? count : 0u, incl - kept, cap, sh,
-                                           list + (size_t)(p >> 5) * 32u * cap))
-                    return;
-            }
-            while (longer) {
-                const uint32_t o = (uint32_t)__ffs(longer) - 1u;
-                longer &= longer - 1u;
-                const uint32_t c = __shfl_sync(FULL, count, o);
-                if (c <= 32u * (uint32_t)KEEP) {
-                    list_by_warp<KEEP>(sorted_slot, sorted_pos, slot_id, kstart, g, n, pwarp + o,
-                                       sh.me[warp * 32u + o], c, cap, &sh.place(warp, 0u, 0u),
-                                       list + (size_t)(p >> 5) * 32u * cap + __shfl_sync(FULL, incl - kept, o));
-                } else if (lane == o) {
-                    list_overflow(sorted_slot, sorted_pos, slot_id, kstart, g, n, p, cap, out);
-                }
-            }
+        // a few in a million in a sparse population, unless entities stand at one point
+        const uint32_t beyond = count > (uint32_t)KEEP ? count : 0u;
+        if (!__any_sync(FULL, beyond != 0u)) return;
+        __syncwarp();  // the kept lists are written out: their words are free
+        if constexpr (DENSE && (PAIRS == kPairsUsed || PAIRS == kPairsKept)) {
+            const uint32_t known = PAIRS == kPairsUsed ? size : near_count <= places ? near_count : kNoPairs;
+            if (known != kNoPairs &&
+                lists_from_pairs<KEEP>(store.pairs + (size_t)(p >> 5) * places, known, sorted_slot, slot_id, sorted_pos,
+                                       g.radius, g.d2_limit, n, pwarp, beyond, incl - kept, cap, sh,
+                                       list + (size_t)(p >> 5) * 32u * cap))
+                return;
         }
+        longer_lists<KEEP>(sorted_slot, sorted_pos, slot_id, kstart, g, reach, n, p, beyond, cap,
+                           &sh.place(warp, 0u, 0u), out);
     }
 }
