@@ -256,6 +256,7 @@ struct msim_ctx {
     TileGrid grid{};
     double expected = 0.0;  // neighbours expected along the road (see msim_create), and the
     uint32_t density = 0;   // query's kernel for that many
+    double expected_area = 0.0;  // the same were the world's area filled evenly
     uint32_t passes = 1;
     uint32_t resort = 16;
     uint32_t since_permute = 0;
@@ -549,12 +550,14 @@ int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
     const int64_t left = (int64_t)std::min(std::floor((double)kWidenLimit * per_reach), 1e9) - since;
     const int64_t best = (int64_t)std::min(std::sqrt(0.5 * (c->density ? kPairCostDense : kPairCost) * per_reach), 1e9);
     const int64_t ticks = std::min(left, std::max(best, kFewest));
-    // a warp keeps about 24 pairs per expected neighbour within the reach (16 pairs per
-    // neighbour, 1.5 neighbours per one along the road), more the further they are kept;
-    // past its places it looks them up all the same (1 M with 192 neighbours, counts alone:
-    // 920 us per tick against 897)
-    if (24.0 * c->expected * (1.0 + 2.0 * (double)ticks / per_reach) > (double)pair_places(query_keep(c->density)))
-        return 0;
+    // a warp keeps about 16 pairs per neighbour within the reach, of which there are 1.5 per
+    // one expected along the road, or, with boxes over many roads, as many as the area
+    // holds; more the further they are kept, and half as many again in many warps.  Past its
+    // places it looks them up all the same (1 M entities, counts alone, kept / not: 65
+    // neighbours 264 / 416 us per tick, 103 neighbours 600 / 567, 570 neighbours 2,797 / 2,630)
+    const double further = 1.0 + 2.0 * (double)ticks / per_reach;
+    const double pairs = 24.0 * further * std::max(1.5 * c->expected, further * c->expected_area);
+    if (pairs > (double)pair_places(query_keep(c->density))) return 0;
     return ticks >= kFewest ? ticks : 0;
 }
 
@@ -1160,6 +1163,8 @@ int msim_create(const msim_map* map, const msim_params* params, msim_ctx** out) 
         road_length += std::sqrt(dx * dx + dy * dy) * (double)every;
     }
     c->expected = road_length > 0.0 ? 2.0 * radius * (double)c->n / road_length : INFINITY;
+    c->expected_area =
+        3.14159265358979 * radius * radius * (double)c->n / std::max((double)c->world_w * (double)c->world_h, 1e-30);
     c->density = c->expected > kCrowdNeighbours ? 2u : c->expected > kDenseNeighbours ? 1u : 0u;
     // y bands inside a tile fill the key up to 24 bits (3 radix passes), at most 64
     // bands, and keep the key-start table within about four entries per entity
