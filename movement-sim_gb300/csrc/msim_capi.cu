@@ -216,6 +216,8 @@ struct msim_ctx {
     uint32_t* pairs_kept = nullptr;
     uint32_t* pair_sizes = nullptr;
     uint32_t* pair_ids = nullptr;
+    uint32_t pair_places = 0;   // per warp
+    bool pairs_failed = false;  // no memory for them
     int64_t pair_until = -1;
     // rank[slot] = sorted position of the slot in the current index, written by the
     // update once allocated (rank_valid: it describes the current index); a reusing
@@ -525,22 +527,36 @@ bool ensure_reuse(msim_ctx* c) {
     return true;
 }
 
-// Buffers of the pair lists: false when their allocation fails (the queries then look
-// their candidates up).
-bool ensure_pairs(msim_ctx* c) {
-    return allocate_parts(c, {part(c->pairs_kept, query_pair_places(c->n, c->density)),
-                              part(c->pair_sizes, query_pair_sizes(c->n)), part(c->pair_ids, c->n)});
+// Buffers of the pair lists, for about that many pairs a warp: false when their allocation
+// fails (the queries then look their candidates up, and it is not tried again: a failing
+// allocation takes longer than a tick).  Up to kPairBytes every warp has all the places
+// its kernel can use, which serves crowded spots; above, twice the pairs expected, to a
+// power of two (16 M entities with 9 neighbours 2 GB for 6).
+bool ensure_pairs(msim_ctx* c, double pairs) {
+    constexpr size_t kPairBytes = size_t(1) << 30;
+    if (c->pairs_kept) return true;
+    if (c->pairs_failed) return false;
+    const size_t warps = query_pair_sizes(c->n);
+    c->pair_places = pair_places(query_keep(c->density));
+    if (warps * c->pair_places * sizeof(uint32_t) > kPairBytes) {
+        uint32_t places = kPairPlacesFewest;
+        while (places < 2.0 * pairs) places *= 2u;
+        c->pair_places = std::min(c->pair_places, places);
+    }
+    c->pairs_failed = !allocate_parts(c, {part(c->pairs_kept, warps * c->pair_places), part(c->pair_sizes, warps),
+                                          part(c->pair_ids, c->n)});
+    return !c->pairs_failed;
 }
 
 // Ticks that pair lists kept `since` move ticks after the index's keys should serve (0:
-// look the candidates up).  More ticks keep more pairs (each one twice its displacement
+// look the candidates up), and about how many pairs a warp then keeps.  More ticks keep more pairs (each one twice its displacement
 // further apart), fewer pay for the keeping query more often: with use cost growing by
 // 2 s / reach per tick and the keeping query worth kPairCost of it, the best count is
 // about the square root of kPairCost x reach / (2 s), as far as the index is reused.
 // Measured with costs 11 / 22 / 44 (sparse): 16 M 388 / 371 / 372 us per tick, 1 M 36.0 /
 // 36.0 / 35.2; 3 / 6 / 12 (dense): 1 M reference mode 105 / 108 / 124, 200,000 with 14.6
 // neighbours 110 / 118 / 122.
-int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
+int64_t pair_list_ticks(const msim_ctx* c, int64_t since, double* pairs) {
     constexpr double kPairCost = 44.0, kPairCostDense = 3.0;
     constexpr int64_t kFewest = 2;
     if (!c->reuse || !c->bounds_valid || !(c->grid.reach > 0.f) || !(c->step_bound > 0.0) ||
@@ -556,8 +572,8 @@ int64_t pair_list_ticks(const msim_ctx* c, int64_t since) {
     // places it looks them up all the same (1 M entities, counts alone, kept / not: 65
     // neighbours 264 / 416 us per tick, 103 neighbours 600 / 567, 570 neighbours 2,797 / 2,630)
     const double further = 1.0 + 2.0 * (double)ticks / per_reach;
-    const double pairs = 24.0 * further * std::max(1.5 * c->expected, further * c->expected_area);
-    if (pairs > (double)pair_places(query_keep(c->density))) return 0;
+    *pairs = 24.0 * further * std::max(1.5 * c->expected, further * c->expected_area);
+    if (*pairs > (double)(c->pairs_kept ? c->pair_places : pair_places(query_keep(c->density)))) return 0;
     return ticks >= kFewest ? ticks : 0;
 }
 
@@ -882,8 +898,9 @@ int reusable_query(msim_ctx* c, int64_t ticks, const float2* pos) {
     if (ticks > 0) g.reach = widened_reach(c, (double)ticks);
     else c->pair_until = -1;  // a new index
     if (ticks <= c->pair_until) return run_query(c, true, nullptr, pos, &g, true);
-    const int64_t serve = pair_list_ticks(c, ticks);
-    if (!serve || !ensure_pairs(c)) return run_query(c, true, nullptr, pos, &g);
+    double pairs = 0.0;
+    const int64_t serve = pair_list_ticks(c, ticks, &pairs);
+    if (!serve || !ensure_pairs(c, pairs)) return run_query(c, true, nullptr, pos, &g);
     g.reach = widened_reach(c, (double)ticks + 2.0 * (double)serve);
     const int rc = run_query(c, true, nullptr, pos, &g, true, widened_reach(c, 2.0 * (double)serve));
     if (rc == MSIM_OK) c->pair_until = ticks + serve;
@@ -1004,7 +1021,7 @@ int run_query(msim_ctx* c, bool overlap, uint32_t* count_by_id, const float2* po
                         c->n, c->nbr_count, c->nbr_list, c->pairs,
                         c->pairs_b[c->pairs == c->pairs_b[0] ? 1 : 0], c->err,
                         c->slots_identity ? count_by_id : nullptr, c->density, pairs ? c->pairs_kept : nullptr,
-                        c->pair_sizes, c->pair_ids, keep_near, disp, kWidenLimit * c->grid.reach),
+                        c->pair_sizes, c->pair_ids, c->pair_places, keep_near, disp, kWidenLimit * c->grid.reach),
            "k_query");
     }
     if (qs != c->stream) {

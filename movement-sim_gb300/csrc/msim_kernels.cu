@@ -953,7 +953,8 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
                          uint32_t* list, unsigned long long* pair_bins, unsigned long long* next_bins, const uint32_t* err,
                          uint32_t* count_by_id,
-                         uint32_t density, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, double keep_near,
+                         uint32_t density, uint32_t* pairs, uint32_t* pair_sizes, uint32_t* pair_ids, uint32_t places,
+                         double keep_near,
                          const uint32_t* disp, float widen_limit) {
     if (n == 0) return cudaSuccess;
     using Query = void (*)(const uint32_t*, const uint32_t*, const float2*, const uint32_t*, TileGrid, uint32_t, uint32_t,
@@ -974,12 +975,14 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
         cudaGetLastError();
         carveout = true;
     }
-    if (pairs && (!pair_sizes || !pair_ids || n > kPairMaxEntities)) return cudaErrorInvalidValue;
+    if (pairs && (!pair_sizes || !pair_ids || n > kPairMaxEntities ||
+                  places < std::min(kPairPlacesFewest, pair_places(query_keep(density)))))
+        return cudaErrorInvalidValue;
     const bool lists = cap > 0 && list;
     if ((pairs && disp) || density > 2u) return cudaErrorInvalidValue;
     const PairLists use = disp ? kPairsWidened : !pairs ? kPairsFound : keep_near > 0.0 ? kPairsKept : kPairsUsed;
     // the squared distance's rounding and its operands' stay far below 2^-18 of it
-    const PairStore store{pairs, pair_sizes, pair_ids, (float)(keep_near * keep_near * (1.0 + 0x1p-18)),
+    const PairStore store{pairs, pair_sizes, pair_ids, places, (float)(keep_near * keep_near * (1.0 + 0x1p-18)),
                           disp, widen_limit};
     kernels[lists][density][use]<<<blocks_for(n, kQueryThreads), kQueryThreads, 0, s>>>(
         kstart, sorted_slot, sorted_pos, slot_id, grid, n, lists ? cap : 0u, count, lists ? list : nullptr, pair_bins,
@@ -988,10 +991,6 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
 }
 
 size_t query_pair_sizes(uint32_t n) { return (size_t)blocks_for(n, kQueryThreads) * (kQueryThreads / 32); }
-size_t query_pair_places(uint32_t n, uint32_t density) {
-    return query_pair_sizes(n) * pair_places(query_keep(density));
-}
-
 cudaError_t launch_check_roads(cudaStream_t s, const uint32_t* head, uint32_t n, uint32_t num_roads,
                                uint32_t* first_bad) {
     cudaError_t e = cudaMemsetAsync(first_bad, 0xff, sizeof(uint32_t), s);

@@ -144,19 +144,20 @@ cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, c
                          // (pairs up to that distance), else read back (the ids then serve as
                          // sorted_slot, slot_id NULL); NULL: not used
                          uint32_t* pairs = nullptr, uint32_t* pair_sizes = nullptr, uint32_t* pair_ids = nullptr,
+                         uint32_t places = 0,  // pairs per warp, kPairPlacesFewest at least where pairs are read
                          double keep_near = 0.0,
                          // boxes widened by the displacement d = *disp (float bits); the query does
                          // nothing when d exceeds widen_limit or is not finite
                          const uint32_t* disp = nullptr, float widen_limit = 0.f);
 constexpr uint32_t kPairMaxEntities = 1u << 27;     // positions that fit a pair's word
-// Places per warp: at least twice what the workloads keep (sparse 1 M and 16 M populations
+// Most places per warp: at least twice what the workloads keep (sparse 1 M and 16 M populations
 // 45 of 128; 4.5 neighbours 170 of 1,024; 15 neighbours 530 of 3,072; with 35 neighbours
 // 1,536 places overflow: 176 us per tick against 138).
+constexpr uint32_t kPairPlacesFewest = 256;  // the dense kernels read the first 192 places unasked, the sparse one 64
 __host__ __device__ constexpr uint32_t pair_places(int keep) {
     return keep == kQueryKeep ? 128u : keep == kQueryKeepDense ? 1024u : 3072u;
 }
-size_t query_pair_places(uint32_t n, uint32_t density);  // pairs of all lists
-size_t query_pair_sizes(uint32_t n);
+size_t query_pair_sizes(uint32_t n);  // warps of a query
 // Index update by counting (msim_indexsort.cuh): the keys' counters become the key-start
 // table (and are zeroed), then every slot goes to its place; sorted_pos and rank may be
 // NULL.  lookback (mark_tiles(num_keys) words) and ticket must be zero when it starts.

@@ -288,7 +288,7 @@ constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 // in range in one of those ticks is among them, and their queries test the kept pairs
 // alone - no tiles, bands or key starts per entity, no search for the run of a pair, and
 // a quarter of the pairs.  One word per pair: owner lane | the candidate's sorted
-// position (pair_places words per warp; kNoPairs: more than that, look them up); and
+// position (PairStore::places words per warp; kNoPairs: more than that, look them up); and
 // the entity id of every sorted position, read beside the candidate's position so that
 // a hit keeps the id itself.
 // Bound by the latency of its three dependent loads (58 % issue active); 378 warp
@@ -306,6 +306,7 @@ struct PairStore {
     uint32_t* pairs;
     uint32_t* sizes;
     uint32_t* ids;
+    uint32_t places;  // per warp
     float near2;  // pairs up to this squared distance are kept
     const uint32_t* disp;  // kPairsWidened: the tick's largest displacement d (float bits)
     float widen_limit;     // and the d up to which the query runs
@@ -365,7 +366,7 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
                                            uint32_t lane, uint32_t warp, uint32_t pwarp, QueryShared<KEEP, LIST>& sh,
                                            const float2* __restrict__ sorted_pos, const TileGrid& g, uint32_t& own,
                                            PairStore store, uint32_t& near_count) {
-    constexpr uint32_t FULL = 0xffffffffu, places = pair_places(KEEP);
+    constexpr uint32_t FULL = 0xffffffffu;
     constexpr bool DENSE = LIST && KEEP != kQueryKeep;
     // A pair of entities of this warp is tested once, by the lower lane, which credits
     // both (the predicate is symmetric, and an in-range pair lies in both entities'
@@ -450,8 +451,8 @@ __device__ __forceinline__ void query_runs(const uint32_t (&lo_in)[kRuns], const
             if constexpr (KEPT) {
                 const uint32_t m = __ballot_sync(FULL, near);
                 const uint32_t at = near_count + (uint32_t)__popc(m & lanemask_lt());
-                if (near && at < places)
-                    store.pairs[(size_t)(pwarp >> 5) * places + at] = q | (owner << kPairOwnerShift);
+                if (near && at < store.places)
+                    store.pairs[(size_t)(pwarp >> 5) * store.places + at] = q | (owner << kPairOwnerShift);
                 near_count += (uint32_t)__popc(m);
             }
             if constexpr (!DENSE) {
@@ -834,11 +835,10 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
     const bool valid = p < n;
     float2 me = make_float2(0.f, 0.f);
     constexpr bool DENSE = LIST && KEEP != kQueryKeep;
-    constexpr uint32_t places = pair_places(KEEP);
     // pairs in flight per lane (dense 2 / 4 / 6: 1 M entities with 4.5 neighbours 90.9 / 87.5 /
     // 85.9 us per tick)
     constexpr uint32_t kPairsAtOnce = KEEP != kQueryKeep ? 6 : 2;
-    const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * places : nullptr;
+    const uint32_t* pairs = PAIRS == kPairsUsed ? store.pairs + (size_t)(p >> 5) * store.places : nullptr;
     uint32_t size = kNoPairs;
     uint32_t pair[kPairsAtOnce], my_id = 0u;
     if (PAIRS == kPairsUsed) {  // the first pairs, their number, position and id in flight together
@@ -957,7 +957,7 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
                                                            store, near_count);
         }
     }
-    if (PAIRS == kPairsKept && lane == 0) store.sizes[p >> 5] = near_count <= places ? near_count : kNoPairs;
+    if (PAIRS == kPairsKept && lane == 0) store.sizes[p >> 5] = near_count <= store.places ? near_count : kNoPairs;
     }
     __syncwarp();
     const uint32_t count = valid ? sh.cnt[tid] + own : 0u;
@@ -1077,9 +1077,9 @@ __global__ __launch_bounds__(kQueryThreads, query_blocks(LIST, KEEP, PAIRS)) voi
         if (!__any_sync(FULL, beyond != 0u)) return;
         __syncwarp();  // the kept lists are written out: their words are free
         if constexpr (DENSE && (PAIRS == kPairsUsed || PAIRS == kPairsKept)) {
-            const uint32_t known = PAIRS == kPairsUsed ? size : near_count <= places ? near_count : kNoPairs;
+            const uint32_t known = PAIRS == kPairsUsed ? size : near_count <= store.places ? near_count : kNoPairs;
             if (known != kNoPairs &&
-                lists_from_pairs<KEEP>(store.pairs + (size_t)(p >> 5) * places, known, sorted_slot, slot_id, sorted_pos,
+                lists_from_pairs<KEEP>(store.pairs + (size_t)(p >> 5) * store.places, known, sorted_slot, slot_id, sorted_pos,
                                        g.radius, g.d2_limit, n, pwarp, beyond, incl - kept, cap, sh,
                                        list + (size_t)(p >> 5) * 32u * cap))
                 return;
