@@ -123,12 +123,66 @@ __global__ __launch_bounds__(256) void k_noalloc_scatter(const float2* __restric
     cell_id[q] = i;
 }
 
-// The query, one thread per entity in cell order: per row of its box one run of
-// positions, four in flight, hits inserted into the thread's ascending list in shared
-// memory.  The lists are written by the whole warp (see k_export_nbr), 16 bytes a lane
-// with QUADS (cap a multiple of 4 and idx_out on a 16-byte boundary).
-template <bool QUADS>
-__global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t* __restrict__ cell_id,
+// A thread's list of ids in shared memory, a column of words.
+struct Column {
+    uint32_t* at0;
+    __device__ __forceinline__ uint32_t& operator[](uint32_t k) const { return at0[k * kQueryThreads]; }
+};
+// id goes down from place k of a heap (largest first) of n ids.
+__device__ __forceinline__ void sift_down(Column c, uint32_t k, uint32_t n, uint32_t id) {
+    for (;;) {
+        uint32_t child = 2u * k + 1u;
+        if (child >= n) break;
+        uint32_t x = c[child];
+        if (child + 1u < n) {
+            const uint32_t y = c[child + 1u];
+            if (y > x) {
+                x = y;
+                child++;
+            }
+        }
+        if (x <= id) break;
+        c[k] = x;
+        k = child;
+    }
+    c[k] = id;
+}
+// The warp puts the m ids of a column in ascending order; m up to 32 K.
+template <uint32_t K>
+__device__ __forceinline__ void order_column(Column c, uint32_t m, uint32_t lane) {
+    uint32_t x[K], rank[K];
+#pragma unroll
+    for (uint32_t k = 0; k < K; k++) {
+        x[k] = lane + 32u * k < m ? c[lane + 32u * k] : MSIM_NO_NEIGHBOUR;
+        rank[k] = 0u;
+    }
+    for (uint32_t j = 0; j < m; j++) {
+        const uint32_t y = c[j];
+#pragma unroll
+        for (uint32_t k = 0; k < K; k++) rank[k] += y < x[k] ? 1u : 0u;
+    }
+    __syncwarp();  // every id is read
+#pragma unroll
+    for (uint32_t k = 0; k < K; k++)
+        if (lane + 32u * k < m) c[rank[k]] = x[k];
+}
+
+// The query, one thread per entity in cell order: per row of its box one run of positions,
+// four loads in flight.  With lists the positions are tested 32 at a time into a mask and
+// the hits taken afterwards, two ids in flight, so that the lanes of a warp take theirs
+// together: the entries of a cell come in no order of ids, and one insertion at a time held
+// up the other lanes (100,003 entities about spots, 42 neighbours, 16 ids 361 -> 193 us).  The
+// thread's list lies in shared memory, ascending up to kAscending ids; longer lists go on in
+// no order (insertion into 200 ids moved 100 for each), become a heap once they are full, and
+// are put in order by the warp in the end (262,144 about spots, 200 ids 2.5 -> 1.2 ms).
+// Registers for 12 and 6 blocks per SM: at 16 the compiler spills (262,144 spread, 4 ids 25.3
+// us for 23.7), and with many ids the shared memory allows no more.
+// The lists are written by the whole warp (see k_export_nbr), 16 bytes a lane with QUADS
+// (cap a multiple of 4 and idx_out on a 16-byte boundary).
+constexpr uint32_t kAscending = 32;
+enum Lists : int { kCounts, kShort, kLong };  // cap 0, up to kAscending, above
+template <Lists LISTS, bool QUADS>
+__global__ __launch_bounds__(kQueryThreads, LISTS == kLong ? 6 : 12) void k_noalloc_query(const uint32_t* __restrict__ cell_id,
                                                                  const float2* __restrict__ cell_pos,
                                                                  const uint32_t* __restrict__ start,
                                                                  const uint32_t* __restrict__ cell_count, CellGrid g,
@@ -140,7 +194,9 @@ __global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t*
     chain_enter();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t p = blockIdx.x * kQueryThreads + tid;
+    const Column list{s_list + tid};
     uint32_t count = 0, id = 0xffffffffu;
+    uint32_t m = 0, last = MSIM_NO_NEIGHBOUR;  // ids held; the largest of a full list
     if (p < n) {
         id = cell_id[p];
         const float2 me = cell_pos[p];
@@ -155,38 +211,80 @@ __global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t*
         for (uint32_t y = y0; y <= y1; y++) {
             const uint32_t c0 = y * g.pitch + x0, c1 = y * g.pitch + x1;
             const uint32_t from = start[c0], to = min(start[c1] + cell_count[c1], n);
-            for (uint32_t q0 = from; q0 < to; q0 += 4u) {
-                float2 o[4];
+            if constexpr (LISTS == kCounts) {
+                for (uint32_t q0 = from; q0 < to; q0 += 4u) {
+                    float2 o[4];
 #pragma unroll
-                for (uint32_t k = 0; k < 4u; k++) o[k] = cell_pos[min(q0 + k, to - 1u)];
+                    for (uint32_t u = 0; u < 4u; u++) o[u] = cell_pos[min(q0 + u, to - 1u)];
 #pragma unroll
-                for (uint32_t k = 0; k < 4u; k++) {
-                    const uint32_t q = q0 + k;
-                    if (q >= to || q == p || !in_range_fast(o[k], me, g.radius, g.d2_limit)) continue;
-                    if (cap) {
-                        const uint32_t other = cell_id[q];
-                        const uint32_t m = count < cap ? count : cap;
-                        if (m < cap || other < s_list[(cap - 1) * kQueryThreads + tid]) {
-                            uint32_t j = m < cap ? m : cap - 1;
-                            while (j > 0) {
-                                const uint32_t prev = s_list[(j - 1) * kQueryThreads + tid];
-                                if (prev <= other) break;
-                                s_list[j * kQueryThreads + tid] = prev;
-                                j--;
-                            }
-                            s_list[j * kQueryThreads + tid] = other;
+                    for (uint32_t u = 0; u < 4u; u++)
+                        if (q0 + u < to && q0 + u != p && in_range_fast(o[u], me, g.radius, g.d2_limit)) count++;
+                }
+            } else {
+                for (uint32_t q0 = from; q0 < to; q0 += 32u) {
+                    uint32_t hits = 0u;
+                    for (uint32_t k = 0; k < 32u && q0 + k < to; k += 4u) {
+                        float2 o[4];
+#pragma unroll
+                        for (uint32_t u = 0; u < 4u; u++) o[u] = cell_pos[min(q0 + k + u, to - 1u)];
+#pragma unroll
+                        for (uint32_t u = 0; u < 4u; u++) {
+                            const uint32_t q = q0 + k + u;
+                            const bool hit = q < to && q != p && in_range_fast(o[u], me, g.radius, g.d2_limit);
+                            hits |= hit ? 1u << (k + u) : 0u;
                         }
                     }
-                    count++;
+                    count += (uint32_t)__popc(hits);
+                    while (hits) {
+                        constexpr uint32_t kIds = 2;
+                        uint32_t other[kIds];
+#pragma unroll
+                        for (uint32_t u = 0; u < kIds; u++) {
+                            other[u] = hits ? cell_id[q0 + (uint32_t)__ffs(hits) - 1u] : MSIM_NO_NEIGHBOUR;
+                            hits &= hits - 1u;
+                        }
+#pragma unroll
+                        for (uint32_t u = 0; u < kIds; u++) {
+                            if (other[u] >= last) continue;
+                            if (LISTS == kLong && m == cap) {
+                                sift_down(list, 0u, cap, other[u]);
+                                last = list[0];
+                                continue;
+                            }
+                            uint32_t j = m < cap ? m++ : cap - 1u;
+                            if (LISTS == kShort || j < kAscending) {
+                                while (j > 0) {
+                                    const uint32_t prev = list[j - 1u];
+                                    if (prev <= other[u]) break;
+                                    list[j] = prev;
+                                    j--;
+                                }
+                            }
+                            list[j] = other[u];
+                            if (m < cap) continue;
+                            if (LISTS == kLong)
+                                for (uint32_t k = cap / 2u; k-- > 0;) sift_down(list, k, cap, list[k]);
+                            last = list[LISTS == kLong ? 0u : cap - 1u];
+                        }
+                    }
                 }
             }
         }
         if (id < n) count_out[id] = count;
     }
-    if (!cap) return;
+    if (LISTS == kCounts) return;
     __syncwarp();
-    const uint32_t kept = count < cap ? count : cap;
-    const uint32_t* col = s_list + warp * 32u;
+    const uint32_t kept = m;
+    const uint32_t* const col = s_list + warp * 32u;
+    if constexpr (LISTS == kLong) {
+        for (uint32_t todo = __ballot_sync(FULL, m > kAscending); todo; todo &= todo - 1u) {
+            const uint32_t e = (uint32_t)__ffs(todo) - 1u, held = __shfl_sync(FULL, m, e);
+            const Column c{s_list + warp * 32u + e};
+            if (held <= 64u) order_column<2>(c, held, lane);
+            else order_column<kMaxCap / 32u>(c, held, lane);
+        }
+        __syncwarp();
+    }
     if constexpr (QUADS) {
         const uint32_t quads = cap >> 2;
         for (uint32_t i = lane; i < quads * 32u; i += 32u) {
@@ -210,6 +308,12 @@ __global__ __launch_bounds__(kQueryThreads) void k_noalloc_query(const uint32_t*
     }
 }
 
+using Query = void (*)(const uint32_t*, const float2*, const uint32_t*, const uint32_t*, CellGrid, uint32_t, uint32_t,
+                       uint32_t*, uint32_t*);
+const Query kQueries[3][2] = {{k_noalloc_query<kCounts, false>, k_noalloc_query<kCounts, false>},
+                              {k_noalloc_query<kShort, false>, k_noalloc_query<kShort, true>},
+                              {k_noalloc_query<kLong, false>, k_noalloc_query<kLong, true>}};
+
 // Per-device set-up: the scratch array's device address (the host-side symbol is
 // only a stand-in, never a usable device pointer) and the query's shared-memory limit.
 // Both end with the device's CUDA context, so another one sets them up again.
@@ -217,6 +321,7 @@ struct DeviceSlot {
     unsigned long long context = 0;  // the CUDA context it was set up in (0: none)
     uint32_t* scratch = nullptr;
 };
+constexpr int kCarveout = 45;  // percent of the largest; 60 and 75: 2 to 5 % slower at 262,144
 std::mutex g_setup_mutex;
 DeviceSlot g_slots[64];
 
@@ -233,11 +338,21 @@ int setup_device(int dev, DeviceSlot** out) {
         if (e != cudaSuccess || !ptr)
             return fail(MSIM_ERR_CUDA, std::string("cudaGetSymbolAddress(no-allocation scratch) failed: ") +
                                            cudaGetErrorString(e));
-        e = cudaFuncSetAttribute(k_noalloc_query<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kMaxCap * kQueryThreads * sizeof(uint32_t)));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_noalloc_query<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kMaxCap * kQueryThreads * sizeof(uint32_t)));
+        for (const Query q : {kQueries[kLong][0], kQueries[kLong][1]})
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(q, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kMaxCap * kQueryThreads * sizeof(uint32_t)));
+        if (e != cudaSuccess)
+            return fail(MSIM_ERR_CUDA, std::string("cudaFuncSetAttribute failed: ") + cudaGetErrorString(e));
+        // The kernels that start under their predecessors' tails find the shared memory of an
+        // SM as those left it.  A small query's blocks were put on the few SMs whose shared
+        // memory had already been set for them (20,000 entities in one cell, 157 blocks, 4 ids:
+        // 11.6 ms for 3.4), so the chain asks for one setting; with longer lists it is the
+        // memory itself that spreads the blocks.
+        for (const void* k : {(const void*)k_noalloc_rank, (const void*)k_noalloc_scan, (const void*)k_noalloc_scatter,
+                              (const void*)kQueries[kShort][0], (const void*)kQueries[kShort][1]})
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
         if (e != cudaSuccess)
             return fail(MSIM_ERR_CUDA, std::string("cudaFuncSetAttribute failed: ") + cudaGetErrorString(e));
         slot.scratch = static_cast<uint32_t*>(ptr);
@@ -305,7 +420,7 @@ extern "C" int msim_query_neighbours_noalloc(const float* d_pos, uint32_t n, flo
                               w + kOffStart, cursor) == cudaSuccess;
     ok = ok && launch_chained(k_noalloc_scatter, blocks, 256, s, pos, n, g, w + kOffStart, w + kOffRank, cell_pos,
                               w + kOffId) == cudaSuccess;
-    ok = ok && launch_chained_shared(quads ? k_noalloc_query<true> : k_noalloc_query<false>,
+    ok = ok && launch_chained_shared(kQueries[cap == 0 ? kCounts : cap <= kAscending ? kShort : kLong][quads],
                               (n + kQueryThreads - 1) / kQueryThreads, kQueryThreads,
                               (size_t)cap * kQueryThreads * sizeof(uint32_t), s, w + kOffId, cell_pos, w + kOffStart,
                               count, g, n, cap, d_count, d_idx) == cudaSuccess;
