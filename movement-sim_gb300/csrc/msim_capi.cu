@@ -629,11 +629,14 @@ T* mapped_range(const void* p, size_t count) {
 // wanted, nullptr.  The state's fields are written in entity
 // order, a line at a time, which keeps the link as busy as a copy and saves the staging
 // (1 M entities 20 us of 470); counts and id lists are written in the order of the query,
-// by id, which crosses the link in pieces, so above kDirectEntities entities counts and
-// lists of fewer than kDirectRow ids are staged (1 M counts 964 us for 25 ticks, 1,250
-// written in place; lists of 64 ids 643 us for five ticks at 200,000, 624 in place, of 16
-// 430 and 433; for few entities the copies' own latency is most of a read-back).
-constexpr uint32_t kDirectEntities = 65536, kDirectRow = 64;
+// by id, which crosses the link in pieces.  So they are staged but where few entities leave
+// the copies' own latency as most of a read-back, and where lists are whole lines.  In place /
+// staged, us: counts of 3,001 entities 15 / 17, of 10,000 17 / 16, of 65,536 33 / 19, of 1 M 315 /
+// 47; with lists of 16 ids 10,000 entities 22 / 25, 20,000 29 / 29, 65,536 60 / 45; the lists alone in
+// place, 65,536 entities: 8 ids 42 / 34, 32 ids 67 / 75, 64 ids 108 / 119, 100 ids 191 / 167; 1 M: 16 ids
+// 419 / 389, 32 ids 705 / 737, 63 ids 2,550 / 1,457, 64 ids 1,371 / 1,415.  Beside such lists the
+// counts' own copy pays later (20,000 entities, 64 ids 48 / 53, 45,000 89 / 81).
+constexpr uint32_t kDirectEntities = 12288, kDirectBesideLines = 32768, kLineIds = 32;
 template <typename T>
 T* direct_out(void* out, size_t count) {
     return out ? mapped_range<T>(out, count) : nullptr;
@@ -1454,11 +1457,11 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     const size_t n = c->n, cap = c->params.cap;
     if (n == 0) return MSIM_OK;
     const bool want_idx = idx && cap;
-    // lists by whole rows, 16 bytes at a time where they allow it
-    const bool direct = n <= kDirectEntities;
+    const bool lines = want_idx && cap % kLineIds == 0;
+    const bool direct = n <= (lines ? kDirectBesideLines : kDirectEntities);
     uint32_t* to_count = direct ? direct_out<uint32_t>(count, n) : nullptr;
     uint32_t* to_idx = nullptr;
-    if (want_idx && (direct || cap >= kDirectRow))
+    if (want_idx && (direct || lines))
         to_idx = reinterpret_cast<uint32_t*>(direct_out<uint4>(idx, std::max<size_t>(n * cap / 4, 1)));
     const bool copy_count = !to_count, copy_idx = want_idx && !to_idx;
     if ((rc = ensure_stage(c, n * sizeof(uint32_t) * ((copy_idx ? cap : 0) + (copy_count ? 1 : 0)))) != MSIM_OK) return rc;

@@ -607,10 +607,11 @@ __global__ __launch_bounds__(256) void k_export_fields(const StateRecord* __rest
     if (speed) speed[id] = __uint_as_float(w[7]);
 }
 
-// The query's list layout: warp w's lists at w * 32 * cap, in lane order.  Every id list
-// goes out by the whole warp, entity after entity, 16 bytes a lane where cap allows: one
+// The query's list layout: warp w's lists at w * 32 * cap, in lane order.  The id lists go
+// out by the whole warp, 16 bytes a lane where cap allows, else entity after entity: one
 // lane writing its own list word by word touched 32 sectors with every store (200,000
-// lists of 64: 78 us).
+// lists of 64: 78 us).  Short lists go end to end, since entity after entity they left most
+// lanes idle (1 M lists of one id, read-back 109 us for 72).
 __global__ __launch_bounds__(kQueryThreads) void k_export_nbr(const uint32_t* sorted_slot, const uint32_t* slot_id,
                                                               const uint32_t* count, const uint32_t* list,
                                                               uint32_t n, uint32_t cap, uint32_t* out_count,
@@ -653,11 +654,20 @@ __global__ __launch_bounds__(kQueryThreads) void k_export_nbr(const uint32_t* so
         }
         return;
     }
-    for (uint32_t e = 0; e < 32u; e++) {
+    if (cap >= 24u) {
+        for (uint32_t e = 0; e < 32u; e++) {
+            const uint32_t eid = __shfl_sync(FULL, id, e), ek = __shfl_sync(FULL, kept, e);
+            const uint32_t* from = src + __shfl_sync(FULL, first, e);
+            if (eid >= n) continue;  // uniform
+            for (uint32_t j = lane; j < cap; j += 32u) out_idx[(size_t)eid * cap + j] = j < ek ? from[j] : 0xffffffffu;
+        }
+        return;
+    }
+    for (uint32_t i = lane; i < cap * 32u; i += 32u) {
+        const uint32_t e = i / cap, j = i - e * cap;
         const uint32_t eid = __shfl_sync(FULL, id, e), ek = __shfl_sync(FULL, kept, e);
         const uint32_t* from = src + __shfl_sync(FULL, first, e);
-        if (eid >= n) continue;  // uniform
-        for (uint32_t j = lane; j < cap; j += 32u) out_idx[(size_t)eid * cap + j] = j < ek ? from[j] : 0xffffffffu;
+        if (eid < n) out_idx[(size_t)eid * cap + j] = j < ek ? from[j] : 0xffffffffu;
     }
 }
 
