@@ -54,7 +54,7 @@ struct BatchArgs {
     const InstanceDesc* inst;
     const WorkItem* items;
     uint32_t num_items;
-    uint32_t* ticket;
+    uint32_t* ticket;  // nullptr: the pieces in turn
     float2* pos;
     uint32_t* head;
     uint4* rng;
@@ -123,13 +123,16 @@ __device__ __forceinline__ void run_piece(const BatchArgs& a, const DeviceMap& m
 // four-entity path (72 registers and 43 % of the warps resident with all three paths
 // in one kernel).
 // Every warp takes its own pieces: no block barrier, and a block's slow warp (road ends)
-// holds up no other.
+// holds up no other.  Without a ticket (see by_turns) the warps take them in turn.
 template <int RNG, int EMAX, bool AHEAD>
 __global__ void __maxnreg__(EMAX == 1 ? 40 : EMAX == 2 ? 56 : 72) k_batch_step(BatchArgs a) {
-    while (true) {
-        uint32_t i = 0;
-        if ((threadIdx.x & 31u) == 0) i = atomicAdd(a.ticket, 1u);
-        i = __shfl_sync(0xffffffffu, i, 0);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (;; i += warps) {
+        if (a.ticket) {
+            if ((threadIdx.x & 31u) == 0) i = atomicAdd(a.ticket, 1u);
+            i = __shfl_sync(0xffffffffu, i, 0);
+        }
         if (i >= a.num_items) return;
         const WorkItem it = a.items[i];
         const InstanceDesc d = a.inst[it.instance];
@@ -179,6 +182,7 @@ struct msim_batch {
     WorkItem* d_items = nullptr;
     uint32_t num_items = 0;   // tiles of the schedule
     uint32_t num_pieces = 0;  // what the warps take: the tiles or parts of them
+    uint32_t piece_rounds = 1;  // of a warp, one entity per thread, in the longest
     size_t items_capacity = 0;
     uint32_t* ticket = nullptr;
     uint32_t* err = nullptr;
@@ -317,6 +321,8 @@ int upload_items(msim_batch* b, const std::vector<WorkItem>& items) {
     }
     b->num_items = (uint32_t)items.size();
     b->num_pieces = (uint32_t)pieces.size();
+    b->piece_rounds = 1;
+    for (const WorkItem& it : pieces) b->piece_rounds = std::max(b->piece_rounds, (it.count + 31u) / 32u);
     if (!pieces.empty())
         BCK(cudaMemcpy(b->d_items, pieces.data(), sizeof(WorkItem) * pieces.size(), cudaMemcpyHostToDevice),
             "upload work items");
@@ -343,12 +349,29 @@ BatchArgs args_of(msim_batch* b, uint32_t ticks) {
     return a;
 }
 
+// Whether the warps take their pieces in turn instead of by tickets: when there is one
+// for each at most, and while a piece is done about as soon as the tickets' word has served
+// the next warp.  Turns / tickets, us: 20 instances of 40,000 entities (25,000 pieces of one
+// round) 1 tick 12.5 / 29.4, 10 ticks 25.8 / 31.3, 32 ticks 57.3 / 54.1; 512 of 50,000 (pieces of 14
+// rounds) 1 tick 196 / 189, 10 ticks 565 / 487; 64 of 1,000 (2,048 pieces) 63 ticks 20.2 / 23.2.
+bool by_turns(const msim_batch* b, uint32_t ticks, uint32_t warps) {
+    constexpr uint64_t kShortPiece = 12;  // rounds of a warp x ticks
+    return b->num_pieces <= warps || (uint64_t)b->piece_rounds * ticks <= kShortPiece;
+}
+
 cudaError_t enqueue(msim_batch* b, uint32_t ticks) {
-    cudaError_t e = cudaMemsetAsync(b->ticket, 0, sizeof(uint32_t), b->stream);
-    if (e != cudaSuccess) return e;
-    const uint32_t threads = b->sched.block_threads;
-    const int grid = b->sms * occupancy(b, threads, ticks);
+    // no more blocks than there are pieces for their warps: each warp asks for one at least,
+    // and those without took 4 us of one small instance's 20
+    const uint32_t threads = b->sched.block_threads, warps = threads / 32u;
+    const uint32_t resident = (uint32_t)(b->sms * occupancy(b, threads, ticks));
+    const uint32_t grid = std::min(resident, (b->num_pieces + warps - 1u) / warps);
     BatchArgs a = args_of(b, ticks);
+    if (by_turns(b, ticks, grid * warps)) {
+        a.ticket = nullptr;
+    } else {
+        cudaError_t e = cudaMemsetAsync(b->ticket, 0, sizeof(uint32_t), b->stream);
+        if (e != cudaSuccess) return e;
+    }
     batch_kernel(b->rng_kind, b->sched, ticks)<<<grid, threads, 0, b->stream>>>(a);
     return cudaGetLastError();
 }
