@@ -307,16 +307,14 @@ std::vector<WorkItem> cut_pieces(msim_batch* b, const std::vector<WorkItem>& ite
 int upload_items(msim_batch* b, const std::vector<WorkItem>& items) {
     const std::vector<WorkItem> pieces = cut_pieces(b, items);
     if (pieces.size() > b->items_capacity || !b->d_items) {
-        drop_graphs(b);
-        b->num_items = b->num_pieces = 0;
+        WorkItem* larger = nullptr;  // the list in use stays until there is another
+        int rc = balloc(b, &larger, pieces.size());
+        if (rc != MSIM_OK) return rc;
         if (b->d_items) {
             cudaFree(b->d_items);
             b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void*)b->d_items));
-            b->d_items = nullptr;
-            b->items_capacity = 0;
         }
-        int rc = balloc(b, &b->d_items, pieces.size());
-        if (rc != MSIM_OK) return rc;
+        b->d_items = larger;
         b->items_capacity = pieces.size();
     }
     b->num_items = (uint32_t)items.size();
@@ -575,8 +573,11 @@ int msim_batch_set_schedule(msim_batch* b, const msim_batch_schedule* s) {
     if (rc != MSIM_OK) return rc;
     cudaSetDevice(b->device);
     BCK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
+    const msim_batch_schedule before = b->sched;
     b->sched = *s;
-    return upload_items(b, make_items(b, b->sched, -1));
+    rc = upload_items(b, make_items(b, b->sched, -1));
+    if (rc != MSIM_OK) b->sched = before;  // as is its work list
+    return rc;
 }
 
 int msim_batch_get_schedule(msim_batch* b, msim_batch_schedule* s) {
@@ -681,6 +682,7 @@ int msim_batch_tune(msim_batch* b, uint32_t ticks, const char* cache_path) {
         BCK(cudaEventElapsedTime(ms, b->t0, b->t1), "cudaEventElapsedTime");
         return MSIM_OK;
     };
+    const msim_batch_schedule before = b->sched;
     msim_batch_schedule best;
     msim_batch_default_schedule(&best);
     int rc = MSIM_OK;
@@ -726,7 +728,11 @@ int msim_batch_tune(msim_batch* b, uint32_t ticks, const char* cache_path) {
     cudaFree(sp);
     cudaFree(sh);
     cudaFree(sr);
-    if (rc != MSIM_OK) return rc;
+    if (rc != MSIM_OK) {  // back from the candidate, one class of instances, that failed
+        const std::string why = msim_last_error();
+        msim_batch_set_schedule(b, &before);
+        return fail(rc, why);
+    }
     rc = msim_batch_set_schedule(b, &best);
     if (rc == MSIM_OK && cache_path) {
         std::ofstream f(cache_path, std::ios::app);
