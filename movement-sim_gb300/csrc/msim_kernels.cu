@@ -174,20 +174,25 @@ __device__ __forceinline__ uint32_t key_rank(uint32_t key, bool valid, uint32_t 
 }
 
 // Move-only ticks: one entity per thread in 128-thread blocks, so a small entity count
-// still spreads over many SMs.  ONE: a single tick (the tick that reuses the index
-// places its positions too); else several ticks with the state and the road's leg in
-// registers between them, bound by the ticks' serial chain (small counts) or by issue:
-// with read-back, 10,000 entities for 1,000 ticks 316 -> 118 us and 1 M for 200 ticks
-// 865 -> 448 us against reloading the road and three intrinsics every tick.  A run's
-// blocks take one entity per thread and no more (the scheduler fills places as they come
-// free; a grid of 16 blocks per SM with 12 resident left its last blocks to run alone: 1 M
-// x 200 ticks 312 us, so 287, with the coordinates in paired instructions 268).
-template <int RNG, bool ONE, bool AHEAD>
-__global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 10) void k_move(StepLaunch a) {
+// still spreads over many SMs.  TICKS: that many, known at compile time; one tick (the tick
+// that reuses the index places its positions too) to four are bound by memory and by the
+// blocks' turnover, so a grid of 16 blocks per SM goes over the entities (three and four
+// ticks 48): 16 M entities 2 ticks 178 -> 108 us, 4 ticks 217 -> 145 against one entity per
+// thread at 10 blocks per SM, 122 and 200 with the road read every tick.
+// TICKS 0: several ticks with the state and the road's leg in registers between them,
+// bound by the ticks' serial chain (small counts) or by issue: with read-back, 10,000
+// entities for 1,000 ticks 316 -> 118 us and 1 M for 200 ticks 865 -> 448 us against reloading
+// the road and three intrinsics every tick.  A run's blocks take one entity per thread and
+// no more (the scheduler fills places as they come free; a grid of 16 blocks per SM with 12
+// resident left its last blocks to run alone: 1 M x 200 ticks 312 us, so 287, with the
+// coordinates in paired instructions 268).
+template <int RNG, int TICKS, bool AHEAD>
+__global__ __launch_bounds__(kMoveThreads, AHEAD ? 10 : 16) void k_move(StepLaunch a) {
+    constexpr bool ONE = TICKS == 1;
     chain_enter();
     const uint32_t thread = blockIdx.x * kMoveThreads + threadIdx.x;
     uint32_t s = thread;
-    if (!ONE) {  // a.lanes entities to a warp
+    if (!TICKS) {  // a.lanes entities to a warp
         const uint32_t lane = thread & 31u;
         if (lane >= a.lanes) return;
         s = (thread >> 5) * a.lanes + lane;
@@ -201,12 +206,12 @@ __global__ __launch_bounds__(kMoveThreads, ONE ? 16 : 10) void k_move(StepLaunch
         const uint32_t q = ONE && a.rank_pos ? a.rank[s] : 0xffffffffu;
         uint4 r = make_uint4(0u, 0u, 0u, 0u);
         bool rd = false;
-        step_entity<RNG, ONE ? 1 : 0, AHEAD>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
+        step_entity<RNG, TICKS, AHEAD>(a.map, a.dt, sp, a.ticks, p, h, r, rd, a.st.rng + s, a.err);
         a.st.pos[s] = p;
         if (h != h0) a.st.head[s] = h;
         if (rd) a.st.rng[s] = r;
         if (ONE && a.rank_pos && q < a.rank_n) a.rank_pos[q] = p;  // a tick that reuses the index
-        if (!ONE) break;
+        if (!TICKS) break;
     }
 }
 
@@ -835,6 +840,7 @@ cudaError_t launch_init_entities(cudaStream_t s, const DeviceMap& m, EntityState
     return cudaGetLastError();
 }
 
+constexpr uint32_t kFewTicks = 4;
 cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
     if (a.n == 0) return cudaSuccess;
     const bool key = a.key != nullptr;
@@ -844,20 +850,21 @@ cudaError_t launch_step(cudaStream_t s, const StepLaunch& a) {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const unsigned most = 16u * (unsigned)std::max(sms, 1);
-        if (a.ticks > 1) {
-            StepLaunch b = a;
-            b.lanes = warp_lanes(a.n, sms);
-            const unsigned blocks = blocks_for(blocks_for(a.n, b.lanes) * 32u, kMoveThreads);
-            if (a.ticks < kAheadTicks)
-                return a.rng_kind == 1 ? launch_chained(k_move<1, false, false>, blocks, kMoveThreads, s, b)
-                                       : launch_chained(k_move<0, false, false>, blocks, kMoveThreads, s, b);
-            return a.rng_kind == 1 ? launch_chained(k_move<1, false, true>, blocks, kMoveThreads, s, b)
-                                   : launch_chained(k_move<0, false, true>, blocks, kMoveThreads, s, b);
+        using Move = void (*)(StepLaunch);
+        static const Move few[2][kFewTicks] = {
+            {k_move<0, 1, false>, k_move<0, 2, false>, k_move<0, 3, false>, k_move<0, 4, false>},
+            {k_move<1, 1, false>, k_move<1, 2, false>, k_move<1, 3, false>, k_move<1, 4, false>}};
+        static const Move many[2][2] = {{k_move<0, 0, false>, k_move<0, 0, true>},
+                                        {k_move<1, 0, false>, k_move<1, 0, true>}};
+        StepLaunch b = a;
+        b.lanes = a.ticks > 1 ? warp_lanes(a.n, sms) : 32u;
+        if (a.ticks <= kFewTicks && b.lanes == 32u) {
+            const unsigned most = (a.ticks <= 2u ? 16u : 48u) * (unsigned)std::max(sms, 1);
+            return launch_chained(few[a.rng_kind == 1][a.ticks - 1u], std::min(most, blocks_for(a.n, kMoveThreads)),
+                                  kMoveThreads, s, b);
         }
-        const unsigned blocks = std::min(most, blocks_for(a.n, kMoveThreads));
-        return a.rng_kind == 1 ? launch_chained(k_move<1, true, false>, blocks, kMoveThreads, s, a)
-                               : launch_chained(k_move<0, true, false>, blocks, kMoveThreads, s, a);
+        return launch_chained(many[a.rng_kind == 1][a.ticks >= kAheadTicks],
+                              blocks_for(blocks_for(a.n, b.lanes) * 32u, kMoveThreads), kMoveThreads, s, b);
     }
     if (a.ticks > 1) return cudaErrorInvalidValue;  // k_step moves one tick at most
     if (a.disp_max) {  // a host tick that queries the previous index (keys, one tick)
