@@ -643,6 +643,7 @@ __global__ void k_adj_gather(const float* __restrict__ in, const uint32_t* __res
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();
     return fail(MSIM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 #define ACK(expr, what)                                    \

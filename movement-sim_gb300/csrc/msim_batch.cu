@@ -150,6 +150,7 @@ __global__ void __maxnreg__(EMAX == 1 ? 40 : EMAX == 2 ? 56 : 72) k_batch_step(B
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();
     return fail(MSIM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 

@@ -312,7 +312,10 @@ struct msim_ctx {
 
 namespace {
 
+// The runtime keeps the error of a refused call for the next launch check; it is reported here
+// and taken from there.
 int cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();
     return fail(MSIM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
