@@ -47,18 +47,22 @@ bool device_malloc(void** p, size_t bytes) {
     return true;
 }
 
+// A function of the driver as of that CUDA version, or nullptr.
+template <typename F>
+static F driver_function(const char* name, unsigned version) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return reinterpret_cast<F>(p);
+}
+
 bool cuda_context_id(unsigned long long* id) {
     using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static const GetId get_id = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-            found != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            p = nullptr;
-        }
-        return reinterpret_cast<GetId>(p);
-    }();
+    static const GetId get_id = driver_function<GetId>("cuCtxGetId", 12000);
     return get_id && get_id(nullptr, id) == CUDA_SUCCESS;
 }
 
@@ -606,25 +610,31 @@ StepLaunch step_args(msim_ctx* c, uint32_t ticks, bool key) {
     return a;
 }
 
-// Device address of page-locked host memory (registered or from cudaMallocHost), or
-// nullptr for any other pointer.
-void* mapped_host(const void* p) {
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
-}
-
-// The same for count elements that all lie in one page-locked range, aligned for the
-// kernels' loads and stores.
+// Device address of count elements that are page-locked throughout and mapped end to end
+// (one allocation or registration, or several side by side), aligned for the kernels' loads
+// and stores; nullptr for any others.  Asked range by range: both ends may be mapped where
+// what lies between them is not.
 template <typename T>
 T* mapped_range(const void* p, size_t count) {
-    char* first = static_cast<char*>(mapped_host(p));
-    if (!first || (reinterpret_cast<uintptr_t>(first) & (sizeof(T) - 1))) return nullptr;
-    const size_t last = count * sizeof(T) - 1;
-    return mapped_host(static_cast<const char*>(p) + last) == first + last ? reinterpret_cast<T*>(first) : nullptr;
+    using GetAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const GetAttributes get = driver_function<GetAttributes>("cuPointerGetAttributes", 7000);
+    if (!p || !get) return nullptr;
+    const CUdeviceptr host = reinterpret_cast<CUdeviceptr>(p);
+    CUdeviceptr first = 0;
+    for (size_t done = 0; done < count * sizeof(T);) {
+        CUmemorytype type{};
+        CUdeviceptr device = 0, start = 0;
+        size_t size = 0;
+        CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                       CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void* to[4] = {&type, &device, &start, &size};
+        // an address that CUDA does not know has zeros for attributes
+        if (get(4u, what, to, host + done) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !device) return nullptr;
+        if (done == 0) first = device;
+        if (device != first + done || device < start || device - start >= size) return nullptr;
+        done += size - (device - start);
+    }
+    return (first & (sizeof(T) - 1u)) ? nullptr : reinterpret_cast<T*>(first);
 }
 
 // Where an export kernel writes an output of count elements: the caller's array itself
@@ -1465,7 +1475,8 @@ int msim_get_neighbours(msim_ctx* c, uint32_t* count, uint32_t* idx) {
     uint32_t* to_count = direct ? direct_out<uint32_t>(count, n) : nullptr;
     uint32_t* to_idx = nullptr;
     if (want_idx && (direct || lines))
-        to_idx = reinterpret_cast<uint32_t*>(direct_out<uint4>(idx, std::max<size_t>(n * cap / 4, 1)));
+        to_idx = direct_out<uint32_t>(idx, n * cap);
+    if (reinterpret_cast<uintptr_t>(to_idx) & 15u) to_idx = nullptr;
     const bool copy_count = !to_count, copy_idx = want_idx && !to_idx;
     if ((rc = ensure_stage(c, n * sizeof(uint32_t) * ((copy_idx ? cap : 0) + (copy_count ? 1 : 0)))) != MSIM_OK) return rc;
     uint32_t* const stage = static_cast<uint32_t*>(c->stage);
@@ -1548,9 +1559,9 @@ int msim_tick_host(msim_ctx* c, const float* in_pos, const uint32_t* in_heading,
     uint4* dev_rng = nullptr;
     if (out_heading && static_cast<const void*>(out_heading) == static_cast<const void*>(in_heading) && out_rng &&
         static_cast<const void*>(out_rng) == static_cast<const void*>(in_rng)) {
-        dev_head = static_cast<uint32_t*>(mapped_host(out_heading));
-        dev_rng = static_cast<uint4*>(mapped_host(out_rng));
-        if (!dev_head || !dev_rng || (reinterpret_cast<uintptr_t>(dev_rng) & 15u)) {
+        dev_head = mapped_range<uint32_t>(out_heading, n);
+        dev_rng = mapped_range<uint4>(out_rng, n);
+        if (!dev_head || !dev_rng) {
             dev_head = nullptr;
             dev_rng = nullptr;
         }
