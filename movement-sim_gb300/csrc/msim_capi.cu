@@ -118,7 +118,7 @@ enum KernelId : uint32_t {
     K_PERMUTE,
     K_EXPORT,
     K_MARK,   // index update: key counts scanned into the key-start table
-    K_MERGE,  // index update: entities to their places
+    K_PLACE,  // index update: entities to their places
     K_GATHER, // host tick: an uploaded chunk's positions into the previous sorted order
     K_MOVE,   // a tick that reuses the index: move + each position at its sorted position
     K_COUNT
@@ -466,7 +466,7 @@ constexpr float kWidenLimit = 1.0f;
 // Measured at 1 M entities, sparse / dense kernel: 0.68 33.1 / 37.6 us, 1.02 40.0 / 40.5,
 // 1.36 46.5 / 45.5, 2.0 55.1 / 52.5, 2.7 81.3 / 63.2, 3.4 170 / 104.
 constexpr double kDenseNeighbours = 1.2;
-// And above which its kernel for crowds is: 48 neighbours kept per entity in 7 blocks per SM
+// And above which its kernel for crowds is: 48 neighbours kept per entity in 6 blocks per SM
 // instead of 32 in 9.  32 / 48, us per tick at 200,000 entities: 5.4 expected (7.2
 // neighbours) 28.4 / 29.6, 7.6 (10.4) 41.0 / 35.6, 10.8 (15.5) 78.5 / 49.9, 15.2 (22.9) 119.6 /
 // 84.8; at 1 M 3.4 (4.8) 60.6 / 71.1, 8.6 (12.3) 155 / 162, 13.8 (21.4) 335 / 301.
@@ -860,7 +860,7 @@ int incremental_update(msim_ctx* c, bool positions, bool ranks) {
         c->sorted_host += c->n;
     }
     {
-        Prof p(c, K_MERGE);
+        Prof p(c, K_PLACE);
         CKL(p, launch_place(c->stream, c->key, c->key_rank, c->kstart, (uint32_t)c->num_keys, c->n,
                             positions ? cur_state(c).pos : nullptr, c->sv[out], positions ? c->sorted_pos : nullptr,
                             ranks ? c->rank : nullptr, c->err),

@@ -8,7 +8,8 @@
 //   k_onesweep  one stable LSD radix pass per 8-bit digit (decoupled look-back,
 //               warp-level multi-split ranking with __match_any_sync; every block
 //               scans the pass's digit counts into offsets itself)
-//   k_kstart    key-start table: first sorted position of every key (tile + band)
+//   k_kstart_pos, k_kstart_fill  key-start table: first sorted position of every key
+//               (tile + band)
 //   k_query     radius neighbour query (random_move.comp:541-719 semantics: the
 //               pair predicate of :551-562), count + the cap smallest ids
 // After the first neighbour tick the sort is replaced by a counting sort
@@ -132,8 +133,8 @@ __global__ void k_init(DeviceMap m, EntityState st, uint32_t n, uint32_t rng_kin
     }
 }
 
-// Move `ticks` ticks (state kept in registers across ticks), then optionally
-// write the tile key and accumulate the radix digit histograms of all passes.
+// The digits of every radix pass of the warp's keys, added to the block's counts: one
+// shared atomic per run of equal digits (neighbouring slots have near-equal keys).
 template <int RNG, bool KEY>
 __device__ __forceinline__ void digit_counts(uint32_t key, bool valid, uint32_t lane, uint32_t passes,
                                              uint32_t* s_hist) {
@@ -931,18 +932,15 @@ uint32_t kstart_chunks(uint64_t num_keys) { return kstart_chunk_cap(num_keys); }
 cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n, uint32_t* kstart, uint32_t num_keys,
                           uint4* chunks, uint32_t* chunk_count, uint32_t* kernels, const uint32_t* sorted_slot,
                           const float2* pos, float2* sorted_pos, const uint32_t* err) {
-    if (kernels) *kernels = 0;
+    *kernels = 0;
     if (num_keys == 0) return cudaSuccess;
-    if (kernels) *kernels = 1;
+    *kernels = 1;
     const uint64_t entries = (uint64_t)num_keys + 1u;
-    const bool gather = sorted_slot && pos && sorted_pos && n > 0;
     if ((uint64_t)n > 8u * entries) {  // many positions per key
         k_kstart_search<<<(unsigned)((entries + 255u) / 256u), 256, 0, s>>>(sorted_key, n, kstart, num_keys, err);
-        if (gather) {
-            k_gather_pos<<<blocks_for(n, 256), 256, 0, s>>>(sorted_slot, pos, n, sorted_pos, err);
-            if (kernels) *kernels = 2;
-        }
-    } else if (chunks && chunk_count) {
+        k_gather_pos<<<blocks_for(n, 256), 256, 0, s>>>(sorted_slot, pos, n, sorted_pos, err);
+        *kernels = 2;
+    } else {
         const uint32_t cap = kstart_chunk_cap(num_keys);
         cudaError_t e = cudaMemsetAsync(chunk_count, 0, sizeof(uint32_t), s);
         if (e != cudaSuccess) return e;
@@ -954,14 +952,7 @@ cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         e = launch_chained(k_kstart_fill, 4u * (sms > 0 ? sms : 1), 256, s, chunks, chunk_count, cap, kstart, err);
         if (e != cudaSuccess) return e;
-        if (kernels) *kernels = 2;
-    } else {
-        const uint64_t warps = (entries + kKstartWindow - 1u) / kKstartWindow;
-        k_kstart<<<(unsigned)((warps + 7u) / 8u), 256, 0, s>>>(sorted_key, n, kstart, num_keys, err);
-        if (gather) {
-            k_gather_pos<<<blocks_for(n, 256), 256, 0, s>>>(sorted_slot, pos, n, sorted_pos, err);
-            if (kernels) *kernels = 2;
-        }
+        *kernels = 2;
     }
     return cudaGetLastError();
 }

@@ -120,16 +120,13 @@ cudaError_t launch_onesweep(cudaStream_t s, const uint32_t* keys_in, const uint3
                             uint32_t* err, const uint32_t* n_dev = nullptr,  // n_dev: count on the device (<= n)
                             const SweepChain* chain = nullptr, uint32_t spin_limit = kDefaultSpinLimit,
                             bool many = false);  // many: with n_dev, 4096-item tiles all the same
-// Key-start table of sorted keys (num_keys + 1 entries).  chunks / chunk_count
-// (kstart_chunks(num_keys) uint4 entries and one counter; may be NULL) enable the
-// per-position kernel, which also gathers pos into sorted order (sorted_pos, n entries)
-// when sorted_slot, pos and sorted_pos are given.  *kernels (may be NULL) receives the
-// number of kernels launched.
+// Key-start table of sorted keys (num_keys + 1 entries), and pos gathered into sorted
+// order (sorted_pos, n entries).  Scratch: kstart_chunks(num_keys) uint4 entries and one
+// counter.  *kernels receives the number of kernels launched.
 uint32_t kstart_chunks(uint64_t num_keys);
 cudaError_t launch_kstart(cudaStream_t s, const uint32_t* sorted_key, uint32_t n, uint32_t* kstart, uint32_t num_keys,
-                          uint4* chunks = nullptr, uint32_t* chunk_count = nullptr, uint32_t* kernels = nullptr,
-                          const uint32_t* sorted_slot = nullptr, const float2* pos = nullptr,
-                          float2* sorted_pos = nullptr, const uint32_t* err = nullptr);
+                          uint4* chunks, uint32_t* chunk_count, uint32_t* kernels, const uint32_t* sorted_slot,
+                          const float2* pos, float2* sorted_pos, const uint32_t* err);
 cudaError_t launch_query(cudaStream_t s, uint32_t cap, const uint32_t* kstart, const uint32_t* sorted_slot,
                          const float2* sorted_pos, const uint32_t* slot_id, TileGrid grid, uint32_t n, uint32_t* count,
                          uint32_t* list,

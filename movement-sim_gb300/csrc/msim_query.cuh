@@ -6,81 +6,10 @@
 // [0, num_keys]; kstart[num_keys] = n.  Keys >= num_keys (never produced by valid
 // inputs) count as num_keys - 1.  A tile's run is [kstart[t << ybits],
 // kstart[(t + 1) << ybits]); a band run inside it is two independent loads.
-constexpr uint32_t kKstartWindow = 1024;  // table entries written by one warp
 
 __device__ __forceinline__ uint32_t clamped_key(const uint32_t* __restrict__ sk, uint32_t q, uint32_t num_keys) {
     const uint32_t k = sk[q];
     return k < num_keys ? k : num_keys - 1u;
-}
-
-// One warp per window of kKstartWindow table entries [B, E): a 32-ary search finds
-// the first position with key >= B, then the warp walks the positions 32 at a time.
-// Position q owns the entries (key[q-1], key[q]] (clipped to the window); the
-// lanes' entry counts are laid end to end (warp prefix sum) and written 32 at a
-// time, each entry's owner found by a binary search over the prefix sums.  Every
-// warp writes exactly its window, so no warp fills a long empty stretch of the key
-// space alone.  For key spaces much smaller than n see k_kstart_search.
-__global__ __launch_bounds__(256) void k_kstart(const uint32_t* __restrict__ sk, uint32_t n,
-                                                uint32_t* __restrict__ kstart, uint32_t num_keys,
-                                                const uint32_t* err) {
-    constexpr uint32_t FULL = 0xffffffffu;
-    if (index_failed(err)) return;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t b64 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kKstartWindow;
-    if (b64 > num_keys) return;  // uniform per warp
-    const uint32_t B = (uint32_t)b64;
-    const uint32_t E = (uint32_t)(b64 + kKstartWindow < (uint64_t)num_keys + 1u ? b64 + kKstartWindow
-                                                                                : (uint64_t)num_keys + 1u);
-    // first position with key >= B: the answer stays in [lo, hi], key[hi] >= B or hi = n
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 32u) {
-        const uint32_t step = (hi - lo + 31u) >> 5;
-        const uint32_t q = min(lo + (lane + 1u) * step - 1u, hi - 1u);
-        const uint32_t m = __ballot_sync(FULL, clamped_key(sk, q, num_keys) >= B);
-        if (m == 0u) {  // the last probe is hi - 1
-            lo = hi;
-            break;
-        }
-        const uint32_t f = __ffs(m) - 1u;
-        const uint32_t qf = min(lo + (f + 1u) * step - 1u, hi - 1u);
-        lo = f ? min(lo + f * step - 1u, hi - 1u) + 1u : lo;
-        hi = qf;
-    }
-    if (hi > lo) {
-        const uint32_t q = lo + lane;
-        const uint32_t m = __ballot_sync(FULL, q < hi && clamped_key(sk, q, num_keys) >= B);
-        lo = m ? lo + __ffs(m) - 1u : hi;
-    }
-    uint32_t cursor = B;  // first entry of the window not yet written
-    for (uint32_t q0 = lo; cursor < E; q0 += 32u) {
-        const uint32_t q = q0 + lane;
-        const uint32_t key = q < n ? clamped_key(sk, q, num_keys) : num_keys;  // n owns the tail up to num_keys
-        const uint32_t prev = __shfl_up_sync(FULL, key, 1);
-        const uint32_t a = lane ? prev + 1u : cursor;
-        const uint32_t b = key < E - 1u ? key : E - 1u;
-        const uint32_t len = b + 1u > a ? b + 1u - a : 0u;
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL, incl, o);
-            if (lane >= (uint32_t)o) incl += y;
-        }
-        const uint32_t excl = incl - len;
-        const uint32_t total = __shfl_sync(FULL, incl, 31);
-        for (uint32_t base = 0; base < total; base += 32u) {
-            const uint32_t i = base + lane;
-            uint32_t owner = 0;  // first lane whose inclusive prefix exceeds i
-#pragma unroll
-            for (uint32_t st = 16; st > 0; st >>= 1) {
-                const uint32_t v = __shfl_sync(FULL, incl, owner + st - 1u);
-                if (v <= i) owner += st;
-            }
-            const uint32_t o_excl = __shfl_sync(FULL, excl, owner);
-            const uint32_t o_a = __shfl_sync(FULL, a, owner);
-            if (i < total) kstart[o_a + (i - o_excl)] = q0 + owner;
-        }
-        cursor = __shfl_sync(FULL, key, 31) + 1u;
-    }
 }
 
 // One thread per position q in [0, n]: q owns the entries (key[q-1], key[q]] (q = n:
@@ -152,26 +81,6 @@ __device__ __forceinline__ void fill_key_gaps(uint32_t from, uint32_t len, uint3
                 }
             }
         }
-    }
-}
-
-// Writes kstart[from + r] = value for r < len by one thread: directly up to kGapWarp
-// entries, in kGapChunk-entry chunks appended to the list beyond that.
-__device__ __forceinline__ void fill_run(uint32_t from, uint32_t len, uint32_t value, uint32_t* __restrict__ kstart,
-                                         uint4* __restrict__ chunks, uint32_t* chunk_count, uint32_t chunk_cap) {
-    if (len <= kGapWarp) {
-        for (uint32_t r = 0; r < len; r++) kstart[from + r] = value;
-        return;
-    }
-    const uint32_t m = (len + kGapChunk - 1u) / kGapChunk;
-    const uint32_t base = atomicAdd(chunk_count, m);
-    if (base + m > chunk_cap) {  // unreachable: chunk_cap bounds every key space; stay correct anyway
-        for (uint32_t r = 0; r < len; r++) kstart[from + r] = value;
-        return;
-    }
-    for (uint32_t c = 0; c < m; c++) {
-        const uint32_t off = c * kGapChunk;
-        chunks[base + c] = make_uint4(from + off, len - off < kGapChunk ? len - off : kGapChunk, value, 0u);
     }
 }
 
