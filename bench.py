@@ -78,21 +78,21 @@ KERNEL_BYTES = {
 }
 
 # warp instructions per entity-step of k_batch_step: smsp__inst_executed.sum of one
-# ncu capture (300.5 M for 64 instances, 2,058,939 entities, 100 ticks, default
+# ncu capture (298.7 M for 64 instances, 2,058,939 entities, 100 ticks, default
 # schedule; profiles/kernels_issue_and_dram.md) over entities x ticks
-NCU_BATCH_WARP_INSTR_PER_ENTITY_STEP = 1.459
+NCU_BATCH_WARP_INSTR_PER_ENTITY_STEP = 1.451
 # warp instructions per entity of k_query, mean over the queries of an index's reuse
-# (two that keep pair lists, 31.8, and 28 that read them, 12.0): smsp__inst_executed.sum
+# (one of 13 keeps pair lists, 32.9; the others read them, 11.7): smsp__inst_executed.sum
 # of an ncu capture of 4,000,000 entities on the 512 x 512 lattice, the 16 M and 1 M
 # workloads' density (profiles/kernels_issue_and_dram.md)
-NCU_QUERY_WARP_INSTR_PER_ENTITY = 13.33
+NCU_QUERY_WARP_INSTR_PER_ENTITY = 13.34
 # warp instructions per entity-tick of the calibration kernels: smsp__inst_executed.sum of
 # one ncu capture (262,144 entities x 200 ticks, K = 100: 154.2 M and 205.8 M)
 NCU_ADJ_WARP_INSTR_PER_ENTITY_TICK = {"k_adj_forward": 2.941, "k_adj_backward": 3.925}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per entity and launch of the
 # same capture (a working set above L2), scaled by the entities of the run
 NCU_DRAM_BYTES_PER_ENTITY = {
-    "scale": {"k_query": 24.2, "k_move": 26.3, "k_step": 34.3, "k_place": 30.0, "k_mark": 9.8},
+    "scale": {"k_query": 23.6, "k_move": 26.2, "k_step": 34.1, "k_place": 29.8, "k_mark": 9.8},
 }
 
 

@@ -200,8 +200,9 @@ constexpr uint32_t kWarpRuns = 32u * kRuns;    // run-list capacity of a warp
 // position (PairStore::places words per warp; kNoPairs: more than that, look them up); and
 // the entity id of every sorted position, read beside the candidate's position so that
 // a hit keeps the id itself.
-// Bound by the latency of its three dependent loads (58 % issue active); 378 warp
-// instructions against 770.  1 M entities at 2 m 30.6 us looked up, 19.3 from pairs, 38
+// Bound by issue in sparse populations (79 % issue active at 4 M entities; 375 warp
+// instructions a warp against 770), by the latency of its three dependent loads in small
+// and in dense ones.  1 M entities at 2 m 30.6 us looked up, 19.3 from pairs, 38
 // for the query that keeps them; the 16 M tick 532 -> 371 us, the 1 M tick 44.3 -> 34.6,
 // reference mode at 1 M 122 -> 105.  Keeping runs instead of pairs gave 31.1 us at 1 M,
 // ids beside the pairs 42 us for the keeping query.
