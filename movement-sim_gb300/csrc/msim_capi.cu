@@ -556,10 +556,11 @@ bool ensure_pairs(msim_ctx* c, double pairs) {
 }
 
 // Ticks that pair lists kept `since` move ticks after the index's keys should serve (0:
-// look the candidates up), and about how many pairs a warp then keeps.  More ticks keep more pairs (each one twice its displacement
-// further apart), fewer pay for the keeping query more often: with use cost growing by
-// 2 s / reach per tick and the keeping query worth kPairCost of it, the best count is
-// about the square root of kPairCost x reach / (2 s), as far as the index is reused.
+// look the candidates up), and about how many pairs a warp then keeps.  More ticks keep
+// more pairs (each one twice its displacement further apart), fewer pay for the keeping
+// query more often: with use cost growing by 2 s / reach per tick and the keeping query
+// worth kPairCost of it, the best count is about the square root of kPairCost x reach /
+// (2 s), as far as the index is reused.
 // Measured with costs 11 / 22 / 44 (sparse): 16 M 388 / 371 / 372 us per tick, 1 M 36.0 /
 // 36.0 / 35.2; 3 / 6 / 12 (dense): 1 M reference mode 105 / 108 / 124, 200,000 with 14.6
 // neighbours 110 / 118 / 122.
